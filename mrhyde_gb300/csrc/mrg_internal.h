@@ -122,6 +122,8 @@ struct mrg_problem {
   std::vector<double> qtab_host;
   std::vector<double> gx1, gw1;  // 1-D Gauss rule of the problem
   void* q2 = nullptr;            // Q2 tensor-product data (mrg_assemble_q2.cu)
+  void* nl1 = nullptr;           // 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
+  void* box_q2 = nullptr;        // thermal Q2 on identical affine cells (mrg_box_q2.cu)
   void* bicg = nullptr;          // BiCGStab workspace (mrg_bicgstab.cu)
   void* bnd = nullptr;           // face boundary conditions (mrg_boundary.cu)
   void* gmg = nullptr;           // multigrid hierarchy and preconditioner choice (mrg_gmg.cu)
@@ -150,6 +152,16 @@ int mrg_launch_kappa32(mrg_problem* p, cudaStream_t s);
 int mrg_q2_setup(mrg_problem* p);
 void mrg_q2_free(mrg_problem* p);
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
+// 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
+bool mrg_nl1_eligible(int dim, int order, int kind, int source_kind, int points_per_axis, bool affine);
+int mrg_nl1_setup(mrg_problem* p);
+void mrg_nl1_free(mrg_problem* p);
+int mrg_launch_nl1(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
+// Thermal Q2 quadrilaterals and hexahedra on identical affine cells (mrg_box_q2.cu)
+bool mrg_box_q2_eligible(int order, int kind, int points_per_axis, bool affine);
+int mrg_box_q2_setup(mrg_problem* p, cudaStream_t s);
+void mrg_box_q2_free(mrg_problem* p);
+int mrg_launch_box_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
 // Q2 element matrices on tcgen05 tensor cores and their row gather (mrg_tc_q2.cu)
 struct Q2Tc;
 int mrg_q2tc_create(mrg_problem* p, const double* tab, const double s[3], Q2Tc** out, cudaStream_t st);

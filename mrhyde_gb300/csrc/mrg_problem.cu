@@ -230,6 +230,7 @@ static void free_problem(mrg_problem* p) {
   mrg_solver_free(p);
   mrg_bicg_free(p);
   mrg_q2_free(p);
+  mrg_box_q2_free(p);
   mrg_boundary_free(p);
   mrg_gmg_free(p);
   cudaFreeAsync(p->d_prefix, s);
@@ -522,7 +523,8 @@ static int create_impl(const mrg_mesh_desc* m, const mrg_physics_desc* ph, cudaS
       return fail_cuda(e, "upload vcoord");
   }
   int st = mrg_launch_kappa32(P, cs);
-  if (st == MRG_OK && P->path == MRG_PATH_TENSOR) st = mrg_q2_setup(P);
+  if (st == MRG_OK && mrg_box_q2_eligible(p, P->kind, n1, P->affine)) st = mrg_box_q2_setup(P, cs);
+  else if (st == MRG_OK && P->path == MRG_PATH_TENSOR) st = mrg_q2_setup(P);
   if (st == MRG_OK && P->path == MRG_PATH_STORED) st = mrg_stored_setup(P, cs);
   if (st != MRG_OK) {
     free_problem(P);
@@ -631,6 +633,9 @@ extern "C" int mrg_assemble(mrg_problem* p, const double* u, double* r, void* J,
   int st;
   if (p->path == MRG_PATH_FACTORED && !(flags & MRG_ASM_FORCE_CELL)) {
     st = mrg_launch_factored(p, u, r, J, flags, s);
+    if (st != MRG_OK) return st;
+  } else if (p->box_q2 && !(flags & MRG_ASM_FORCE_CELL) && (p->path == MRG_PATH_TENSOR || !(flags & MRG_ASM_ATOMIC))) {
+    st = mrg_launch_box_q2(p, u, r, J, flags, s);
     if (st != MRG_OK) return st;
   } else if (p->path == MRG_PATH_TENSOR && !(flags & MRG_ASM_FORCE_CELL)) {
     st = mrg_launch_q2(p, u, r, J, flags, s);
