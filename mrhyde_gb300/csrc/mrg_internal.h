@@ -122,6 +122,9 @@ struct mrg_problem {
   std::vector<double> qtab_host;
   std::vector<double> gx1, gw1;  // 1-D Gauss rule of the problem
   void* q2 = nullptr;            // Q2 tensor-product data (mrg_assemble_q2.cu)
+  // Pool of the workspaces that one assembly call takes and returns in stream order, so that calls of one handle
+  // may overlap on several streams or be captured; it keeps its memory until the handle is destroyed
+  cudaMemPool_t pool = nullptr;
   void* nl1 = nullptr;           // 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
   void* box_q2 = nullptr;        // thermal Q2 on identical affine cells (mrg_box_q2.cu)
   void* bicg = nullptr;          // BiCGStab workspace (mrg_bicgstab.cu)
@@ -152,8 +155,8 @@ int mrg_launch_kappa32(mrg_problem* p, cudaStream_t s);
 int mrg_q2_setup(mrg_problem* p);
 void mrg_q2_free(mrg_problem* p);
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
+int mrg_pool_create(mrg_problem* p);  // once, on the current device
 // 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
-bool mrg_nl1_eligible(int dim, int order, int kind, int source_kind, int points_per_axis, bool affine);
 int mrg_nl1_setup(mrg_problem* p);
 void mrg_nl1_free(mrg_problem* p);
 int mrg_launch_nl1(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);

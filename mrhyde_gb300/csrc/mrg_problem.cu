@@ -230,6 +230,7 @@ static void free_problem(mrg_problem* p) {
   mrg_solver_free(p);
   mrg_bicg_free(p);
   mrg_q2_free(p);
+  mrg_nl1_free(p);
   mrg_box_q2_free(p);
   mrg_boundary_free(p);
   mrg_gmg_free(p);
@@ -246,7 +247,20 @@ static void free_problem(mrg_problem* p) {
   cudaFreeAsync(p->d_khat32, s);
   cudaFreeAsync(p->d_bload, s);
   cudaStreamSynchronize(s);
+  if (p->pool) cudaMemPoolDestroy(p->pool);
   delete p;
+}
+
+int mrg_pool_create(mrg_problem* p) {
+  if (p->pool) return MRG_OK;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  MRG_CUDA(cudaGetDevice(&props.location.id));
+  MRG_CUDA(cudaMemPoolCreate(&p->pool, &props));
+  uint64_t keep = UINT64_MAX;  // without it the memory would go back to the driver at every synchronisation
+  MRG_CUDA(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  return MRG_OK;
 }
 
 static int create_impl(const mrg_mesh_desc* m, const mrg_physics_desc* ph, cudaStream_t cs, mrg_problem** out) {
@@ -524,7 +538,7 @@ static int create_impl(const mrg_mesh_desc* m, const mrg_physics_desc* ph, cudaS
   }
   int st = mrg_launch_kappa32(P, cs);
   if (st == MRG_OK && mrg_box_q2_eligible(p, P->kind, n1, P->affine)) st = mrg_box_q2_setup(P, cs);
-  else if (st == MRG_OK && P->path == MRG_PATH_TENSOR) st = mrg_q2_setup(P);
+  else if (st == MRG_OK && P->path == MRG_PATH_TENSOR) st = p == 1 ? mrg_nl1_setup(P) : mrg_q2_setup(P);
   if (st == MRG_OK && P->path == MRG_PATH_STORED) st = mrg_stored_setup(P, cs);
   if (st != MRG_OK) {
     free_problem(P);
@@ -638,7 +652,7 @@ extern "C" int mrg_assemble(mrg_problem* p, const double* u, double* r, void* J,
     st = mrg_launch_box_q2(p, u, r, J, flags, s);
     if (st != MRG_OK) return st;
   } else if (p->path == MRG_PATH_TENSOR && !(flags & MRG_ASM_FORCE_CELL)) {
-    st = mrg_launch_q2(p, u, r, J, flags, s);
+    st = p->nl1 ? mrg_launch_nl1(p, u, r, J, flags, s) : mrg_launch_q2(p, u, r, J, flags, s);
     if (st != MRG_OK) return st;
   } else if (p->path == MRG_PATH_STORED && !(flags & (MRG_ASM_FORCE_CELL | MRG_ASM_ATOMIC))) {
     st = mrg_launch_stored(p, u, r, J, flags, s);
