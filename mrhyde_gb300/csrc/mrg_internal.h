@@ -125,6 +125,7 @@ struct mrg_problem {
   // Pool of the workspaces that one assembly call takes and returns in stream order, so that calls of one handle
   // may overlap on several streams or be captured; it keeps its memory until the handle is destroyed
   cudaMemPool_t pool = nullptr;
+  void* general = nullptr;       // cell matrices with stored geometry (mrg_general.cu)
   void* nl1 = nullptr;           // 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
   void* box_q2 = nullptr;        // thermal Q2 on identical affine cells (mrg_box_q2.cu)
   void* bicg = nullptr;          // BiCGStab workspace (mrg_bicgstab.cu)
@@ -156,6 +157,11 @@ int mrg_q2_setup(mrg_problem* p);
 void mrg_q2_free(mrg_problem* p);
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
 int mrg_pool_create(mrg_problem* p);  // once, on the current device
+// Cell matrices with stored geometry: the forms and shapes without a path of their own (mrg_general.cu)
+bool mrg_general_eligible(const mrg_problem* p, int points_per_axis);
+int mrg_general_setup(mrg_problem* p, cudaStream_t s);
+void mrg_general_free(mrg_problem* p);
+int mrg_launch_general(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
 // 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
 int mrg_nl1_setup(mrg_problem* p);
 void mrg_nl1_free(mrg_problem* p);

@@ -231,6 +231,7 @@ static void free_problem(mrg_problem* p) {
   mrg_bicg_free(p);
   mrg_q2_free(p);
   mrg_nl1_free(p);
+  mrg_general_free(p);
   mrg_box_q2_free(p);
   mrg_boundary_free(p);
   mrg_gmg_free(p);
@@ -540,6 +541,7 @@ static int create_impl(const mrg_mesh_desc* m, const mrg_physics_desc* ph, cudaS
   if (st == MRG_OK && mrg_box_q2_eligible(p, P->kind, n1, P->affine)) st = mrg_box_q2_setup(P, cs);
   else if (st == MRG_OK && P->path == MRG_PATH_TENSOR) st = p == 1 ? mrg_nl1_setup(P) : mrg_q2_setup(P);
   if (st == MRG_OK && P->path == MRG_PATH_STORED) st = mrg_stored_setup(P, cs);
+  if (st == MRG_OK && !P->box_q2 && mrg_general_eligible(P, n1)) st = mrg_general_setup(P, cs);
   if (st != MRG_OK) {
     free_problem(P);
     return st;
@@ -656,6 +658,9 @@ extern "C" int mrg_assemble(mrg_problem* p, const double* u, double* r, void* J,
     if (st != MRG_OK) return st;
   } else if (p->path == MRG_PATH_STORED && !(flags & (MRG_ASM_FORCE_CELL | MRG_ASM_ATOMIC))) {
     st = mrg_launch_stored(p, u, r, J, flags, s);
+    if (st != MRG_OK) return st;
+  } else if (p->general && !(flags & (MRG_ASM_FORCE_CELL | MRG_ASM_ATOMIC))) {
+    st = mrg_launch_general(p, u, r, J, flags, s);
     if (st != MRG_OK) return st;
   } else {
     if (flags & MRG_ASM_OVERWRITE) {
