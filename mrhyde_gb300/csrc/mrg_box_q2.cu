@@ -10,40 +10,40 @@
 // the contraction over the Gauss points takes 27 * 81 operations per row and cell.  The residual is
 // r_i = b_i - sum over the distance classes of K[class] * (sum of S(off) u(i+off) over the class).
 //
+// FP32 Jacobians: FP32 sums and products in 3-D; in 2-D, where a row has 16 entries on average, the FP64 products
+// rounded once.
+//
 // What bounds it: the FP64 pipe (16 SM cycles a warp instruction), with about 64 multiplications and 87 FMAs a
-// row in 3-D; so warps are filled with rows of one kind (8 kinds in 3-D, 4 in 2-D, each a grid of its own,
-// flattened), which keeps all 32 lanes on the same unrolled code whatever the mesh size.  Rows of a kind are
-// not neighbours in CSR: each warp stages one z plane of its 32 rows (25, 15 or 9 values each) in shared memory
-// and writes it with consecutive lanes on consecutive addresses.  Measured, FP64 Jacobian and residual:
+// row in 3-D; so warps are filled with rows of one kind (mrg_q2_rows.cuh), which keeps all 32 lanes on the same
+// unrolled code whatever the mesh size.  Measured, FP64 Jacobian and residual:
 // 33 x 30 x 27 cells 6081 -> 78 us (FP64 floor 66), 300 x 211 cells with two flux sides 1146 -> 39 us.
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
-#include "mrg_device.cuh"
-#include "mrg_internal.h"
+#include "mrg_fixmul.cuh"
+#include "mrg_q2_rows.cuh"
 
 namespace {
 
-constexpr int BT = 128;   // threads per CTA: 4 warps of 32 rows of one kind
-constexpr int PLANE = 25;  // most entries of a row in one z plane
+using mrgq2::cells;
+using mrgq2::half;
+using mrgq2::PLANE;
+
+constexpr int BT = 128;  // threads per CTA: 4 warps of 32 rows of one kind
 
 struct BoxArgs {
   Grid g;
-  double K[125];    // class coefficients of the 8 node kinds, kind by kind, z slowest
+  mrgq2::Kinds kinds;
+  double K[125];  // class coefficients of the 8 node kinds, kind by kind, z slowest
   float K32[125];
-  int koff[8];      // first coefficient of a kind
-  int m[8][3];      // nodes of a kind per axis
-  int64_t block0[9];  // first CTA of a kind
+  int koff[8];    // first coefficient of a kind
   const double* B[3];  // per-axis load factors
   double amp;
 };
 
-// Along one axis a row of kind PX (0: vertex, 1: mid-side) has up to len(PX) couplings from up to 2 - PX cells
-__host__ __device__ constexpr int len(int P) { return P ? 3 : 5; }
-__host__ __device__ constexpr int half(int P) { return P ? 1 : 2; }
-__host__ __device__ constexpr int classes(int P) { return P ? 2 : 3; }
-__host__ __device__ constexpr int sums(int P) { return P ? 1 : 3; }  // distinct sets of cells: left, both, right
-__host__ __device__ constexpr int cells(int P) { return P ? 1 : 2; }
+__host__ __device__ constexpr int classes(int P) { return P ? 2 : 3; }  // distances along an axis
+__host__ __device__ constexpr int sums(int P) { return P ? 1 : 3; }     // distinct sets of cells: left, both, right
 __host__ __device__ constexpr int cls_of(int P, int e) { return e < half(P) ? half(P) - e : e - half(P); }
 __host__ __device__ constexpr int sum_of(int P, int e) { return P ? 0 : (e < 2 ? 0 : (e == 2 ? 1 : 2)); }
 
@@ -78,34 +78,18 @@ __device__ __forceinline__ void kappa_sums(const T (&k)[cells(PZ)][cells(PY)][ce
       for (int x = 0; x < sums(PX); ++x) S[z][y][x] = axis_sum<PZ>(&b[0][y][x], sums(PY) * sums(PX), z);
 }
 
-// The rows of one warp: kind (PX, PY, PZ), row number `at` of the kind (x fastest).  2-D problems run as one
-// z plane (PZ = 1, D3 = false).
+// The rows of one warp: kind (PX, PY, PZ), row number `at` of the kind.  2-D problems run as one z plane (PZ = 1,
+// D3 = false).
 template <bool D3, int PX, int PY, int PZ, typename JT, bool DOJ, bool DOR, bool OVW>
 __device__ __forceinline__ void box_rows(const BoxArgs& A, int kind, int64_t at, const double* __restrict__ u,
                                          const double* __restrict__ kap, const float* __restrict__ kap32,
                                          double* __restrict__ r, JT* __restrict__ J, JT* stage) {
-  constexpr bool MIXED = sizeof(JT) == 4;
-  constexpr int LX = len(PX), LY = len(PY), LZ = D3 ? len(PZ) : 1, N = LX * LY;
+  constexpr bool F32 = sizeof(JT) == 4 && D3;  // FP32 products
+  constexpr bool K64 = !F32 || DOR;            // FP64 sums of kappa
+  using R = mrgq2::Row<D3, PX, PY, PZ>;
   const Grid& g = A.g;
-  const int lane = threadIdx.x & 31;
-  const int mx = A.m[kind][0], my = A.m[kind][1];
-  const bool on = at < (int64_t)mx * my * A.m[kind][2];
-  int ix = PX, iy = PY, iz = D3 ? PZ : 0;
-  if (on) {
-    const unsigned a = (unsigned)at, t = a / (unsigned)mx;
-    ix += 2 * (int)(a - t * (unsigned)mx);
-    iy += 2 * (int)(t % (unsigned)my);
-    if (D3) iz += 2 * (int)(t / (unsigned)my);
-  }
-  const int NX = g.nn[0], NY = g.nn[1], NZ = g.nn[2];
-  // couplings that exist: a vertex at an end of its axis has one cell only
-  const bool xl = PX || ix > 0, xr = PX || ix < NX - 1, yl = PY || iy > 0, yr = PY || iy < NY - 1;
-  const bool zl = !D3 || PZ || iz > 0, zr = !D3 || PZ || iz < NZ - 1;
-  const int cx = (xl && xr) ? LX : 3, cy = (yl && yr) ? LY : 3, cz = D3 ? ((zl && zr) ? LZ : 3) : 1;
-  const bool fixed = on && node_fixed(g, ix, iy, iz);
-  const int64_t n = ix + (int64_t)NX * (iy + (int64_t)NY * iz);
-  int64_t rp = 0;
-  if (DOJ && on) rp = g.P[2][iz] * g.T[1] * g.T[0] + (int64_t)cz * (g.P[1][iy] * g.T[0] + (int64_t)cy * g.P[0][ix]);
+  const R row(g, A.kinds.m[kind], at);
+  const int NX = g.nn[0], NY = g.nn[1];
   // kappa of the row's cells, 0 outside the mesh
   double k[cells(PZ)][cells(PY)][cells(PX)];
   float k32[cells(PZ)][cells(PY)][cells(PX)];
@@ -115,33 +99,27 @@ __device__ __forceinline__ void box_rows(const BoxArgs& A, int kind, int64_t at,
     for (int y = 0; y < cells(PY); ++y)
 #pragma unroll
       for (int x = 0; x < cells(PX); ++x) {
-        const int ccx = PX ? ix / 2 : ix / 2 - 1 + x, ccy = PY ? iy / 2 : iy / 2 - 1 + y;
-        const int ccz = !D3 ? 0 : (PZ ? iz / 2 : iz / 2 - 1 + z);
-        const bool ok = on && ccx >= 0 && ccx < g.nc[0] && ccy >= 0 && ccy < g.nc[1] && ccz >= 0 && ccz < g.nc[2];
-        const int64_t c = ccx + (int64_t)g.nc[0] * (ccy + (int64_t)g.nc[1] * ccz);
-        if (!MIXED || DOR) k[z][y][x] = ok ? __ldg(kap + c) : 0.0;
-        if (MIXED && DOJ) k32[z][y][x] = ok ? __ldg(kap32 + c) : 0.0f;
+        int64_t c;
+        const bool ok = row.cell(g, x, y, z, c);
+        if (K64) k[z][y][x] = ok ? __ldg(kap + c) : 0.0;
+        if (F32 && DOJ) k32[z][y][x] = ok ? __ldg(kap32 + c) : 0.0f;
       }
   double S[sums(PZ)][sums(PY)][sums(PX)];
   float S32[sums(PZ)][sums(PY)][sums(PX)];
-  if constexpr (!MIXED || DOR) kappa_sums<PX, PY, PZ, double>(k, S);
-  if constexpr (MIXED && DOJ) kappa_sums<PX, PY, PZ, float>(k32, S32);
+  if constexpr (K64) kappa_sums<PX, PY, PZ, double>(k, S);
+  if constexpr (F32 && DOJ) kappa_sums<PX, PY, PZ, float>(k32, S32);
   const double* K = A.K + A.koff[kind];
   const float* K32 = A.K32 + A.koff[kind];
   double acc = 0.0;
-  if (DOR) {
-    acc = on ? A.amp * __ldg(A.B[0] + ix) * __ldg(A.B[1] + iy) : 0.0;
-    if (D3 && on) acc *= __ldg(A.B[2] + iz);
+  if (DOR && row.on) {
+    acc = A.amp * __ldg(A.B[0] + row.ix) * __ldg(A.B[1] + row.iy);
+    if (D3) acc *= __ldg(A.B[2] + row.iz);
   }
-  const bool whole = cx == LX && cy == LY && cz == LZ && on;
-  const bool all_whole = __all_sync(0xffffffffu, whole);
-  const double* un = u + n;
+  const double* un = u + row.n;
 #pragma unroll
-  for (int ez = 0; ez < LZ; ++ez) {
+  for (int ez = 0; ez < R::LZ; ++ez) {
     const int oz = D3 ? ez - half(PZ) : 0;
     const int sz = D3 ? sum_of(PZ, ez) : 0, kz = D3 ? cls_of(PZ, ez) : 0;
-    const bool vz = !D3 || PZ || oz == 0 || (oz < 0 ? zl : zr);
-    const int xmin = xl ? 0 : half(PX), ymin = yl ? 0 : half(PY);
 #pragma unroll
     for (int ky = 0; ky < classes(PY); ++ky)
 #pragma unroll
@@ -149,61 +127,34 @@ __device__ __forceinline__ void box_rows(const BoxArgs& A, int kind, int64_t at,
         double t = 0.0;
         const int kc = (kz * classes(PY) + ky) * classes(PX) + kx;
 #pragma unroll
-        for (int ey = 0; ey < LY; ++ey) {
+        for (int ey = 0; ey < R::LY; ++ey) {
           if (cls_of(PY, ey) != ky) continue;
 #pragma unroll
-          for (int ex = 0; ex < LX; ++ex) {
+          for (int ex = 0; ex < R::LX; ++ex) {
             if (cls_of(PX, ex) != kx) continue;
             const int oy = ey - half(PY), ox = ex - half(PX);
-            const bool v = vz && (PY || oy == 0 || (oy < 0 ? yl : yr)) && (PX || ox == 0 || (ox < 0 ? xl : xr));
             if (DOJ) {
               JT val;
-              if constexpr (MIXED) val = K32[kc] * S32[sz][sum_of(PY, ey)][sum_of(PX, ex)];
+              if constexpr (F32) val = K32[kc] * S32[sz][sum_of(PY, ey)][sum_of(PX, ex)];
+              else if constexpr (sizeof(JT) == 4) val = mrgfix::f64_to_f32_rn(K[kc] * S[sz][sum_of(PY, ey)][sum_of(PX, ex)]);
               else val = K[kc] * S[sz][sum_of(PY, ey)][sum_of(PX, ex)];
-              if (fixed) val = (OVW && ox == 0 && oy == 0 && oz == 0) ? JT(1) : JT(0);
-              if (all_whole) stage[lane * N + ey * LX + ex] = val;
-              else if (v) stage[lane * PLANE + (ey - ymin) * cx + (ex - xmin)] = val;
+              if (row.fixed) val = (OVW && ox == 0 && oy == 0 && oz == 0) ? JT(1) : JT(0);
+              row.put(stage, ez, ey, ex, val);
             }
-            if (DOR && v && on) t = fma(S[sz][sum_of(PY, ey)][sum_of(PX, ex)], __ldg(un + ox + (int64_t)NX * (oy + (int64_t)NY * oz)), t);
+            if (DOR && row.on && row.has_z(oz) && row.has_y(oy) && row.has_x(ox))
+              t = fma(S[sz][sum_of(PY, ey)][sum_of(PX, ex)], __ldg(un + ox + (int64_t)NX * (oy + (int64_t)NY * oz)), t);
           }
         }
         if (DOR) acc = fma(-K[kc], t, acc);
       }
-    if (DOJ) {
-      __syncwarp();
-      if (all_whole) {
-        // 32 rows of N values, value by value: consecutive lanes on consecutive addresses
-        const int64_t base = rp + (int64_t)ez * N;
-#pragma unroll 5
-        for (int i = 0; i < N; ++i) {
-          const int e = i * 32 + lane, row = e / N;
-          const int64_t d = __shfl_sync(0xffffffffu, base, row) + (e - row * N);
-          if (OVW) __stcs(J + d, stage[e]); else J[d] += stage[e];
-        }
-      } else {
-        const int64_t base = rp + (int64_t)(ez - (zl ? 0 : half(PZ))) * cx * cy;
-        const int count = (on && vz) ? cx * cy : 0;
-        for (int row = 0; row < 32; ++row) {
-          const int64_t d = __shfl_sync(0xffffffffu, base, row);
-          const int c = __shfl_sync(0xffffffffu, count, row);
-          if (lane < c) {
-            if (OVW) J[d + lane] = stage[row * PLANE + lane]; else J[d + lane] += stage[row * PLANE + lane];
-          }
-        }
-      }
-      __syncwarp();
-    }
+    if (DOJ) row.template store_plane<OVW>(J, stage, ez);
   }
-  if (DOJ && !OVW && fixed) {
-    // the row's values were left as they were; its diagonal is 1 (written after this warp's additions)
-    const int dx = xl ? half(PX) : 0, dy = yl ? half(PY) : 0, dz = !D3 ? 0 : (zl ? half(PZ) : 0);
-    J[rp + ((int64_t)dz * cy + dy) * cx + dx] = JT(1);
-  }
-  if (DOR && on) {
-    if (fixed) {
-      if (OVW) r[n] = 0.0;
+  if (DOJ && !OVW) row.fix_diagonal(J);
+  if (DOR && row.on) {
+    if (row.fixed) {
+      if (OVW) r[row.n] = 0.0;
     } else {
-      if (OVW) r[n] = acc; else r[n] += acc;
+      if (OVW) r[row.n] = acc; else r[row.n] += acc;
     }
   }
 }
@@ -214,45 +165,23 @@ __global__ void __launch_bounds__(BT) k_box_q2(const __grid_constant__ BoxArgs A
                                                double* __restrict__ r, JT* __restrict__ J) {
   __shared__ JT stage_all[DOJ ? (BT / 32) * 32 * PLANE : 1];
   JT* stage = stage_all + (DOJ ? (threadIdx.x >> 5) * 32 * PLANE : 0);
-  constexpr int KINDS = D3 ? 8 : 4;
-  int kind = 0;
-#pragma unroll
-  for (int t = 1; t < KINDS; ++t)
-    if ((int64_t)blockIdx.x >= A.block0[t]) kind = t;
-  const int64_t at = ((int64_t)blockIdx.x - A.block0[kind]) * BT + threadIdx.x;
-#define MRG_BOX_KIND(T)                                                                                           \
-  case T:                                                                                                         \
-    box_rows<D3, (T) & 1, ((T) >> 1) & 1, D3 ? ((T) >> 2) & 1 : 1, JT, DOJ, DOR, OVW>(A, T, at, u, kap, kap32, r, \
-                                                                                     J, stage);                  \
-    break;
-  switch (kind) {
-    MRG_BOX_KIND(0)
-    MRG_BOX_KIND(1)
-    MRG_BOX_KIND(2)
-    MRG_BOX_KIND(3)
-    default:
-      if constexpr (D3) {
-        switch (kind) {
-          MRG_BOX_KIND(4)
-          MRG_BOX_KIND(5)
-          MRG_BOX_KIND(6)
-          MRG_BOX_KIND(7)
-        }
-      }
-  }
-#undef MRG_BOX_KIND
+  const int kind = mrgq2::kind_of(A.kinds, blockIdx.x);
+  const int64_t at = ((int64_t)blockIdx.x - A.kinds.block0[kind]) * BT + threadIdx.x;
+  mrgq2::with_kind<D3>(kind, [&](auto px, auto py, auto pz) {
+    box_rows<D3, decltype(px)::value, decltype(py)::value, decltype(pz)::value, JT, DOJ, DOR, OVW>(A, kind, at, u, kap,
+                                                                                                  kap32, r, J, stage);
+  });
 }
 
 struct BoxQ2 {
   BoxArgs A;
-  int64_t blocks = 0;
   double* d_B = nullptr;
 };
 
 template <bool D3, typename JT>
 cudaError_t launch(const mrg_problem* p, const BoxQ2& Q, const double* u, double* r, JT* J, bool doJ, bool doR, bool ovw,
                    cudaStream_t s) {
-  const unsigned grid = (unsigned)Q.blocks;
+  const unsigned grid = (unsigned)Q.A.kinds.block0[8];
 #define MRG_BOX_LAUNCH(DJ, DR, OV) \
   k_box_q2<D3, JT, DJ, DR, OV><<<grid, BT, 0, s>>>(Q.A, u, p->d_kappa, p->d_kappa32, r, J)
   if (doJ && doR) { if (ovw) MRG_BOX_LAUNCH(true, true, true); else MRG_BOX_LAUNCH(true, true, false); }
@@ -289,7 +218,6 @@ int mrg_box_q2_setup(mrg_problem* p, cudaStream_t s) {
   // distance c from a vertex: its own row [0][c]; from a mid-side node: [1][1] and [1][0]
   auto at = [](const double (&m)[2][3], int mid, int c) { return mid ? m[1][1 - c] : m[0][c]; };
   int off = 0;
-  int64_t blocks = 0;
   for (int t = 0; t < (d == 3 ? 8 : 4); ++t) {
     const int P[3] = {t & 1, (t >> 1) & 1, d == 3 ? (t >> 2) & 1 : 1};
     A.koff[t] = off;
@@ -306,16 +234,8 @@ int mrg_box_q2_setup(mrg_problem* p, cudaStream_t s) {
           A.K[off] = v;
           A.K32[off++] = (float)v;
         }
-    int64_t rows = 1;
-    for (int k = 0; k < 3; ++k) {
-      A.m[t][k] = k < d ? (P[k] ? p->g.nc[k] : p->g.nc[k] + 1) : 1;
-      rows *= A.m[t][k];
-    }
-    A.block0[t] = blocks;
-    blocks += (rows + BT - 1) / BT;
   }
-  for (int t = (d == 3 ? 8 : 4); t <= 8; ++t) A.block0[t] = blocks;
-  Q->blocks = blocks;
+  A.kinds = mrgq2::make_kinds(p->g, BT);
   // load factors: b_i = amp * prod_k B_k[i_k], B_k[i] the 1-D integral of f_k phi_i over the node's cells with
   // f_k = 1 or sin(freq x)
   std::vector<double> B;
