@@ -33,9 +33,9 @@
  *     sorted columns).
  *   - All work is enqueued on the caller's stream; nothing synchronises the host except the calls that
  *     return host-visible results (mrg_solve_pcg / mrg_newton statistics).  mrg_assemble can be captured
- *     in a CUDA graph once a first call has created its workspace (the Q2 FP32 Jacobian allocates its
- *     tensor-core workspace on first use); a time-out inside the tensor-core kernel is reported by a
- *     later Q2 FP32 Jacobian call instead of synchronising.
+ *     in a CUDA graph (with MRG_ASM_TENSOR_CORES once a first call has created the tensor-core
+ *     workspace); a time-out inside the tensor-core kernel is reported by a later MRG_ASM_TENSOR_CORES
+ *     call instead of synchronising.
  *   - Every call returns an mrg_status; no C++ exception crosses the ABI.  mrg_last_error() gives text.
  *   - A handle is thread-compatible (one host thread at a time per handle).
  */
@@ -132,9 +132,9 @@ enum {
   MRG_ASM_ATOMIC = 512u,       /* per-cell AD path with atomic scatter instead of the 8-colour scatter */
   MRG_ASM_ADJOINT = 1024u,     /* not supported -> MRG_ENOTSUP                   */
   MRG_ASM_SENS = 2048u,        /* not supported -> MRG_ENOTSUP                   */
-  MRG_ASM_TENSOR_CORES = 4096u,/* Q2 FP32 Jacobian: element contractions on tcgen05 tensor cores (3xTF32);
-                                  the default for Q2 FP32 Jacobians, kept for explicitness */
-  MRG_ASM_CUDA_CORES = 8192u,  /* Q2 FP32 Jacobian: force the CUDA-core contraction instead */
+  MRG_ASM_TENSOR_CORES = 4096u,/* 1 + u^2 Q2 hexahedra, FP32 Jacobian: dense element contractions on tcgen05 tensor
+                                  cores (3xTF32) instead of the sum-factorised FP32 ones */
+  MRG_ASM_CUDA_CORES = 8192u,  /* the sum-factorised contractions (the default), kept for explicitness */
   MRG_ASM_NATIVE_FP64 = 16384u /* Q1 factored path: every kappa sum, product and residual FMA as an FP64
                                   instruction.  By default each S(off) is the exact sum (64-bit fixed point
                                   on the integer pipes) rounded once to FP64, for every row whose kappa lie

@@ -222,7 +222,7 @@ class AssemblyManager:
             flags |= L.MRG_ASM_FORCE_CELL
         if atomic:
             flags |= L.MRG_ASM_ATOMIC
-        if tensor_cores is not None:  # Q2 FP32 Jacobians use the tensor cores unless told otherwise
+        if tensor_cores is not None:  # 1 + u^2 Q2 FP32 Jacobians: True takes the tensor cores
             flags |= L.MRG_ASM_TENSOR_CORES if tensor_cores else L.MRG_ASM_CUDA_CORES
         if native_fp64:
             flags |= L.MRG_ASM_NATIVE_FP64

@@ -121,7 +121,7 @@ struct mrg_problem {
   double cell_load;             // factored path: int_cell phi_l for one node (vol / 2^dim)
   std::vector<double> qtab_host;
   std::vector<double> gx1, gw1;  // 1-D Gauss rule of the problem
-  void* q2 = nullptr;            // Q2 tensor-product data (mrg_assemble_q2.cu)
+  void* q2 = nullptr;            // 1 + u^2 Q2 hexahedra on identical affine cells (mrg_assemble_q2.cu)
   // Pool of the workspaces that one assembly call takes and returns in stream order, so that calls of one handle
   // may overlap on several streams or be captured; it keeps its memory until the handle is destroyed
   cudaMemPool_t pool = nullptr;
@@ -152,7 +152,7 @@ int mrg_launch_cell(mrg_problem* p, const double* u, double* r, void* J, uint32_
 int mrg_launch_constraints(mrg_problem* p, void* J, bool fp32, cudaStream_t s);
 int mrg_launch_fix_zero_rows(mrg_problem* p, void* J, bool fp32, cudaStream_t s);
 int mrg_launch_kappa32(mrg_problem* p, cudaStream_t s);
-// Q2 hexahedra on identical affine cells (mrg_assemble_q2.cu)
+// 1 + u^2 Q2 hexahedra on identical affine cells (mrg_assemble_q2.cu)
 int mrg_q2_setup(mrg_problem* p);
 void mrg_q2_free(mrg_problem* p);
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
@@ -173,7 +173,7 @@ void mrg_box_q2_free(mrg_problem* p);
 int mrg_launch_box_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
 // Q2 element matrices on tcgen05 tensor cores and their row gather (mrg_tc_q2.cu)
 struct Q2Tc;
-int mrg_q2tc_create(mrg_problem* p, const double* tab, const double s[3], Q2Tc** out, cudaStream_t st);
+int mrg_q2tc_create(mrg_problem* p, Q2Tc** out, cudaStream_t st);
 void mrg_q2tc_free(Q2Tc* T, cudaStream_t st);
 float* mrg_q2tc_w_image(Q2Tc* T);  // [tile][hi, lo][K chunk 28][cell 128][4] TF32 operand image
 int mrg_q2tc_launch(const mrg_problem* p, Q2Tc* T, float* J, bool ovw, int* err, cudaStream_t s);

@@ -6,19 +6,18 @@
 // residual, differentiated by the workset AD types of assemblyManager_jacres.hpp:121-630) the element
 // Jacobian is
 //     K_c[l][j] = sum_q cw_q sum_d s_d^2 G_d[q][l] G_d[q][j]  +  sum_{d,q} ew_{q,d} G_d[q][l] Phi[q][j]
-// with per-point coefficients W_c = (cw_q | ew_{q,x} | ew_{q,y} | ew_{q,z}) (108 values, written by the
-// residual pass; the ew block is zero for the linear thermal form) and the constant reference tables G_d
-// (gradients) and Phi (values).  All element matrices together are ONE GEMM with a constant right operand:
+// with per-point coefficients W_c = (cw_q | ew_{q,x} | ew_{q,y} | ew_{q,z}) (108 values, written by
+// k_q2_cell) and the constant reference tables G_d (gradients) and Phi (values).  All element matrices together are ONE GEMM with a constant right operand:
 //     E (ncell x 768) = W (ncell x K) * H (K x 768),   H[k][28 l + j] = the products above,
-// K = 108 (nonlinear) or 27 (thermal), the 27 x 27 element matrix stored with rows padded to 28 so that
+// K = 108, the 27 x 27 element matrix stored with rows padded to 28 so that
 // each row starts on 16 bytes.  The GEMM runs in FP32-class precision as 3xTF32: every operand is split
 // x = hi + lo (hi = x rounded to TF32, lo = the rounded remainder) and E = Wh Hh + Wh Hl + Wl Hh.
 //
 // k_q2_elem_tc is a persistent warp-specialised kernel (one CTA per SM, 6 warps):
 //   warp 0  producer: 1-D bulk copies (cp.async.bulk) of the 128-cell W tile (hi and lo planes) and of
 //           256-column slices of H in a 5-stage ring (K = 8 per stage).  Both operands are kept in global
-//           memory as the exact shared-memory image of the K-major no-swizzle core-matrix layout (the
-//           residual pass writes W that way; H is a constant built on the host), so each copy is one
+//           memory as the exact shared-memory image of the K-major no-swizzle core-matrix layout (k_q2_cell
+//           writes W that way; H is a constant built on the host), so each copy is one
 //           contiguous transfer instead of hundreds of 16-byte rows;
 //   warp 1  owns TMEM (512 columns = two 128 x 256 FP32 accumulators) and issues tcgen05.mma from one
 //           thread: per 256-column slice, K/8 steps x 3 products, then tcgen05.commit to the mbarriers
@@ -547,14 +546,15 @@ struct Q2Tc {
   int ntiles = 0, ksteps = 0;
 };
 
-// Builds H^T (hi/lo) from the reference tables tab[(d*27 + q)*28 + j] (d = 0..2 gradients, 3 = values)
-// and the axis scalings s[d] = 2 / h_d, allocates the coefficient and element buffers and encodes the
-// tensor maps.  W is written by the residual pass into q2tc_w_planes().
-int mrg_q2tc_create(mrg_problem* p, const double* tab, const double s[3], Q2Tc** out, cudaStream_t st) {
+// Builds H^T (hi/lo) from the reference tables and the axis scalings s[d] = 2 / h_d, allocates the coefficient and
+// element buffers and encodes the tensor map.  W is written by k_q2_cell into mrg_q2tc_w_image().
+int mrg_q2tc_create(mrg_problem* p, Q2Tc** out, cudaStream_t st) {
   Q2Tc* T = new Q2Tc();
-  const bool thermal = p->kind == MRG_THERMAL;
   T->ntiles = (int)((p->ncell + TM - 1) / TM);
-  T->ksteps = thermal ? 4 : KH / 8;
+  T->ksteps = KH / 8;
+  const double* phi = p->qtab_host.data() + 27;  // [node][point], then gradients [node][point][axis]
+  const double* dphi = phi + 27 * 27;
+  const double s[3] = {2.0 / p->h[0], 2.0 / p->h[1], 2.0 / p->h[2]};
   std::vector<float> h((size_t)NNCH * KSTEPS_MAX * H_STAGE_FLOATS, 0.0f);
   // position of H^T[n][k] (plane 0 = hi, 1 = lo) in the stage image
   auto at = [&](int n, int k, int plane) {
@@ -562,7 +562,7 @@ int mrg_q2tc_create(mrg_problem* p, const double* tab, const double s[3], Q2Tc**
     return (size_t)(sl * KSTEPS_MAX + ks) * H_STAGE_FLOATS + (size_t)plane * (B_PLANE / 4) + (size_t)c * NCH * 4 +
            (size_t)col * 4 + (size_t)(k % 4);
   };
-  auto G = [&](int d, int q, int j) { return tab[(d * 27 + q) * 28 + j]; };
+  auto G = [&](int d, int q, int j) { return d < 3 ? dphi[(j * 27 + q) * 3 + d] : phi[j * 27 + q]; };
   for (int l = 0; l < 27; ++l)
     for (int j = 0; j < 27; ++j) {
       const int n = 28 * l + j;
@@ -589,8 +589,7 @@ int mrg_q2tc_create(mrg_problem* p, const double* tab, const double s[3], Q2Tc**
   };
   const size_t wbytes = (size_t)T->ntiles * W_TILE_FLOATS * sizeof(float);
   cudaError_t e = cudaMallocAsync(&T->d_w, wbytes, st);
-  // slots never written by the residual pass (K padding, the ew block of the thermal form, cells past
-  // the end of the last tile) must read as zero
+  // slots never written (K padding, cells past the end of the last tile) must read as zero
   if (e == cudaSuccess) e = cudaMemsetAsync(T->d_w, 0, wbytes, st);
   if (e == cudaSuccess) e = cudaMallocAsync(&T->d_h, h.size() * sizeof(float), st);
   if (e == cudaSuccess) e = cudaMallocAsync(&T->d_e, (size_t)T->ntiles * TM * NE * sizeof(float), st);
