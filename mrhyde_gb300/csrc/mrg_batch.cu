@@ -484,6 +484,18 @@ extern "C" int mrg_batch_create(const mrg_batch_desc* d, mrg_batch** out) {
       delete B;
       return mrg_fail(MRG_ENUMERIC, "mrg_batch_create: kappa contains NaN or Inf");
     }
+  // CTAs per SM: two share an SM's issue slots and FP64 pipe, so each runs slower but more is in flight.  While the
+  // batch is little more than its largest problem for every SM, that problem's own time is the batch's: one.  Work is
+  // taken as interior rows times the longest axis (the inner iterations grow with it); the line lies where both measured
+  // the same.  Per-axis cells 4 to 16, one / two CTAs: 300 problems (0.35 of the largest one's work per SM) 343 / 532 us,
+  // 700 (0.8) 637 / 622, 2000 (2.3) 1677 / 1129; cells 4 to 8: 700 (1.5) 211 / 153.
+  double total = 0.0, largest = 0.0;
+  for (const BatchProb& P : B->probs) {
+    const double w = (double)(P.nx - 1) * (P.ny - 1) * (P.nz - 1) * std::max(P.nx, std::max(P.ny, P.nz));
+    total += w;
+    largest = std::max(largest, w);
+  }
+  if (total < 0.75 * largest * mrg_device_sms()) B->ctas_per_sm = 1;
   // largest problems first (longest-processing-time order for the work queue)
   std::vector<int32_t> order(B->nprob);
   std::iota(order.begin(), order.end(), 0);
