@@ -448,7 +448,7 @@ int mrg_q2_setup(mrg_problem* p) {
   cudaStream_t s = p->stream;
   MRG_CUDA(cudaMallocAsync(&Q->d_err, sizeof(int), s));
   MRG_CUDA(cudaMemsetAsync(Q->d_err, 0, sizeof(int), s));
-  return mrg_pool_create(p);
+  return mrg_ws_open(p);
 }
 
 void mrg_q2_free(mrg_problem* p) {
@@ -537,7 +537,7 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
   const size_t ebytes = doJ && !tc ? slots * ENT * (fp32 ? sizeof(float) : sizeof(double)) : 0;
   const size_t bytes = ebytes + (doR ? slots * 27 * sizeof(double) : 0);
   void* ws = nullptr;
-  if (bytes) MRG_CUDA(cudaMallocFromPoolAsync(&ws, bytes, p->pool, s));
+  if (bytes) MRG_CUDA(mrg_ws_take(p, bytes, s, &ws));
   double* rbuf = doR ? reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + ebytes) : nullptr;
   int st = MRG_OK;
   cudaError_t e = cudaSuccess;
@@ -556,7 +556,7 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
     if (e == cudaSuccess) e = launch_rows<double>(p, Q, eb, rbuf, r, (double*)J, doJ, doR, ovw, s);
   }
   if (ws) {
-    const cudaError_t ef = cudaFreeAsync(ws, s);
+    const cudaError_t ef = mrg_ws_give(ws, s);
     if (e == cudaSuccess) e = ef;
   }
   if (st) return st;

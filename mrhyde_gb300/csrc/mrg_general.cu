@@ -20,8 +20,8 @@
 //                 written once
 // Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 259 us (cells 231, FP64
 // pipe 87 % active, rows 27).
-// The workspace is taken from the handle's own pool in stream order for each call, so calls of one handle may
-// overlap on several streams and may be captured.
+// The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
+// on several streams and may be captured.
 #include <cmath>
 #include <type_traits>
 
@@ -668,7 +668,7 @@ int mrg_general_setup(mrg_problem* p, cudaStream_t s) {
   Q->A.kap = p->d_kappa;
   Q->A.thermal = p->kind == MRG_THERMAL;
   Q->A.ncell = p->ncell;
-  return mrg_pool_create(p);
+  return mrg_ws_open(p);
 }
 
 void mrg_general_free(mrg_problem* p) {
@@ -687,7 +687,7 @@ int mrg_launch_general(mrg_problem* p, const double* u, double* r, void* J, uint
   const size_t cells = (size_t)((p->ncell + CB - 1) / CB) * CB;
   const size_t ebytes = doJ ? cells * p->npe * p->npe * (fp32 ? sizeof(float) : sizeof(double)) : 0;
   void* ws = nullptr;
-  MRG_CUDA(cudaMallocFromPoolAsync(&ws, ebytes + (doR ? cells * p->npe * sizeof(double) : 0), p->pool, s));
+  MRG_CUDA(mrg_ws_take(p, ebytes + (doR ? cells * p->npe * sizeof(double) : 0), s, &ws));
   double* rbuf = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + ebytes);
   cudaError_t e;
   auto go = [&](auto* Jt) {
@@ -699,7 +699,7 @@ int mrg_launch_general(mrg_problem* p, const double* u, double* r, void* J, uint
   };
   if (fp32) e = go(reinterpret_cast<float*>(J));
   else e = go(reinterpret_cast<double*>(J));
-  const cudaError_t ef = cudaFreeAsync(ws, s);
+  const cudaError_t ef = mrg_ws_give(ws, s);
   if (e == cudaSuccess) e = ef;
   return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "general assembly launch");
 }

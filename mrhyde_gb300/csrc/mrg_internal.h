@@ -122,9 +122,10 @@ struct mrg_problem {
   std::vector<double> qtab_host;
   std::vector<double> gx1, gw1;  // 1-D Gauss rule of the problem
   void* q2 = nullptr;            // 1 + u^2 Q2 hexahedra on identical affine cells (mrg_assemble_q2.cu)
-  // Pool of the workspaces that one assembly call takes and returns in stream order, so that calls of one handle
-  // may overlap on several streams or be captured; it keeps its memory until the handle is destroyed
-  cudaMemPool_t pool = nullptr;
+  // Workspaces that one assembly call takes and returns in stream order (mrg_ws_take, mrg_ws_give), so that calls of
+  // one handle may overlap on several streams or be captured
+  struct WsPool* ws_pool = nullptr;
+  size_t ws_need = 0;            // largest request so far
   void* general = nullptr;       // cell matrices with stored geometry (mrg_general.cu)
   void* nl1 = nullptr;           // 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
   void* box_q2 = nullptr;        // thermal Q2 on identical affine cells (mrg_box_q2.cu)
@@ -156,7 +157,14 @@ int mrg_launch_kappa32(mrg_problem* p, cudaStream_t s);
 int mrg_q2_setup(mrg_problem* p);
 void mrg_q2_free(mrg_problem* p);
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
-int mrg_pool_create(mrg_problem* p);  // once, on the current device
+// Assembly workspaces come from one pool per device, shared by the handles on it: a new handle finds memory that is
+// mapped already (mapping 40 MB takes longer than most assembly calls).  Whenever a handle is destroyed the pool gives
+// back what exceeds the live handles' largest requests by more than 1 GiB, and everything with the last one.  Safe from any thread and
+// stream: take and give are ordered on the call's stream, and memory in use on one stream is never handed to another.
+int mrg_ws_open(mrg_problem* p);   // at creation, on the current device
+void mrg_ws_close(mrg_problem* p); // after the handle's streams have drained
+cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, void** out);
+cudaError_t mrg_ws_give(void* ws, cudaStream_t s);
 // Cell matrices with stored geometry: the forms and shapes without a path of their own (mrg_general.cu)
 bool mrg_general_eligible(const mrg_problem* p, int points_per_axis);
 int mrg_general_setup(mrg_problem* p, cudaStream_t s);

@@ -21,8 +21,8 @@
 // Measured, FP64 Jacobian and residual on 95^3 cells: 3506 -> 1046 us (cells 704, rows 340, FP64 pipe 84 and 83 %
 // active; the row-by-row contraction took 2712 and eight coloured residual launches 780); FP32 Jacobian alone on
 // 96^3 cells 865 -> about 40 us.
-// The workspace is taken from the handle's own pool in stream order for each call, so calls of one handle may
-// overlap on several streams and may be captured.
+// The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
+// on several streams and may be captured.
 #include <cmath>
 
 #include "mrg_device.cuh"
@@ -341,7 +341,7 @@ int mrg_nl1_setup(mrg_problem* p) {
     A.wf[a] = (float)A.w[a];
   }
   A.load = p->source_amp * vol;  // the 8 basis values at the 8 equal-weight points add up to 1 for each node
-  return mrg_pool_create(p);
+  return mrg_ws_open(p);
 }
 
 void mrg_nl1_free(mrg_problem* p) {
@@ -356,11 +356,11 @@ int mrg_launch_nl1(mrg_problem* p, const double* u, double* r, void* J, uint32_t
   const size_t cells = (size_t)((p->ncell + CB - 1) / CB) * CB;
   const size_t zbytes = doJ ? cells * NZ_ * (fp32 ? sizeof(float) : sizeof(double)) : 0;
   void* ws = nullptr;
-  MRG_CUDA(cudaMallocFromPoolAsync(&ws, zbytes + (doR ? cells * 8 * sizeof(double) : 0), p->pool, s));
+  MRG_CUDA(mrg_ws_take(p, zbytes + (doR ? cells * 8 * sizeof(double) : 0), s, &ws));
   double* rb = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + zbytes);
   cudaError_t e = fp32 && doJ ? launch<float>(p, A, u, r, (float*)J, (float*)ws, rb, doJ, doR, ovw, s)
                               : launch<double>(p, A, u, r, (double*)J, (double*)ws, rb, doJ, doR, ovw, s);
-  const cudaError_t ef = cudaFreeAsync(ws, s);
+  const cudaError_t ef = mrg_ws_give(ws, s);
   if (e == cudaSuccess) e = ef;
   return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "nonlinear Q1 assembly launch");
 }

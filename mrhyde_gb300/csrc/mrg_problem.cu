@@ -248,21 +248,74 @@ static void free_problem(mrg_problem* p) {
   cudaFreeAsync(p->d_khat32, s);
   cudaFreeAsync(p->d_bload, s);
   cudaStreamSynchronize(s);
-  if (p->pool) cudaMemPoolDestroy(p->pool);
+  mrg_ws_close(p);
   delete p;
 }
 
-int mrg_pool_create(mrg_problem* p) {
-  if (p->pool) return MRG_OK;
-  cudaMemPoolProps props = {};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  MRG_CUDA(cudaGetDevice(&props.location.id));
-  MRG_CUDA(cudaMemPoolCreate(&p->pool, &props));
-  uint64_t keep = UINT64_MAX;  // without it the memory would go back to the driver at every synchronisation
-  MRG_CUDA(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+// ------------------------------------------------------------------------------------------------
+// assembly workspaces
+// ------------------------------------------------------------------------------------------------
+struct WsPool {
+  cudaMemPool_t pool = nullptr;
+  size_t wanted = 0;  // sum of the live handles' largest requests
+  int users = 0;      // live handles
+};
+constexpr size_t WS_SLACK = (size_t)1 << 30;
+namespace {
+std::mutex g_ws_mu;
+WsPool g_ws[SM_CACHE];  // by device ordinal
+}  // namespace
+
+int mrg_ws_open(mrg_problem* p) {
+  int dev = 0;
+  MRG_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= SM_CACHE) return mrg_fail(MRG_ECUDA, "device ordinal out of range");
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  WsPool& w = g_ws[dev];
+  if (!w.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    MRG_CUDA(cudaMemPoolCreate(&pool, &props));
+    // keep memory over synchronisations (trimmed when a handle goes); never make one stream wait for another to
+    // reuse its memory
+    uint64_t keep = UINT64_MAX;
+    int no = 0;
+    cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return mrg_cuda_check(e, "workspace pool");
+    }
+    w.pool = pool;
+  }
+  ++w.users;
+  p->ws_pool = &w;
   return MRG_OK;
 }
+
+void mrg_ws_close(mrg_problem* p) {
+  if (!p->ws_pool) return;
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  WsPool& w = *p->ws_pool;
+  w.wanted -= p->ws_need;
+  --w.users;
+  cudaMemPoolTrimTo(w.pool, w.users ? w.wanted + WS_SLACK : 0);
+  p->ws_pool = nullptr;
+}
+
+cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, void** out) {
+  if (bytes > p->ws_need) {
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    p->ws_pool->wanted += bytes - p->ws_need;
+    p->ws_need = bytes;
+  }
+  return cudaMallocFromPoolAsync(out, bytes, p->ws_pool->pool, s);
+}
+
+cudaError_t mrg_ws_give(void* ws, cudaStream_t s) { return cudaFreeAsync(ws, s); }
 
 static int create_impl(const mrg_mesh_desc* m, const mrg_physics_desc* ph, cudaStream_t cs, mrg_problem** out) {
   if (!m || !ph || !out) return mrg_fail(MRG_EINVAL, "mrg_problem_create: null argument");
