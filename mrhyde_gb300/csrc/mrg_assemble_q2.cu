@@ -19,7 +19,7 @@
 // k_q2_row: one thread a CSR row, rows of one kind per warp (mrg_q2_rows.cuh): its 1, 2, 4 or 8 cells' entries, lane by
 // lane consecutive, added in a fixed order and written once.
 //
-// Measured on 64^3 cells, FP32 Jacobian and FP64 residual: 1818 -> 1347 us (the tensor-core path with eight coloured
+// Measured on 64^3 cells, FP32 Jacobian and FP64 residual: 1818 -> 1156 us (the tensor-core path with eight coloured
 // residual launches before), and the FP32 matrix's error fell from 2.4e-7 to 2.1e-8.
 // MRG_ASM_TENSOR_CORES takes the FP32 element matrices from the tcgen05 kernel instead (mrg_tc_q2.cu), for which
 // k_q2_cell writes the coefficients as TF32 operand images.
@@ -352,27 +352,38 @@ __device__ __forceinline__ void q2_row(const Grid& g, const int (&m)[3], int64_t
       }
   if (DOR && row.on) r[row.n] = res;  // a Dirichlet row is left alone (overwrite: 0)
   if constexpr (DOJ) {
+    // Rows with all their cells: no predicates and no branches, so that a plane's loads are in flight together (the
+    // kernel waits on memory: with a branch at every entry it took 623 us on 64^3 cells)
+    const bool fast = row.all_whole && !__any_sync(0xffffffffu, row.fixed);
+    auto plane = [&](int ez, auto fast_tag) {
+      constexpr bool FAST = decltype(fast_tag)::value;
+      JT v[R::N];
+#pragma unroll
+      for (int n = 0; n < R::N; ++n) {
+        const int oz = ez - half(PZ), oy = n / R::LX - half(PY), ox = n % R::LX - half(PX);
+        v[n] = JT(0);
+#pragma unroll
+        for (int z = 0; z < cells(PZ); ++z)
+#pragma unroll
+          for (int y = 0; y < cells(PY); ++y)
+#pragma unroll
+            for (int x = 0; x < cells(PX); ++x) {
+              const int jx = local(PX, x) + ox, jy = local(PY, y) + oy, jz = local(PZ, z) + oz;
+              if (jx < 0 || jx > 2 || jy < 0 || jy > 2 || jz < 0 || jz > 2) continue;
+              if (FAST || ok[z][y][x]) v[n] += __ldg(e[z][y][x] + (jx + 3 * jy + 9 * jz) * CB);
+            }
+        if (!FAST && OVW && row.fixed && ox == 0 && oy == 0 && oz == 0) v[n] = JT(1);
+      }
+#pragma unroll
+      for (int n = 0; n < R::N; ++n) {
+        if (FAST) stage[(threadIdx.x & 31) * R::N + n] = v[n];
+        else row.put(stage, ez, n / R::LX, n % R::LX, v[n]);
+      }
+    };
 #pragma unroll
     for (int ez = 0; ez < R::LZ; ++ez) {
-#pragma unroll
-      for (int ey = 0; ey < R::LY; ++ey)
-#pragma unroll
-        for (int ex = 0; ex < R::LX; ++ex) {
-          const int oz = ez - half(PZ), oy = ey - half(PY), ox = ex - half(PX);
-          JT v = JT(0);
-#pragma unroll
-          for (int z = 0; z < cells(PZ); ++z)
-#pragma unroll
-            for (int y = 0; y < cells(PY); ++y)
-#pragma unroll
-              for (int x = 0; x < cells(PX); ++x) {
-                const int jx = local(PX, x) + ox, jy = local(PY, y) + oy, jz = local(PZ, z) + oz;
-                if (jx < 0 || jx > 2 || jy < 0 || jy > 2 || jz < 0 || jz > 2) continue;
-                if (ok[z][y][x]) v += __ldg(e[z][y][x] + (jx + 3 * jy + 9 * jz) * CB);
-              }
-          if (OVW && row.fixed && ox == 0 && oy == 0 && oz == 0) v = JT(1);
-          row.put(stage, ez, ey, ex, v);
-        }
+      if (fast) plane(ez, std::true_type{});
+      else plane(ez, std::false_type{});
       row.template store_plane<OVW>(J, stage, ez);
     }
     if (!OVW) row.fix_diagonal(J);
