@@ -37,6 +37,10 @@ using namespace mrgdev;
 constexpr int ST = WST;          // rows per CTA
 constexpr int CHUNK = 16;        // PCG iterations per captured graph
 
+// CTAs per SM the SpMV grid is sized for (shared-memory bound for P = 1)
+template <int P, typename JT>
+constexpr int spmv_per_sm() { return P == 1 ? (sizeof(JT) == 8 ? 4 : 7) : 16; }
+
 // device scalars of one PCG instance
 struct PcgScal {
   double rho, rho_old, pq, alpha, beta, r0, rnorm, tol;
@@ -48,7 +52,7 @@ struct PcgScal {
 // y = J x (FP64 accumulation), Q1 rows through the per-warp staged loop.  err (may be null) is set to 1 if a
 // staging copy did not complete within its time bound.
 template <typename JT>
-__global__ void __launch_bounds__(ST) k_spmv(Grid g, int64_t nrows, const JT* __restrict__ J, const double* __restrict__ x,
+__global__ void __launch_bounds__(ST, spmv_per_sm<1, JT>()) k_spmv(Grid g, int64_t nrows, const JT* __restrict__ J, const double* __restrict__ x,
                                              double* __restrict__ y, int* err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (ST / 32)];
@@ -194,7 +198,7 @@ __global__ void __launch_bounds__(ST) k_pcg64_init(Grid g, int64_t nrows, PcgVec
 
 // q = J p ; pq partial ; last block: alpha = rho / pq
 template <int P>
-__global__ void __launch_bounds__(ST) k_pcg64_spmv(Grid g, int64_t nrows, PcgVec64 V) {
+__global__ void __launch_bounds__(ST, P == 1 ? spmv_per_sm<1, double>() : 1) k_pcg64_spmv(Grid g, int64_t nrows, PcgVec64 V) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (ST / 32)];
   if (((volatile PcgScal*)V.s)->done) return;
@@ -356,7 +360,7 @@ __global__ void __launch_bounds__(ST) k_pcg32_init(Grid g, int64_t nrows, PcgVec
 // iteration is this kernel plus k_pcg32_update.  Partial p.q; last block: alpha = rho / (p.q).
 // Before the first iteration p = z, q = 0 and beta = 0.
 template <int P>
-__global__ void __launch_bounds__(ST) k_pcg32_spmv(Grid g, int64_t nrows, PcgVec32 V) {
+__global__ void __launch_bounds__(ST, P == 1 ? spmv_per_sm<1, float>() : 1) k_pcg32_spmv(Grid g, int64_t nrows, PcgVec32 V) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (ST / 32)];
   if (((volatile PcgScal*)V.s)->done) return;
@@ -509,9 +513,6 @@ inline unsigned pcg_grid(const mrg_problem* p, int per_sm = 16) {
 // dynamic shared memory of the PCG SpMV: two staging buffers for P = 1
 template <int P, typename JT>
 constexpr int spmv_smem() { return P == 1 ? wspmv_smem<JT>() : 0; }
-// CTAs per SM the SpMV grid is sized for (shared-memory bound for P = 1)
-template <int P, typename JT>
-constexpr int spmv_per_sm() { return P == 1 ? (sizeof(JT) == 8 ? 4 : 7) : 16; }
 
 }  // namespace
 
