@@ -30,6 +30,7 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "mrg_device.cuh"
@@ -46,6 +47,10 @@ constexpr int GCHUNK = 2;          // Krylov iterations per captured graph (2: f
 constexpr int MAXC = 32;           // largest coarsest level solved densely
 constexpr int MAXLEV = 16;
 constexpr int64_t RAP_WARP_ROWS = 24576;  // Galerkin sweeps with fewer output rows: one warp per row
+
+// CTAs per SM of the kernels with the staged row loop: what their shared buffers allow
+template <typename T>
+constexpr int staged_per_sm() { return sizeof(T) == 8 ? 4 : 7; }
 
 // ---- 1-D transfer along one axis ----------------------------------------------------------------
 // Parents of fine node i (fine nodes 0..nnf-1, coarse nodes 0..nnc-1) with interpolation weights.
@@ -100,13 +105,15 @@ __device__ __forceinline__ auto row_prod(const Grid& g, const RowInfo& R, const 
   else return row_apply<P, double, double>(g, R, vals, x);
 }
 
-// f(n, R, vals) for every row: Q1 rows through the per-warp staged loop, Q2 rows (125-point) read directly.
-template <int P, typename T, typename F>
+// f(n, R, vals) for every row: Q1 rows through the per-warp staged loop, Q2 rows (125-point) read directly.  gate
+// waits for the predecessor (pdl_wait) and says whether to go on.
+template <int P, typename T, typename F, typename Gate>
 __device__ __forceinline__ bool level_rows(const Grid& g, int64_t n, const T* __restrict__ A, unsigned char* smem_raw,
-                                           uint64_t* mbar, F&& f) {
+                                           uint64_t* mbar, F&& f, Gate&& gate) {
   if constexpr (P == 1) {
-    return warp_staged_rows<T>(g, n, A, smem_raw, mbar, f);
+    return warp_staged_rows<T>(g, n, A, smem_raw, mbar, f, gate);
   } else {
+    if (!gate()) return true;
     for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
       int ix, iy, iz;
       decompose(g, i, ix, iy, iz);
@@ -134,6 +141,12 @@ __device__ __forceinline__ RowInfo row_info_p3(const Grid& g, const P3& pp, int 
 
 __device__ __forceinline__ bool is_done(const GScal* S) { return ((volatile const GScal*)S)->done != 0; }
 
+// whether coordinate i of axis a lies on no Dirichlet face of that axis
+__device__ __forceinline__ bool axis_free(const Grid& g, int a, int i) {
+  if (a >= g.dim) return true;
+  return !(((g.faces >> (2 * a)) & 1u) && i == 0) && !(((g.faces >> (2 * a + 1)) & 1u) && i == g.nn[a] - 1);
+}
+
 // ---- setup kernels ------------------------------------------------------------------------------
 // One axis of the Galerkin product, one thread per row of the output grid gc (gc = gf coarsened along
 // `axis` only).  The free nodes form a Cartesian product (Dirichlet faces are axis-aligned), so the
@@ -141,63 +154,36 @@ __device__ __forceinline__ bool is_done(const GScal* S) { return ((volatile cons
 // each keeping the 27-point layout on an intermediate grid: ~160 multiply-adds per output row instead
 // of ~5,800 for the direct triple product.
 //
-// Rows away from the faces take a fast path: every fine column and coarse parent there is free and has the
-// standard weights (1/2, 1, 1/2), and every row has its full width, so the loops unroll with
-// compile-time accumulator positions (registers instead of a local-memory array).  Row widths along an
-// axis: 3 on a p = 1 axis; on a p = 2 axis 5 at even (vertex) nodes and 3 at odd (mid-edge) nodes.  The
-// swept axis A goes from p = QA ? 2 : 1 to p = 1; the other two axes keep their widths WB, WC (B < C).
-// The fast path adds the same products in the same order as the general loop (children ascending, then
-// the row's entries in storage order, then the lower and upper parent), so the result is bit-identical.
-template <typename T, int A, bool QA, int WB, int WC, int DC>
-__device__ __forceinline__ void rap_child(const Grid& gf, const P3& pf, const int I[3], const T* __restrict__ Af,
-                                          T* acc) {
-  constexpr int B = (A == 0) ? 1 : 0;  // the lower of the two other axes (C is the remaining one)
-  constexpr int WA = (QA && DC == 0) ? 5 : 3;  // child 2I is a vertex node, 2I +- 1 mid-edge nodes
-  constexpr int W0 = (A == 0) ? WA : (B == 0 ? WB : WC);
-  constexpr int W1 = (A == 1) ? WA : (B == 1 ? WB : WC);
-  constexpr int W2 = (A == 2) ? WA : (B == 2 ? WB : WC);
-  constexpr int O0 = (A == 0) ? 3 : W0, O1 = (A == 1) ? 3 : W1, O2 = (A == 2) ? 3 : W2;  // output widths
-  int f[3] = {I[0], I[1], I[2]};
-  f[A] = 2 * I[A] + DC;
-  const T* vals = Af + row_info_p3(gf, pf, f[0], f[1], f[2]).rp;
-  const T wc = (DC == 0) ? T(1) : T(0.5);
+// The h-levels (order 1) take k_rap_line, which adds the same products in the same order as the general loop (children
+// ascending, then the row's entries in storage order, then the lower and upper parent).
+// One child's contribution to an output row of an order-1 grid: the child at 2 I + DC along A, vals its row.  The row's
+// neighbours along an axis that do not exist or are fixed have m[axis][.] false; plo, phi: the weights with which the
+// fine column at 2 I + s (s = -2 .. 2) goes to the coarse columns I + floor(s / 2) and I + ceil(s / 2) (0: fixed or none).
+template <typename T, int A, int DC>
+__device__ __forceinline__ void rap_child(const T* vals, const RowInfo& R, const int (&lo)[3], const bool (&m)[3][3],
+                                          const float (&plo)[5], const float (&phi)[5], T wc, T* acc) {
+  // lo[a]: 1 if the row has a coupling at offset -1 along a
+  const T* v0 = vals + (lo[2] * R.cy + lo[1]) * R.cx + lo[0];
 #pragma unroll
-  for (int ez = -(W2 - 1) / 2; ez <= (W2 - 1) / 2; ++ez)
+  for (int ez = -1; ez <= 1; ++ez)
 #pragma unroll
-    for (int ey = -(W1 - 1) / 2; ey <= (W1 - 1) / 2; ++ey)
+    for (int ey = -1; ey <= 1; ++ey) {
+      const T* v1 = v0 + (ez * R.cy + ey) * R.cx;
 #pragma unroll
-      for (int ex = -(W0 - 1) / 2; ex <= (W0 - 1) / 2; ++ex) {
-        const T a = vals[((ez + (W2 - 1) / 2) * W1 + (ey + (W1 - 1) / 2)) * W0 + (ex + (W0 - 1) / 2)] * wc;
+      for (int ex = -1; ex <= 1; ++ex) {
+        const bool in = m[0][ex + 1] && m[1][ey + 1] && m[2][ez + 1];
+        const T a = (in ? v1[ex] : T(0)) * wc;
         const int e[3] = {ex, ey, ez};
-        const int sft = DC + e[A];  // fine column along A relative to 2I: -2..2
+        const int sft = DC + e[A];
         int o[3] = {ex, ey, ez};
-        if ((sft & 1) == 0) {
-          o[A] = sft / 2;
-          T& t = acc[((o[2] + (O2 - 1) / 2) * O1 + (o[1] + (O1 - 1) / 2)) * O0 + (o[0] + (O0 - 1) / 2)];
-          t += a * T(1);
-        } else {
-          o[A] = (sft - 1) / 2;
-          T& t0 = acc[((o[2] + (O2 - 1) / 2) * O1 + (o[1] + (O1 - 1) / 2)) * O0 + (o[0] + (O0 - 1) / 2)];
-          t0 += a * T(0.5);
-          o[A] = (sft + 1) / 2;
-          T& t1 = acc[((o[2] + (O2 - 1) / 2) * O1 + (o[1] + (O1 - 1) / 2)) * O0 + (o[0] + (O0 - 1) / 2)];
-          t1 += a * T(0.5);
+        o[A] = sft >= 0 ? sft / 2 : -((1 - sft) / 2);  // floor
+        acc[(o[2] + 1) * 9 + (o[1] + 1) * 3 + (o[0] + 1)] += a * (T)plo[sft + 2];
+        if (sft & 1) {
+          o[A] += 1;
+          acc[(o[2] + 1) * 9 + (o[1] + 1) * 3 + (o[0] + 1)] += a * (T)phi[sft + 2];
         }
       }
-}
-
-template <typename T, int A, bool QA, int WB, int WC>
-__device__ __forceinline__ void rap_interior(const Grid& gf, const P3& pf, const int I[3], const T* __restrict__ Af,
-                                             T* __restrict__ out) {
-  constexpr int LEN = 3 * WB * WC;
-  T acc[LEN];
-#pragma unroll
-  for (int k = 0; k < LEN; ++k) acc[k] = T(0);
-  rap_child<T, A, QA, WB, WC, -1>(gf, pf, I, Af, acc);
-  rap_child<T, A, QA, WB, WC, 0>(gf, pf, I, Af, acc);
-  rap_child<T, A, QA, WB, WC, 1>(gf, pf, I, Af, acc);
-#pragma unroll
-  for (int k = 0; k < LEN; ++k) out[k] = acc[k];
+    }
 }
 
 template <typename T>
@@ -215,22 +201,6 @@ __global__ void __launch_bounds__(NT) k_rap_axis(Grid gf, P3 pf, Grid gc, P3 pc,
     const int dg = (int)(diag_pos(Rc, I[0], I[1], I[2]) - Rc.rp);
     for (int e = 0; e < lenc; ++e) out[e] = (e == dg) ? T(1) : T(0);
     return;
-  }
-  // fast path: 3-D, order 1 throughout (the h-levels).  The same template covers order-2 rows, but
-  // instantiating those variants in this kernel raised it from 64 to 128 (FP32) / 254 (FP64) registers
-  // and slowed every sweep; on the Q2 -> Q1 sweeps it was no faster than the loop below (1.66 vs 1.40 ms
-  // for the first sweep of a 64^3 Q2 grid).
-  if (gf.dim == 3 && pf.p[0] == 1 && pf.p[1] == 1 && pf.p[2] == 1 && pc.p[0] == 1 && pc.p[1] == 1 && pc.p[2] == 1) {
-    bool inner = I[axis] >= 2 && 2 * I[axis] + 2 <= gf.nn[axis] - 2;
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      if (b != axis) inner = inner && I[b] >= 2 && I[b] <= gf.nn[b] - 3;
-    if (inner) {
-      if (axis == 0) rap_interior<T, 0, false, 3, 3>(gf, pf, I, Af, out);
-      else if (axis == 1) rap_interior<T, 1, false, 3, 3>(gf, pf, I, Af, out);
-      else rap_interior<T, 2, false, 3, 3>(gf, pf, I, Af, out);
-      return;
-    }
   }
   constexpr int MAXROW = 75;  // 3 x 5 x 5: the widest output row (one axis swept from a Q2 grid)
   if (lenc > MAXROW) { atomicExch(err, 1); return; }
@@ -265,6 +235,132 @@ __global__ void __launch_bounds__(NT) k_rap_axis(Grid gf, P3 pf, Grid gc, P3 pc,
         }
   }
   for (int e = 0; e < lenc; ++e) out[e] = acc[e];
+}
+
+// The sweep of the 3-D h-levels (order 1 throughout), one warp per 32 output rows of a grid line.  The children's rows
+// are consecutive in CSR (axis 0: the fine rows 2 x0 - 1 .. 2 x1 + 1 of the line; otherwise 32 rows of each of the three
+// child lines), so the warp copies them into its shared buffer with consecutive lanes on consecutive addresses, each
+// lane works on its row there, and the output rows leave the same way.  Read and written row by row from global memory
+// the first sweep of a 97^3 grid took 239 us (every load instruction on 32 lines).
+__device__ __forceinline__ bool col_at(const bool (&col)[5], int s) { return s < -2 || s > 2 ? false : col[s + 2]; }
+
+constexpr int RAP_W = 4;             // warps per CTA
+constexpr int RAP_BUF = 3 * 32 * 27;  // the longest copy: three lines of 32 rows (axis 0: 65 rows)
+template <typename T>
+constexpr int rap_smem() { return RAP_W * RAP_BUF * (int)sizeof(T); }
+template <typename T, int A>
+__global__ void __launch_bounds__(RAP_W * 32) k_rap_line(Grid gf, Grid gc, int tiles, int64_t ntile,
+                                                         const T* __restrict__ Af, T* __restrict__ Ac,
+                                                         int* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* buf = reinterpret_cast<T*>(smem_raw) + (threadIdx.x >> 5) * RAP_BUF;
+  const int lane = threadIdx.x & 31;
+  const int64_t tile = (int64_t)blockIdx.x * RAP_W + (threadIdx.x >> 5);
+  if (tile >= ntile) return;  // uniform over the warp
+  const int64_t line = tile / tiles;
+  const int x0 = (int)(tile - line * tiles) * 32, x1 = min(x0 + 32, gc.nn[0]) - 1;
+  int I[3] = {min(x0 + lane, x1), (int)(line % gc.nn[1]), (int)(line / gc.nn[1])};
+  const bool on = x0 + lane <= x1;
+  int fixed_at = -1;  // a Dirichlet row: its diagonal's position
+  // the children's rows: shared offset of the first row of each copied segment
+  const int clo = A == 0 ? 0 : max(2 * I[A] - 1, 0), chi = A == 0 ? 0 : min(2 * I[A] + 1, gf.nn[A] - 1);
+  int64_t seg[3];
+  int at[3], used = 0;
+#pragma unroll
+  for (int c = 0; c < (A == 0 ? 1 : 3); ++c) {
+    int f0[3] = {x0, I[1], I[2]}, f1[3] = {x1, I[1], I[2]};
+    if (A == 0) {
+      f0[0] = max(2 * x0 - 1, 0);
+      f1[0] = min(2 * x1 + 1, gf.nn[0] - 1);
+    } else {
+      if (clo + c > chi) break;
+      f0[A] = f1[A] = clo + c;
+    }
+    const RowInfo R0 = row_info<1>(gf, f0[0], f0[1], f0[2]), R1 = row_info<1>(gf, f1[0], f1[1], f1[2]);
+    const int n = (int)(R1.rp + R1.cx * R1.cy * R1.cz - R0.rp);
+    seg[c] = R0.rp;
+    at[c] = used;
+#pragma unroll 8
+    for (int k = lane; k < n; k += 32) buf[used + k] = __ldg(Af + R0.rp + k);
+    used += n;
+  }
+  __syncwarp();
+  const RowInfo Rc = row_info<1>(gc, I[0], I[1], I[2]);
+  const int lenc = Rc.cx * Rc.cy * Rc.cz;
+  T acc[27];
+#pragma unroll
+  for (int k = 0; k < 27; ++k) acc[k] = T(0);
+  auto fine = [&](int f, int64_t rp) {  // values of the fine row at coordinate f along A
+    if constexpr (A == 0) return buf + (rp - seg[0]);
+    else {
+      const int c = f - clo;
+      return c == 0 ? buf + at[0] + (rp - seg[0]) : (c == 1 ? buf + at[1] + (rp - seg[1]) : buf + at[2] + (rp - seg[2]));
+    }
+  };
+  if (on) {
+    if (node_fixed(gc, I[0], I[1], I[2])) {
+      const int dg = (int)(diag_pos(Rc, I[0], I[1], I[2]) - Rc.rp);
+      fixed_at = dg;
+    } else {
+      // fine columns along A relative to 2 I: they exist, are free, and go to free coarse columns with these weights
+      float plo[5], phi[5];
+      bool col[5];
+#pragma unroll
+      for (int s = -2; s <= 2; ++s) {
+        const int f = 2 * I[A] + s, p0 = I[A] + (s >= 0 ? s / 2 : -((1 - s) / 2));
+        col[s + 2] = f >= 0 && f < gf.nn[A] && axis_free(gf, A, f);
+        plo[s + 2] = phi[s + 2] = 0.0f;
+        if (s & 1) {
+          const bool last = f == gf.nn[A] - 1;  // an odd last node is kept: its parent is the last coarse node, weight 1
+          if (p0 >= 0 && !last && axis_free(gc, A, p0)) plo[s + 2] = 0.5f;
+          if (p0 + 1 < gc.nn[A] && axis_free(gc, A, p0 + 1)) phi[s + 2] = last ? 1.0f : 0.5f;
+        } else if (p0 >= 0 && p0 < gc.nn[A] && axis_free(gc, A, p0)) {
+          plo[s + 2] = 1.0f;
+        }
+      }
+      bool m[3][3];
+      int lo[3];
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        lo[b] = I[b] > 0 ? 1 : 0;
+#pragma unroll
+        for (int e = -1; e <= 1; ++e) m[b][e + 1] = I[b] + e >= 0 && I[b] + e < gf.nn[b] && axis_free(gf, b, I[b] + e);
+      }
+      auto child = [&](auto dc_tag) {
+        constexpr int DC = decltype(dc_tag)::value;
+        int f[3] = {I[0], I[1], I[2]};
+        f[A] = 2 * I[A] + DC;
+        // the child exists, is free and has this row among its parents
+        const float wc = DC == 0 ? plo[2] : (DC < 0 ? phi[1] : plo[3]);
+        if (!col[DC + 2] || wc == 0.0f) return;
+        lo[A] = f[A] > 0 ? 1 : 0;
+#pragma unroll
+        for (int e = -1; e <= 1; ++e) m[A][e + 1] = col_at(col, DC + e);
+        const RowInfo R = row_info<1>(gf, f[0], f[1], f[2]);
+        rap_child<T, A, DC>(fine(f[A], R.rp), R, lo, m, plo, phi, (T)wc, acc);
+      };
+      child(std::integral_constant<int, -1>{});
+      child(std::integral_constant<int, 0>{});
+      child(std::integral_constant<int, 1>{});
+    }
+  }
+  __syncwarp();
+  // the output rows are one segment of CSR
+  const int64_t out0 = __shfl_sync(0xffffffffu, Rc.rp, 0);
+  const int total = (int)(__shfl_sync(0xffffffffu, Rc.rp + lenc, x1 - x0) - out0);
+  T* mine = buf + (Rc.rp - out0);
+  if (on && fixed_at >= 0) {
+    for (int e = 0; e < lenc; ++e) mine[e] = e == fixed_at ? T(1) : T(0);
+  } else if (on) {
+#pragma unroll
+    for (int e = 0; e < 27; ++e) {  // the couplings the row has, in storage order
+      const int x = I[0] + e % 3 - 1, y = I[1] + e / 3 % 3 - 1, z = I[2] + e / 9 - 1;
+      if (x >= 0 && x < gc.nn[0] && y >= 0 && y < gc.nn[1] && z >= 0 && z < gc.nn[2])
+        mine[((z - Rc.lz) * Rc.cy + (y - Rc.ly)) * Rc.cx + (x - Rc.lx)] = acc[e];
+    }
+  }
+  __syncwarp();
+  for (int k = lane; k < total; k += 32) Ac[out0 + k] = buf[k];
 }
 
 // The same sweep with one warp per output row and the lanes over the row's entries: an entry sums, over
@@ -354,23 +450,26 @@ __global__ void __launch_bounds__(NT) k_rap_axis_w(Grid gf, P3 pf, Grid gc, P3 p
 
 // minv = 1 / diag; Gershgorin bound max_i sum_j |a_ij| / |a_ii| into lmax (as float bits, atomicMax)
 template <int P, typename T>
-__global__ void __launch_bounds__(NT) k_diag(Grid g, const T* __restrict__ A, T* __restrict__ minv,
-                                             unsigned int* __restrict__ lmax_bits) {
-  const int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x;
+__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_diag(Grid g, const T* __restrict__ A, T* __restrict__ minv,
+                                                                 unsigned int* __restrict__ lmax_bits, int* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t mbar[2 * (NT / 32)];
   const int64_t nrows = (int64_t)g.nn[0] * g.nn[1] * g.nn[2];
   float v = 0.0f;
-  if (n < nrows) {
-    int ix, iy, iz;
-    decompose(g, n, ix, iy, iz);
-    const RowInfo R = row_info<P>(g, ix, iy, iz);
-    const T* vals = A + R.rp;
-    const int len = R.cx * R.cy * R.cz;
-    const T dgv = vals[diag_pos(R, ix, iy, iz) - R.rp];
-    T s = T(0);  // a bound: the level's precision is enough
-    for (int e = 0; e < len; ++e) s += fabs(vals[e]);
-    minv[n] = T(1) / dgv;
-    v = (float)(s / fabs(dgv));
-  }
+  const bool ok = level_rows<P, T>(
+      g, nrows, A, smem_raw, mbar,
+      [&](int64_t n, const RowInfo& R, const T* vals) {
+        int ix, iy, iz;
+        decompose(g, n, ix, iy, iz);
+        const int len = R.cx * R.cy * R.cz;
+        const T dgv = vals[diag_pos(R, ix, iy, iz) - R.rp];
+        T s = T(0);  // a bound: the level's precision is enough
+        for (int e = 0; e < len; ++e) s += fabs(vals[e]);
+        minv[n] = T(1) / dgv;
+        v = fmaxf(v, (float)(s / fabs(dgv)));
+      },
+      AlwaysGo{});
+  if (!ok) atomicExch(err, 3);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
   if ((threadIdx.x & 31) == 0 && v > 0.0f) atomicMax(lmax_bits, __float_as_uint(v));
@@ -495,34 +594,38 @@ __device__ __forceinline__ void resid_row(const LevDev<T>& L, int64_t n, T ax) {
 }
 
 template <int P, typename T>
-__global__ void __launch_bounds__(NT) k_cheb(LevDev<T> L, const T* __restrict__ xin, T* __restrict__ xout, int k,
+__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cheb(LevDev<T> L, const T* __restrict__ xin, T* __restrict__ xout, int k,
                                              int zero_x, const double* __restrict__ coef,
                                              const GScal* __restrict__ S, int* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (NT / 32)];
-  if (is_done(S)) return;
+  pdl_trigger();
   const T c_first = (T)coef[3 * k], c_old = (T)coef[3 * k + 1], c_new = (T)coef[3 * k + 2];
   auto fin = [&](int64_t n, T ax) { cheb_row<T>(L, n, ax, xin, xout, k, zero_x, c_first, c_old, c_new); };
   if (zero_x) {
+    pdl_wait();
+    if (is_done(S)) return;
     for (int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x; n < L.n; n += (int64_t)gridDim.x * NT) fin(n, T(0));
     return;
   }
-  const bool ok = level_rows<P, T>(L.g, L.n, L.A, smem_raw, mbar, [&](int64_t n, const RowInfo& R, const T* vals) {
-    fin(n, (T)row_prod<P, T>(L.g, R, vals, xin));
-  });
+  const bool ok = level_rows<P, T>(
+      L.g, L.n, L.A, smem_raw, mbar,
+      [&](int64_t n, const RowInfo& R, const T* vals) { fin(n, (T)row_prod<P, T>(L.g, R, vals, xin)); },
+      [&] { pdl_wait(); return !is_done(S); });
   if (!ok) atomicExch(err, 3);
 }
 
 // r = b - A x
 template <int P, typename T>
-__global__ void __launch_bounds__(NT) k_resid(LevDev<T> L, const T* __restrict__ x, const GScal* __restrict__ S,
+__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_resid(LevDev<T> L, const T* __restrict__ x, const GScal* __restrict__ S,
                                               int* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (NT / 32)];
-  if (is_done(S)) return;
-  const bool ok = level_rows<P, T>(L.g, L.n, L.A, smem_raw, mbar, [&](int64_t n, const RowInfo& R, const T* vals) {
-    resid_row<T>(L, n, (T)row_prod<P, T>(L.g, R, vals, x));
-  });
+  pdl_trigger();
+  const bool ok = level_rows<P, T>(
+      L.g, L.n, L.A, smem_raw, mbar,
+      [&](int64_t n, const RowInfo& R, const T* vals) { resid_row<T>(L, n, (T)row_prod<P, T>(L.g, R, vals, x)); },
+      [&] { pdl_wait(); return !is_done(S); });
   if (!ok) atomicExch(err, 3);
 }
 
@@ -568,36 +671,46 @@ __device__ __forceinline__ void parent_slots(int i, int nnf, int nnc, int co, bo
 }
 
 // b_c = P^T r_f, coarse row n (shared by k_restrict and k_vcycle_tail)
+// The free nodes are a Cartesian product, so a child counts if it exists and is free along each axis; the others are
+// loaded as zeros (no branches: the lanes of a warp have children missing at different places).
 template <typename T>
 __device__ __forceinline__ void restrict_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* __restrict__ rf,
                                              T* __restrict__ bc, int64_t n) {
   int I[3];
   decompose(gc, n, I[0], I[1], I[2]);
   if (node_fixed(gc, I[0], I[1], I[2])) { bc[n] = T(0); return; }
-  int c0[3], c1[3], c2[3];
-  float w0[3], w1[3], w2[3];
-  bool k0[3], k1[3], k2[3];
-  child_slots(I[0], gf.nn[0], gc.nn[0], X.co[0], gf.dim > 0, c0, w0, k0);
-  child_slots(I[1], gf.nn[1], gc.nn[1], X.co[1], gf.dim > 1, c1, w1, k1);
-  child_slots(I[2], gf.nn[2], gc.nn[2], X.co[2], gf.dim > 2, c2, w2, k2);
+  int c[3][3];
+  float w[3][3];
+  bool k[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    child_slots(I[a], gf.nn[a], gc.nn[a], X.co[a], gf.dim > a, c[a], w[a], k[a]);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) k[a][e] = k[a][e] && axis_free(gf, a, c[a][e]);
+  }
+  const int NX = gf.nn[0];
+  const int64_t plane = (int64_t)NX * gf.nn[1];
   T s = T(0);
 #pragma unroll
   for (int a2 = 0; a2 < 3; ++a2)
 #pragma unroll
-    for (int a1 = 0; a1 < 3; ++a1)
+    for (int a1 = 0; a1 < 3; ++a1) {
+      const T* r = rf + NX * c[1][a1] + plane * c[2][a2];
+      const float w12 = w[1][a1] * w[2][a2];
 #pragma unroll
       for (int a0 = 0; a0 < 3; ++a0) {
-        if (!(k2[a2] && k1[a1] && k0[a0])) continue;
-        const int ix = c0[a0], iy = c1[a1], iz = c2[a2];
-        if (node_fixed(gf, ix, iy, iz)) continue;
-        s = fma((T)(w0[a0] * w1[a1] * w2[a2]), rf[ix + (int64_t)gf.nn[0] * (iy + (int64_t)gf.nn[1] * iz)], s);
+        const bool in = k[2][a2] && k[1][a1] && k[0][a0];
+        s = fma((T)(w[0][a0] * w12), in ? r[c[0][a0]] : T(0), s);  // the weights are powers of two
       }
+    }
   bc[n] = s;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(NT) k_restrict(Grid gf, Grid gc, Xfer X, const T* __restrict__ rf, T* __restrict__ bc,
                                                  const GScal* __restrict__ S) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(S)) return;
   const int64_t nc = (int64_t)gc.nn[0] * gc.nn[1] * gc.nn[2];
   for (int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x; n < nc; n += (int64_t)gridDim.x * NT)
@@ -611,29 +724,38 @@ __device__ __forceinline__ void prolong_row(const Grid& gf, const Grid& gc, cons
   int i[3];
   decompose(gf, n, i[0], i[1], i[2]);
   if (node_fixed(gf, i[0], i[1], i[2])) return;
-  int p0[2], p1[2], p2[2];
-  float w0[2], w1[2], w2[2];
-  bool k0[2], k1[2], k2[2];
-  parent_slots(i[0], gf.nn[0], gc.nn[0], X.co[0], gf.dim > 0, p0, w0, k0);
-  parent_slots(i[1], gf.nn[1], gc.nn[1], X.co[1], gf.dim > 1, p1, w1, k1);
-  parent_slots(i[2], gf.nn[2], gc.nn[2], X.co[2], gf.dim > 2, p2, w2, k2);
+  int p[3][2];
+  float w[3][2];
+  bool k[3][2];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    parent_slots(i[a], gf.nn[a], gc.nn[a], X.co[a], gf.dim > a, p[a], w[a], k[a]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) k[a][e] = k[a][e] && axis_free(gc, a, p[a][e]);
+  }
+  const int NX = gc.nn[0];
+  const int64_t plane = (int64_t)NX * gc.nn[1];
   T s = T(0);
 #pragma unroll
   for (int b2 = 0; b2 < 2; ++b2)
 #pragma unroll
-    for (int b1 = 0; b1 < 2; ++b1)
+    for (int b1 = 0; b1 < 2; ++b1) {
+      const T* r = xc + NX * p[1][b1] + plane * p[2][b2];
+      const float w12 = w[1][b1] * w[2][b2];
 #pragma unroll
       for (int b0 = 0; b0 < 2; ++b0) {
-        if (!(k2[b2] && k1[b1] && k0[b0])) continue;
-        if (node_fixed(gc, p0[b0], p1[b1], p2[b2])) continue;
-        s = fma((T)(w0[b0] * w1[b1] * w2[b2]), xc[p0[b0] + (int64_t)gc.nn[0] * (p1[b1] + (int64_t)gc.nn[1] * p2[b2])], s);
+        const bool in = k[2][b2] && k[1][b1] && k[0][b0];
+        s = fma((T)(w[0][b0] * w12), in ? r[p[0][b0]] : T(0), s);
       }
+    }
   xf[n] = add_rn(xf[n], s);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(NT) k_prolong(Grid gf, Grid gc, Xfer X, const T* __restrict__ xc, T* __restrict__ xf,
                                                 const GScal* __restrict__ S) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(S)) return;
   const int64_t nf = (int64_t)gf.nn[0] * gf.nn[1] * gf.nn[2];
   for (int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x; n < nf; n += (int64_t)gridDim.x * NT)
@@ -652,6 +774,8 @@ __device__ __forceinline__ void coarse_row(int n, const T* __restrict__ inv, con
 template <typename T>
 __global__ void __launch_bounds__(NT) k_coarse_apply(int n, const T* __restrict__ inv, const T* __restrict__ b,
                                                      T* __restrict__ x, const GScal* __restrict__ S) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(S)) return;
   for (int i = threadIdx.x; i < n; i += NT) coarse_row<T>(n, inv, b, x, i);
 }
@@ -660,16 +784,18 @@ __global__ void __launch_bounds__(NT) k_coarse_apply(int n, const T* __restrict_
 // The smallest levels take a microsecond of work per step but a launch each (seven per level and cycle).
 // k_vcycle_tail runs the whole cycle below the first such level -- pre-smoothing, residual and restriction
 // down to the coarsest level, the dense coarsest solve, prolongation and post-smoothing back up -- in one
-// CTA, with a CTA barrier between steps.  Every row is computed by the same device functions, in the same
-// order, as by the per-step kernels, so the result is bit-identical (MRG_PREC_GMG_SPLIT keeps the per-step
-// launches for comparison).
+// CTA, with a CTA barrier between steps.  What bounds it is the chain of steps, so everything they touch is in
+// shared memory: the levels' operators and diagonals are copied there before the kernel waits for its predecessor
+// (no kernel of a solve writes them), the vectors live there, and each row's start and extents are worked out once.
+// From global memory, with the row decoding at every step, the tail of a 97^3 hierarchy (7^3 nodes) took 42 us.  Every
+// row's arithmetic is that of the per-step kernels, in the same order, so the result is bit-identical
+// (MRG_PREC_GMG_SPLIT keeps the per-step launches for comparison).
 constexpr int TT = 1024;               // threads of the tail CTA
 constexpr int MAXTAIL = 8;             // levels the tail can hold
 constexpr int64_t TAIL_ROWS32 = 1024;  // FP32: first level taken into the tail has at most this many rows
-// A level's sweep in one SM must cost less than the launches it replaces.  Measured on the C2 mixed
-// multigrid Newton solve (128^3): FP32 tail from 9^3 nodes 9.62 ms, none 9.83 ms, from 17^3 nodes
-// 10.66 ms.  FP64 takes none: its pipe (1/64 of the FP32 rate) makes a single-SM sweep of a 729-row
-// level as long as a launch, and from 17^3 nodes the FP64 solve went 26.4 -> 31.9 ms.
+constexpr size_t TAIL_SMEM = 200 * 1024;
+// A level's sweep in one SM must cost less than the launches it replaces.  FP64 takes no tail: its pipe (1/64 of the
+// FP32 rate) makes a single-SM sweep of a 729-row level as long as a launch.
 template <typename T>
 constexpr int64_t tail_rows() { return sizeof(T) == 4 ? TAIL_ROWS32 : 0; }
 
@@ -682,53 +808,137 @@ struct TailArgs {
   const T* cinv = nullptr;       // dense inverse of the coarsest operator
 };
 
+// shared memory of one smoothed level: row records, operator, 1/diag and five vectors
 template <typename T>
-__device__ __forceinline__ void tail_cheb(const LevDev<T>& D, const T* xin, T* xout, int k, int zero_x,
+__host__ __device__ inline size_t tail_level_bytes(const Grid& g, int64_t n) {
+  const size_t nnz = (size_t)(g.T[0] * g.T[1] * g.T[2]);
+  return (size_t)n * sizeof(int4) + (((nnz + 6 * (size_t)n) * sizeof(T) + 15) & ~(size_t)15);
+}
+template <typename T>
+inline size_t tail_smem(const TailArgs<T>& A) {
+  size_t b = 0;
+  for (int j = 0; j + 1 < A.nlev; ++j) b += tail_level_bytes<T>(A.L[j].g, A.L[j].n);
+  const size_t n = (size_t)A.L[A.nlev - 1].n;
+  return b + n * (n + 2) * sizeof(T);
+}
+
+// a level in shared memory; LevDev with row records
+template <typename T>
+struct TailLev {
+  LevDev<T> D;
+  const int4* row;  // start in A, first coupled node, extents cx | cy << 2 | cz << 4
+};
+
+template <typename T>
+__device__ __forceinline__ T tail_prod(const TailLev<T>& L, int n, const T* x) {
+  const int4 q = L.row[n];
+  const T* a = L.D.A + q.x;
+  const T* xb = x + q.y;
+  const int NX = L.D.g.nn[0], plane = NX * L.D.g.nn[1];
+  T acc = T(0);
+  if (q.z == (3 | 3 << 2 | 3 << 4)) {
+#pragma unroll
+    for (int k = 0; k < 27; ++k) acc = fma(a[k], xb[(k % 3) + NX * ((k / 3) % 3) + plane * (k / 9)], acc);
+    return acc;
+  }
+  const int cx = q.z & 3, cy = (q.z >> 2) & 3, cz = q.z >> 4;
+  int pos = 0;
+#pragma unroll
+  for (int z = 0; z < 3; ++z)
+    if (z < cz)
+#pragma unroll
+      for (int y = 0; y < 3; ++y)
+        if (y < cy)
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            if (i < cx) acc = fma(a[pos++], xb[i + NX * y + plane * z], acc);
+  return acc;
+}
+
+template <typename T>
+__device__ __forceinline__ void tail_cheb(const TailLev<T>& L, const T* xin, T* xout, int k, int zero_x,
                                           const double* __restrict__ coef) {
   const T c_first = (T)coef[3 * k], c_old = (T)coef[3 * k + 1], c_new = (T)coef[3 * k + 2];
-  for (int64_t n = threadIdx.x; n < D.n; n += TT) {
-    T ax = T(0);
-    if (!zero_x) {
-      int ix, iy, iz;
-      decompose(D.g, n, ix, iy, iz);
-      const RowInfo R = row_info<1>(D.g, ix, iy, iz);
-      ax = (T)row_prod<1, T>(D.g, R, D.A + R.rp, xin);
-    }
-    cheb_row<T>(D, n, ax, xin, xout, k, zero_x, c_first, c_old, c_new);
-  }
+  for (int n = threadIdx.x; n < (int)L.D.n; n += TT)
+    cheb_row<T>(L.D, n, zero_x ? T(0) : tail_prod<T>(L, n, xin), xin, xout, k, zero_x, c_first, c_old, c_new);
   __syncthreads();
 }
 
 template <typename T>
-__global__ void __launch_bounds__(TT) k_vcycle_tail(const TailArgs<T> A, const GScal* __restrict__ S) {
-  if (is_done(S)) return;
+__global__ void __launch_bounds__(TT) k_vcycle_tail(const __grid_constant__ TailArgs<T> A, const GScal* __restrict__ S) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ TailLev<T> lev[MAXTAIL];
+  pdl_trigger();
   const int nl = A.nlev;
-  for (int j = 0; j < nl - 1; ++j) {
-    const LevDev<T>& D = A.L[j];
-    tail_cheb<T>(D, D.xa, D.xa, 0, 1, A.coef[j]);
-    tail_cheb<T>(D, D.xa, D.xb, 1, 0, A.coef[j]);
-    for (int64_t n = threadIdx.x; n < D.n; n += TT) {
-      int ix, iy, iz;
-      decompose(D.g, n, ix, iy, iz);
-      const RowInfo R = row_info<1>(D.g, ix, iy, iz);
-      resid_row<T>(D, n, (T)row_prod<1, T>(D.g, R, D.A + R.rp, D.xb));
+  {
+    unsigned char* at = smem_raw;
+    for (int j = 0; j < nl; ++j) {
+      const LevDev<T>& G = A.L[j];
+      const int n = (int)G.n;
+      TailLev<T> L;
+      L.D = G;
+      if (j == nl - 1) {  // coarsest: inverse, right-hand side, solution
+        T* v = reinterpret_cast<T*>(at);
+        for (int k = threadIdx.x; k < n * n; k += TT) v[k] = A.cinv[k];
+        L.D.A = v;
+        L.D.b = v + n * n;
+        L.D.xb = L.D.b + n;
+        L.row = nullptr;
+      } else {
+        int4* row = reinterpret_cast<int4*>(at);
+        T* v = reinterpret_cast<T*>(row + n);
+        const int nnz = (int)(G.g.T[0] * G.g.T[1] * G.g.T[2]);
+        for (int k = threadIdx.x; k < nnz; k += TT) v[k] = G.A[k];
+        L.D.A = v;
+        L.D.minv = v + nnz;
+        L.D.xa = L.D.minv + n;
+        L.D.xb = L.D.xa + n;
+        L.D.d = L.D.xb + n;
+        L.D.b = L.D.d + n;
+        L.D.r = L.D.b + n;
+        for (int k = threadIdx.x; k < n; k += TT) {
+          L.D.minv[k] = G.minv[k];
+          int ix, iy, iz;
+          decompose(G.g, k, ix, iy, iz);
+          const RowInfo R = row_info<1>(G.g, ix, iy, iz);
+          row[k] = make_int4((int)R.rp, R.lx + G.g.nn[0] * (R.ly + G.g.nn[1] * R.lz), R.cx | R.cy << 2 | R.cz << 4, 0);
+        }
+        L.row = row;
+        at += tail_level_bytes<T>(G.g, n);
+      }
+      if (threadIdx.x == 0) lev[j] = L;
     }
+  }
+  pdl_wait();
+  if (is_done(S)) return;
+  __syncthreads();
+  for (int n = threadIdx.x; n < (int)A.L[0].n; n += TT) lev[0].D.b[n] = A.L[0].b[n];
+  __syncthreads();
+  for (int j = 0; j < nl - 1; ++j) {
+    const TailLev<T>& L = lev[j];
+    const LevDev<T>& D = L.D;
+    tail_cheb<T>(L, D.xa, D.xa, 0, 1, A.coef[j]);
+    tail_cheb<T>(L, D.xa, D.xb, 1, 0, A.coef[j]);
+    for (int n = threadIdx.x; n < (int)D.n; n += TT) resid_row<T>(D, n, tail_prod<T>(L, n, D.xb));
     __syncthreads();
-    const LevDev<T>& C = A.L[j + 1];
+    const LevDev<T>& C = lev[j + 1].D;
     for (int64_t n = threadIdx.x; n < C.n; n += TT) restrict_row<T>(D.g, C.g, A.X[j + 1], D.r, C.b, n);
     __syncthreads();
   }
-  const LevDev<T>& Lc = A.L[nl - 1];
-  for (int i = threadIdx.x; i < (int)Lc.n; i += TT) coarse_row<T>((int)Lc.n, A.cinv, Lc.b, Lc.xb, i);
+  const LevDev<T>& Lc = lev[nl - 1].D;
+  for (int i = threadIdx.x; i < (int)Lc.n; i += TT) coarse_row<T>((int)Lc.n, Lc.A, Lc.b, Lc.xb, i);
   __syncthreads();
   for (int j = nl - 2; j >= 0; --j) {
-    const LevDev<T>& D = A.L[j];
-    const LevDev<T>& C = A.L[j + 1];
+    const TailLev<T>& L = lev[j];
+    const LevDev<T>& D = L.D;
+    const LevDev<T>& C = lev[j + 1].D;
     for (int64_t n = threadIdx.x; n < D.n; n += TT) prolong_row<T>(D.g, C.g, A.X[j + 1], C.xb, D.xb, n);
     __syncthreads();
-    tail_cheb<T>(D, D.xb, D.xa, 0, 0, A.coef[j]);
-    tail_cheb<T>(D, D.xa, D.xb, 1, 0, A.coef[j]);
+    tail_cheb<T>(L, D.xb, D.xa, 0, 0, A.coef[j]);
+    tail_cheb<T>(L, D.xa, D.xb, 1, 0, A.coef[j]);
   }
+  // what the level above reads
+  for (int n = threadIdx.x; n < (int)A.L[0].n; n += TT) A.L[0].xb[n] = lev[0].D.xb[n];
 }
 
 // ---- CG kernels -----------------------------------------------------------------------------------
@@ -773,6 +983,8 @@ __global__ void __launch_bounds__(NT) k_cg_init(int64_t n, const double* __restr
 // rho_new = r . z ; beta = rho_new / rho (0 on the first call)
 template <typename T>
 __global__ void __launch_bounds__(NT) k_cg_rz(int64_t n, CgVec<T> V, int first) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(V.S)) return;
   T rz = T(0);
   for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
@@ -792,20 +1004,28 @@ __global__ void __launch_bounds__(NT) k_cg_rz(int64_t n, CgVec<T> V, int first) 
 
 // w = A z ; p = z + beta p ; q = w + beta q ; partial p.q ; alpha = rho / p.q
 template <int P, typename T>
-__global__ void __launch_bounds__(NT) k_cg_spmv(Grid g, int64_t n, const T* __restrict__ A, CgVec<T> V) {
+__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cg_spmv(Grid g, int64_t n, const T* __restrict__ A, CgVec<T> V) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (NT / 32)];
-  if (is_done(V.S)) return;
-  const T beta = (T)V.S->beta;
-  T pq = T(0);
-  const bool ok = level_rows<P, T>(g, n, A, smem_raw, mbar, [&](int64_t i, const RowInfo& R, const T* vals) {
-    const T w = (T)row_prod<P, T>(g, R, vals, V.z);
-    const T pn = V.z[i] + beta * V.p[i];
-    const T qn = w + beta * V.q[i];
-    V.p[i] = pn;
-    V.q[i] = qn;
-    pq = fma(pn, qn, pq);
-  });
+  pdl_trigger();
+  T beta = T(0), pq = T(0);
+  bool go = false;
+  const bool ok = level_rows<P, T>(
+      g, n, A, smem_raw, mbar,
+      [&](int64_t i, const RowInfo& R, const T* vals) {
+        const T w = (T)row_prod<P, T>(g, R, vals, V.z);
+        const T pn = V.z[i] + beta * V.p[i];
+        const T qn = w + beta * V.q[i];
+        V.p[i] = pn;
+        V.q[i] = qn;
+        pq = fma(pn, qn, pq);
+      },
+      [&] {
+        pdl_wait();
+        beta = (T)V.S->beta;
+        return go = !is_done(V.S);
+      });
+  if (!go) return;
   if (!ok) atomicExch(&V.S->err, 3);
   double m[1] = {block_sum((double)pq)};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
@@ -824,6 +1044,8 @@ __global__ void __launch_bounds__(NT) k_cg_spmv(Grid g, int64_t n, const T* __re
 // x += alpha p ; r -= alpha q ; |r| ; stopping test
 template <typename T>
 __global__ void __launch_bounds__(NT) k_cg_update(int64_t n, CgVec<T> V) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(V.S)) return;
   const T alpha = (T)V.S->alpha;
   T rr = T(0);
@@ -897,6 +1119,8 @@ __global__ void __launch_bounds__(NT) k_bg_init(int64_t n, const double* __restr
 // p = r + beta (p - omega v)
 template <typename T>
 __global__ void __launch_bounds__(NT) k_bg_p(int64_t n, BgVec<T> V) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(V.S)) return;
   const T beta = (T)V.S->beta, omega = (T)V.S->omega;
   for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
@@ -905,23 +1129,31 @@ __global__ void __launch_bounds__(NT) k_bg_p(int64_t n, BgVec<T> V) {
 
 // STEP 0: v = A ph, rv = rh . v, alpha = rho / rv.   STEP 1: t = A sh, omega = (t . s) / (t . t).
 template <int P, typename T, int STEP>
-__global__ void __launch_bounds__(NT) k_bg_spmv(Grid g, int64_t n, const T* __restrict__ A, BgVec<T> V) {
+__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_bg_spmv(Grid g, int64_t n, const T* __restrict__ A, BgVec<T> V) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (NT / 32)];
-  if (is_done(V.S)) return;
+  pdl_trigger();
   const T* in = STEP == 0 ? V.ph : V.sh;
   T* out = STEP == 0 ? V.v : V.t;
   T d0 = T(0), d1 = T(0);
-  const bool ok = level_rows<P, T>(g, n, A, smem_raw, mbar, [&](int64_t i, const RowInfo& R, const T* vals) {
-    const T y = (T)row_prod<P, T>(g, R, vals, in);
-    out[i] = y;
-    if (STEP == 0) {
-      d0 = fma(V.rh[i], y, d0);
-    } else {
-      d0 = fma(y, V.s[i], d0);
-      d1 = fma(y, y, d1);
-    }
-  });
+  bool go = false;
+  const bool ok = level_rows<P, T>(
+      g, n, A, smem_raw, mbar,
+      [&](int64_t i, const RowInfo& R, const T* vals) {
+        const T y = (T)row_prod<P, T>(g, R, vals, in);
+        out[i] = y;
+        if (STEP == 0) {
+          d0 = fma(V.rh[i], y, d0);
+        } else {
+          d0 = fma(y, V.s[i], d0);
+          d1 = fma(y, y, d1);
+        }
+      },
+      [&] {
+        pdl_wait();
+        return go = !is_done(V.S);
+      });
+  if (!go) return;
   if (!ok) atomicExch(&V.S->err, 3);
   double m[2] = {block_sum((double)d0), block_sum((double)d1)};
   if (last_block<2>(V.parts, m, &V.S->counter)) {
@@ -944,6 +1176,8 @@ __global__ void __launch_bounds__(NT) k_bg_spmv(Grid g, int64_t n, const T* __re
 // s = r - alpha v
 template <typename T>
 __global__ void __launch_bounds__(NT) k_bg_s(int64_t n, BgVec<T> V) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(V.S)) return;
   const T alpha = (T)V.S->alpha;
   for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
@@ -953,6 +1187,8 @@ __global__ void __launch_bounds__(NT) k_bg_s(int64_t n, BgVec<T> V) {
 // x += alpha ph + omega sh ; r = s - omega t ; |r|, rh . r -> beta for the next direction; stopping test
 template <typename T>
 __global__ void __launch_bounds__(NT) k_bg_update(int64_t n, BgVec<T> V) {
+  pdl_trigger();
+  pdl_wait();
   if (is_done(V.S)) return;
   const T alpha = (T)V.S->alpha, omega = (T)V.S->omega;
   T rr = T(0), rhr = T(0);
@@ -988,9 +1224,6 @@ unsigned grid_for(int64_t n, int per_sm) {
   const unsigned need = nblk(n, NT), cap = (unsigned)(per_sm * num_sms());
   return need < cap ? need : cap;
 }
-
-template <typename T>
-constexpr int staged_per_sm() { return sizeof(T) == 8 ? 4 : 7; }
 
 // ---- hierarchy ------------------------------------------------------------------------------------
 struct HLevel {
@@ -1219,14 +1452,17 @@ void set_tail(Hier<T>* H, bool split) {
     for (int l = t; l < nl; ++l)
       if (H->L[l].pp.p[0] != 1 || H->L[l].pp.p[1] != 1 || H->L[l].pp.p[2] != 1) t = nl;
   }
-  H->tail = t;
   TailArgs<T>& A = H->targs;
-  A.nlev = nl - t;
-  for (int j = 0; j < A.nlev; ++j) {
-    A.L[j] = levdev<T>(H->L[t + j]);
-    A.X[j] = H->L[t + j].X;
-    A.coef[j] = H->coef + (size_t)(t + j) * NU * 3;
+  for (;; ++t) {  // a first level that does not fit the shared memory stays with the launches
+    A.nlev = nl - t;
+    for (int j = 0; j < A.nlev; ++j) {
+      A.L[j] = levdev<T>(H->L[t + j]);
+      A.X[j] = H->L[t + j].X;
+      A.coef[j] = H->coef + (size_t)(t + j) * NU * 3;
+    }
+    if (A.nlev == 0 || tail_smem<T>(A) <= TAIL_SMEM) break;
   }
+  H->tail = t;
   A.cinv = H->cinv;
 }
 
@@ -1237,6 +1473,11 @@ int set_staged_attr() {
   std::call_once(once, [] {
     const int smem = (NT / 32) * 2 * wbuf_elems<T>() * (int)sizeof(T);
     e = cudaFuncSetAttribute(k_cheb<1, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_diag<1, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rap_line<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, rap_smem<T>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rap_line<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, rap_smem<T>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rap_line<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, rap_smem<T>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_vcycle_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_resid<1, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cg_spmv<1, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_bg_spmv<1, T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1255,8 +1496,8 @@ int setup_level0(Hier<T>* H, const T* J, cudaStream_t s) {
   HLevel& L = H->L[0];
   L.A = const_cast<T*>(J);
   MRG_CUDA(cudaMemsetAsync(H->lmax, 0, sizeof(unsigned int), s));
-  if (L.pp.p[0] == 2) k_diag<2, T><<<nblk(L.n, NT), NT, 0, s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax);
-  else k_diag<1, T><<<nblk(L.n, NT), NT, 0, s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax);
+  if (L.pp.p[0] == 2) k_diag<2, T><<<grid_for(L.n, 16), NT, 0, s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax, H->err);
+  else k_diag<1, T><<<grid_for(L.n, staged_per_sm<T>()), NT, staged_smem<T>(), s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax, H->err);
   k_cheb_coef<<<1, 32, 0, s>>>(H->lmax, (int)H->L.size(), H->coef);
   MRG_CUDA(cudaGetLastError());
   return MRG_OK;
@@ -1281,21 +1522,31 @@ int setup_values(Hier<T>* H, const T* J, cudaStream_t s) {
         const P3 pout = last ? L.pp : L.mid_pp[w];
         T* aout = last ? (T*)L.A : H->mid[w];
         const int64_t nout = (int64_t)gout.nn[0] * gout.nn[1] * gout.nn[2];
-        if (nout < RAP_WARP_ROWS) {
+        const bool line = gout.dim == 3 && pin.p[0] == 1 && pin.p[1] == 1 && pin.p[2] == 1;
+        if (!line && nout < RAP_WARP_ROWS) {
           const unsigned nb = nblk(nout * 32, NT);
           if (L.sweep_axis[w] == 0) k_rap_axis_w<T, 0><<<nb, NT, 0, s>>>(*gin, pin, gout, pout, ain, aout);
           else if (L.sweep_axis[w] == 1) k_rap_axis_w<T, 1><<<nb, NT, 0, s>>>(*gin, pin, gout, pout, ain, aout);
           else k_rap_axis_w<T, 2><<<nb, NT, 0, s>>>(*gin, pin, gout, pout, ain, aout);
-        } else
+        } else if (line) {
+          const int tiles = (gout.nn[0] + 31) / 32;
+          const int64_t nt = (int64_t)tiles * gout.nn[1] * gout.nn[2];
+          const unsigned nb = nblk(nt, RAP_W);
+          constexpr int smem = rap_smem<T>();
+          if (L.sweep_axis[w] == 0) k_rap_line<T, 0><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout, H->err);
+          else if (L.sweep_axis[w] == 1) k_rap_line<T, 1><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout, H->err);
+          else k_rap_line<T, 2><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout, H->err);
+        } else {
           k_rap_axis<T><<<nblk(nout, NT), NT, 0, s>>>(*gin, pin, gout, pout, L.sweep_axis[w], ain, aout, H->err);
+        }
         MRG_CUDA(cudaGetLastError());
         gin = &gout;
         pin = pout;
         ain = aout;
       }
     }
-    if (L.pp.p[0] == 2) k_diag<2, T><<<nblk(L.n, NT), NT, 0, s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax + l);
-    else k_diag<1, T><<<nblk(L.n, NT), NT, 0, s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax + l);
+    if (L.pp.p[0] == 2) k_diag<2, T><<<grid_for(L.n, 16), NT, 0, s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax + l, H->err);
+    else k_diag<1, T><<<grid_for(L.n, staged_per_sm<T>()), NT, staged_smem<T>(), s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax + l, H->err);
     MRG_CUDA(cudaGetLastError());
   }
   k_coarse_inv<T><<<1, NT, 0, s>>>(H->L.back().g, (const T*)H->L.back().A, H->cinv, H->err);
@@ -1310,17 +1561,17 @@ template <typename T>
 void launch_cheb(const HLevel& L, const LevDev<T>& D, const T* xin, T* xout, int k, int zero_x,
                  const double* coef, const GScal* S, int* err, cudaStream_t s) {
   if (zero_x)
-    k_cheb<1, T><<<grid_for(D.n, 16), NT, 0, s>>>(D, xin, xout, k, 1, coef, S, err);
+    launch_pdl(k_cheb<1, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 1, coef, S, err);
   else if (L.pp.p[0] == 2)
-    k_cheb<2, T><<<grid_for(D.n, 16), NT, 0, s>>>(D, xin, xout, k, 0, coef, S, err);
+    launch_pdl(k_cheb<2, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 0, coef, S, err);
   else
-    k_cheb<1, T><<<grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s>>>(D, xin, xout, k, 0, coef, S, err);
+    launch_pdl(k_cheb<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, xin, xout, k, 0, coef, S, err);
 }
 
 template <typename T>
 void launch_resid(const HLevel& L, const LevDev<T>& D, const T* x, const GScal* S, int* err, cudaStream_t s) {
-  if (L.pp.p[0] == 2) k_resid<2, T><<<grid_for(D.n, 16), NT, 0, s>>>(D, x, S, err);
-  else k_resid<1, T><<<grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s>>>(D, x, S, err);
+  if (L.pp.p[0] == 2) launch_pdl(k_resid<2, T>, grid_for(D.n, 16), NT, 0, s, D, x, S, err);
+  else launch_pdl(k_resid<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, x, S, err);
 }
 
 // One V(NU, NU) cycle: out = M^{-1} in on level 0 (in, out: level-0 vectors not used by the cycle).
@@ -1337,19 +1588,19 @@ void enqueue_vcycle(Hier<T>* H, const T* in, T* out, cudaStream_t s) {
     launch_cheb<T>(H->L[l], D, D.xa, D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
     launch_resid<T>(H->L[l], D, D.xb, S, H->err, s);
     const HLevel& C = H->L[l + 1];
-    k_restrict<T><<<grid_for(C.n, 16), NT, 0, s>>>(D.g, C.g, C.X, D.r, (T*)C.b, S);
+    launch_pdl(k_restrict<T>, grid_for(C.n, 16), NT, 0, s, D.g, C.g, C.X, D.r, (T*)C.b, S);
   }
   if (tail < nl) {
-    k_vcycle_tail<T><<<1, TT, 0, s>>>(H->targs, S);
+    launch_pdl(k_vcycle_tail<T>, 1, TT, tail_smem<T>(H->targs), s, H->targs, S);
   } else {
     const HLevel& Lc = H->L[nl - 1];
-    k_coarse_apply<T><<<1, NT, 0, s>>>((int)Lc.n, H->cinv, (const T*)Lc.b, (T*)Lc.xb, S);
+    launch_pdl(k_coarse_apply<T>, 1, NT, 0, s, (int)Lc.n, H->cinv, (const T*)Lc.b, (T*)Lc.xb, S);
   }
   for (int l = std::min(tail, nl - 1) - 1; l >= 0; --l) {
     LevDev<T> D = levdev<T>(H->L[l]);
     if (l == 0) D.b = const_cast<T*>(in);
     const HLevel& C = H->L[l + 1];
-    k_prolong<T><<<grid_for(D.n, 16), NT, 0, s>>>(D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
+    launch_pdl(k_prolong<T>, grid_for(D.n, 16), NT, 0, s, D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
     // post-smoothing: xb -> xa (step 0), xa -> xb (step 1; level 0: -> out)
     launch_cheb<T>(H->L[l], D, D.xb, D.xa, 0, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
     launch_cheb<T>(H->L[l], D, D.xa, l == 0 ? out : D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
@@ -1367,11 +1618,11 @@ void enqueue_iters(Hier<T>* H, int count, cudaStream_t s) {
   CgVec<T> V = cgvec(H);
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>());
   for (int it = 0; it < count; ++it) {
-    if (L0.pp.p[0] == 2) k_cg_spmv<2, T><<<ge, NT, 0, s>>>(L0.g, L0.n, (const T*)L0.A, V);
-    else k_cg_spmv<1, T><<<gs, NT, staged_smem<T>(), s>>>(L0.g, L0.n, (const T*)L0.A, V);
-    k_cg_update<T><<<ge, NT, 0, s>>>(L0.n, V);
+    if (L0.pp.p[0] == 2) launch_pdl(k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    else launch_pdl(k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_pdl(k_cg_update<T>, ge, NT, 0, s, L0.n, V);
     enqueue_vcycle(H, H->r, (T*)H->L[0].xb, s);
-    k_cg_rz<T><<<ge, NT, 0, s>>>(L0.n, V, 0);
+    launch_pdl(k_cg_rz<T>, ge, NT, 0, s, L0.n, V, 0);
   }
 }
 
@@ -1478,15 +1729,15 @@ void enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
   BgVec<T> V = bgvec(H);
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>());
   for (int it = 0; it < count; ++it) {
-    k_bg_p<T><<<ge, NT, 0, s>>>(L0.n, V);
+    launch_pdl(k_bg_p<T>, ge, NT, 0, s, L0.n, V);
     enqueue_vcycle(H, H->p, H->ph, s);
-    if (L0.pp.p[0] == 2) k_bg_spmv<2, T, 0><<<ge, NT, 0, s>>>(L0.g, L0.n, (const T*)L0.A, V);
-    else k_bg_spmv<1, T, 0><<<gs, NT, staged_smem<T>(), s>>>(L0.g, L0.n, (const T*)L0.A, V);
-    k_bg_s<T><<<ge, NT, 0, s>>>(L0.n, V);
+    if (L0.pp.p[0] == 2) launch_pdl(k_bg_spmv<2, T, 0>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    else launch_pdl(k_bg_spmv<1, T, 0>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_pdl(k_bg_s<T>, ge, NT, 0, s, L0.n, V);
     enqueue_vcycle(H, H->sv, H->sh, s);
-    if (L0.pp.p[0] == 2) k_bg_spmv<2, T, 1><<<ge, NT, 0, s>>>(L0.g, L0.n, (const T*)L0.A, V);
-    else k_bg_spmv<1, T, 1><<<gs, NT, staged_smem<T>(), s>>>(L0.g, L0.n, (const T*)L0.A, V);
-    k_bg_update<T><<<ge, NT, 0, s>>>(L0.n, V);
+    if (L0.pp.p[0] == 2) launch_pdl(k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    else launch_pdl(k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_pdl(k_bg_update<T>, ge, NT, 0, s, L0.n, V);
   }
 }
 
