@@ -73,7 +73,6 @@ __device__ __forceinline__ double neg_int(double v) {
   return __hiloint2double(hi, __double2loint(v));
 }
 
-using mrgdev::row_ptr_of;
 using mrgdev::seg_store;
 
 struct FactArgs {
@@ -478,8 +477,9 @@ __global__ void __launch_bounds__(FT) k_fact_quad(const FactArgs A, const double
   const int64_t n0 = (int64_t)blockIdx.x * FT;
   const int64_t n = n0 + threadIdx.x;
   const int64_t nend = (n0 + FT < A.nrows) ? n0 + FT : A.nrows;
-  const int64_t seg0 = row_ptr_of(g, n0, A.nrows);
-  const int64_t seg1 = row_ptr_of(g, nend, A.nrows);
+  // row starts in closed form: no table loads ahead of the coefficients' (32 x 32 cells wait on nothing but latency)
+  const int64_t seg0 = mrgdev::row_ptr_at<1>(g, n0, A.nrows);
+  const int64_t seg1 = mrgdev::row_ptr_at<1>(g, nend, A.nrows);
   const int phase = DOJ ? (int)(((uintptr_t)(J + seg0) & 15) / sizeof(JT)) : 0;
   JT* sv = reinterpret_cast<JT*>(smem_raw) + phase;
   bool active = n < A.nrows, fixed = false;
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(FT) k_fact_quad(const FactArgs A, const double
     int lo, cx, cy;
     axis_range(ix, NX, 1, lo, cx);
     axis_range(iy, NY, 1, lo, cy);
-    myrow = g.P[1][iy] * g.T[0] + (int64_t)cy * g.P[0][ix];
+    myrow = (int64_t)max(3 * iy - 1, 0) * g.T[0] + (int64_t)cy * max(3 * ix - 1, 0);
     const int64_t loc = myrow - seg0;
     fixed = node_fixed(g, ix, iy, 0);
     const bool vx[3] = {ix > 0, true, ix < NX - 1};

@@ -16,17 +16,6 @@ __device__ __forceinline__ void decompose(const Grid& g, int64_t n, int& ix, int
   iz = (int)(t / ny);
 }
 
-__device__ __forceinline__ int64_t row_ptr_of(const Grid& g, int64_t n, int64_t nrows) {
-  if (n >= nrows) return g.T[0] * g.T[1] * g.T[2];
-  int ix, iy, iz;
-  decompose(g, n, ix, iy, iz);
-  int lo, cx, cy, cz;
-  axis_range(ix, g.nn[0], g.p, lo, cx);
-  axis_range(iy, g.nn[1], g.p, lo, cy);
-  if (g.dim == 3) axis_range(iz, g.nn[2], g.p, lo, cz); else cz = 1;
-  return g.P[2][iz] * g.T[1] * g.T[0] + (int64_t)cz * (g.P[1][iy] * g.T[0] + (int64_t)cy * g.P[0][ix]);
-}
-
 // Copy (or add) a contiguous segment from shared memory to global memory.  src[k] <-> dst[k]; both
 // pointers have the same address phase modulo 16 bytes, so the body uses aligned 16-byte accesses.
 template <typename T, bool ADD>

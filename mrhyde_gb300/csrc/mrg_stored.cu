@@ -351,8 +351,8 @@ __global__ void __launch_bounds__(ST_T, stored_minb<JT, DOJ, DOR>())
   int64_t seg0 = 0, seg1 = 0;
   JT* sv = nullptr;
   if (STAGE) {
-    seg0 = row_ptr_of(g, n0, A.nrows);
-    seg1 = row_ptr_of(g, nend, A.nrows);
+    seg0 = row_ptr_at<1>(g, n0, A.nrows);
+    seg1 = row_ptr_at<1>(g, nend, A.nrows);
     sv = reinterpret_cast<JT*>(smem_raw) + (int)(((uintptr_t)(J + seg0) & 15) / sizeof(JT));
   }
   const bool active = n < A.nrows;
