@@ -101,10 +101,30 @@ __device__ __forceinline__ int64_t diag_pos(const RowInfo& R, int ix, int iy, in
   return R.rp + ((int64_t)(iz - R.lz) * R.cy + (iy - R.ly)) * R.cx + (ix - R.lx);
 }
 
+// FP32 -> FP64 on the integer pipes (the conversion instruction issues at the FP64 rate): exact for zeros and normal
+// numbers; subnormal, infinite and NaN values (widen_special) take the instruction.
+__device__ __forceinline__ bool widen_special(double) { return false; }
+__device__ __forceinline__ bool widen_special(float v) {
+  const uint32_t t = __float_as_uint(v) & 0x7fffffffu;
+  return t - 1u < 0x7fffffu || t >= 0x7f800000u;
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+  const uint32_t b = __float_as_uint(v), t = b & 0x7fffffffu;
+  return __hiloint2double((int)((t ? (t >> 3) + 0x38000000u : 0u) | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double widen_any(double v) { return v; }
+__device__ __forceinline__ double widen_any(float v) {
+  double d;  // volatile: not to be hoisted out of the branch that rarely needs it
+  asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d) : "f"(v));
+  return d;
+}
+
 // Row product of a Q1 row (2 or 3 couplings along each axis; 1 along z in 2-D) without branches: the couplings past a
 // row's extents are loaded as zeros, so that a warp whose rows include boundary nodes (any tile of a short grid line)
 // runs the row once instead of once for its interior and once for its boundary lanes (y = J x on 80^3 cells: FP32 matrix
-// 92 -> 71 us, FP64 54 -> 46).  Terms in storage order.
+// 92 -> 71 us, FP64 54 -> 46).  FP32 values against an FP64 vector are widened on the integer pipes: 27 conversions a row
+// took as long as its 27 FMAs (71 -> 39 us).  Terms in storage order.
 template <typename AT, typename JT, typename XT>
 __device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* __restrict__ vals,
                                      const XT* __restrict__ x) {
@@ -129,10 +149,23 @@ __device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* 
   for (int z = 0; z < 3; ++z) {
     if (z == 0 || z < R.cz) {
       const JT* vr = vals + z * R.cy * R.cx;
+      JT v[9];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const bool in = (k % 3 < 2 || x2) && (k < 6 || y2);
-        acc = fma(in ? (AT)vr[(k / 3) * R.cx + k % 3] : AT(0), (AT)b[z * 9 + k], acc);
+      for (int k = 0; k < 9; ++k) v[k] = (k % 3 < 2 || x2) && (k < 6 || y2) ? vr[(k / 3) * R.cx + k % 3] : JT(0);
+      if constexpr (sizeof(AT) == 8 && sizeof(JT) == 4) {
+        bool odd = false;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) odd |= widen_special(v[k]);
+        if (odd) {
+#pragma unroll
+          for (int k = 0; k < 9; ++k) acc = fma(widen_any(v[k]), (AT)b[z * 9 + k], acc);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 9; ++k) acc = fma(widen(v[k]), (AT)b[z * 9 + k], acc);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) acc = fma((AT)v[k], (AT)b[z * 9 + k], acc);
       }
     }
   }
@@ -463,20 +496,6 @@ __device__ __forceinline__ bool warp_staged_rows(const Grid& g, int64_t nrows, c
     if (armed1) wbar_wait(mb1, ph1, limit);
   }
   return ok;
-}
-
-__device__ __forceinline__ double block_max(double v) {
-  __shared__ double sh[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s = fmax(s, sh[i]);
-  __syncthreads();
-  return s;
 }
 
 }  // namespace mrgdev

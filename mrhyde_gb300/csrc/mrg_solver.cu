@@ -41,6 +41,10 @@ constexpr int CHUNK = 16;        // PCG iterations per captured graph
 template <int P, typename JT>
 constexpr int spmv_per_sm() { return P == 1 ? (sizeof(JT) == 8 ? 4 : 7) : 16; }
 
+// and of k_spmv, whose 27 FP64 source values a row need the registers of 5 CTAs per SM
+template <typename JT>
+constexpr int apply_per_sm() { return sizeof(JT) == 8 ? 4 : 5; }
+
 // device scalars of one PCG instance
 struct PcgScal {
   double rho, rho_old, pq, alpha, beta, r0, rnorm, tol;
@@ -52,7 +56,7 @@ struct PcgScal {
 // y = J x (FP64 accumulation), Q1 rows through the per-warp staged loop.  err (may be null) is set to 1 if a
 // staging copy did not complete within its time bound.
 template <typename JT>
-__global__ void __launch_bounds__(ST, spmv_per_sm<1, JT>()) k_spmv(Grid g, int64_t nrows, const JT* __restrict__ J, const double* __restrict__ x,
+__global__ void __launch_bounds__(ST, apply_per_sm<JT>()) k_spmv(Grid g, int64_t nrows, const JT* __restrict__ J, const double* __restrict__ x,
                                              double* __restrict__ y, int* err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (ST / 32)];
@@ -76,21 +80,6 @@ struct Q2Kinds {
   int m[8][3];       // nodes of a kind per axis
   int64_t tile0[9];  // first step of QR rows of a kind
 };
-
-// zero, subnormal, infinite or NaN: widened by the conversion instruction
-__device__ __forceinline__ bool special(double) { return false; }
-__device__ __forceinline__ bool special(float v) { return (__float_as_uint(v) << 1) - 0x01000000u >= 0xfe000000u; }
-__device__ __forceinline__ double widen(double v) { return v; }
-__device__ __forceinline__ double widen(float v) {
-  const uint32_t b = __float_as_uint(v);
-  return __hiloint2double((int)((((b >> 3) & 0x0fffffffu) + 0x38000000u) | (b & 0x80000000u)), (int)(b << 29));
-}
-__device__ __forceinline__ double widen_any(double v) { return v; }
-__device__ __forceinline__ double widen_any(float v) {
-  double d;  // volatile: not to be hoisted out of the branch that rarely needs it
-  asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d) : "f"(v));
-  return d;
-}
 
 template <typename JT>
 __global__ void __launch_bounds__(ST) k_spmv_q2(Grid g, const __grid_constant__ Q2Kinds Q, const JT* __restrict__ J,
@@ -132,7 +121,7 @@ __global__ void __launch_bounds__(ST) k_spmv_q2(Grid g, const __grid_constant__ 
           const bool in = i + k * QL < len;
           a[k] = in ? __ldcs(v + i + k * QL) : JT(1);
           b[k] = in ? __ldg(xb + o[i + k * QL]) : 0.0;
-          odd |= special(a[k]);
+          odd |= widen_special(a[k]);
         }
         if (odd) {
 #pragma unroll
@@ -743,8 +732,8 @@ extern "C" int mrg_spmv(const mrg_problem* p, const void* J, int32_t fp32, const
   });
   MRG_CUDA(attr_err);
   if (p->g.p == 1) {
-    if (fp32) k_spmv<float><<<pcg_grid(p, spmv_per_sm<1, float>()), ST, spmv_smem<1, float>(), s>>>(p->g, p->ndof, (const float*)J, x, y, nullptr);
-    else k_spmv<double><<<pcg_grid(p, spmv_per_sm<1, double>()), ST, spmv_smem<1, double>(), s>>>(p->g, p->ndof, (const double*)J, x, y, nullptr);
+    if (fp32) k_spmv<float><<<pcg_grid(p, apply_per_sm<float>()), ST, spmv_smem<1, float>(), s>>>(p->g, p->ndof, (const float*)J, x, y, nullptr);
+    else k_spmv<double><<<pcg_grid(p, apply_per_sm<double>()), ST, spmv_smem<1, double>(), s>>>(p->g, p->ndof, (const double*)J, x, y, nullptr);
   } else {
     // rows of one kind per step, kinds one after the other (2-D: 4 kinds)
     Q2Kinds Q;
