@@ -94,10 +94,25 @@ struct LevDev {
 struct GScal {
   double rho, pq, alpha, beta, r0, rnorm, tol;
   double omega, rv;  // BiCGStab
+  float alpha32, beta32, omega32;  // FP32 copies, rounded once by the thread that sets the scalar
   int iter, maxiter, done, status;
   unsigned int counter;
   int err;
 };
+
+// a scalar in the vectors' precision
+template <typename T>
+__device__ __forceinline__ T alpha_of(const GScal* S) {
+  if constexpr (sizeof(T) == 4) return S->alpha32; else return S->alpha;
+}
+template <typename T>
+__device__ __forceinline__ T beta_of(const GScal* S) {
+  if constexpr (sizeof(T) == 4) return S->beta32; else return S->beta;
+}
+template <typename T>
+__device__ __forceinline__ T omega_of(const GScal* S) {
+  if constexpr (sizeof(T) == 4) return S->omega32; else return S->omega;
+}
 
 template <int P, typename T>
 __device__ __forceinline__ auto row_prod(const Grid& g, const RowInfo& R, const T* vals, const T* x) {
@@ -479,15 +494,18 @@ __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_diag(Grid g, const T
 // the hierarchy's precision (FP32 for the inner solve's hierarchy: FP64 arithmetic there cost the FP64
 // pipe's latency on every step for a preconditioner that is FP32 anyway).  The pivot is the first row
 // of largest magnitude, found by warp 0 with shuffles.
+// A thread owns one column (of MAXC + n) of two rows, so a pivot step is three barriers and no index arithmetic (with
+// 128 threads walking the elements a step took 2.2 us).
+constexpr int IT = 1024;
 template <typename T>
-__global__ void __launch_bounds__(NT) k_coarse_inv(Grid g, const T* __restrict__ A, T* __restrict__ inv,
+__global__ void __launch_bounds__(IT) k_coarse_inv(Grid g, const T* __restrict__ A, T* __restrict__ inv,
                                                    int* __restrict__ err) {
-  __shared__ T M[MAXC][2 * MAXC];
+  __shared__ T M[MAXC][2 * MAXC];  // [A | inverse]; the inverse begins at column MAXC
   __shared__ int piv;
   const int n = g.nn[0] * g.nn[1] * g.nn[2];
-  for (int k = threadIdx.x; k < MAXC * 2 * MAXC; k += NT) (&M[0][0])[k] = T(0);
+  for (int k = threadIdx.x; k < MAXC * 2 * MAXC; k += IT) (&M[0][0])[k] = T(0);
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += NT) {
+  for (int i = threadIdx.x; i < n; i += IT) {
     int ix, iy, iz;
     decompose(g, i, ix, iy, iz);
     const RowInfo R = row_info<1>(g, ix, iy, iz);
@@ -496,9 +514,11 @@ __global__ void __launch_bounds__(NT) k_coarse_inv(Grid g, const T* __restrict__
       for (int jy = R.ly; jy < R.ly + R.cy; ++jy)
         for (int jx = R.lx; jx < R.lx + R.cx; ++jx, ++e)
           M[i][jx + g.nn[0] * (jy + g.nn[1] * jz)] = A[R.rp + e];
-    M[i][n + i] = T(1);
+    M[i][MAXC + i] = T(1);
   }
   __syncthreads();
+  const int k = threadIdx.x & (2 * MAXC - 1), r0 = threadIdx.x / (2 * MAXC);
+  constexpr int RS = IT / (2 * MAXC);  // rows per pass
   for (int c = 0; c < n; ++c) {
     if (threadIdx.x < 32) {
       const int r = threadIdx.x;
@@ -519,36 +539,29 @@ __global__ void __launch_bounds__(NT) k_coarse_inv(Grid g, const T* __restrict__
       }
     }
     __syncthreads();
+    // rows c and pr change places; row c is scaled, column c leaves the other rows
     const int pr = piv;
-    if (pr != c)
-      for (int k = threadIdx.x; k < 2 * n; k += NT) {
-        const T t = M[c][k];
-        M[c][k] = M[pr][k];
-        M[pr][k] = t;
-      }
-    __syncthreads();
-    const T inv_p = T(1) / M[c][c];
-    __syncthreads();
-    for (int k = threadIdx.x; k < 2 * n; k += NT) M[c][k] *= inv_p;
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < n * 2 * n; idx += NT) {
-      const int r = idx / (2 * n), k = idx % (2 * n);
-      if (r != c && k != c) M[r][k] -= M[r][c] * M[c][k];
+    const T pk = M[pr][k] * (T(1) / M[pr][c]), qk = M[c][k], qc = M[c][c];
+    T out[MAXC / RS];
+#pragma unroll
+    for (int j = 0; j < MAXC / RS; ++j) {
+      const int r = r0 + j * RS;
+      const T f = r == pr ? qc : M[r][c], v = r == pr ? qk : M[r][k];
+      out[j] = r == c ? pk : (k == c ? T(0) : v - f * pk);
     }
     __syncthreads();
-    for (int r = threadIdx.x; r < n; r += NT)
-      if (r != c) M[r][c] = T(0);
+#pragma unroll
+    for (int j = 0; j < MAXC / RS; ++j) M[r0 + j * RS][k] = out[j];
     __syncthreads();
   }
-  for (int idx = threadIdx.x; idx < n * n; idx += NT) inv[idx] = M[idx / n][n + idx % n];
+  for (int idx = threadIdx.x; idx < n * n; idx += IT) inv[idx] = M[idx / n][MAXC + idx % n];
 }
 
-// ---- cycle kernels --------------------------------------------------------------------------------
-// Chebyshev step `k` (0..NU-1): d = rho_k rho_{k-1} d + (2 rho_k / delta) D^{-1}(b - A x)  (k = 0:
-// d = D^{-1}(b - A x) / theta); xout = x + d.  zero_x: x = 0 (no SpMV).
 // Chebyshev coefficients of every level and step (one thread per level, at setup): coef[(l NU + k) 3 + m]
 // = {1/theta, rho_k rho_{k-1}, 2 rho_k / delta} on [CHEB_LO L, L], L the level's Gershgorin bound.
-__global__ void k_cheb_coef(const unsigned int* __restrict__ lmax_bits, int nlev, double* __restrict__ coef) {
+// in the levels' precision: converted once here, not by every thread that uses them (a conversion takes the FP64 pipe).
+template <typename T>
+__global__ void k_cheb_coef(const unsigned int* __restrict__ lmax_bits, int nlev, T* __restrict__ coef) {
   const int l = threadIdx.x;
   if (l >= nlev) return;
   const double hi = (double)__uint_as_float(lmax_bits[l]), lo = CHEB_LO * hi;
@@ -560,7 +573,7 @@ __global__ void k_cheb_coef(const unsigned int* __restrict__ lmax_bits, int nlev
       rho_prev = rho;
       rho = rn;
     }
-    double* c = coef + ((size_t)l * NU + k) * 3;
+    T* c = coef + ((size_t)l * NU + k) * 3;
     c[0] = 1.0 / theta;
     c[1] = rho * rho_prev;
     c[2] = 2.0 * rho / delta;
@@ -595,12 +608,12 @@ __device__ __forceinline__ void resid_row(const LevDev<T>& L, int64_t n, T ax) {
 
 template <int P, typename T>
 __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cheb(LevDev<T> L, const T* __restrict__ xin, T* __restrict__ xout, int k,
-                                             int zero_x, const double* __restrict__ coef,
+                                             int zero_x, const T* __restrict__ coef,
                                              const GScal* __restrict__ S, int* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (NT / 32)];
   pdl_trigger();
-  const T c_first = (T)coef[3 * k], c_old = (T)coef[3 * k + 1], c_new = (T)coef[3 * k + 2];
+  const T c_first = coef[3 * k], c_old = coef[3 * k + 1], c_new = coef[3 * k + 2];
   auto fin = [&](int64_t n, T ax) { cheb_row<T>(L, n, ax, xin, xout, k, zero_x, c_first, c_old, c_new); };
   if (zero_x) {
     pdl_wait();
@@ -804,7 +817,7 @@ struct TailArgs {
   int nlev = 0;                  // levels in the tail; the last is the coarsest
   LevDev<T> L[MAXTAIL];
   Xfer X[MAXTAIL];               // X[j]: how tail level j was coarsened from level j - 1
-  const double* coef[MAXTAIL];   // Chebyshev coefficients of each level
+  const T* coef[MAXTAIL];        // Chebyshev coefficients of each level
   const T* cinv = nullptr;       // dense inverse of the coarsest operator
 };
 
@@ -857,8 +870,8 @@ __device__ __forceinline__ T tail_prod(const TailLev<T>& L, int n, const T* x) {
 
 template <typename T>
 __device__ __forceinline__ void tail_cheb(const TailLev<T>& L, const T* xin, T* xout, int k, int zero_x,
-                                          const double* __restrict__ coef) {
-  const T c_first = (T)coef[3 * k], c_old = (T)coef[3 * k + 1], c_new = (T)coef[3 * k + 2];
+                                          const T* __restrict__ coef) {
+  const T c_first = coef[3 * k], c_old = coef[3 * k + 1], c_new = coef[3 * k + 2];
   for (int n = threadIdx.x; n < (int)L.D.n; n += TT)
     cheb_row<T>(L.D, n, zero_x ? T(0) : tail_prod<T>(L, n, xin), xin, xout, k, zero_x, c_first, c_old, c_new);
   __syncthreads();
@@ -941,6 +954,25 @@ __global__ void __launch_bounds__(TT) k_vcycle_tail(const __grid_constant__ Tail
   for (int n = threadIdx.x; n < (int)A.L[0].n; n += TT) A.L[0].xb[n] = lev[0].D.xb[n];
 }
 
+// Vector updates with a dot product: RED_PER_SM CTAs per SM (each CTA's FP64 tree takes the FP64 pipe for 320 cycles, so
+// 16 per SM spent more time on the trees than on the vectors), four elements of a thread in flight.
+constexpr int RED_PER_SM = 4;
+template <typename L, typename F>
+__device__ __forceinline__ void each4(int64_t n, L&& load, F&& use) {
+  const int64_t st = (int64_t)gridDim.x * NT;
+  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += 4 * st) {
+    decltype(load(i)) v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * st < n) v[k] = load(i + k * st);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * st < n) use(i + k * st, v[k]);
+  }
+}
+template <typename T, int N>
+struct Vals { T v[N]; };
+
 // ---- CG kernels -----------------------------------------------------------------------------------
 template <typename T>
 struct CgVec {
@@ -973,6 +1005,7 @@ __global__ void __launch_bounds__(NT) k_cg_init(int64_t n, const double* __restr
       S->iter = 0;
       S->status = MRG_OK;
       S->beta = 0.0;
+      S->beta32 = 0.0f;
       S->rho = 0.0;
       S->done = (S->r0 == 0.0 || S->maxiter <= 0) ? 1 : 0;
       if (!isfinite(S->r0)) { S->done = 1; S->status = MRG_ENUMERIC; }
@@ -987,8 +1020,8 @@ __global__ void __launch_bounds__(NT) k_cg_rz(int64_t n, CgVec<T> V, int first) 
   pdl_wait();
   if (is_done(V.S)) return;
   T rz = T(0);
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
-    rz = fma(V.r[i], V.z[i], rz);
+  each4(n, [&](int64_t i) { return Vals<T, 2>{{V.r[i], V.z[i]}}; },
+        [&](int64_t, const Vals<T, 2>& e) { rz = fma(e.v[0], e.v[1], rz); });
   double m[1] = {block_sum((double)rz)};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
     double t[1];
@@ -996,6 +1029,7 @@ __global__ void __launch_bounds__(NT) k_cg_rz(int64_t n, CgVec<T> V, int first) 
     if (threadIdx.x == 0) {
       GScal* S = V.S;
       S->beta = first ? 0.0 : t[0] / S->rho;
+      S->beta32 = (float)S->beta;
       S->rho = t[0];
       if (!(t[0] > 0.0) || !isfinite(t[0])) { S->status = MRG_ENUMERIC; S->done = 1; }
     }
@@ -1022,7 +1056,7 @@ __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cg_spmv(Grid g, int6
       },
       [&] {
         pdl_wait();
-        beta = (T)V.S->beta;
+        beta = beta_of<T>(V.S);
         return go = !is_done(V.S);
       });
   if (!go) return;
@@ -1035,6 +1069,7 @@ __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cg_spmv(Grid g, int6
       GScal* S = V.S;
       S->pq = t[0];
       S->alpha = S->rho / t[0];
+      S->alpha32 = (float)S->alpha;
       if (!(t[0] > 0.0) || !isfinite(S->alpha)) { S->status = MRG_ENUMERIC; S->done = 1; }
       if (S->err) { S->status = MRG_ETIMEOUT; S->done = 1; }
     }
@@ -1047,14 +1082,15 @@ __global__ void __launch_bounds__(NT) k_cg_update(int64_t n, CgVec<T> V) {
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
-  const T alpha = (T)V.S->alpha;
+  const T alpha = alpha_of<T>(V.S);
   T rr = T(0);
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
-    V.x[i] += alpha * V.p[i];
-    const T r = V.r[i] - alpha * V.q[i];
-    V.r[i] = r;
-    rr = fma(r, r, rr);
-  }
+  each4(n, [&](int64_t i) { return Vals<T, 4>{{V.x[i], V.p[i], V.r[i], V.q[i]}}; },
+        [&](int64_t i, const Vals<T, 4>& e) {
+          V.x[i] = e.v[0] + alpha * e.v[1];
+          const T r = e.v[2] - alpha * e.v[3];
+          V.r[i] = r;
+          rr = fma(r, r, rr);
+        });
   double m[1] = {block_sum((double)rr)};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
     double t[1];
@@ -1108,6 +1144,8 @@ __global__ void __launch_bounds__(NT) k_bg_init(int64_t n, const double* __restr
       S->alpha = 1.0;
       S->omega = 1.0;
       S->beta = 0.0;
+      S->alpha32 = S->omega32 = 1.0f;
+      S->beta32 = 0.0f;
       S->iter = 0;
       S->status = MRG_OK;
       S->done = (S->r0 == 0.0 || S->maxiter <= 0) ? 1 : 0;
@@ -1122,7 +1160,7 @@ __global__ void __launch_bounds__(NT) k_bg_p(int64_t n, BgVec<T> V) {
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
-  const T beta = (T)V.S->beta, omega = (T)V.S->omega;
+  const T beta = beta_of<T>(V.S), omega = omega_of<T>(V.S);
   for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
     V.p[i] = V.r[i] + beta * (V.p[i] - omega * V.v[i]);
 }
@@ -1164,9 +1202,11 @@ __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_bg_spmv(Grid g, int6
       if (STEP == 0) {
         S->rv = t[0];
         S->alpha = S->rho / t[0];
+        S->alpha32 = (float)S->alpha;
         if (!(t[0] != 0.0) || !isfinite(S->alpha)) { S->status = MRG_ENUMERIC; S->done = 1; }
       } else {
         S->omega = (t[1] > 0.0) ? t[0] / t[1] : 0.0;
+        S->omega32 = (float)S->omega;
       }
       if (S->err) { S->status = MRG_ETIMEOUT; S->done = 1; }
     }
@@ -1179,7 +1219,7 @@ __global__ void __launch_bounds__(NT) k_bg_s(int64_t n, BgVec<T> V) {
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
-  const T alpha = (T)V.S->alpha;
+  const T alpha = alpha_of<T>(V.S);
   for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
     V.s[i] = V.r[i] - alpha * V.v[i];
 }
@@ -1190,15 +1230,16 @@ __global__ void __launch_bounds__(NT) k_bg_update(int64_t n, BgVec<T> V) {
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
-  const T alpha = (T)V.S->alpha, omega = (T)V.S->omega;
+  const T alpha = alpha_of<T>(V.S), omega = omega_of<T>(V.S);
   T rr = T(0), rhr = T(0);
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
-    V.x[i] += alpha * V.ph[i] + omega * V.sh[i];
-    const T r = V.s[i] - omega * V.t[i];
-    V.r[i] = r;
-    rr = fma(r, r, rr);
-    rhr = fma(V.rh[i], r, rhr);
-  }
+  each4(n, [&](int64_t i) { return Vals<T, 6>{{V.x[i], V.ph[i], V.sh[i], V.s[i], V.t[i], V.rh[i]}}; },
+        [&](int64_t i, const Vals<T, 6>& e) {
+          V.x[i] = e.v[0] + (alpha * e.v[1] + omega * e.v[2]);
+          const T r = e.v[3] - omega * e.v[4];
+          V.r[i] = r;
+          rr = fma(r, r, rr);
+          rhr = fma(e.v[5], r, rhr);
+        });
   double m[2] = {block_sum((double)rr), block_sum((double)rhr)};
   if (last_block<2>(V.parts, m, &V.S->counter)) {
     double t[2];
@@ -1208,6 +1249,7 @@ __global__ void __launch_bounds__(NT) k_bg_update(int64_t n, BgVec<T> V) {
       S->rnorm = sqrt(t[0]);
       S->iter += 1;
       S->beta = (t[1] / S->rho) * (S->alpha / S->omega);
+      S->beta32 = (float)S->beta;
       S->rho = t[1];
       if (!(S->rnorm / S->r0 > S->tol) || S->iter >= S->maxiter) S->done = 1;
       if (!isfinite(S->rnorm)) { S->done = 1; S->status = MRG_ENUMERIC; }
@@ -1247,7 +1289,7 @@ struct Hier {
   T* cinv = nullptr;
   T* mid[2] = {nullptr, nullptr};  // intermediate operators of the Galerkin sweeps
   unsigned int* lmax = nullptr;   // [nlev] float bits
-  double* coef = nullptr;         // [nlev][NU][3] Chebyshev coefficients
+  T* coef = nullptr;              // [nlev][NU][3] Chebyshev coefficients
   int* err = nullptr;             // setup / cycle error word
   T *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr;  // CG vectors (level-0 size)
   double* parts = nullptr;
@@ -1417,7 +1459,7 @@ int build_hier(const mrg_problem* p, Hier<T>*& out, cudaStream_t s) {
   const size_t nparts = (size_t)2 * grid_for(n0, 16) + 64;
   if (cudaMallocAsync(&H->cinv, (size_t)nc * nc * sizeof(T), s) != cudaSuccess ||
       cudaMallocAsync(&H->lmax, MAXLEV * sizeof(unsigned int), s) != cudaSuccess ||
-      cudaMallocAsync(&H->coef, (size_t)MAXLEV * NU * 3 * sizeof(double), s) != cudaSuccess ||
+      cudaMallocAsync(&H->coef, (size_t)MAXLEV * NU * 3 * sizeof(T), s) != cudaSuccess ||
       cudaMallocAsync(&H->err, sizeof(int), s) != cudaSuccess ||
       cudaMallocAsync(&H->x, n0 * sizeof(T), s) != cudaSuccess || cudaMallocAsync(&H->r, n0 * sizeof(T), s) != cudaSuccess ||
       cudaMallocAsync(&H->p, n0 * sizeof(T), s) != cudaSuccess || cudaMallocAsync(&H->q, n0 * sizeof(T), s) != cudaSuccess ||
@@ -1498,7 +1540,7 @@ int setup_level0(Hier<T>* H, const T* J, cudaStream_t s) {
   MRG_CUDA(cudaMemsetAsync(H->lmax, 0, sizeof(unsigned int), s));
   if (L.pp.p[0] == 2) k_diag<2, T><<<grid_for(L.n, 16), NT, 0, s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax, H->err);
   else k_diag<1, T><<<grid_for(L.n, staged_per_sm<T>()), NT, staged_smem<T>(), s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax, H->err);
-  k_cheb_coef<<<1, 32, 0, s>>>(H->lmax, (int)H->L.size(), H->coef);
+  k_cheb_coef<T><<<1, 32, 0, s>>>(H->lmax, (int)H->L.size(), H->coef);
   MRG_CUDA(cudaGetLastError());
   return MRG_OK;
 }
@@ -1549,8 +1591,8 @@ int setup_values(Hier<T>* H, const T* J, cudaStream_t s) {
     else k_diag<1, T><<<grid_for(L.n, staged_per_sm<T>()), NT, staged_smem<T>(), s>>>(L.g, (const T*)L.A, (T*)L.minv, H->lmax + l, H->err);
     MRG_CUDA(cudaGetLastError());
   }
-  k_coarse_inv<T><<<1, NT, 0, s>>>(H->L.back().g, (const T*)H->L.back().A, H->cinv, H->err);
-  k_cheb_coef<<<1, 32, 0, s>>>(H->lmax, nl, H->coef);
+  k_coarse_inv<T><<<1, IT, 0, s>>>(H->L.back().g, (const T*)H->L.back().A, H->cinv, H->err);
+  k_cheb_coef<T><<<1, 32, 0, s>>>(H->lmax, nl, H->coef);
   MRG_CUDA(cudaGetLastError());
   return MRG_OK;
 }
@@ -1559,7 +1601,7 @@ int setup_values(Hier<T>* H, const T* J, cudaStream_t s) {
 // CTAs per SM), a Q2 level 0 the direct row loop.
 template <typename T>
 void launch_cheb(const HLevel& L, const LevDev<T>& D, const T* xin, T* xout, int k, int zero_x,
-                 const double* coef, const GScal* S, int* err, cudaStream_t s) {
+                 const T* coef, const GScal* S, int* err, cudaStream_t s) {
   if (zero_x)
     launch_pdl(k_cheb<1, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 1, coef, S, err);
   else if (L.pp.p[0] == 2)
@@ -1616,13 +1658,13 @@ template <typename T>
 void enqueue_iters(Hier<T>* H, int count, cudaStream_t s) {
   const HLevel& L0 = H->L[0];
   CgVec<T> V = cgvec(H);
-  const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>());
+  const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
     if (L0.pp.p[0] == 2) launch_pdl(k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_pdl(k_cg_update<T>, ge, NT, 0, s, L0.n, V);
+    launch_pdl(k_cg_update<T>, gr, NT, 0, s, L0.n, V);
     enqueue_vcycle(H, H->r, (T*)H->L[0].xb, s);
-    launch_pdl(k_cg_rz<T>, ge, NT, 0, s, L0.n, V, 0);
+    launch_pdl(k_cg_rz<T>, gr, NT, 0, s, L0.n, V, 0);
   }
 }
 
@@ -1688,10 +1730,10 @@ int gmg_cg(mrg_problem* p, Hier<T>* H, const T* J, const double* b, double* x, d
   MRG_CUDA(cudaMemcpyAsync(H->S, &init, sizeof(GScal), cudaMemcpyHostToDevice, s));
   const int64_t n = p->ndof;
   CgVec<T> V = cgvec(H);
-  k_cg_init<T><<<grid_for(n, 16), NT, 0, s>>>(n, b, V);
+  k_cg_init<T><<<grid_for(n, RED_PER_SM), NT, 0, s>>>(n, b, V);
   MRG_CUDA(cudaGetLastError());
   enqueue_vcycle(H, H->r, (T*)H->L[0].xb, s);
-  k_cg_rz<T><<<grid_for(n, 16), NT, 0, s>>>(n, V, 1);
+  k_cg_rz<T><<<grid_for(n, RED_PER_SM), NT, 0, s>>>(n, V, 1);
   MRG_CUDA(cudaGetLastError());
   // captured chunk of iterations (re-captured when the Jacobian pointer or the stream changes)
   if (!H->graph || H->graph_A != (const void*)J || H->graph_stream != s || H->graph_tail != H->tail) {
@@ -1727,7 +1769,7 @@ template <typename T>
 void enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
   const HLevel& L0 = H->L[0];
   BgVec<T> V = bgvec(H);
-  const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>());
+  const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
     launch_pdl(k_bg_p<T>, ge, NT, 0, s, L0.n, V);
     enqueue_vcycle(H, H->p, H->ph, s);
@@ -1737,7 +1779,7 @@ void enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
     enqueue_vcycle(H, H->sv, H->sh, s);
     if (L0.pp.p[0] == 2) launch_pdl(k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_pdl(k_bg_update<T>, ge, NT, 0, s, L0.n, V);
+    launch_pdl(k_bg_update<T>, gr, NT, 0, s, L0.n, V);
   }
 }
 
@@ -1757,7 +1799,7 @@ int gmg_bicgstab(mrg_problem* p, Hier<T>* H, const T* J, const double* b, double
   init.tol = rtol;
   init.maxiter = maxiter;
   MRG_CUDA(cudaMemcpyAsync(H->S, &init, sizeof(GScal), cudaMemcpyHostToDevice, s));
-  k_bg_init<T><<<grid_for(n, 16), NT, 0, s>>>(n, b, bgvec(H));
+  k_bg_init<T><<<grid_for(n, RED_PER_SM), NT, 0, s>>>(n, b, bgvec(H));
   MRG_CUDA(cudaGetLastError());
   if (!H->bgraph || H->bgraph_A != (const void*)J || H->bgraph_stream != s || H->bgraph_tail != H->tail) {
     if (H->bgraph) {

@@ -459,20 +459,38 @@ __global__ void k_f32_to_f64(int64_t n, const float* __restrict__ a, double* __r
   if (i < n) b[i] = (double)a[i];
 }
 
-// inf-norm with the last-block pattern; result in s->rnorm
+// inf-norm with the last-block pattern; result in s->rnorm.  Magnitudes are compared as integers (non-negative doubles
+// order like their bits), off the FP64 pipe; anything not finite counts as infinity.
+__device__ __forceinline__ unsigned long long block_umax(unsigned long long v) {
+  __shared__ unsigned long long sh[ST / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_down_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  for (int k = 0; k < ST / 32; ++k) v = max(v, sh[k]);
+  __syncthreads();
+  return v;  // valid in thread 0
+}
+
 __global__ void __launch_bounds__(ST) k_norminf(int64_t n, const double* __restrict__ v, double* parts, PcgScal* s) {
-  double a = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * ST + threadIdx.x; i < n; i += (int64_t)gridDim.x * ST) {
-    const double x = v[i];
-    a = isfinite(x) ? fmax(a, fabs(x)) : INFINITY;
+  constexpr unsigned long long INF = 0x7ff0000000000000ull;
+  unsigned long long a = 0;
+  const int64_t st = (int64_t)gridDim.x * ST;
+  for (int64_t i = (int64_t)blockIdx.x * ST + threadIdx.x; i < n; i += 4 * st) {
+    unsigned long long b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) b[k] = i + k * st < n ? (unsigned long long)__double_as_longlong(v[i + k * st]) & ~(1ull << 63) : 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a = max(a, min(b[k], INF));
   }
-  double m[1] = {block_max(a)};
+  double m[1] = {__longlong_as_double((long long)block_umax(a))};
   if (last_block<1>(parts, m, &s->counter)) {
-    double mx = 0.0;
-    for (unsigned int k = threadIdx.x; k < gridDim.x; k += blockDim.x) mx = fmax(mx, __ldcg(parts + k));
-    mx = block_max(mx);
+    unsigned long long mx = 0;
+    for (unsigned int k = threadIdx.x; k < gridDim.x; k += blockDim.x)
+      mx = max(mx, (unsigned long long)__double_as_longlong(__ldcg(parts + k)));
+    mx = block_umax(mx);
     if (threadIdx.x == 0) {
-      s->rnorm = mx;
+      s->rnorm = __longlong_as_double((long long)mx);
       s->counter = 0u;
     }
   }
@@ -815,7 +833,7 @@ int mrg_residual_from(mrg_problem* p, const double* b, double* res, cudaStream_t
 
 static int norm_inf(mrg_problem* p, const double* v, double* out, cudaStream_t s) {
   SolverWork* w = p->work;
-  k_norminf<<<pcg_grid(p), ST, 0, s>>>(p->ndof, v, w->parts, w->s);
+  k_norminf<<<pcg_grid(p, 4), ST, 0, s>>>(p->ndof, v, w->parts, w->s);
   MRG_CUDA(cudaGetLastError());
   MRG_CUDA(cudaMemcpyAsync(w->h_s, w->s, sizeof(PcgScal), cudaMemcpyDeviceToHost, s));
   MRG_CUDA(cudaStreamSynchronize(s));
