@@ -10,15 +10,15 @@
 //     Z_a[j] = pairs over (q_b, q_c) of  w_a ( sigma(j) sum_{q_a} c + 2 d_a sum_{q_a} u L[q_a][j] ),
 // where b, c are the other two axes, sigma(0) = -1, sigma(1) = +1 and t the unordered pair of the two nodes' ends
 // along an axis (00, 01 or 11: the weight of a Gauss point is L[q][l] L[q][j]).  So 54 numbers a cell give its 64
-// entries: about 250 operations, and 2 additions an entry when the rows gather them (the row-by-row contraction
-// took about 200 operations a row and cell, 1600 a cell).  The residual shares c and d_a with it: about 150
+// entries: about 230 operations, and 2 additions an entry when the rows gather them (the row-by-row contraction
+// took about 200 operations a row and cell, 1600 a cell).  The residual shares c and d_a with it: about 130
 // operations a cell against 360 with one lane per Gauss point.
 //
 //   k_nl1_cell   one thread a cell: the 54 numbers and the 8 residual entries to a workspace in blocks of 32 cells,
 //                so that lanes write and read consecutive addresses and every offset is an immediate
 //   k_nl1_row    one thread a CSR row: 24 loads from each of its 8 cells, the CTA's rows staged in shared memory
 //                and written once; the residual adds the cells' entries in the same order
-// Measured, FP64 Jacobian and residual on 95^3 cells: 3506 -> 1046 us (cells 704, rows 340, FP64 pipe 84 and 83 %
+// Measured, FP64 Jacobian and residual on 95^3 cells: 3506 -> 1001 us (cells 660, rows 340, FP64 pipe 84 and 83 %
 // active; the row-by-row contraction took 2712 and eight coloured residual launches 780); FP32 Jacobian alone on
 // 96^3 cells 865 -> about 40 us.
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
@@ -39,7 +39,6 @@ constexpr int CB = 32;    // cells per workspace block
 // products and sums that must not be contracted differently from one instance to the next (the residual of the
 // separate and of the fused call has the same bits)
 __device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double addr(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float addr(float a, float b) { return __fadd_rn(a, b); }
 
@@ -57,6 +56,8 @@ struct Nl1Args {
   double w[3];       // |J| w_q / h_a^2
   double load;       // f * int(phi_l) over one cell
   float betaf, wf[3];
+  double m[3], m02;  // L L at the Gauss point near node 0 for the pairs 00, 01, 11; m[0] + m[2]
+  float m32[3][2];   // m in FP32: value and what it lacks
   int64_t ncell;
 };
 
@@ -78,12 +79,22 @@ __device__ __forceinline__ void lerp2(T beta, T a, T b, T& p0, T& p1, T& d) {
   p1 = fma(-beta, d, b);
 }
 
-// sums of two Gauss points' values against L[q][l] L[q][j]: (00, 01, 11)
-template <typename T>
-__device__ __forceinline__ void pair3(T aa, T bb, T ab, T v0, T v1, T& t00, T& t01, T& t11) {
-  t00 = fma(bb, v1, aa * v0);
-  t11 = fma(aa, v1, bb * v0);
-  t01 = ab * (v0 + v1);
+// Sums of two Gauss points' values against L[q][l] L[q][j]: (00, 01, 11).  FP64: t00 and t11 add up to
+// (aa + bb)(v0 + v1), 5 operations.  FP32 is not short of operations: the table's values come in two parts, because
+// their rounding would shift every entry the same way (FP32 matrix's error at 16 x 16 x 16 cells 8.8e-8 with values
+// rounded once, 5.7e-8 so; 5.8e-8 for the row-by-row contraction).
+__device__ __forceinline__ void pair3(const Nl1Args& A, double v0, double v1, double& t00, double& t01, double& t11) {
+  const double s = v0 + v1;
+  t00 = fma(A.m[2], v1, A.m[0] * v0);
+  t11 = fma(A.m02, s, -t00);
+  t01 = A.m[1] * s;
+}
+__device__ __forceinline__ void pair3(const Nl1Args& A, float v0, float v1, float& t00, float& t01, float& t11) {
+  const float (&m)[3][2] = A.m32;
+  const float s = v0 + v1;
+  t00 = fmaf(m[2][0], v1, fmaf(m[0][0], v0, fmaf(m[0][1], v0, m[2][1] * v1)));
+  t11 = fmaf(m[0][0], v1, fmaf(m[2][0], v0, fmaf(m[0][1], v1, m[2][1] * v0)));
+  t01 = fmaf(m[1][0], s, m[1][1] * s);
 }
 
 // JT: type of the 54 numbers.  CT: type of the fields at the Gauss points (double whenever the residual is
@@ -144,7 +155,7 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
 #pragma unroll
     for (int q = 0; q < 2; ++q)
 #pragma unroll
-      for (int p = 0; p < 2; ++p) C[q][p] = mulr(w_of<CT>(A, a), addr(at(cw, a, q, p, 0), at(cw, a, q, p, 1)));
+      for (int p = 0; p < 2; ++p) C[q][p] = addr(at(cw, a, q, p, 0), at(cw, a, q, p, 1));
     if constexpr (DOR) {
       CT m[2][2], unused;
 #pragma unroll
@@ -156,8 +167,8 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
       for (int p = 0; p < 2; ++p) lerp2(be, m[0][p], m[1][p], R[a][0][p], R[a][1][p], unused);
     }
     if constexpr (DOJ) {
-      const JT bj = beta_of<JT>(A), al = JT(1) - bj, aa = al * al, bb = bj * bj, ab = al * bj;
-      const JT w2 = JT(2) * w_of<JT>(A, a);
+      const JT bj = beta_of<JT>(A);
+      const JT w = w_of<JT>(A, a), w2 = JT(2) * w;
       JT* out = zbuf + ((cl >> 5) * NZ_ + a * 18) * CB + (cl & 31);
       JT Z[2][2][2];  // [j][q][p]
 #pragma unroll
@@ -166,7 +177,7 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
         for (int p = 0; p < 2; ++p) {
           JT U[2], unused;
           lerp2(bj, as<JT>(at(u, a, q, p, 0)), as<JT>(at(u, a, q, p, 1)), U[0], U[1], unused);
-          const JT D = w2 * as<JT>(gd[a][q][p]), Cj = as<JT>(C[q][p]);
+          const JT D = w2 * as<JT>(gd[a][q][p]), Cj = w * as<JT>(C[q][p]);
           Z[0][q][p] = fma(D, U[0], -Cj);
           Z[1][q][p] = fma(D, U[1], Cj);
         }
@@ -174,11 +185,11 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
       for (int j = 0; j < 2; ++j) {
         JT P[2][3];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) pair3(aa, bb, ab, Z[j][q][0], Z[j][q][1], P[q][0], P[q][1], P[q][2]);
+        for (int q = 0; q < 2; ++q) pair3(A, Z[j][q][0], Z[j][q][1], P[q][0], P[q][1], P[q][2]);
 #pragma unroll
         for (int t = 0; t < 3; ++t) {
           JT o[3];
-          pair3(aa, bb, ab, P[0][t], P[1][t], o[0], o[1], o[2]);
+          pair3(A, P[0][t], P[1][t], o[0], o[1], o[2]);
 #pragma unroll
           for (int s = 0; s < 3; ++s) out[(j * 9 + s * 3 + t) * CB] = o[s];  // [j][second other axis][first]
         }
@@ -189,19 +200,19 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
 #pragma unroll
     for (int l = 0; l < 8; ++l) {
       const int x = l & 1, y = (l >> 1) & 1, z = l >> 2;
-      CT v = addr(x ? R[0][z][y] : -R[0][z][y], (CT)(-A.load));
-      v = addr(v, y ? R[1][z][x] : -R[1][z][x]);
-      v = addr(v, z ? R[2][y][x] : -R[2][y][x]);
+      CT v = fma(w_of<CT>(A, 0), x ? R[0][z][y] : -R[0][z][y], (CT)(-A.load));
+      v = fma(w_of<CT>(A, 1), y ? R[1][z][x] : -R[1][z][x], v);
+      v = fma(w_of<CT>(A, 2), z ? R[2][y][x] : -R[2][y][x], v);
       rbuf[((cl >> 5) * 8 + l) * CB + (cl & 31)] = v;
     }
   }
 }
 
-// 4 CTAs per SM (128 registers): 27 accumulators and a cell's 24 loads in flight
+// FP64: 4 CTAs per SM (128 registers): 27 accumulators and a cell's 24 loads in flight; FP32 needs 80 registers
 template <typename JT, bool DOJ, bool DOR, bool OVW>
-__global__ void __launch_bounds__(RT, DOJ ? 4 : 8) k_nl1_row(const Grid g, int64_t nrows, const JT* __restrict__ zbuf,
-                                                   const double* __restrict__ rbuf, double* __restrict__ r,
-                                                   JT* __restrict__ J) {
+__global__ void __launch_bounds__(RT, !DOJ ? 8 : (sizeof(JT) == 4 ? 6 : 4))
+    k_nl1_row(const Grid g, int64_t nrows, const JT* __restrict__ zbuf, const double* __restrict__ rbuf,
+              double* __restrict__ r, JT* __restrict__ J) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int64_t s_seg[2];
   const int64_t n0 = (int64_t)blockIdx.x * RT, n = n0 + threadIdx.x;
@@ -252,14 +263,16 @@ __global__ void __launch_bounds__(RT, DOJ ? 4 : 8) k_nl1_row(const Grid g, int64
             for (int j = 0; j < 8; ++j) {
               const int jj[3] = {j & 1, (j >> 1) & 1, j >> 2};
               const int t[3] = {l[0] + jj[0], l[1] + jj[1], l[2] + jj[2]};  // 00, 01, 11
-              JT v = acc[(jj[2] - l[2] + 1) * 9 + (jj[1] - l[1] + 1) * 3 + (jj[0] - l[0] + 1)];
+              // the cell's entry first, then the row's sum: fewer roundings at the size of the sum
+              JT v = JT(0);
 #pragma unroll
               for (int a = 0; a < 3; ++a) {
                 const int p = a == 0 ? 1 : 0, q = a == 2 ? 1 : 2;
                 const JT x = __ldg(z + (a * 18 + jj[a] * 9 + t[q] * 3 + t[p]) * CB);
-                v += l[a] ? x : -x;
+                if (a == 0) v = l[a] ? x : -x;
+                else v += l[a] ? x : -x;
               }
-              acc[(jj[2] - l[2] + 1) * 9 + (jj[1] - l[1] + 1) * 3 + (jj[0] - l[0] + 1)] = v;
+              acc[(jj[2] - l[2] + 1) * 9 + (jj[1] - l[1] + 1) * 3 + (jj[0] - l[0] + 1)] += v;
             }
           }
         }
@@ -334,6 +347,13 @@ int mrg_nl1_setup(mrg_problem* p) {
   mrg_lagrange_1d(1, p->gx1[0], l, dl);
   A.beta = l[1];
   A.betaf = (float)A.beta;
+  const double m[3] = {l[0] * l[0], l[0] * l[1], l[1] * l[1]};
+  A.m02 = m[0] + m[2];
+  for (int k = 0; k < 3; ++k) {
+    A.m[k] = m[k];
+    A.m32[k][0] = (float)m[k];
+    A.m32[k][1] = (float)(m[k] - (double)A.m32[k][0]);
+  }
   double vol = 1.0;
   for (int a = 0; a < 3; ++a) vol *= 0.5 * p->h[a] * p->gw1[0];  // both weights are 1
   for (int a = 0; a < 3; ++a) {
