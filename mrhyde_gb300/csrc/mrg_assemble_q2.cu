@@ -19,11 +19,14 @@
 // k_q2_row: one thread a CSR row, rows of one kind per warp (mrg_q2_rows.cuh): its 1, 2, 4 or 8 cells' entries, lane by
 // lane consecutive, added in a fixed order and written once.
 //
-// Measured on 64^3 cells, FP32 Jacobian and FP64 residual: 1818 -> 1156 us (the tensor-core path with eight coloured
-// residual launches before), and the FP32 matrix's error fell from 2.4e-7 to 2.1e-8.
+// Measured on 64^3 cells, FP32 Jacobian and FP64 residual: 1818 -> 1025 us (the tensor-core path with eight coloured
+// residual launches before), and the FP32 matrix's error fell from 2.4e-7 to 2.1e-8.  Cells take 730 us of it (FP64 pipe),
+// rows 390 (memory); the rows of a slab run beside the next slab's cells.
 // MRG_ASM_TENSOR_CORES takes the FP32 element matrices from the tcgen05 kernel instead (mrg_tc_q2.cu), for which
 // k_q2_cell writes the coefficients as TF32 operand images.
+#include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <vector>
 
 #include "mrg_fixmul.cuh"
@@ -36,6 +39,11 @@ constexpr int LINES = 9;     // warps: lines of one direction, pairs (l_x, j_x)
 constexpr int ET = LINES * 32;
 constexpr int ENT = 729;     // entries of an element matrix
 constexpr int QRT = 128;     // threads per CTA of the row kernel
+// Slabs of cell layers (64^3 cells, FP32 Jacobian and FP64 residual: one slab 1151 us, 4 1074, 8 1050, 12 1059, 16 1086).
+// A slab of 16384 cells is 512 CTAs, a little more than the GPU holds at 3 CTAs per SM: below that the launches' ends cost
+// more than the overlap gives.
+constexpr int MAXSLAB = 8;
+constexpr int64_t SLAB_CELLS = 16384;
 
 // Tables in the arithmetic type.  Gauss points -s, 0, s; node values l(q, a), derivatives d(q, a).
 template <typename T>
@@ -51,6 +59,7 @@ struct Tab {
 struct Q2Args {
   Grid g;
   int64_t ncell;
+  int64_t blk0;        // first block of 32 cells of the launch
   Tab<double> t64;
   Tab<float> t32;
 };
@@ -129,8 +138,9 @@ constexpr int cell_smem() {
 // Jacobian alone).  out: element matrices [cell / 32][27 l + j][32], or the operand image
 // [cell / 128][hi, lo][k / 4][128][4].  rbuf: residual entries [cell / 32][27][32].
 template <typename JT, typename CT, int OUT, bool DOR>
-__global__ void __launch_bounds__(ET, 2) k_q2_cell(const __grid_constant__ Q2Args A, const double* __restrict__ u,
-                                                   JT* __restrict__ out, double* __restrict__ rbuf) {
+__global__ void __launch_bounds__(ET, sizeof(JT) == 4 ? 3 : 2)  // FP32: 1106 -> 1074 us against 2 CTAs per SM
+    k_q2_cell(const __grid_constant__ Q2Args A, const double* __restrict__ u, JT* __restrict__ out,
+              double* __restrict__ rbuf) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CT* const a0 = reinterpret_cast<CT*>(smem_raw) + (threadIdx.x & 31);  // three fields of 27 values a cell
   CT* const b0 = a0 + 3 * 27 * CB;
@@ -139,7 +149,7 @@ __global__ void __launch_bounds__(ET, 2) k_q2_cell(const __grid_constant__ Q2Arg
   const Tab<CT>& t = tab<CT>(A);
   const Grid& g = A.g;
   const int line = threadIdx.x >> 5, lane = threadIdx.x & 31, i = line % 3, k = line / 3;
-  const int64_t blk = blockIdx.x, slot = blk * CB + lane;
+  const int64_t blk = A.blk0 + blockIdx.x, slot = blk * CB + lane;
   const int64_t c = slot < A.ncell ? slot : A.ncell - 1;  // the last block's spare lanes repeat a cell
   {
     const unsigned c32 = (unsigned)c, r = c32 / (unsigned)g.nc[0];
@@ -325,13 +335,13 @@ __global__ void __launch_bounds__(ET, 2) k_q2_cell(const __grid_constant__ Q2Arg
 
 // One row of kind (PX, PY, PZ)
 template <int PX, int PY, int PZ, typename JT, bool DOJ, bool DOR, bool OVW>
-__device__ __forceinline__ void q2_row(const Grid& g, const int (&m)[3], int64_t at, const JT* __restrict__ ebuf,
+__device__ __forceinline__ void q2_row(const Grid& g, const mrgq2::Kinds& K, int kind, int64_t at, const JT* __restrict__ ebuf,
                                        const double* __restrict__ rbuf, double* __restrict__ r, JT* __restrict__ J,
                                        JT* stage) {
   using mrgq2::cells;
   using mrgq2::half;
   using R = mrgq2::Row<true, PX, PY, PZ>;
-  const R row(g, m, at);
+  const R row(g, K, kind, at);
   // local index along an axis: a mid-side node is 1; a vertex is 2 in the cell on its left, 0 in the one on its right
   auto local = [](int P, int s) { return P ? 1 : (s ? 0 : 2); };
   const JT* e[cells(PZ)][cells(PY)][cells(PX)];
@@ -384,7 +394,7 @@ __device__ __forceinline__ void q2_row(const Grid& g, const int (&m)[3], int64_t
     for (int ez = 0; ez < R::LZ; ++ez) {
       if (fast) plane(ez, std::true_type{});
       else plane(ez, std::false_type{});
-      row.template store_plane<OVW>(J, stage, ez);
+      row.template store_plane<OVW, false>(J, stage, ez);
     }
     if (!OVW) row.fix_diagonal(J);
   }
@@ -399,7 +409,7 @@ __global__ void __launch_bounds__(QRT) k_q2_row(const Grid g, const __grid_const
   const int kind = mrgq2::kind_of(K, blockIdx.x);
   const int64_t at = ((int64_t)blockIdx.x - K.block0[kind]) * QRT + threadIdx.x;
   mrgq2::with_kind<true>(kind, [&](auto px, auto py, auto pz) {
-    q2_row<decltype(px)::value, decltype(py)::value, decltype(pz)::value, JT, DOJ, DOR, OVW>(g, K.m[kind], at, ebuf, rbuf,
+    q2_row<decltype(px)::value, decltype(py)::value, decltype(pz)::value, JT, DOJ, DOR, OVW>(g, K, kind, at, ebuf, rbuf,
                                                                                              r, J, stage);
   });
 }
@@ -411,7 +421,11 @@ __global__ void __launch_bounds__(QRT) k_q2_row(const Grid g, const __grid_const
 // ------------------------------------------------------------------------------------------------
 struct Q2Data {
   Q2Args A;
-  mrgq2::Kinds kinds;
+  std::vector<int> slab;            // cell layers at which the slabs begin, and the last one's end
+  std::vector<mrgq2::Kinds> kinds;  // the slabs' rows; kinds.back(): all rows
+  std::mutex side_use;              // held by the call that launches on the side stream
+  cudaStream_t side = nullptr;      // rows of a slab while the next slab's cells are worked on (several slabs only)
+  std::vector<cudaEvent_t> ev;      // a slab's cells are done; the last: all rows are
   int* d_err = nullptr;          // tensor-core kernel status (bounded waits), sticky until reported
   int* h_err = nullptr;          // pinned mirror, refreshed asynchronously after every tensor-core launch
   cudaEvent_t err_ev = nullptr;  // recorded after the refresh
@@ -426,7 +440,7 @@ int mrg_q2_setup(mrg_problem* p) {
   p->q2 = Q;
   Q->A.g = p->g;
   Q->A.ncell = p->ncell;
-  Q->kinds = mrgq2::make_kinds(p->g, QRT);
+  Q->A.blk0 = 0;
   Tab<double>& t = Q->A.t64;
   double l[3][3], d[3][3], detJ = 1.0;
   for (int q = 0; q < 3; ++q) mrg_lagrange_1d(2, p->gx1[q], l[q], d[q]);
@@ -456,6 +470,20 @@ int mrg_q2_setup(mrg_problem* p) {
   const double* src = reinterpret_cast<const double*>(&t);
   float* dst = reinterpret_cast<float*>(&Q->A.t32);
   for (size_t k = 0; k < sizeof(t) / sizeof(double); ++k) dst[k] = (float)src[k];
+  const int nz = p->g.nc[2];
+  const int64_t layer = (int64_t)p->g.nc[0] * p->g.nc[1];
+  const int slabs = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(nz, MAXSLAB), layer * nz / SLAB_CELLS));
+  for (int k = 0; k <= slabs; ++k) Q->slab.push_back((int)((int64_t)nz * k / slabs));
+  if (slabs > 1) {
+    for (int k = 0; k < slabs; ++k) Q->kinds.push_back(mrgq2::make_kinds(p->g, QRT, Q->slab[k], Q->slab[k + 1]));
+    MRG_CUDA(cudaStreamCreateWithFlags(&Q->side, cudaStreamNonBlocking));
+    for (int k = 0; k <= slabs; ++k) {
+      cudaEvent_t e = nullptr;
+      MRG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      Q->ev.push_back(e);
+    }
+  }
+  Q->kinds.push_back(mrgq2::make_kinds(p->g, QRT));
   cudaStream_t s = p->stream;
   MRG_CUDA(cudaMallocAsync(&Q->d_err, sizeof(int), s));
   MRG_CUDA(cudaMemsetAsync(Q->d_err, 0, sizeof(int), s));
@@ -465,6 +493,8 @@ int mrg_q2_setup(mrg_problem* p) {
 void mrg_q2_free(mrg_problem* p) {
   Q2Data* Q = q2data(p);
   if (!Q) return;
+  if (Q->side) cudaStreamDestroy(Q->side);
+  for (cudaEvent_t e : Q->ev) cudaEventDestroy(e);
   cudaFreeAsync(Q->d_err, p->stream);
   if (Q->err_ev) cudaEventDestroy(Q->err_ev);
   mrg_pinned_release(Q->h_err);
@@ -474,25 +504,63 @@ void mrg_q2_free(mrg_problem* p) {
 }
 
 template <typename JT, typename CT, int OUT, bool DOR>
-static cudaError_t launch_cell(const Q2Data& Q, const double* u, JT* out, double* rbuf, cudaStream_t s) {
+static cudaError_t launch_cell(const Q2Data& Q, const double* u, JT* out, double* rbuf, cudaStream_t s, int64_t b0 = 0,
+                               int64_t b1 = -1) {
   constexpr int smem = cell_smem<JT, CT, OUT>();
   auto kern = k_q2_cell<JT, CT, OUT, DOR>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  kern<<<(unsigned)((Q.A.ncell + CB - 1) / CB), ET, smem, s>>>(Q.A, u, out, rbuf);
+  Q2Args A = Q.A;
+  A.blk0 = b0;
+  if (b1 < 0) b1 = (Q.A.ncell + CB - 1) / CB;
+  if (b1 > b0) kern<<<(unsigned)(b1 - b0), ET, smem, s>>>(A, u, out, rbuf);
   return cudaGetLastError();
 }
 
 template <typename JT>
-static cudaError_t launch_rows(const mrg_problem* p, const Q2Data& Q, const JT* ebuf, const double* rbuf, double* r, JT* J,
+static cudaError_t launch_rows(const mrg_problem* p, const mrgq2::Kinds& K, const JT* ebuf, const double* rbuf, double* r, JT* J,
                                bool doJ, bool doR, bool ovw, cudaStream_t s) {
-  const unsigned grid = (unsigned)Q.kinds.block0[8];
-#define MRG_Q2_ROW(DJ, DR, OV) k_q2_row<JT, DJ, DR, OV><<<grid, QRT, 0, s>>>(p->g, Q.kinds, ebuf, rbuf, r, J)
+  const unsigned grid = (unsigned)K.block0[8];
+#define MRG_Q2_ROW(DJ, DR, OV) k_q2_row<JT, DJ, DR, OV><<<grid, QRT, 0, s>>>(p->g, K, ebuf, rbuf, r, J)
   if (doJ && doR) { if (ovw) MRG_Q2_ROW(true, true, true); else MRG_Q2_ROW(true, true, false); }
   else if (doJ) { if (ovw) MRG_Q2_ROW(true, false, true); else MRG_Q2_ROW(true, false, false); }
   else { if (ovw) MRG_Q2_ROW(false, true, true); else MRG_Q2_ROW(false, true, false); }
 #undef MRG_Q2_ROW
   return cudaGetLastError();
+}
+
+// Cells, then rows; in slabs of cell layers on a large mesh, the rows of a slab on the side stream while the next slab's
+// cells are worked on: the cells are bound by arithmetic and the rows by memory, so the two overlap.  The bits are the
+// same either way.  The side stream and its events serve one call at a time: a call that finds them taken by another
+// thread's, or that is being captured (its graph would hold on to the stream until the capture ends), goes without.
+template <typename JT, typename CT, bool DOR>
+static cudaError_t launch_slabs(const mrg_problem* p, Q2Data& Q, const double* u, JT* eb, double* rb, double* r, JT* J,
+                                bool ovw, cudaStream_t s) {
+  const int slabs = (int)Q.slab.size() - 1;
+  std::unique_lock<std::mutex> use(Q.side_use, std::defer_lock);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (slabs > 1) {
+    const cudaError_t e = cudaStreamIsCapturing(s, &cap);
+    if (e != cudaSuccess) return e;
+  }
+  if (slabs == 1 || cap != cudaStreamCaptureStatusNone || !use.try_lock()) {
+    const cudaError_t e = launch_cell<JT, CT, OUT_MATRIX, DOR>(Q, u, eb, rb, s);
+    return e != cudaSuccess ? e : launch_rows<JT>(p, Q.kinds.back(), eb, rb, r, J, true, DOR, ovw, s);
+  }
+  const int64_t layer = (int64_t)p->g.nc[0] * p->g.nc[1];
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < slabs && e == cudaSuccess; ++k) {
+    // blocks of 32 cells up to the slab's last cell (they may reach into the next layer)
+    const int64_t b0 = (layer * Q.slab[k] + CB - 1) / CB, b1 = (layer * Q.slab[k + 1] + CB - 1) / CB;
+    e = launch_cell<JT, CT, OUT_MATRIX, DOR>(Q, u, eb, rb, s, k ? b0 : 0, b1);
+    if (e == cudaSuccess) e = cudaEventRecord(Q.ev[k], s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(Q.side, Q.ev[k], 0);
+    if (e == cudaSuccess) e = launch_rows<JT>(p, Q.kinds[k], eb, rb, r, J, true, DOR, ovw, Q.side);
+  }
+  // the caller's stream goes on when the rows are written, whatever was launched
+  cudaError_t j = cudaEventRecord(Q.ev[slabs], Q.side);
+  if (j == cudaSuccess) j = cudaStreamWaitEvent(s, Q.ev[slabs], 0);
+  return e != cudaSuccess ? e : j;
 }
 
 // FP32 Jacobian with the element matrices from the tensor cores; rbuf is null when no residual is asked for.
@@ -525,7 +593,7 @@ static int launch_tensor_cores(mrg_problem* p, const double* u, double* r, float
   float* w = mrg_q2tc_w_image(Q.tc);
   if (rbuf) {
     MRG_CUDA((launch_cell<float, double, OUT_TF32, true>(Q, u, w, rbuf, s)));
-    MRG_CUDA(launch_rows<float>(p, Q, nullptr, rbuf, r, nullptr, false, true, ovw, s));
+    MRG_CUDA(launch_rows<float>(p, Q.kinds.back(), nullptr, rbuf, r, nullptr, false, true, ovw, s));
   } else {
     MRG_CUDA((launch_cell<float, float, OUT_TF32, false>(Q, u, w, nullptr, s)));
   }
@@ -540,7 +608,7 @@ static int launch_tensor_cores(mrg_problem* p, const double* u, double* r, float
 }
 
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s) {
-  const Q2Data& Q = *q2data(p);
+  Q2Data& Q = *q2data(p);
   const bool doJ = flags & MRG_ASM_JAC, doR = flags & MRG_ASM_RES, ovw = flags & MRG_ASM_OVERWRITE;
   const bool fp32 = (flags & MRG_ASM_J_FP32) && doJ;
   const bool tc = fp32 && (flags & MRG_ASM_TENSOR_CORES) && !(flags & MRG_ASM_CUDA_CORES);
@@ -554,17 +622,15 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
   cudaError_t e = cudaSuccess;
   if (tc) {
     st = launch_tensor_cores(p, u, r, (float*)J, rbuf, ovw, s);
+  } else if (!doJ) {
+    e = launch_cell<double, double, OUT_NONE, true>(Q, u, nullptr, rbuf, s);
+    if (e == cudaSuccess) e = launch_rows<double>(p, Q.kinds.back(), nullptr, rbuf, r, nullptr, false, true, ovw, s);
   } else if (fp32) {
-    float* eb = reinterpret_cast<float*>(ws);
-    e = doR ? launch_cell<float, double, OUT_MATRIX, true>(Q, u, eb, rbuf, s)
-            : launch_cell<float, float, OUT_MATRIX, false>(Q, u, eb, nullptr, s);
-    if (e == cudaSuccess) e = launch_rows<float>(p, Q, eb, rbuf, r, (float*)J, true, doR, ovw, s);
+    e = doR ? launch_slabs<float, double, true>(p, Q, u, reinterpret_cast<float*>(ws), rbuf, r, (float*)J, ovw, s)
+            : launch_slabs<float, float, false>(p, Q, u, reinterpret_cast<float*>(ws), nullptr, r, (float*)J, ovw, s);
   } else {
-    double* eb = reinterpret_cast<double*>(ws);
-    if (!doJ) e = launch_cell<double, double, OUT_NONE, true>(Q, u, nullptr, rbuf, s);
-    else if (doR) e = launch_cell<double, double, OUT_MATRIX, true>(Q, u, eb, rbuf, s);
-    else e = launch_cell<double, double, OUT_MATRIX, false>(Q, u, eb, nullptr, s);
-    if (e == cudaSuccess) e = launch_rows<double>(p, Q, eb, rbuf, r, (double*)J, doJ, doR, ovw, s);
+    e = doR ? launch_slabs<double, double, true>(p, Q, u, reinterpret_cast<double*>(ws), rbuf, r, (double*)J, ovw, s)
+            : launch_slabs<double, double, false>(p, Q, u, reinterpret_cast<double*>(ws), nullptr, r, (double*)J, ovw, s);
   }
   if (ws) {
     const cudaError_t ef = mrg_ws_give(ws, s);

@@ -88,7 +88,7 @@ __device__ __forceinline__ void box_rows(const BoxArgs& A, int kind, int64_t at,
   constexpr bool K64 = !F32 || DOR;            // FP64 sums of kappa
   using R = mrgq2::Row<D3, PX, PY, PZ>;
   const Grid& g = A.g;
-  const R row(g, A.kinds.m[kind], at);
+  const R row(g, A.kinds, kind, at);
   const int NX = g.nn[0], NY = g.nn[1];
   // kappa of the row's cells, 0 outside the mesh
   double k[cells(PZ)][cells(PY)][cells(PX)];
@@ -147,7 +147,7 @@ __device__ __forceinline__ void box_rows(const BoxArgs& A, int kind, int64_t at,
         }
         if (DOR) acc = fma(-K[kc], t, acc);
       }
-    if (DOJ) row.template store_plane<OVW>(J, stage, ez);
+    if (DOJ) row.template store_plane<OVW, true>(J, stage, ez);
   }
   if (DOJ && !OVW) row.fix_diagonal(J);
   if (DOR && row.on) {

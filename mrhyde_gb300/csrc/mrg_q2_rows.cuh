@@ -20,17 +20,23 @@ __host__ __device__ constexpr int cells(int P) { return P ? 1 : 2; }
 
 struct Kinds {
   int m[8][3];        // nodes of a kind per axis
+  int z0;             // first cell layer
   int64_t block0[9];  // first block of a kind; block0[8]: all blocks
 };
 
-inline Kinds make_kinds(const Grid& g, int rows_per_block) {
+// the rows of all nodes, or of the node planes 2 c0 .. 2 c1 - 1 (with the last plane when c1 is the last layer)
+inline Kinds make_kinds(const Grid& g, int rows_per_block, int c0 = 0, int c1 = -1) {
   Kinds K;
   int64_t blocks = 0;
+  if (c1 < 0) c1 = g.nc[2];
+  K.z0 = c0;
   for (int t = 0; t < 8; ++t) {
     int64_t rows = 1;
     for (int k = 0; k < 3; ++k) {
       const int mid = (t >> k) & 1;
-      K.m[t][k] = k < g.dim ? (mid ? g.nc[k] : g.nc[k] + 1) : (mid ? 0 : 1);  // 2-D: kinds 0 to 3 only
+      const int n = k == 2 ? c1 - c0 : g.nc[k];
+      const bool end = k != 2 || c1 == g.nc[2];
+      K.m[t][k] = k < g.dim ? (mid || !end ? n : n + 1) : (mid ? 0 : 1);  // 2-D: kinds 0 to 3 only
       rows *= K.m[t][k];
     }
     K.block0[t] = blocks;
@@ -57,7 +63,8 @@ struct Row {
   bool xl, xr, yl, yr, zl, zr;          // cells on either side of a vertex
   int64_t n, rp;
 
-  __device__ __forceinline__ Row(const Grid& g, const int (&m)[3], int64_t at) {
+  __device__ __forceinline__ Row(const Grid& g, const Kinds& K, int kind, int64_t at) {
+    const int (&m)[3] = K.m[kind];
     on = at < (int64_t)m[0] * m[1] * m[2];
     ix = PX;
     iy = PY;
@@ -66,7 +73,7 @@ struct Row {
       const unsigned a = (unsigned)at, t = a / (unsigned)m[0];
       ix += 2 * (int)(a - t * (unsigned)m[0]);
       iy += 2 * (int)(t % (unsigned)m[1]);
-      if (D3) iz += 2 * (int)(t / (unsigned)m[1]);
+      if (D3) iz += 2 * (K.z0 + (int)(t / (unsigned)m[1]));
     }
     xl = PX || ix > 0;
     xr = PX || ix < g.nn[0] - 1;
@@ -101,8 +108,9 @@ struct Row {
     else if (has_z(D3 ? ez - half(PZ) : 0) && has_y(ey - half(PY)) && has_x(ex - half(PX)))
       stage[lane * PLANE + (ey - (yl ? 0 : half(PY))) * cx + (ex - (xl ? 0 : half(PX)))] = v;
   }
-  // write (or add) the staged plane ez of the warp's rows
-  template <bool OVW, typename JT>
+  // write (or add) the staged plane ez of the warp's rows; STREAM: past the caches (thermal rows, 33 x 30 x 27 cells:
+  // 80.0 -> 78.3 us; rows gathered from element matrices, 64^3 cells: 1050 -> 1061, so not there)
+  template <bool OVW, bool STREAM, typename JT>
   __device__ __forceinline__ void store_plane(JT* __restrict__ J, const JT* stage, int ez) const {
     const int lane = threadIdx.x & 31;
     __syncwarp();
@@ -112,7 +120,9 @@ struct Row {
       for (int i = 0; i < N; ++i) {
         const int e = i * 32 + lane, row = e / N;
         const int64_t d = __shfl_sync(0xffffffffu, base, row) + (e - row * N);
-        if (OVW) __stcs(J + d, stage[e]); else J[d] += stage[e];
+        if constexpr (!OVW) J[d] += stage[e];
+        else if constexpr (STREAM) __stcs(J + d, stage[e]);
+        else J[d] = stage[e];
       }
     } else {
       const int64_t base = rp + (int64_t)(ez - (zl ? 0 : half(PZ))) * cx * cy;
