@@ -10,15 +10,15 @@
 //     res_i  = sum_q k sum_ab M_ab d_a phi_i d_b u - load_i
 //     J_ij   = sum_q k sum_ab M_ab d_a phi_i d_b phi_j  +  sum_q 2 u (sum_ab M_ab d_b u d_a phi_i) phi_j .
 // FP64 arithmetic bounds these passes (1/64 of the FP32 rate), so the sums over the tensor-product points are taken
-// axis by axis, one thread a cell: about 1050 operations for a Q1 hexahedron and 1500 for a Q2 quadrilateral,
-// where forward differentiation row by row took about 7000 and 8500.
+// axis by axis, one thread a cell (small meshes of quadrilaterals: one thread a cell and l_x): about 1000 operations for
+// a Q1 hexahedron and 1500 for a Q2 quadrilateral, where forward differentiation row by row took about 7000 and 8500.
 //
 //   k_metric      (setup) one thread a Gauss point
 //   k_cell_hex1,  one thread a cell: the cell matrix and residual to a workspace in blocks of 32 cells, so that
 //   k_cell_quad   lanes write and read consecutive addresses
 //   k_gather      one thread a CSR row: adds its cells' entries in a fixed order; rows staged in shared memory and
 //                 written once
-// Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 259 us (cells 231, FP64
+// Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 249 us (cells 222, FP64
 // pipe 87 % active, rows 27).
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
 // on several streams and may be captured.
@@ -200,9 +200,10 @@ __device__ __forceinline__ void lerp2(double be, double a, double b, double& p0,
   p1 = fma(-be, d, b);
 }
 __device__ __forceinline__ void pair3(double aa, double bb, double ab, double v0, double v1, double* t) {
+  const double s = v0 + v1;
   t[0] = fma(bb, v1, aa * v0);
-  t[2] = fma(aa, v1, bb * v0);
-  t[1] = ab * (v0 + v1);
+  t[2] = fma(aa + bb, s, -t[0]);  // the two add up to (aa + bb)(v0 + v1): 5 operations for 6 (259 -> 249 us)
+  t[1] = ab * s;
 }
 
 template <typename JT, bool DOJ, bool DOR>
@@ -373,7 +374,8 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
 // Sums over q_x for each pair of x indices, then over q_y: an entry's terms have four kinds of factor along y
 // (value or derivative of either function), so with a, b the combinations for the row's function
 //     E[l][j] = sum_qy a(qy) L_{jy}(qy) + b(qy) D_{jy}(qy).
-template <int P, typename JT, bool DOJ, bool DOR>
+// SPLIT (small meshes): a thread forms the rows of one l_x, blockIdx.y.
+template <int P, typename JT, bool DOJ, bool DOR, bool SPLIT>
 __global__ void __launch_bounds__(CT_) k_cell_quad(const __grid_constant__ GenArgs A, const double* __restrict__ u_,
                                                    JT* __restrict__ ebuf, double* __restrict__ rbuf) {
   constexpr int N1 = P + 1, NL = N1 * N1;
@@ -432,7 +434,7 @@ __global__ void __launch_bounds__(CT_) k_cell_quad(const __grid_constant__ GenAr
         v1[qy][qx] = u2 * h1;
       }
   }
-  if constexpr (DOR) {
+  if (DOR && (!SPLIT || blockIdx.y == 0)) {
     double* out = rbuf + (c >> 5) * (NL * CB) + (c & 31);
 #pragma unroll
     for (int lx = 0; lx < N1; ++lx) {
@@ -459,7 +461,8 @@ __global__ void __launch_bounds__(CT_) k_cell_quad(const __grid_constant__ GenAr
   }
   if constexpr (DOJ) {
     JT* out = ebuf + (c >> 5) * (NL * NL * CB) + (c & 31);
-    for (int lx = 0; lx < N1; ++lx)  // not unrolled: the code of one (l_x, j_x) is already some hundred operations
+    // not unrolled: the code of one (l_x, j_x) is already some hundred operations
+    for (int lx = SPLIT ? (int)blockIdx.y : 0; lx < (SPLIT ? (int)blockIdx.y + 1 : N1); ++lx)
 #pragma unroll 1
       for (int jx = 0; jx < N1; ++jx) {
         double LL[N1], DD[N1], LD[N1], DL[N1];  // factors along y: row's function first
@@ -608,16 +611,25 @@ int setup_t(mrg_problem* p, General* Q, MetricArgs& M, cudaStream_t s) {
   return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "cell geometry launch");
 }
 
-template <int DIM, int P, typename JT>
+// FP64 work issues at 64 cycles a warp instruction on each of an SM's four schedulers, so a mesh with fewer cells than
+// 32 lanes on all of them (19456 on 152 SMs) leaves schedulers idle and takes a cell's whole chain.  A quadrilateral's
+// matrix is then split by its rows over P + 1 threads, each forming the fields again, as long as that gives a scheduler
+// two warps at most (Q2).  FP64 Jacobian and residual, whole -> split: Q2, 60 x 60 cells 86 -> 57 us, 100 x 100 94 -> 85,
+// 120 x 120 95 -> 104; Q1, 60 x 60 36 -> 31, 120 x 120 37.7 -> 36.8, 139 x 139 38 -> 42.  A hexahedron's rows share too
+// much: one axis's and one mixed part a thread with the parts added by the gather took 62 us against 50 on 20 x 22 x 19.
+constexpr int64_t FILL = 32 * 4 * 2 / 3 - 1;  // cells per SM
+
+template <int DIM, int P, typename JT, bool SPLIT>
 cudaError_t launch_t(const mrg_problem* p, const General& Q, const double* u, double* r, JT* J, JT* ebuf, double* rbuf,
                      bool doJ, bool doR, bool ovw, cudaStream_t s) {
-  const unsigned gc = nblk(p->ncell, CT_), gr = nblk(p->ndof, RT);
-#define MRG_GEN_CELL(DJ, DR)                                                        \
-  if constexpr (DIM == 3) k_cell_hex1<JT, DJ, DR><<<gc, CT_, 0, s>>>(Q.A, u, ebuf, rbuf); \
-  else k_cell_quad<P, JT, DJ, DR><<<gc, CT_, 0, s>>>(Q.A, u, ebuf, rbuf)
-  if (doJ && doR) { MRG_GEN_CELL(true, true); }
-  else if (doJ) { MRG_GEN_CELL(true, false); }
-  else { MRG_GEN_CELL(false, true); }
+  const dim3 gc(nblk(p->ncell, CT_), SPLIT && doJ ? P + 1 : 1);
+  const unsigned gr = nblk(p->ndof, RT);
+#define MRG_GEN_CELL(DJ, DR, SP)                                                              \
+  if constexpr (DIM == 3) k_cell_hex1<JT, DJ, DR><<<gc, CT_, 0, s>>>(Q.A, u, ebuf, rbuf);     \
+  else k_cell_quad<P, JT, DJ, DR, SP><<<gc, CT_, 0, s>>>(Q.A, u, ebuf, rbuf)
+  if (doJ && doR) { MRG_GEN_CELL(true, true, SPLIT); }
+  else if (doJ) { MRG_GEN_CELL(true, false, SPLIT); }
+  else { MRG_GEN_CELL(false, true, false); }
 #undef MRG_GEN_CELL
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -693,9 +705,13 @@ int mrg_launch_general(mrg_problem* p, const double* u, double* r, void* J, uint
   auto go = [&](auto* Jt) {
     using JT = std::remove_pointer_t<decltype(Jt)>;
     JT* eb = reinterpret_cast<JT*>(ws);
-    if (p->g.dim == 3) return launch_t<3, 1, JT>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
-    if (p->g.p == 1) return launch_t<2, 1, JT>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
-    return launch_t<2, 2, JT>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
+    if (p->g.dim == 3) return launch_t<3, 1, JT, false>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
+    const bool split = p->ncell < FILL * mrg_device_sms();
+    if (p->g.p == 1)
+      return split ? launch_t<2, 1, JT, true>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s)
+                   : launch_t<2, 1, JT, false>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
+    return split ? launch_t<2, 2, JT, true>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s)
+                 : launch_t<2, 2, JT, false>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
   };
   if (fp32) e = go(reinterpret_cast<float*>(J));
   else e = go(reinterpret_cast<double*>(J));
