@@ -10,15 +10,15 @@
 //     Z_a[j] = pairs over (q_b, q_c) of  w_a ( sigma(j) sum_{q_a} c + 2 d_a sum_{q_a} u L[q_a][j] ),
 // where b, c are the other two axes, sigma(0) = -1, sigma(1) = +1 and t the unordered pair of the two nodes' ends
 // along an axis (00, 01 or 11: the weight of a Gauss point is L[q][l] L[q][j]).  So 54 numbers a cell give its 64
-// entries: about 230 operations, and 2 additions an entry when the rows gather them (the row-by-row contraction
-// took about 200 operations a row and cell, 1600 a cell).  The residual shares c and d_a with it: about 130
-// operations a cell against 360 with one lane per Gauss point.
+// entries: about 225 operations, and 2 additions an entry when the rows gather them (the row-by-row contraction
+// took about 200 operations a row and cell, 1600 a cell).  The residual shares c and d_a with it: about 80
+// operations a cell besides the 54 of the fields, against 360 with one lane per Gauss point.
 //
 //   k_nl1_cell   one thread a cell: the 54 numbers and the 8 residual entries to a workspace in blocks of 32 cells,
 //                so that lanes write and read consecutive addresses and every offset is an immediate
 //   k_nl1_row    one thread a CSR row: 24 loads from each of its 8 cells, the CTA's rows staged in shared memory
 //                and written once; the residual adds the cells' entries in the same order
-// Measured, FP64 Jacobian and residual on 95^3 cells: 3506 -> 1001 us (cells 660, rows 340, FP64 pipe 84 and 83 %
+// Measured, FP64 Jacobian and residual on 95^3 cells: 3506 -> 950 us (cells 610, rows 340, FP64 pipe 84 and 83 %
 // active; the row-by-row contraction took 2712 and eight coloured residual launches 780); FP32 Jacobian alone on
 // 96^3 cells 865 -> about 40 us.
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
@@ -53,9 +53,10 @@ __device__ __forceinline__ T as(float v) { return (T)v; }
 struct Nl1Args {
   Grid g;
   double beta;       // L[0][1] = L[1][0]: the far node's weight at a Gauss point
+  double alpha, slope;  // 1 - beta, beta (1 - 2 beta)
   double w[3];       // |J| w_q / h_a^2
   double load;       // f * int(phi_l) over one cell
-  float betaf, wf[3];
+  float betaf, slopef, wf[3];
   double m[3], m02;  // L L at the Gauss point near node 0 for the pairs 00, 01, 11; m[0] + m[2]
   float m32[3][2];   // m in FP32: value and what it lacks
   int64_t ncell;
@@ -64,6 +65,10 @@ struct Nl1Args {
 template <typename T>
 __device__ __forceinline__ T beta_of(const Nl1Args& A) {
   if constexpr (sizeof(T) == 4) return A.betaf; else return A.beta;
+}
+template <typename T>
+__device__ __forceinline__ T slope_of(const Nl1Args& A) {
+  if constexpr (sizeof(T) == 4) return A.slopef; else return A.slope;
 }
 template <typename T>
 __device__ __forceinline__ T w_of(const Nl1Args& A, int a) {
@@ -137,11 +142,12 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
 #pragma unroll
     for (int x = 0; x < 2; ++x) lerp2(be, dy[0][x], dy[1][x], gd[1][0][x], gd[1][1][x], unused);  // [qz][qx]
   }
-  CT cw[2][2][2];
+  // 2 + u^2 at the points of even x + y + z: each pair of neighbours has one of them
+  CT c2[2][2][2];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const CT q = u[k >> 2][(k >> 1) & 1][k & 1];
-    cw[k >> 2][(k >> 1) & 1][k & 1] = fma(q, q, CT(1));
+    const int x = k & 1, y = (k >> 1) & 1, z = k >> 2;
+    if ((x + y + z) % 2 == 0) c2[z][y][x] = fma(u[z][y][x], u[z][y][x], CT(2));
   }
   // element (first other axis p, second other axis q, own axis a) of a [z][y][x] array
   auto at = [](const auto& v, int a, int q, int p, int o) {
@@ -155,19 +161,24 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
 #pragma unroll
     for (int q = 0; q < 2; ++q)
 #pragma unroll
-      for (int p = 0; p < 2; ++p) C[q][p] = addr(at(cw, a, q, p, 0), at(cw, a, q, p, 1));
+      for (int p = 0; p < 2; ++p) {  // sum of 1 + u^2 along the axis
+        const int even = (p + q) & 1;
+        const CT v = at(u, a, q, p, 1 - even);
+        C[q][p] = fma(v, v, at(c2, a, q, p, even));
+      }
     if constexpr (DOR) {
       CT m[2][2], unused;
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const CT f0 = mulr(C[q][0], gd[a][q][0]), f1 = mulr(C[q][1], gd[a][q][1]);
-        lerp2(be, f0, f1, m[q][0], m[q][1], unused);
+        const CT f0 = mulr(C[q][0], gd[a][q][0]), d = fma(C[q][1], gd[a][q][1], -f0);
+        m[q][0] = fma(be, d, f0);
+        m[q][1] = fma((CT)A.alpha, d, f0);
       }
 #pragma unroll
       for (int p = 0; p < 2; ++p) lerp2(be, m[0][p], m[1][p], R[a][0][p], R[a][1][p], unused);
     }
     if constexpr (DOJ) {
-      const JT bj = beta_of<JT>(A);
+      const JT kj = slope_of<JT>(A);
       const JT w = w_of<JT>(A, a), w2 = JT(2) * w;
       JT* out = zbuf + ((cl >> 5) * NZ_ + a * 18) * CB + (cl & 31);
       JT Z[2][2][2];  // [j][q][p]
@@ -175,11 +186,10 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
       for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-          JT U[2], unused;
-          lerp2(bj, as<JT>(at(u, a, q, p, 0)), as<JT>(at(u, a, q, p, 1)), U[0], U[1], unused);
-          const JT D = w2 * as<JT>(gd[a][q][p]), Cj = w * as<JT>(C[q][p]);
-          Z[0][q][p] = fma(D, U[0], -Cj);
-          Z[1][q][p] = fma(D, U[1], Cj);
+          // u's sums along the axis against the end nodes: u is linear there, u(1) - u(0) = (1 - 2 beta) gd
+          const JT gj = as<JT>(gd[a][q][p]), D = w2 * gj, Cj = w * as<JT>(C[q][p]);
+          Z[0][q][p] = fma(D, fma(kj, gj, as<JT>(at(u, a, q, p, 0))), -Cj);
+          Z[1][q][p] = fma(D, fma(-kj, gj, as<JT>(at(u, a, q, p, 1))), Cj);
         }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
@@ -346,7 +356,10 @@ int mrg_nl1_setup(mrg_problem* p) {
   double l[2], dl[2];
   mrg_lagrange_1d(1, p->gx1[0], l, dl);
   A.beta = l[1];
+  A.alpha = l[0];
+  A.slope = l[1] * (l[0] - l[1]);
   A.betaf = (float)A.beta;
+  A.slopef = (float)A.slope;
   const double m[3] = {l[0] * l[0], l[0] * l[1], l[1] * l[1]};
   A.m02 = m[0] + m[2];
   for (int k = 0; k < 3; ++k) {
