@@ -6,9 +6,10 @@
 // every shared-memory access 32 consecutive values.
 //   Fields and residual (FP64).  u and its scaled reference gradient at the Gauss points by sum factorisation, a warp
 //   for each of the 9 lines of a direction; the middle Gauss point is the middle node, and the outer two are mirror
-//   images, so a line takes 10 operations for values and derivatives (18 by the 3 x 3 tables) and 13 back.  About 1,200
-//   FP64 operations a cell against 1,650 with one lane per Gauss point, and all 32 lanes work instead of 27: the FP64
-//   pipe bounds this part.
+//   images, so a line takes 9 operations for values and derivatives (18 by the 3 x 3 tables) and 13 back for a pair of
+//   fluxes.  1,060 FP64 operations a cell (1,300, and 1025 us for the call below, with the products of the fluxes formed by
+//   themselves and the doublings and constants left in the lines) against 1,650 with one lane per Gauss point, and all 32 lanes work instead of 27: the
+//   FP64 pipe bounds this part.
 //   Element matrix (FP64 or FP32, the Jacobian's type).  Warp w owns the pair (l_x, j_x) = (w % 3, w / 3).  With the
 //   coefficients c = W (1 + u^2) and e_a = W 2 u s_a^2 d_a u at the points, sums over q_x, q_y and q_z in turn give
 //       J[l][j] = sum_q c sum_a s_a^2 d_a phi_l d_a phi_j + sum_q sum_a e_a d_a phi_l phi_j
@@ -19,8 +20,8 @@
 // k_q2_row: one thread a CSR row, rows of one kind per warp (mrg_q2_rows.cuh): its 1, 2, 4 or 8 cells' entries, lane by
 // lane consecutive, added in a fixed order and written once.
 //
-// Measured on 64^3 cells, FP32 Jacobian and FP64 residual: 1818 -> 1025 us (the tensor-core path with eight coloured
-// residual launches before), and the FP32 matrix's error fell from 2.4e-7 to 2.1e-8.  Cells take 730 us of it (FP64 pipe),
+// Measured on 64^3 cells, FP32 Jacobian and FP64 residual: 1818 -> 933 us (the tensor-core path with eight coloured
+// residual launches before), and the FP32 matrix's error fell from 2.4e-7 to 2.1e-8.  Cells take 600 us of it (FP64 pipe),
 // rows 390 (memory); the rows of a slab run beside the next slab's cells.
 // MRG_ASM_TENSOR_CORES takes the FP32 element matrices from the tcgen05 kernel instead (mrg_tc_q2.cu), for which
 // k_q2_cell writes the coefficients as TF32 operand images.
@@ -39,20 +40,25 @@ constexpr int LINES = 9;     // warps: lines of one direction, pairs (l_x, j_x)
 constexpr int ET = LINES * 32;
 constexpr int ENT = 729;     // entries of an element matrix
 constexpr int QRT = 128;     // threads per CTA of the row kernel
-// Slabs of cell layers (64^3 cells, FP32 Jacobian and FP64 residual: one slab 1151 us, 4 1074, 8 1050, 12 1059, 16 1086).
+// Slabs of cell layers (64^3 cells, FP32 Jacobian and FP64 residual, with 1,300 operations a cell: one slab 1151 us,
+// 4 1074, 8 1050, 12 1059, 16 1086).
 // A slab of 16384 cells is 512 CTAs, a little more than the GPU holds at 3 CTAs per SM: below that the launches' ends cost
 // more than the overlap gives.
 constexpr int MAXSLAB = 8;
 constexpr int64_t SLAB_CELLS = 16384;
 
+// k_q2_cell hands over e_a / E_SCALE (half the derivatives, and W u for 2 W u)
+constexpr double E_SCALE = 4.0;
+
 // Tables in the arithmetic type.  Gauss points -s, 0, s; node values l(q, a), derivatives d(q, a).
 template <typename T>
 struct Tab {
-  T ea, oa, w, s;      // l(q, outer) = ea -+ oa, l(outer q, middle) = w, l(middle q, middle) = 1
-  T sc[3];             // (2 / h_a)^2
+  T ea, oa, w;         // l(q, outer) = ea -+ oa, l(outer q, middle) = w = 1 - 2 ea, l(middle q, middle) = 1
+  T hc[3], zc[3];      // c / 4 and c s / 2 with c = (2 / h_a)^2: half the scaled derivative
+  T s2, s4;            // 2 s and -4 s: twice the transposed derivative
   T W[27];             // w_q |det J|
   T load[27];          // f * sum_q W_q phi_l(q)
-  T LL[3][9], DL[3][9];  // [q][l + 3 j]: l_l l_j, d_l l_j
+  T LL[3][9], DL[3][9];  // [q][l + 3 j]: l_l l_j, E_SCALE d_l l_j
   T DD[3][3][9];       // [axis][q][l + 3 j]: sc d_l d_j
 };
 
@@ -91,39 +97,68 @@ __device__ __forceinline__ float tf32_rn(float x) {
   return __uint_as_float(r);
 }
 
-// values at the three Gauss points of a line, and derivatives times c
+// Line operations, with explicit operations throughout.  Powers of two go where they cost nothing: derivatives are taken at
+// half and their transposes at twice their size, exactly.
+// values at the three Gauss points of a line: with z = v0 - 2 v1 + v2 the even part is v1 + ea z
+template <typename T>
+__device__ __forceinline__ T even_odd(const T v[3], T& o) {
+  o = addr(v[2], -v[0]);
+  return fma(T(-2), v[1], addr(v[0], v[2]));
+}
 template <typename T>
 __device__ __forceinline__ void values(const Tab<T>& t, const T v[3], T q[3]) {
-  const T e = addr(v[0], v[2]), o = addr(v[2], -v[0]), m = fma(t.ea, e, mulr(t.w, v[1]));
+  T o;
+  const T z = even_odd(v, o), m = fma(t.ea, z, v[1]);
   q[0] = fma(-t.oa, o, m);
   q[1] = v[1];
   q[2] = fma(t.oa, o, m);
 }
+// values, and half the derivatives along axis a
 template <typename T>
-__device__ __forceinline__ void values_derivs(const Tab<T>& t, T c, const T v[3], T q[3], T d[3]) {
-  const T e = addr(v[0], v[2]), o = addr(v[2], -v[0]), m = fma(t.ea, e, mulr(t.w, v[1]));
+__device__ __forceinline__ void values_derivs(const Tab<T>& t, int a, const T v[3], T q[3], T d[3]) {
+  T o;
+  const T z = even_odd(v, o), m = fma(t.ea, z, v[1]), h = mulr(t.hc[a], o);
   q[0] = fma(-t.oa, o, m);
   q[1] = v[1];
   q[2] = fma(t.oa, o, m);
-  const T z = fma(T(-2), v[1], e), h = mulr(mulr(T(0.5), c), o), sc = mulr(t.s, c);
-  d[0] = fma(-sc, z, h);
+  d[0] = fma(-t.zc[a], z, h);
   d[1] = h;
-  d[2] = fma(sc, z, h);
+  d[2] = fma(t.zc[a], z, h);
 }
-// the transposes: node sums of Gauss-point values against node values / derivatives
+// the transposes: node sums of Gauss-point values against node values
 template <typename T>
-__device__ __forceinline__ void values_t(const Tab<T>& t, const T f[3], T v[3]) {
-  const T e = addr(f[0], f[2]), o = addr(f[2], -f[0]), m = mulr(t.ea, e);
+__device__ __forceinline__ void values_t(const Tab<T>& t, T f1, T e, T o, T v[3]) {  // e = f0 + f2, o = f2 - f0
+  const T m = mulr(t.ea, e);
   v[0] = fma(-t.oa, o, m);
-  v[1] = fma(t.w, e, f[1]);
+  v[1] = fma(t.w, e, f1);
   v[2] = fma(t.oa, o, m);
 }
 template <typename T>
-__device__ __forceinline__ void derivs_t(const Tab<T>& t, const T f[3], T v[3]) {
-  const T so = mulr(t.s, addr(f[2], -f[0])), m = addr(addr(f[0], f[2]), f[1]);
-  v[0] = fma(T(-0.5), m, so);
-  v[1] = mulr(T(-2), so);
-  v[2] = fma(T(0.5), m, so);
+__device__ __forceinline__ void values_t(const Tab<T>& t, const T f[3], T v[3]) {
+  values_t<T>(t, f[1], addr(f[0], f[2]), addr(f[2], -f[0]), v);
+}
+// of the products c g
+template <typename T>
+__device__ __forceinline__ void values_t(const Tab<T>& t, const T c[3], const T g[3], T v[3]) {
+  const T f0 = mulr(c[0], g[0]);
+  values_t<T>(t, mulr(c[1], g[1]), fma(c[2], g[2], f0), fma(c[2], g[2], -f0), v);
+}
+// twice the sums against node derivatives, of the products c g
+template <typename T>
+__device__ __forceinline__ void derivs_t(const Tab<T>& t, const T c[3], const T g[3], T v[3]) {
+  const T f0 = mulr(c[0], g[0]), o = fma(c[2], g[2], -f0), m = fma(c[1], g[1], fma(c[2], g[2], f0));
+  v[0] = fma(t.s2, o, -m);
+  v[1] = mulr(t.s4, o);
+  v[2] = fma(t.s2, o, m);
+}
+// twice the sums of fd against derivatives plus the sums of fv against values
+template <typename T>
+__device__ __forceinline__ void derivs_values_t(const Tab<T>& t, const T fd[3], const T fv[3], T v[3]) {
+  const T o = addr(fd[2], -fd[0]), m = addr(addr(fd[0], fd[2]), fd[1]);
+  const T e = addr(fv[0], fv[2]), ov = addr(fv[2], -fv[0]);
+  v[0] = fma(t.s2, o, fma(-t.oa, ov, fma(t.ea, e, -m)));
+  v[1] = fma(t.s4, o, fma(t.w, e, fv[1]));
+  v[2] = fma(t.s2, o, fma(t.oa, ov, fma(t.ea, e, m)));
 }
 
 // What k_q2_cell leaves behind besides the residual entries
@@ -159,7 +194,7 @@ __global__ void __launch_bounds__(ET, sizeof(JT) == 4 ? 3 : 2)  // FP32: 1106 ->
     CT v[3], q[3], d[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) v[a] = (CT)__ldg(un + a);
-    values_derivs<CT>(t, t.sc[0], v, q, d);
+    values_derivs<CT>(t, 0, v, q, d);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       a0[(3 * line + a) * CB] = q[a];
@@ -172,7 +207,7 @@ __global__ void __launch_bounds__(ET, sizeof(JT) == 4 ? 3 : 2)  // FP32: 1106 ->
     CT v[3], q[3], d[3];
 #pragma unroll
     for (int b = 0; b < 3; ++b) v[b] = a0[at + 3 * b * CB];
-    values_derivs<CT>(t, t.sc[1], v, q, d);
+    values_derivs<CT>(t, 1, v, q, d);
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       b0[at + 3 * b * CB] = q[b];
@@ -189,47 +224,43 @@ __global__ void __launch_bounds__(ET, sizeof(JT) == 4 ? 3 : 2)  // FP32: 1106 ->
     CT v[3], uq[3], gx[3], gy[3], gz[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) v[q] = b0[at + 9 * q * CB];
-    values_derivs<CT>(t, t.sc[2], v, uq, gz);
+    values_derivs<CT>(t, 2, v, uq, gz);
 #pragma unroll
     for (int q = 0; q < 3; ++q) v[q] = b0[F + at + 9 * q * CB];
     values<CT>(t, v, gx);
 #pragma unroll
     for (int q = 0; q < 3; ++q) v[q] = b0[2 * F + at + 9 * q * CB];
     values<CT>(t, v, gy);
-    CT fx[3], fy[3], fz[3];
+    CT cw[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const CT W = t.W[line + 9 * q], cw = mulr(W, fma(uq[q], uq[q], CT(1)));
-      if constexpr (DOR) {
-        fx[q] = mulr(cw, gx[q]);
-        fy[q] = mulr(cw, gy[q]);
-        fz[q] = mulr(cw, gz[q]);
-      }
+      const CT W = t.W[line + 9 * q], e = mulr(W, uq[q]);
+      cw[q] = fma(e, uq[q], W);
       if constexpr (OUT != OUT_NONE) {
-        const CT e = mulr(CT(2) * W, uq[q]);
-        co[(line + 9 * q) * CB] = as<JT>(cw);
+        co[(line + 9 * q) * CB] = as<JT>(cw[q]);
         co[(27 + line + 9 * q) * CB] = as<JT>(mulr(e, gx[q]));
         co[(54 + line + 9 * q) * CB] = as<JT>(mulr(e, gy[q]));
         co[(81 + line + 9 * q) * CB] = as<JT>(mulr(e, gz[q]));
       }
     }
     if constexpr (DOR) {
-      values_t<CT>(t, fx, v);
+      values_t<CT>(t, cw, gx, v);
 #pragma unroll
       for (int q = 0; q < 3; ++q) a0[at + 9 * q * CB] = v[q];
-      values_t<CT>(t, fy, v);
+      values_t<CT>(t, cw, gy, v);
 #pragma unroll
       for (int q = 0; q < 3; ++q) a0[F + at + 9 * q * CB] = v[q];
-      derivs_t<CT>(t, fz, v);
+      derivs_t<CT>(t, cw, gz, v);
 #pragma unroll
       for (int q = 0; q < 3; ++q) a0[2 * F + at + 9 * q * CB] = v[q];
     }
   }
   __syncthreads();
   if constexpr (DOR) {
+    // the x and y fluxes come at half their size and are doubled by their transposed derivatives; the z flux is whole
     {  // back along y: line (q_x, node z)
       const int at = (i + 9 * k) * CB;
-      CT f[3], v[3], w[3];
+      CT f[3], w[3], v[3];
 #pragma unroll
       for (int b = 0; b < 3; ++b) f[b] = a0[at + 3 * b * CB];
       values_t<CT>(t, f, v);
@@ -237,26 +268,23 @@ __global__ void __launch_bounds__(ET, sizeof(JT) == 4 ? 3 : 2)  // FP32: 1106 ->
       for (int b = 0; b < 3; ++b) {
         b0[at + 3 * b * CB] = v[b];
         f[b] = a0[F + at + 3 * b * CB];
+        w[b] = a0[2 * F + at + 3 * b * CB];
       }
-      derivs_t<CT>(t, f, v);
+      derivs_values_t<CT>(t, f, w, v);
 #pragma unroll
-      for (int b = 0; b < 3; ++b) f[b] = a0[2 * F + at + 3 * b * CB];
-      values_t<CT>(t, f, w);
-#pragma unroll
-      for (int b = 0; b < 3; ++b) b0[F + at + 3 * b * CB] = addr(v[b], w[b]);
+      for (int b = 0; b < 3; ++b) b0[F + at + 3 * b * CB] = v[b];
     }
     __syncthreads();
     {  // back along x: line (node y, node z)
-      CT f[3], v[3], w[3];
+      CT f[3], w[3], v[3];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) f[a] = b0[(3 * line + a) * CB];
-      derivs_t<CT>(t, f, v);
+      for (int a = 0; a < 3; ++a) {
+        f[a] = b0[(3 * line + a) * CB];
+        w[a] = b0[F + (3 * line + a) * CB];
+      }
+      derivs_values_t<CT>(t, f, w, v);
 #pragma unroll
-      for (int a = 0; a < 3; ++a) f[a] = b0[F + (3 * line + a) * CB];
-      values_t<CT>(t, f, w);
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-        rbuf[(blk * 27 + 3 * line + a) * CB + lane] = addr(addr(v[a], w[a]), -t.load[3 * line + a]);
+      for (int a = 0; a < 3; ++a) rbuf[(blk * 27 + 3 * line + a) * CB + lane] = addr(v[a], -t.load[3 * line + a]);
     }
   }
   if constexpr (OUT == OUT_TF32) {
@@ -442,15 +470,19 @@ int mrg_q2_setup(mrg_problem* p) {
   Q->A.ncell = p->ncell;
   Q->A.blk0 = 0;
   Tab<double>& t = Q->A.t64;
-  double l[3][3], d[3][3], detJ = 1.0;
+  double l[3][3], d[3][3], sc[3], detJ = 1.0;
   for (int q = 0; q < 3; ++q) mrg_lagrange_1d(2, p->gx1[q], l[q], d[q]);
-  t.s = p->gx1[2];
+  const double gs = p->gx1[2];
+  t.s2 = 2.0 * gs;
+  t.s4 = -4.0 * gs;
   t.ea = 0.5 * (l[0][0] + l[0][2]);
   t.oa = 0.5 * (l[0][0] - l[0][2]);
   t.w = l[0][1];
   for (int a = 0; a < 3; ++a) {
     detJ *= 0.5 * p->h[a];
-    t.sc[a] = (2.0 / p->h[a]) * (2.0 / p->h[a]);
+    sc[a] = (2.0 / p->h[a]) * (2.0 / p->h[a]);
+    t.hc[a] = 0.25 * sc[a];
+    t.zc[a] = 0.5 * gs * sc[a];
   }
   const double* tw = p->qtab_host.data();
   const double* tphi = tw + p->nq;
@@ -463,8 +495,8 @@ int mrg_q2_setup(mrg_problem* p) {
   for (int q = 0; q < 3; ++q)
     for (int n = 0; n < 9; ++n) {
       t.LL[q][n] = l[q][n % 3] * l[q][n / 3];
-      t.DL[q][n] = d[q][n % 3] * l[q][n / 3];
-      for (int a = 0; a < 3; ++a) t.DD[a][q][n] = t.sc[a] * d[q][n % 3] * d[q][n / 3];
+      t.DL[q][n] = E_SCALE * (d[q][n % 3] * l[q][n / 3]);
+      for (int a = 0; a < 3; ++a) t.DD[a][q][n] = sc[a] * d[q][n % 3] * d[q][n / 3];
     }
   static_assert(sizeof(Tab<double>) == 2 * sizeof(Tab<float>), "the two tables hold the same values");
   const double* src = reinterpret_cast<const double*>(&t);

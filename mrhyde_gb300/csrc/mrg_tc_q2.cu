@@ -573,7 +573,7 @@ int mrg_q2tc_create(mrg_problem* p, Q2Tc** out, cudaStream_t st) {
           for (int d = 0; d < 3; ++d) v += s[d] * s[d] * G(d, k, l) * G(d, k, j);
         } else {
           const int d = (k - 27) / 27, q = (k - 27) % 27;
-          v = G(d, q, l) * G(3, q, j);
+          v = 4.0 * (G(d, q, l) * G(3, q, j));  // k_q2_cell writes ew / 4
         }
         const float hi = tf32_round_host((float)v);
         h[at(n, k, 0)] = hi;
