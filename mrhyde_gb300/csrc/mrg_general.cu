@@ -18,7 +18,7 @@
 //   k_cell_quad   lanes write and read consecutive addresses
 //   k_gather      one thread a CSR row: adds its cells' entries in a fixed order; rows staged in shared memory and
 //                 written once
-// Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 249 us (cells 222, FP64
+// Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 241 us (cells 214, FP64
 // pipe 87 % active, rows 27).
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
 // on several streams and may be captured.
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(128) k_metric(const __grid_constant__ MetricAr
     C[1][1] = Jm[0][0];
     det = Jm[0][0] * Jm[1][1] - Jm[0][1] * Jm[1][0];
   }
-  const double ad = fabs(det), sc = wq / ad;
+  const double ad = fabs(det), sc = (DIM == 3 ? 0.25 : 1.0) * (wq / ad);  // k_cell_hex1 uses a quarter of M
   double* out = A.metric + ((c >> 5) * Gen<DIM, P>::MROW + q) * CB + (c & 31);
   int k = 0;
 #pragma unroll
@@ -192,12 +192,18 @@ __global__ void __launch_bounds__(128) k_loads(const __grid_constant__ MetricArg
 
 // ---- Q1 hexahedra ----------------------------------------------------------------------------------
 // A linear node's reference gradient along its own axis is the constant +-1/2, so with differences d_b in place of
-// reference gradients a quarter of M is used (folded in below), sigma = -1 or +1 stands for the derivative, and the
+// reference gradients a quarter of M is used (stored so), sigma = -1 or +1 stands for the derivative, and the
 // weights of a pair of nodes at a Gauss point depend on the unordered pair alone (00, 01 or 11).
 __device__ __forceinline__ void lerp2(double be, double a, double b, double& p0, double& p1, double& d) {
   d = __dadd_rn(b, -a);
   p0 = fma(be, d, a);
   p1 = fma(-be, d, b);
+}
+// the same of the values c0 g0 and c1 g1, al = 1 - be: an operation less
+__device__ __forceinline__ void lerp2(double be, double al, double c0, double g0, double c1, double g1, double& p0, double& p1) {
+  const double f0 = __dmul_rn(c0, g0), d = fma(c1, g1, -f0);
+  p0 = fma(be, d, f0);
+  p1 = fma(al, d, f0);
 }
 __device__ __forceinline__ void pair3(double aa, double bb, double ab, double v0, double v1, double* t) {
   const double s = v0 + v1;
@@ -215,7 +221,7 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
   int cx, cy, cz;
   cell_of(g, c, cx, cy, cz);
   const int64_t NX = g.nn[0], plane = NX * g.nn[1], n0 = cx + NX * cy + plane * cz;
-  const double be = A.t.l[0][1];
+  const double be = A.t.l[0][1], al = A.t.l[0][0];
   double u[8], gd[3][4];  // u at the points q = qx + 2 qy + 4 qz; differences at the points of the other two axes
   {
     double v[8], X[8], Y[8], dx[4], dy[4], t[4], unused;
@@ -244,7 +250,7 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int x = q & 1, y = (q >> 1) & 1, z = q >> 2;
-    k[q] = 0.25 * fma(u[q], u[q], 1.0);
+    k[q] = fma(u[q], u[q], 1.0);
     const double d0 = gd[0][y + 2 * z], d1 = gd[1][x + 2 * z], d2 = gd[2][x + 2 * y];
     const double m01 = m(1, q), m02 = m(2, q), m12 = m(4, q);
     h[0][q] = fma(m(0, q), d0, fma(m01, d1, m02 * d2));
@@ -279,7 +285,7 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
     }
   }
   if constexpr (DOJ) {
-    const double al = 1.0 - be, aa = al * al, bb = be * be, ab = al * be;
+    const double aa = al * al, bb = be * be, ab = al * be;
     double E[64];
     // same-axis and advective parts: E[l][j] gets sigma(l_a) Z[j_a][pair b][pair c]
 #pragma unroll
@@ -291,11 +297,9 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
         for (int p = 0; p < 2; ++p) {
           const int q0 = pt(a, q, p, 0), q1 = pt(a, q, p, 1), ca = a == 0 ? 0 : (a == 1 ? 3 : 5);
           const double C = fma(k[q1], m(ca, q1), k[q0] * m(ca, q0));
-          // 2 u h / 4 (k carries the quarter, h does not)
-          double d, x0, x1;
-          lerp2(be, 0.5 * u[q0] * h[a][q0], 0.5 * u[q1] * h[a][q1], x0, x1, d);
-          Z[0][q][p] = x0 - C;
-          Z[1][q][p] = x1 + C;
+          const double f0 = (u[q0] + u[q0]) * h[a][q0], d = fma(u[q1] + u[q1], h[a][q1], -f0);  // 2 u h
+          Z[0][q][p] = fma(be, d, f0 - C);
+          Z[1][q][p] = fma(al, d, f0 + C);
         }
 #pragma unroll
       for (int ja = 0; ja < 2; ++ja) {
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
 #pragma unroll
           for (int qb = 0; qb < 2; ++qb) {
             const int q0 = (qb << b) | (qo << o), q1 = q0 | (1 << a);
-            lerp2(be, k[q0] * m(comp(a, b), q0), k[q1] * m(comp(a, b), q1), W[0][qb], W[1][qb], unused);
+            lerp2(be, al, k[q0], m(comp(a, b), q0), k[q1], m(comp(a, b), q1), W[0][qb], W[1][qb]);
           }
 #pragma unroll
           for (int i = 0; i < 2; ++i) lerp2(be, W[i][0], W[i][1], V[qo][i][0], V[qo][i][1], unused);
