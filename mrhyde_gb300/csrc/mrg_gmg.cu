@@ -599,6 +599,20 @@ __device__ __forceinline__ void cheb_row(const LevDev<T>& L, int64_t n, T ax, co
   L.d[n] = d;
   xout[n] = add_rn(zero_x ? T(0) : xin[n], d);
 }
+// Step 0 from x = 0, taken by the kernel that writes b: a launch and a pass over b less for each level of a cycle.  coef is
+// null where the cycle does not smooth (coarsest level, levels of k_vcycle_tail).
+template <typename T>
+struct FirstStep {
+  const T *coef, *minv;
+  T *d, *xa;
+  __device__ __forceinline__ T diag(int64_t n) const { return coef ? minv[n] : T(0); }  // to be in flight with b's terms
+  __device__ __forceinline__ void operator()(int64_t n, T b, T mi) const {
+    if (!coef) return;
+    const T v = mul_rn(coef[0], mul_rn(mi, b));
+    d[n] = v;
+    xa[n] = add_rn(T(0), v);
+  }
+};
 
 // r = b - A x, row n
 template <typename T>
@@ -687,11 +701,10 @@ __device__ __forceinline__ void parent_slots(int i, int nnf, int nnc, int co, bo
 // The free nodes are a Cartesian product, so a child counts if it exists and is free along each axis; the others are
 // loaded as zeros (no branches: the lanes of a warp have children missing at different places).
 template <typename T>
-__device__ __forceinline__ void restrict_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* __restrict__ rf,
-                                             T* __restrict__ bc, int64_t n) {
+__device__ __forceinline__ T restrict_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* __restrict__ rf, int64_t n) {
   int I[3];
   decompose(gc, n, I[0], I[1], I[2]);
-  if (node_fixed(gc, I[0], I[1], I[2])) { bc[n] = T(0); return; }
+  if (node_fixed(gc, I[0], I[1], I[2])) return T(0);
   int c[3][3];
   float w[3][3];
   bool k[3][3];
@@ -716,21 +729,25 @@ __device__ __forceinline__ void restrict_row(const Grid& gf, const Grid& gc, con
         s = fma((T)(w[0][a0] * w12), in ? r[c[0][a0]] : T(0), s);  // the weights are powers of two
       }
     }
-  bc[n] = s;
+  return s;
 }
 
+// and the coarse level's first smoothing step
 template <typename T>
 __global__ void __launch_bounds__(NT) k_restrict(Grid gf, Grid gc, Xfer X, const T* __restrict__ rf, T* __restrict__ bc,
-                                                 const GScal* __restrict__ S) {
+                                                 FirstStep<T> first, const GScal* __restrict__ S) {
   pdl_trigger();
   pdl_wait();
   if (is_done(S)) return;
   const int64_t nc = (int64_t)gc.nn[0] * gc.nn[1] * gc.nn[2];
-  for (int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x; n < nc; n += (int64_t)gridDim.x * NT)
-    restrict_row<T>(gf, gc, X, rf, bc, n);
+  for (int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x; n < nc; n += (int64_t)gridDim.x * NT) {
+    const T mi = first.diag(n), b = restrict_row<T>(gf, gc, X, rf, n);
+    bc[n] = b;
+    first(n, b, mi);
+  }
 }
 
-// x_f += P x_c, fine row n (shared by k_prolong and k_vcycle_tail)
+// x_f += P x_c, fine row n (k_vcycle_tail; k_prolong takes two rows at once)
 template <typename T>
 __device__ __forceinline__ void prolong_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* __restrict__ xc,
                                             T* __restrict__ xf, int64_t n) {
@@ -764,15 +781,63 @@ __device__ __forceinline__ void prolong_row(const Grid& gf, const Grid& gc, cons
   xf[n] = add_rn(xf[n], s);
 }
 
+// FP32: two neighbours along x a thread (nodes 2 j and 2 j + 1).  Their parents are the nodes j and j + 1 (2 j and 2 j + 1
+// where x is not coarsened), so 8 loads and one set of index arithmetic serve two rows (97^3 nodes: 14.2 -> 9.2 us).
+// Terms in prolong_row's order; those it multiplies by a weight of 0 are left out.  FP64: a row a thread; pairs halve the
+// warps that the FP64 pipe's latency is hidden behind (Newton solves on 48^3 cells with pairs 2 % slower).
 template <typename T>
 __global__ void __launch_bounds__(NT) k_prolong(Grid gf, Grid gc, Xfer X, const T* __restrict__ xc, T* __restrict__ xf,
                                                 const GScal* __restrict__ S) {
   pdl_trigger();
   pdl_wait();
   if (is_done(S)) return;
-  const int64_t nf = (int64_t)gf.nn[0] * gf.nn[1] * gf.nn[2];
-  for (int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x; n < nf; n += (int64_t)gridDim.x * NT)
-    prolong_row<T>(gf, gc, X, xc, xf, n);
+  if constexpr (sizeof(T) == 8) {
+    const int64_t nf = (int64_t)gf.nn[0] * gf.nn[1] * gf.nn[2];
+    for (int64_t n = (int64_t)blockIdx.x * NT + threadIdx.x; n < nf; n += (int64_t)gridDim.x * NT)
+      prolong_row<T>(gf, gc, X, xc, xf, n);
+    return;
+  }
+  const unsigned NXF = (unsigned)gf.nn[0], pairs = (NXF + 1) / 2, NY = (unsigned)gf.nn[1];
+  const unsigned np = pairs * NY * (unsigned)gf.nn[2];  // at most the number of rows, which is at most INT32_MAX
+  const int NX = gc.nn[0];
+  const int64_t plane = (int64_t)NX * gc.nn[1];
+  for (unsigned m = blockIdx.x * NT + threadIdx.x; m < np; m += gridDim.x * NT) {
+    const unsigned line = m / pairs, j = m - line * pairs;
+    const int i0 = 2 * (int)j, i[3] = {i0, (int)(line % NY), (int)(line / NY)};
+    int p[3][2], p1[2];
+    float w[3][2], w1[2];
+    bool k[3][2], k1[2];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      parent_slots(i[a], gf.nn[a], gc.nn[a], X.co[a], gf.dim > a, p[a], w[a], k[a]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) k[a][e] = k[a][e] && axis_free(gc, a, p[a][e]);
+    }
+    const bool second = i0 + 1 < (int)NXF;
+    parent_slots(min(i0 + 1, (int)NXF - 1), gf.nn[0], gc.nn[0], X.co[0], true, p1, w1, k1);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) k1[e] = k1[e] && axis_free(gc, 0, p1[e]);
+    const int b0 = p[0][0], b1 = min(b0 + 1, NX - 1);  // parents of both
+    const bool f0 = axis_free(gc, 0, b0), f1 = axis_free(gc, 0, b1);
+    T s0 = T(0), s1 = T(0);
+#pragma unroll
+    for (int e2 = 0; e2 < 2; ++e2)
+#pragma unroll
+      for (int e1 = 0; e1 < 2; ++e1) {
+        const T* r = xc + NX * p[1][e1] + plane * p[2][e2];
+        const float w12 = w[1][e1] * w[2][e2];
+        const bool in = k[2][e2] && k[1][e1];
+        const T t0 = in && f0 ? r[b0] : T(0), t1 = in && f1 ? r[b1] : T(0);
+        s0 = fma((T)(w[0][0] * w12), t0, s0);
+        s1 = fma((T)(w1[0] * w12), k1[0] ? (p1[0] == b0 ? t0 : t1) : T(0), s1);
+        s1 = fma((T)(w1[1] * w12), k1[1] ? t1 : T(0), s1);
+      }
+    const bool fr = !node_fixed(gf, i0, i[1], i[2]), fr1 = second && !node_fixed(gf, i0 + 1, i[1], i[2]);
+    T* x = xf + (int64_t)line * NXF + i0;
+    const T v0 = fr ? x[0] : T(0), v1 = fr1 ? x[1] : T(0);
+    if (fr) x[0] = add_rn(v0, s0);
+    if (fr1) x[1] = add_rn(v1, s1);
+  }
 }
 
 // x = inv b on the coarsest level, row i (shared by k_coarse_apply and k_vcycle_tail)
@@ -935,7 +1000,7 @@ __global__ void __launch_bounds__(TT) k_vcycle_tail(const __grid_constant__ Tail
     for (int n = threadIdx.x; n < (int)D.n; n += TT) resid_row<T>(D, n, tail_prod<T>(L, n, D.xb));
     __syncthreads();
     const LevDev<T>& C = lev[j + 1].D;
-    for (int64_t n = threadIdx.x; n < C.n; n += TT) restrict_row<T>(D.g, C.g, A.X[j + 1], D.r, C.b, n);
+    for (int64_t n = threadIdx.x; n < C.n; n += TT) C.b[n] = restrict_row<T>(D.g, C.g, A.X[j + 1], D.r, n);
     __syncthreads();
   }
   const LevDev<T>& Lc = lev[nl - 1].D;
@@ -1078,18 +1143,19 @@ __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cg_spmv(Grid g, int6
 
 // x += alpha p ; r -= alpha q ; |r| ; stopping test
 template <typename T>
-__global__ void __launch_bounds__(NT) k_cg_update(int64_t n, CgVec<T> V) {
+__global__ void __launch_bounds__(NT) k_cg_update(int64_t n, CgVec<T> V, FirstStep<T> first) {
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
   const T alpha = alpha_of<T>(V.S);
   T rr = T(0);
-  each4(n, [&](int64_t i) { return Vals<T, 4>{{V.x[i], V.p[i], V.r[i], V.q[i]}}; },
-        [&](int64_t i, const Vals<T, 4>& e) {
+  each4(n, [&](int64_t i) { return Vals<T, 5>{{V.x[i], V.p[i], V.r[i], V.q[i], first.diag(i)}}; },
+        [&](int64_t i, const Vals<T, 5>& e) {
           V.x[i] = e.v[0] + alpha * e.v[1];
           const T r = e.v[2] - alpha * e.v[3];
           V.r[i] = r;
           rr = fma(r, r, rr);
+          first(i, r, e.v[4]);
         });
   double m[1] = {block_sum((double)rr)};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
@@ -1156,13 +1222,17 @@ __global__ void __launch_bounds__(NT) k_bg_init(int64_t n, const double* __restr
 
 // p = r + beta (p - omega v)
 template <typename T>
-__global__ void __launch_bounds__(NT) k_bg_p(int64_t n, BgVec<T> V) {
+__global__ void __launch_bounds__(NT) k_bg_p(int64_t n, BgVec<T> V, FirstStep<T> first) {
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
   const T beta = beta_of<T>(V.S), omega = omega_of<T>(V.S);
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
-    V.p[i] = V.r[i] + beta * (V.p[i] - omega * V.v[i]);
+  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
+    const T mi = first.diag(i);
+    const T b = V.r[i] + beta * (V.p[i] - omega * V.v[i]);
+    V.p[i] = b;
+    first(i, b, mi);
+  }
 }
 
 // STEP 0: v = A ph, rv = rh . v, alpha = rho / rv.   STEP 1: t = A sh, omega = (t . s) / (t . t).
@@ -1215,13 +1285,17 @@ __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_bg_spmv(Grid g, int6
 
 // s = r - alpha v
 template <typename T>
-__global__ void __launch_bounds__(NT) k_bg_s(int64_t n, BgVec<T> V) {
+__global__ void __launch_bounds__(NT) k_bg_s(int64_t n, BgVec<T> V, FirstStep<T> first) {
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
   const T alpha = alpha_of<T>(V.S);
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT)
-    V.s[i] = V.r[i] - alpha * V.v[i];
+  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
+    const T mi = first.diag(i);
+    const T b = V.r[i] - alpha * V.v[i];
+    V.s[i] = b;
+    first(i, b, mi);
+  }
 }
 
 // x += alpha ph + omega sh ; r = s - omega t ; |r|, rh . r -> beta for the next direction; stopping test
@@ -1616,21 +1690,29 @@ void launch_resid(const HLevel& L, const LevDev<T>& D, const T* x, const GScal* 
   else launch_pdl(k_resid<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, x, S, err);
 }
 
-// One V(NU, NU) cycle: out = M^{-1} in on level 0 (in, out: level-0 vectors not used by the cycle).
 template <typename T>
-void enqueue_vcycle(Hier<T>* H, const T* in, T* out, cudaStream_t s) {
+FirstStep<T> first_step(const Hier<T>* H, int l) {
+  const int nl = (int)H->L.size(), tail = H->tail < 1 ? nl : H->tail;
+  const HLevel& L = H->L[l];
+  return FirstStep<T>{l < nl - 1 && l < tail ? H->coef + (size_t)l * NU * 3 : nullptr, (const T*)L.minv, (T*)L.d, (T*)L.xa};
+}
+
+// One V(NU, NU) cycle: out = M^{-1} in on level 0 (in, out: level-0 vectors not used by the cycle).  begun: level 0's first
+// step is done.
+template <typename T>
+void enqueue_vcycle(Hier<T>* H, const T* in, T* out, bool begun, cudaStream_t s) {
   const int nl = (int)H->L.size();
   const int tail = H->tail < 1 ? nl : H->tail;  // levels >= tail: k_vcycle_tail
   const GScal* S = H->S;
   for (int l = 0; l < nl - 1 && l < tail; ++l) {
     LevDev<T> D = levdev<T>(H->L[l]);
     if (l == 0) D.b = const_cast<T*>(in);
-    // pre-smoothing from x = 0: xa <- step 0, xb <- step 1
-    launch_cheb<T>(H->L[l], D, D.xa, D.xa, 0, 1, H->coef + (size_t)l * NU * 3, S, H->err, s);
+    // pre-smoothing from x = 0: xa <- step 0 (with the kernel that wrote b), xb <- step 1
+    if (l == 0 && !begun) launch_cheb<T>(H->L[l], D, D.xa, D.xa, 0, 1, H->coef + (size_t)l * NU * 3, S, H->err, s);
     launch_cheb<T>(H->L[l], D, D.xa, D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
     launch_resid<T>(H->L[l], D, D.xb, S, H->err, s);
     const HLevel& C = H->L[l + 1];
-    launch_pdl(k_restrict<T>, grid_for(C.n, 16), NT, 0, s, D.g, C.g, C.X, D.r, (T*)C.b, S);
+    launch_pdl(k_restrict<T>, grid_for(C.n, 16), NT, 0, s, D.g, C.g, C.X, D.r, (T*)C.b, first_step(H, l + 1), S);
   }
   if (tail < nl) {
     launch_pdl(k_vcycle_tail<T>, 1, TT, tail_smem<T>(H->targs), s, H->targs, S);
@@ -1642,7 +1724,7 @@ void enqueue_vcycle(Hier<T>* H, const T* in, T* out, cudaStream_t s) {
     LevDev<T> D = levdev<T>(H->L[l]);
     if (l == 0) D.b = const_cast<T*>(in);
     const HLevel& C = H->L[l + 1];
-    launch_pdl(k_prolong<T>, grid_for(D.n, 16), NT, 0, s, D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
+    launch_pdl(k_prolong<T>, grid_for(sizeof(T) == 4 ? (D.n + 1) / 2 : D.n, 16), NT, 0, s, D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
     // post-smoothing: xb -> xa (step 0), xa -> xb (step 1; level 0: -> out)
     launch_cheb<T>(H->L[l], D, D.xb, D.xa, 0, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
     launch_cheb<T>(H->L[l], D, D.xa, l == 0 ? out : D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
@@ -1662,8 +1744,8 @@ void enqueue_iters(Hier<T>* H, int count, cudaStream_t s) {
   for (int it = 0; it < count; ++it) {
     if (L0.pp.p[0] == 2) launch_pdl(k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_pdl(k_cg_update<T>, gr, NT, 0, s, L0.n, V);
-    enqueue_vcycle(H, H->r, (T*)H->L[0].xb, s);
+    launch_pdl(k_cg_update<T>, gr, NT, 0, s, L0.n, V, first_step(H, 0));
+    enqueue_vcycle(H, H->r, (T*)H->L[0].xb, true, s);
     launch_pdl(k_cg_rz<T>, gr, NT, 0, s, L0.n, V, 0);
   }
 }
@@ -1732,7 +1814,7 @@ int gmg_cg(mrg_problem* p, Hier<T>* H, const T* J, const double* b, double* x, d
   CgVec<T> V = cgvec(H);
   k_cg_init<T><<<grid_for(n, RED_PER_SM), NT, 0, s>>>(n, b, V);
   MRG_CUDA(cudaGetLastError());
-  enqueue_vcycle(H, H->r, (T*)H->L[0].xb, s);
+  enqueue_vcycle(H, H->r, (T*)H->L[0].xb, false, s);
   k_cg_rz<T><<<grid_for(n, RED_PER_SM), NT, 0, s>>>(n, V, 1);
   MRG_CUDA(cudaGetLastError());
   // captured chunk of iterations (re-captured when the Jacobian pointer or the stream changes)
@@ -1771,12 +1853,12 @@ void enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
   BgVec<T> V = bgvec(H);
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
-    launch_pdl(k_bg_p<T>, ge, NT, 0, s, L0.n, V);
-    enqueue_vcycle(H, H->p, H->ph, s);
+    launch_pdl(k_bg_p<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
+    enqueue_vcycle(H, H->p, H->ph, true, s);
     if (L0.pp.p[0] == 2) launch_pdl(k_bg_spmv<2, T, 0>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_bg_spmv<1, T, 0>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_pdl(k_bg_s<T>, ge, NT, 0, s, L0.n, V);
-    enqueue_vcycle(H, H->sv, H->sh, s);
+    launch_pdl(k_bg_s<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
+    enqueue_vcycle(H, H->sv, H->sh, true, s);
     if (L0.pp.p[0] == 2) launch_pdl(k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
     launch_pdl(k_bg_update<T>, gr, NT, 0, s, L0.n, V);
