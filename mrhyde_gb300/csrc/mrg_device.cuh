@@ -432,6 +432,14 @@ inline cudaError_t launch_pdl(void (*kernel)(KA...), unsigned grid, unsigned blo
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
 }
 
+// A kernel of such a chain that starts on idle SMs.  Q2 rows are read one a thread and live on the L1 cache, and an SM
+// gives its storage to L1 only when nothing else is resident: behind a programmatic launch they ran with the split of
+// the bulk-staged kernels before them (Newton on 64^3 Q2 cells 126 ms so, 49 launched whole).
+template <typename... KA, typename... A>
+inline void launch_whole(void (*kernel)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+  kernel<<<grid, block, smem, s>>>(static_cast<KA>(args)...);
+}
+
 struct AlwaysGo {
   __device__ __forceinline__ bool operator()() const { return true; }
 };

@@ -1679,14 +1679,14 @@ void launch_cheb(const HLevel& L, const LevDev<T>& D, const T* xin, T* xout, int
   if (zero_x)
     launch_pdl(k_cheb<1, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 1, coef, S, err);
   else if (L.pp.p[0] == 2)
-    launch_pdl(k_cheb<2, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 0, coef, S, err);
+    launch_whole(k_cheb<2, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 0, coef, S, err);
   else
     launch_pdl(k_cheb<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, xin, xout, k, 0, coef, S, err);
 }
 
 template <typename T>
 void launch_resid(const HLevel& L, const LevDev<T>& D, const T* x, const GScal* S, int* err, cudaStream_t s) {
-  if (L.pp.p[0] == 2) launch_pdl(k_resid<2, T>, grid_for(D.n, 16), NT, 0, s, D, x, S, err);
+  if (L.pp.p[0] == 2) launch_whole(k_resid<2, T>, grid_for(D.n, 16), NT, 0, s, D, x, S, err);
   else launch_pdl(k_resid<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, x, S, err);
 }
 
@@ -1742,7 +1742,7 @@ void enqueue_iters(Hier<T>* H, int count, cudaStream_t s) {
   CgVec<T> V = cgvec(H);
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
-    if (L0.pp.p[0] == 2) launch_pdl(k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    if (L0.pp.p[0] == 2) launch_whole(k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
     launch_pdl(k_cg_update<T>, gr, NT, 0, s, L0.n, V, first_step(H, 0));
     enqueue_vcycle(H, H->r, (T*)H->L[0].xb, true, s);
@@ -1855,11 +1855,11 @@ void enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
   for (int it = 0; it < count; ++it) {
     launch_pdl(k_bg_p<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
     enqueue_vcycle(H, H->p, H->ph, true, s);
-    if (L0.pp.p[0] == 2) launch_pdl(k_bg_spmv<2, T, 0>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    if (L0.pp.p[0] == 2) launch_whole(k_bg_spmv<2, T, 0>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_bg_spmv<1, T, 0>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
     launch_pdl(k_bg_s<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
     enqueue_vcycle(H, H->sv, H->sh, true, s);
-    if (L0.pp.p[0] == 2) launch_pdl(k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    if (L0.pp.p[0] == 2) launch_whole(k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
     else launch_pdl(k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
     launch_pdl(k_bg_update<T>, gr, NT, 0, s, L0.n, V);
   }
