@@ -1673,21 +1673,33 @@ int setup_values(Hier<T>* H, const T* J, cudaStream_t s) {
 
 // Launches of the row kernels for a level: Q1 levels use the staged loop (dynamic shared memory, fewer
 // CTAs per SM), a Q2 level 0 the direct row loop.
+// A kernel of the cycle on a level of n rows (grid transfers: of the finer level).  Chained launches hide the launch and the
+// first copies: FP32 Newton on 16^3 cells 1.63 -> 1.44 ms, 96^3 10 % faster, 128^3 alike.  On a large FP64 level they cost
+// more than that: the next kernel's CTAs take their places one by one as the FP64-bound ones end.  FP64 thermal Newton, ms,
+// all chained / none / levels up to 2^15 rows / up to 2^13: 128^3 50.3, 39.6, 39.1, 39.1; 48^3 6.94, 6.74, 6.36, 6.30;
+// 40^3 5.44, 5.49, 4.96, 5.15; 26^3 3.78, 4.09, 3.77, 3.66; 20^3 1.92, 2.12, 1.93, 1.94 (1+u^2 7.17, 7.42, 7.17, 6.74).
+constexpr int64_t CHAIN_ROWS64 = 1 << 13;
+template <typename T, typename... A>
+void launch_level(int64_t n, A&&... args) {
+  if (sizeof(T) == 4 || n <= CHAIN_ROWS64) launch_pdl(args...);
+  else launch_whole(args...);
+}
+
 template <typename T>
 void launch_cheb(const HLevel& L, const LevDev<T>& D, const T* xin, T* xout, int k, int zero_x,
                  const T* coef, const GScal* S, int* err, cudaStream_t s) {
   if (zero_x)
-    launch_pdl(k_cheb<1, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 1, coef, S, err);
+    launch_level<T>(D.n, k_cheb<1, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 1, coef, S, err);
   else if (L.pp.p[0] == 2)
     launch_whole(k_cheb<2, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 0, coef, S, err);
   else
-    launch_pdl(k_cheb<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, xin, xout, k, 0, coef, S, err);
+    launch_level<T>(D.n, k_cheb<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, xin, xout, k, 0, coef, S, err);
 }
 
 template <typename T>
 void launch_resid(const HLevel& L, const LevDev<T>& D, const T* x, const GScal* S, int* err, cudaStream_t s) {
   if (L.pp.p[0] == 2) launch_whole(k_resid<2, T>, grid_for(D.n, 16), NT, 0, s, D, x, S, err);
-  else launch_pdl(k_resid<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, x, S, err);
+  else launch_level<T>(D.n, k_resid<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, x, S, err);
 }
 
 template <typename T>
@@ -1712,19 +1724,19 @@ void enqueue_vcycle(Hier<T>* H, const T* in, T* out, bool begun, cudaStream_t s)
     launch_cheb<T>(H->L[l], D, D.xa, D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
     launch_resid<T>(H->L[l], D, D.xb, S, H->err, s);
     const HLevel& C = H->L[l + 1];
-    launch_pdl(k_restrict<T>, grid_for(C.n, 16), NT, 0, s, D.g, C.g, C.X, D.r, (T*)C.b, first_step(H, l + 1), S);
+    launch_level<T>(D.n, k_restrict<T>, grid_for(C.n, 16), NT, 0, s, D.g, C.g, C.X, D.r, (T*)C.b, first_step(H, l + 1), S);
   }
   if (tail < nl) {
-    launch_pdl(k_vcycle_tail<T>, 1, TT, tail_smem<T>(H->targs), s, H->targs, S);
+    launch_level<T>(H->L[tail - 1].n, k_vcycle_tail<T>, 1, TT, tail_smem<T>(H->targs), s, H->targs, S);
   } else {
     const HLevel& Lc = H->L[nl - 1];
-    launch_pdl(k_coarse_apply<T>, 1, NT, 0, s, (int)Lc.n, H->cinv, (const T*)Lc.b, (T*)Lc.xb, S);
+    launch_level<T>(Lc.n, k_coarse_apply<T>, 1, NT, 0, s, (int)Lc.n, H->cinv, (const T*)Lc.b, (T*)Lc.xb, S);
   }
   for (int l = std::min(tail, nl - 1) - 1; l >= 0; --l) {
     LevDev<T> D = levdev<T>(H->L[l]);
     if (l == 0) D.b = const_cast<T*>(in);
     const HLevel& C = H->L[l + 1];
-    launch_pdl(k_prolong<T>, grid_for(sizeof(T) == 4 ? (D.n + 1) / 2 : D.n, 16), NT, 0, s, D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
+    launch_level<T>(D.n, k_prolong<T>, grid_for(sizeof(T) == 4 ? (D.n + 1) / 2 : D.n, 16), NT, 0, s, D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
     // post-smoothing: xb -> xa (step 0), xa -> xb (step 1; level 0: -> out)
     launch_cheb<T>(H->L[l], D, D.xb, D.xa, 0, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
     launch_cheb<T>(H->L[l], D, D.xa, l == 0 ? out : D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
@@ -1743,10 +1755,10 @@ void enqueue_iters(Hier<T>* H, int count, cudaStream_t s) {
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
     if (L0.pp.p[0] == 2) launch_whole(k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
-    else launch_pdl(k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_pdl(k_cg_update<T>, gr, NT, 0, s, L0.n, V, first_step(H, 0));
+    else launch_level<T>(L0.n, k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_level<T>(L0.n, k_cg_update<T>, gr, NT, 0, s, L0.n, V, first_step(H, 0));
     enqueue_vcycle(H, H->r, (T*)H->L[0].xb, true, s);
-    launch_pdl(k_cg_rz<T>, gr, NT, 0, s, L0.n, V, 0);
+    launch_level<T>(L0.n, k_cg_rz<T>, gr, NT, 0, s, L0.n, V, 0);
   }
 }
 
@@ -1853,15 +1865,15 @@ void enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
   BgVec<T> V = bgvec(H);
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
-    launch_pdl(k_bg_p<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
+    launch_level<T>(L0.n, k_bg_p<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
     enqueue_vcycle(H, H->p, H->ph, true, s);
     if (L0.pp.p[0] == 2) launch_whole(k_bg_spmv<2, T, 0>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
-    else launch_pdl(k_bg_spmv<1, T, 0>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_pdl(k_bg_s<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
+    else launch_level<T>(L0.n, k_bg_spmv<1, T, 0>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_level<T>(L0.n, k_bg_s<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
     enqueue_vcycle(H, H->sv, H->sh, true, s);
     if (L0.pp.p[0] == 2) launch_whole(k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
-    else launch_pdl(k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_pdl(k_bg_update<T>, gr, NT, 0, s, L0.n, V);
+    else launch_level<T>(L0.n, k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_level<T>(L0.n, k_bg_update<T>, gr, NT, 0, s, L0.n, V);
   }
 }
 
