@@ -648,7 +648,7 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
   const size_t ebytes = doJ && !tc ? slots * ENT * (fp32 ? sizeof(float) : sizeof(double)) : 0;
   const size_t bytes = ebytes + (doR ? slots * 27 * sizeof(double) : 0);
   void* ws = nullptr;
-  if (bytes) MRG_CUDA(mrg_ws_take(p, bytes, s, &ws));
+  if (bytes) MRG_TAKE_WS(p, bytes, s, &ws);
   double* rbuf = doR ? reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + ebytes) : nullptr;
   int st = MRG_OK;
   cudaError_t e = cudaSuccess;

@@ -656,6 +656,14 @@ bool mrg_general_eligible(const mrg_problem* p, int points_per_axis) {
 }
 
 int mrg_general_setup(mrg_problem* p, cudaStream_t s) {
+  // a metric of more than a quarter of the device's memory (hexahedra: 384 bytes a cell) is left to the per-cell kernels,
+  // which form it anew: the caller's matrix is to fit as it would without it
+  const size_t bytes = (size_t)p->ncell * (p->g.dim == 3 ? 6 : 3) * p->npe * sizeof(double);
+  if (bytes > (size_t)1 << 30) {
+    size_t avail = 0, total = 0;
+    MRG_CUDA(cudaMemGetInfo(&avail, &total));
+    if (bytes > total / 4) return MRG_OK;
+  }
   General* Q = new General();
   p->general = Q;
   GenTab& t = Q->A.t;
@@ -677,6 +685,11 @@ int mrg_general_setup(mrg_problem* p, cudaStream_t s) {
   M.freq = p->source_freq;
   M.ncell = p->ncell;
   const int st = p->g.dim == 3 ? setup_t<3, 1>(p, Q, M, s) : (p->g.p == 1 ? setup_t<2, 1>(p, Q, M, s) : setup_t<2, 2>(p, Q, M, s));
+  if (st == MRG_ENOMEM) {  // likewise
+    cudaGetLastError();
+    mrg_general_free(p);
+    return MRG_OK;
+  }
   if (st) return st;
   Q->A.g = p->g;
   Q->A.metric = Q->d_metric;
@@ -703,7 +716,7 @@ int mrg_launch_general(mrg_problem* p, const double* u, double* r, void* J, uint
   const size_t cells = (size_t)((p->ncell + CB - 1) / CB) * CB;
   const size_t ebytes = doJ ? cells * p->npe * p->npe * (fp32 ? sizeof(float) : sizeof(double)) : 0;
   void* ws = nullptr;
-  MRG_CUDA(mrg_ws_take(p, ebytes + (doR ? cells * p->npe * sizeof(double) : 0), s, &ws));
+  MRG_TAKE_WS(p, ebytes + (doR ? cells * p->npe * sizeof(double) : 0), s, &ws);
   double* rbuf = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + ebytes);
   cudaError_t e;
   auto go = [&](auto* Jt) {

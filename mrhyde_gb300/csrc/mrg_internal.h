@@ -165,6 +165,18 @@ int mrg_ws_open(mrg_problem* p);   // at creation, on the current device
 void mrg_ws_close(mrg_problem* p); // after the handle's streams have drained
 cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, void** out);
 cudaError_t mrg_ws_give(void* ws, cudaStream_t s);
+// A launcher's return when there is no memory for its workspace; nothing has been launched then, and the call takes the
+// per-cell kernels, which need none: a mesh whose matrix nearly fills the device is assembled all the same.
+constexpr int MRG_NO_WORKSPACE = -1;
+#define MRG_TAKE_WS(p, bytes, s, out)                                       \
+  do {                                                                      \
+    const cudaError_t e__ = mrg_ws_take(p, bytes, s, out);                  \
+    if (e__ == cudaErrorMemoryAllocation) {                                 \
+      cudaGetLastError(); /* not to be found by the next launch's check */  \
+      return MRG_NO_WORKSPACE;                                              \
+    }                                                                       \
+    if (e__ != cudaSuccess) return mrg_cuda_check(e__, "workspace");        \
+  } while (0)
 // Cell matrices with stored geometry: the forms and shapes without a path of their own (mrg_general.cu)
 bool mrg_general_eligible(const mrg_problem* p, int points_per_axis);
 int mrg_general_setup(mrg_problem* p, cudaStream_t s);

@@ -389,7 +389,7 @@ int mrg_launch_nl1(mrg_problem* p, const double* u, double* r, void* J, uint32_t
   const size_t cells = (size_t)((p->ncell + CB - 1) / CB) * CB;
   const size_t zbytes = doJ ? cells * NZ_ * (fp32 ? sizeof(float) : sizeof(double)) : 0;
   void* ws = nullptr;
-  MRG_CUDA(mrg_ws_take(p, zbytes + (doR ? cells * 8 * sizeof(double) : 0), s, &ws));
+  MRG_TAKE_WS(p, zbytes + (doR ? cells * 8 * sizeof(double) : 0), s, &ws);
   double* rb = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + zbytes);
   cudaError_t e = fp32 && doJ ? launch<float>(p, A, u, r, (float*)J, (float*)ws, rb, doJ, doR, ovw, s)
                               : launch<double>(p, A, u, r, (double*)J, (double*)ws, rb, doJ, doR, ovw, s);

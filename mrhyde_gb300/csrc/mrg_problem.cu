@@ -261,6 +261,7 @@ struct WsPool {
   int users = 0;      // live handles
 };
 constexpr size_t WS_SLACK = (size_t)1 << 30;
+constexpr uint64_t WS_KEEP = 8ull << 30;
 namespace {
 std::mutex g_ws_mu;
 WsPool g_ws[SM_CACHE];  // by device ordinal
@@ -279,9 +280,10 @@ int mrg_ws_open(mrg_problem* p) {
     props.location.id = dev;
     cudaMemPool_t pool = nullptr;
     MRG_CUDA(cudaMemPoolCreate(&pool, &props));
-    // keep memory over synchronisations (trimmed when a handle goes); never make one stream wait for another to
-    // reuse its memory
-    uint64_t keep = UINT64_MAX;
+    // keep up to WS_KEEP over synchronisations (less when a handle goes): beyond that a call takes tens of milliseconds
+    // and can afford to map its memory, which the caller may want back; never make one stream wait for another to reuse
+    // its memory
+    uint64_t keep = WS_KEEP;
     int no = 0;
     cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no);
@@ -699,7 +701,7 @@ extern "C" int mrg_assemble(mrg_problem* p, const double* u, double* r, void* J,
   cudaStream_t s = (cudaStream_t)stream;
   p->last_stream = s;
   const bool fp32 = flags & MRG_ASM_J_FP32;
-  int st;
+  int st = MRG_NO_WORKSPACE;
   if (p->path == MRG_PATH_FACTORED && !(flags & MRG_ASM_FORCE_CELL)) {
     st = mrg_launch_factored(p, u, r, J, flags, s);
     if (st != MRG_OK) return st;
@@ -708,25 +710,22 @@ extern "C" int mrg_assemble(mrg_problem* p, const double* u, double* r, void* J,
     if (st != MRG_OK) return st;
   } else if (p->path == MRG_PATH_TENSOR && !(flags & MRG_ASM_FORCE_CELL)) {
     st = p->nl1 ? mrg_launch_nl1(p, u, r, J, flags, s) : mrg_launch_q2(p, u, r, J, flags, s);
-    if (st != MRG_OK) return st;
   } else if (p->path == MRG_PATH_STORED && !(flags & (MRG_ASM_FORCE_CELL | MRG_ASM_ATOMIC))) {
     st = mrg_launch_stored(p, u, r, J, flags, s);
     if (st != MRG_OK) return st;
   } else if (p->general && !(flags & (MRG_ASM_FORCE_CELL | MRG_ASM_ATOMIC))) {
     st = mrg_launch_general(p, u, r, J, flags, s);
-    if (st != MRG_OK) return st;
-  } else {
+  }
+  if (st == MRG_NO_WORKSPACE) {
     if (flags & MRG_ASM_OVERWRITE) {
       if (doJ) MRG_CUDA(cudaMemsetAsync(J, 0, p->nnz * (fp32 ? sizeof(float) : sizeof(double)), s));
       if (doR) MRG_CUDA(cudaMemsetAsync(r, 0, p->ndof * sizeof(double), s));
     }
     st = mrg_launch_cell(p, u, doR ? r : nullptr, doJ ? J : nullptr, flags, s);
     if (st != MRG_OK) return st;
-    if (doJ) {
-      st = mrg_launch_constraints(p, J, fp32, s);
-      if (st != MRG_OK) return st;
-    }
+    if (doJ) st = mrg_launch_constraints(p, J, fp32, s);
   }
+  if (st != MRG_OK) return st;
   // boundary workset loop (jacres:485-603): Neumann / weak-Dirichlet faces, after the volume terms
   if (mrg_boundary_active(p)) {
     st = mrg_launch_boundary(p, u, doR ? r : nullptr, doJ ? J : nullptr, fp32, s);
