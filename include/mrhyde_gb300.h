@@ -84,7 +84,8 @@ typedef struct mrg_mesh_desc {
   int32_t nx, ny, nz;
   double lo[3], hi[3];
   /* Optional host array [(nx+1)(ny+1)(nz+1) * dim] of vertex coordinates (x fastest).  NULL = uniform
-     box.  When given, cells may be non-affine and the exact per-cell AD path is used. */
+     box.  When given, cells may be non-affine: their geometry is stored at creation (thermal Q1 cells,
+     1 + u^2 on Q1 hexahedra and all quadrilaterals), Q2 hexahedra take the per-cell AD path. */
   const double* vertex_coords;
 } mrg_mesh_desc;
 
@@ -111,9 +112,11 @@ typedef struct mrg_problem_info {
 
 enum {
   MRG_PATH_FACTORED = 1,   /* identical affine cells: K_e = kappa_c * K_ref, row-gather assembly */
-  MRG_PATH_CELL = 2,       /* per-cell geometry + forward-AD tangents in registers, colored scatter */
-  MRG_PATH_TENSOR = 3,     /* identical affine hexahedra, Q2 or nonlinear Q1: sum-factorised FP64 residual,
-                              row-gather Jacobian (each (row, cell) pair one row of a constant-operand GEMM) */
+  MRG_PATH_CELL = 2,       /* any geometry and form: cell matrices from a stored metric, gathered row by row (Q1
+                              hexahedra, quadrilaterals); other cells, MRG_ASM_FORCE_CELL and MRG_ASM_ATOMIC:
+                              per-cell geometry + forward-AD tangents in registers, colored scatter */
+  MRG_PATH_TENSOR = 3,     /* identical affine hexahedra, Q2 or nonlinear Q1: sum-factorised cell numbers or
+                              matrices gathered row by row; thermal Q2: kappa sums times class coefficients */
   MRG_PATH_STORED = 4      /* thermal Q1 hexahedra of general geometry: each cell's kappa-free stiffness (FP64
                               and FP32) and the node loads computed once at creation (the reference's stored
                               per-cell basis data, "storage proportion" 1.0; 432 bytes a cell and 8 a node),

@@ -20,7 +20,8 @@
 //      4, an exponent shift), with the sign set on the integer pipe.  The only FP64 instructions of a row
 //      are then the residual's 21 FMAs (42 with the products).
 //
-//  (2) Per-cell path (any geometry; any physics form; Q1 or Q2).  One CTA slice per cell: one
+//  (2) Per-cell path (general Q2 hexahedra; any cells for MRG_ASM_FORCE_CELL and MRG_ASM_ATOMIC; the other forms are
+//      in mrg_stored.cu, mrg_general.cu, mrg_box_q2.cu, mrg_nonlinear_q1.cu and mrg_assemble_q2.cu).  One CTA slice per cell: one
 //      thread per quadrature point computes the geometric Jacobian from the cell vertices, the
 //      physical gradients and the fields at that point into shared memory; then one thread per
 //      element row i runs the reference's forward-AD residual literally -- res_i as a dual number with

@@ -8,8 +8,8 @@
 //   for each of the 9 lines of a direction; the middle Gauss point is the middle node, and the outer two are mirror
 //   images, so a line takes 9 operations for values and derivatives (18 by the 3 x 3 tables) and 13 back for a pair of
 //   fluxes.  1,060 FP64 operations a cell (1,300, and 1025 us for the call below, with the products of the fluxes formed by
-//   themselves and the doublings and constants left in the lines) against 1,650 with one lane per Gauss point, and all 32 lanes work instead of 27: the
-//   FP64 pipe bounds this part.
+//   themselves and the doublings and constants left in the lines) against 1,650 with one lane per Gauss point, and all
+//   32 lanes work instead of 27: the FP64 pipe bounds this part.
 //   Element matrix (FP64 or FP32, the Jacobian's type).  Warp w owns the pair (l_x, j_x) = (w % 3, w / 3).  With the
 //   coefficients c = W (1 + u^2) and e_a = W 2 u s_a^2 d_a u at the points, sums over q_x, q_y and q_z in turn give
 //       J[l][j] = sum_q c sum_a s_a^2 d_a phi_l d_a phi_j + sum_q sum_a e_a d_a phi_l phi_j

@@ -7,7 +7,8 @@
 // Jacobian is
 //     K_c[l][j] = sum_q cw_q sum_d s_d^2 G_d[q][l] G_d[q][j]  +  sum_{d,q} ew_{q,d} G_d[q][l] Phi[q][j]
 // with per-point coefficients W_c = (cw_q | ew_{q,x} | ew_{q,y} | ew_{q,z}) (108 values, written by
-// k_q2_cell) and the constant reference tables G_d (gradients) and Phi (values).  All element matrices together are ONE GEMM with a constant right operand:
+// k_q2_cell, ew at a quarter of its size) and the constant reference tables G_d (gradients) and Phi (values).  All
+// element matrices together are ONE GEMM with a constant right operand:
 //     E (ncell x 768) = W (ncell x K) * H (K x 768),   H[k][28 l + j] = the products above,
 // K = 108, the 27 x 27 element matrix stored with rows padded to 28 so that
 // each row starts on 16 bytes.  The GEMM runs in FP32-class precision as 3xTF32: every operand is split
