@@ -1674,14 +1674,16 @@ int setup_values(Hier<T>* H, const T* J, cudaStream_t s) {
 // Launches of the row kernels for a level: Q1 levels use the staged loop (dynamic shared memory, fewer
 // CTAs per SM), a Q2 level 0 the direct row loop.
 // A kernel of the cycle on a level of n rows (grid transfers: of the finer level).  Chained launches hide the launch and the
-// first copies: FP32 Newton on 16^3 cells 1.63 -> 1.44 ms, 96^3 10 % faster, 128^3 alike.  On a large FP64 level they cost
-// more than that: the next kernel's CTAs take their places one by one as the FP64-bound ones end.  FP64 thermal Newton, ms,
-// all chained / none / levels up to 2^15 rows / up to 2^13: 128^3 50.3, 39.6, 39.1, 39.1; 48^3 6.94, 6.74, 6.36, 6.30;
-// 40^3 5.44, 5.49, 4.96, 5.15; 26^3 3.78, 4.09, 3.77, 3.66; 20^3 1.92, 2.12, 1.93, 1.94 (1+u^2 7.17, 7.42, 7.17, 6.74).
-constexpr int64_t CHAIN_ROWS64 = 1 << 13;
+// first copies, but the next kernel's CTAs take their places one by one as those of the one before end, which costs a large
+// level, and a large FP64 level more, than that.  Newton solves in ms.
+// FP64 thermal, all chained / none / levels up to 2^15 rows / up to 2^13: 128^3 50.3, 39.6, 39.1, 39.1; 48^3 6.94, 6.74,
+// 6.36, 6.30; 40^3 5.44, 5.49, 4.96, 5.15; 26^3 3.78, 4.09, 3.77, 3.66; 20^3 1.92, 2.12, 1.93, 1.94 (1+u^2 7.17, 7.42, 7.17,
+// 6.74).  FP32 thermal, all / up to 2^20 / 2^19 / 2^16 / 2^12: 192^3 36.8, 32.5; 128^3 11.4, 10.92, 10.93, 11.06, 11.45;
+// 96^3 6.42, 6.41, 6.35, 6.49, 6.62; 64^3 3.46, 3.47, 3.47, 3.58, 3.92; 28^3 1.89, 1.89, 1.88, 1.88, 1.94.
+constexpr int64_t CHAIN_ROWS64 = 1 << 13, CHAIN_ROWS32 = 1 << 19;
 template <typename T, typename... A>
 void launch_level(int64_t n, A&&... args) {
-  if (sizeof(T) == 4 || n <= CHAIN_ROWS64) launch_pdl(args...);
+  if (n <= (sizeof(T) == 4 ? CHAIN_ROWS32 : CHAIN_ROWS64)) launch_pdl(args...);
   else launch_whole(args...);
 }
 
