@@ -1731,8 +1731,10 @@ void enqueue_vcycle(Hier<T>* H, const T* in, T* out, bool begun, cudaStream_t s)
   if (tail < nl) {
     launch_level<T>(H->L[tail - 1].n, k_vcycle_tail<T>, 1, TT, tail_smem<T>(H->targs), s, H->targs, S);
   } else {
+    // a mesh of at most MAXC nodes is its own coarsest level: the inverse takes the cycle's input to its output
     const HLevel& Lc = H->L[nl - 1];
-    launch_level<T>(Lc.n, k_coarse_apply<T>, 1, NT, 0, s, (int)Lc.n, H->cinv, (const T*)Lc.b, (T*)Lc.xb, S);
+    launch_level<T>(Lc.n, k_coarse_apply<T>, 1, NT, 0, s, (int)Lc.n, H->cinv, nl == 1 ? in : (const T*)Lc.b,
+                    nl == 1 ? out : (T*)Lc.xb, S);
   }
   for (int l = std::min(tail, nl - 1) - 1; l >= 0; --l) {
     LevDev<T> D = levdev<T>(H->L[l]);
