@@ -440,8 +440,13 @@ const KCfg kCfgs[] = {
     {1024, 4, k_batch<1024, 4>},
 };
 
-int batch_smem(const mrg_batch* B, const KCfg& c) {
-  return (2 * c.threads * c.rows + B->max_nodes + B->max_cells) * (int)sizeof(float);  // x, 1/diag; p; kappa
+int batch_smem(const KCfg& c, int nodes, int cells) {
+  return (2 * c.threads * c.rows + nodes + cells) * (int)sizeof(float);  // x, 1/diag; p; kappa
+}
+// of the largest problem that a batch may hold
+constexpr int MAX_EDGE = 16;
+int batch_smem_most(const KCfg& c) {
+  return batch_smem(c, (MAX_EDGE + 1) * (MAX_EDGE + 1) * (MAX_EDGE + 1), MAX_EDGE * MAX_EDGE * MAX_EDGE);
 }
 
 }  // namespace
@@ -460,7 +465,7 @@ extern "C" int mrg_batch_create(const mrg_batch_desc* d, mrg_batch** out) {
     P.ny = d->sizes[3 * k + 1];
     P.nz = d->sizes[3 * k + 2];
     P.pad = 0;
-    if (P.nx < 2 || P.ny < 2 || P.nz < 2 || P.nx > 16 || P.ny > 16 || P.nz > 16) {
+    if (P.nx < 2 || P.ny < 2 || P.nz < 2 || P.nx > MAX_EDGE || P.ny > MAX_EDGE || P.nz > MAX_EDGE) {
       delete B;
       return mrg_fail(MRG_EINVAL, "mrg_batch_create: local problem cells per axis must be in [2, 16]");
     }
@@ -528,8 +533,9 @@ extern "C" int mrg_batch_create(const mrg_batch_desc* d, mrg_batch** out) {
     return fail(e, "upload kappa32");
   if ((e = cudaMemcpy(B->d_g, d->dirichlet, B->nnode * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess)
     return fail(e, "upload dirichlet");
+  // the limit belongs to the kernel, not to the batch: always the same, so that no batch takes it from another
   for (const KCfg& c : kCfgs)
-    if ((e = cudaFuncSetAttribute(c.k, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_smem(B, c))) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(c.k, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_smem_most(c))) != cudaSuccess)
       return fail(e, "batch kernel shared memory");
   *out = B;
   return MRG_OK;
@@ -575,7 +581,7 @@ static int launch_batch(mrg_batch* B, double* u, float* J, const mrg_batch_opts*
   if (!cfg) return mrg_fail(MRG_EINVAL, "mrg_batch: unsupported thread count");
   BatchArgs A{B->d_probs, B->d_order, B->nprob, B->d_kappa, B->d_kappa32, B->d_g, u, J, B->d_counter, B->d_stats,
               o->tol, o->inner_tol, o->max_outer, o->max_inner, B->max_nodes, B->max_cells};
-  const int smem = batch_smem(B, *cfg);
+  const int smem = batch_smem(*cfg, B->max_nodes, B->max_cells);
   const int grid = std::max(1, std::min(B->nprob, nsm * ctas_per_sm));
   MRG_CUDA(cudaMemsetAsync(B->d_counter, 0, sizeof(int), s));
   cfg->k<<<grid, cfg->threads, smem, s>>>(A);
