@@ -281,7 +281,10 @@ static int bicg_run(mrg_problem* p, const JT* J, const double* b, VT* x, bool x0
     MRG_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     if (p->g.p == 1) enqueue_iters<1, VT, JT>(p, V, cs);
     else enqueue_iters<2, VT, JT>(p, V, cs);
-    cudaError_t e = cudaStreamEndCapture(cs, &graph);
+    cudaError_t e = cudaGetLastError();  // a refused launch leaves the capture intact, without that kernel
+    const cudaError_t ended = cudaStreamEndCapture(cs, &graph);
+    if (e == cudaSuccess) e = ended;
+    else if (ended == cudaSuccess) cudaGraphDestroy(graph);
     if (own) cudaStreamDestroy(cs);
     if (e != cudaSuccess) return mrg_cuda_check(e, "capture BiCGStab chunk");
     e = cudaGraphInstantiate(&w->g[gi], graph, 0);

@@ -418,7 +418,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... KA, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+inline cudaError_t launch_as(bool chained, void (*kernel)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                             A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
@@ -428,17 +429,17 @@ inline cudaError_t launch_pdl(void (*kernel)(KA...), unsigned grid, unsigned blo
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
 }
+template <typename... A>
+inline cudaError_t launch_pdl(A... args) { return launch_as(true, args...); }
 
 // A kernel of such a chain that starts on idle SMs.  Q2 rows are read one a thread and live on the L1 cache, and an SM
 // gives its storage to L1 only when nothing else is resident: behind a programmatic launch they ran with the split of
 // the bulk-staged kernels before them (Newton on 64^3 Q2 cells 126 ms so, 49 launched whole).
-template <typename... KA, typename... A>
-inline void launch_whole(void (*kernel)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
-  kernel<<<grid, block, smem, s>>>(static_cast<KA>(args)...);
-}
+template <typename... A>
+inline cudaError_t launch_whole(A... args) { return launch_as(false, args...); }
 
 struct AlwaysGo {
   __device__ __forceinline__ bool operator()() const { return true; }

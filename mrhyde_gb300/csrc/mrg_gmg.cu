@@ -1681,27 +1681,33 @@ int setup_values(Hier<T>* H, const T* J, cudaStream_t s) {
 // 6.74).  FP32 thermal, all / up to 2^20 / 2^19 / 2^16 / 2^12: 192^3 36.8, 32.5; 128^3 11.4, 10.92, 10.93, 11.06, 11.45;
 // 96^3 6.42, 6.41, 6.35, 6.49, 6.62; 64^3 3.46, 3.47, 3.47, 3.58, 3.92; 28^3 1.89, 1.89, 1.88, 1.88, 1.94.
 constexpr int64_t CHAIN_ROWS64 = 1 << 13, CHAIN_ROWS32 = 1 << 19;
+// A refused launch inside a capture leaves the capture intact, without that kernel: so every launch is looked at, the first
+// error is kept in e, and nothing is launched after it.
+template <typename... A>
+void launch_q2(cudaError_t& e, A&&... args) {
+  if (e == cudaSuccess) e = launch_whole(args...);
+}
 template <typename T, typename... A>
-void launch_level(int64_t n, A&&... args) {
-  if (n <= (sizeof(T) == 4 ? CHAIN_ROWS32 : CHAIN_ROWS64)) launch_pdl(args...);
-  else launch_whole(args...);
+void launch_level(cudaError_t& e, int64_t n, A&&... args) {
+  if (e != cudaSuccess) return;
+  e = n <= (sizeof(T) == 4 ? CHAIN_ROWS32 : CHAIN_ROWS64) ? launch_pdl(args...) : launch_whole(args...);
 }
 
 template <typename T>
-void launch_cheb(const HLevel& L, const LevDev<T>& D, const T* xin, T* xout, int k, int zero_x,
+void launch_cheb(cudaError_t& e, const HLevel& L, const LevDev<T>& D, const T* xin, T* xout, int k, int zero_x,
                  const T* coef, const GScal* S, int* err, cudaStream_t s) {
   if (zero_x)
-    launch_level<T>(D.n, k_cheb<1, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 1, coef, S, err);
+    launch_level<T>(e, D.n, k_cheb<1, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 1, coef, S, err);
   else if (L.pp.p[0] == 2)
-    launch_whole(k_cheb<2, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 0, coef, S, err);
+    launch_q2(e, k_cheb<2, T>, grid_for(D.n, 16), NT, 0, s, D, xin, xout, k, 0, coef, S, err);
   else
-    launch_level<T>(D.n, k_cheb<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, xin, xout, k, 0, coef, S, err);
+    launch_level<T>(e, D.n, k_cheb<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, xin, xout, k, 0, coef, S, err);
 }
 
 template <typename T>
-void launch_resid(const HLevel& L, const LevDev<T>& D, const T* x, const GScal* S, int* err, cudaStream_t s) {
-  if (L.pp.p[0] == 2) launch_whole(k_resid<2, T>, grid_for(D.n, 16), NT, 0, s, D, x, S, err);
-  else launch_level<T>(D.n, k_resid<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, x, S, err);
+void launch_resid(cudaError_t& e, const HLevel& L, const LevDev<T>& D, const T* x, const GScal* S, int* err, cudaStream_t s) {
+  if (L.pp.p[0] == 2) launch_q2(e, k_resid<2, T>, grid_for(D.n, 16), NT, 0, s, D, x, S, err);
+  else launch_level<T>(e, D.n, k_resid<1, T>, grid_for(D.n, staged_per_sm<T>()), NT, staged_smem<T>(), s, D, x, S, err);
 }
 
 template <typename T>
@@ -1714,7 +1720,7 @@ FirstStep<T> first_step(const Hier<T>* H, int l) {
 // One V(NU, NU) cycle: out = M^{-1} in on level 0 (in, out: level-0 vectors not used by the cycle).  begun: level 0's first
 // step is done.
 template <typename T>
-void enqueue_vcycle(Hier<T>* H, const T* in, T* out, bool begun, cudaStream_t s) {
+void enqueue_vcycle(cudaError_t& e, Hier<T>* H, const T* in, T* out, bool begun, cudaStream_t s) {
   const int nl = (int)H->L.size();
   const int tail = H->tail < 1 ? nl : H->tail;  // levels >= tail: k_vcycle_tail
   const GScal* S = H->S;
@@ -1722,28 +1728,28 @@ void enqueue_vcycle(Hier<T>* H, const T* in, T* out, bool begun, cudaStream_t s)
     LevDev<T> D = levdev<T>(H->L[l]);
     if (l == 0) D.b = const_cast<T*>(in);
     // pre-smoothing from x = 0: xa <- step 0 (with the kernel that wrote b), xb <- step 1
-    if (l == 0 && !begun) launch_cheb<T>(H->L[l], D, D.xa, D.xa, 0, 1, H->coef + (size_t)l * NU * 3, S, H->err, s);
-    launch_cheb<T>(H->L[l], D, D.xa, D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
-    launch_resid<T>(H->L[l], D, D.xb, S, H->err, s);
+    if (l == 0 && !begun) launch_cheb<T>(e, H->L[l], D, D.xa, D.xa, 0, 1, H->coef + (size_t)l * NU * 3, S, H->err, s);
+    launch_cheb<T>(e, H->L[l], D, D.xa, D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
+    launch_resid<T>(e, H->L[l], D, D.xb, S, H->err, s);
     const HLevel& C = H->L[l + 1];
-    launch_level<T>(D.n, k_restrict<T>, grid_for(C.n, 16), NT, 0, s, D.g, C.g, C.X, D.r, (T*)C.b, first_step(H, l + 1), S);
+    launch_level<T>(e, D.n, k_restrict<T>, grid_for(C.n, 16), NT, 0, s, D.g, C.g, C.X, D.r, (T*)C.b, first_step(H, l + 1), S);
   }
   if (tail < nl) {
-    launch_level<T>(H->L[tail - 1].n, k_vcycle_tail<T>, 1, TT, tail_smem<T>(H->targs), s, H->targs, S);
+    launch_level<T>(e, H->L[tail - 1].n, k_vcycle_tail<T>, 1, TT, tail_smem<T>(H->targs), s, H->targs, S);
   } else {
     // a mesh of at most MAXC nodes is its own coarsest level: the inverse takes the cycle's input to its output
     const HLevel& Lc = H->L[nl - 1];
-    launch_level<T>(Lc.n, k_coarse_apply<T>, 1, NT, 0, s, (int)Lc.n, H->cinv, nl == 1 ? in : (const T*)Lc.b,
+    launch_level<T>(e, Lc.n, k_coarse_apply<T>, 1, NT, 0, s, (int)Lc.n, H->cinv, nl == 1 ? in : (const T*)Lc.b,
                     nl == 1 ? out : (T*)Lc.xb, S);
   }
   for (int l = std::min(tail, nl - 1) - 1; l >= 0; --l) {
     LevDev<T> D = levdev<T>(H->L[l]);
     if (l == 0) D.b = const_cast<T*>(in);
     const HLevel& C = H->L[l + 1];
-    launch_level<T>(D.n, k_prolong<T>, grid_for(sizeof(T) == 4 ? (D.n + 1) / 2 : D.n, 16), NT, 0, s, D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
+    launch_level<T>(e, D.n, k_prolong<T>, grid_for(sizeof(T) == 4 ? (D.n + 1) / 2 : D.n, 16), NT, 0, s, D.g, C.g, C.X, (const T*)C.xb, D.xb, S);
     // post-smoothing: xb -> xa (step 0), xa -> xb (step 1; level 0: -> out)
-    launch_cheb<T>(H->L[l], D, D.xb, D.xa, 0, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
-    launch_cheb<T>(H->L[l], D, D.xa, l == 0 ? out : D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
+    launch_cheb<T>(e, H->L[l], D, D.xb, D.xa, 0, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
+    launch_cheb<T>(e, H->L[l], D, D.xa, l == 0 ? out : D.xb, 1, 0, H->coef + (size_t)l * NU * 3, S, H->err, s);
   }
 }
 
@@ -1753,17 +1759,19 @@ CgVec<T> cgvec(Hier<T>* H) {
 }
 
 template <typename T>
-void enqueue_iters(Hier<T>* H, int count, cudaStream_t s) {
+cudaError_t enqueue_iters(Hier<T>* H, int count, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   const HLevel& L0 = H->L[0];
   CgVec<T> V = cgvec(H);
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
-    if (L0.pp.p[0] == 2) launch_whole(k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
-    else launch_level<T>(L0.n, k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_level<T>(L0.n, k_cg_update<T>, gr, NT, 0, s, L0.n, V, first_step(H, 0));
-    enqueue_vcycle(H, H->r, (T*)H->L[0].xb, true, s);
-    launch_level<T>(L0.n, k_cg_rz<T>, gr, NT, 0, s, L0.n, V, 0);
+    if (L0.pp.p[0] == 2) launch_q2(e, k_cg_spmv<2, T>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    else launch_level<T>(e, L0.n, k_cg_spmv<1, T>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_level<T>(e, L0.n, k_cg_update<T>, gr, NT, 0, s, L0.n, V, first_step(H, 0));
+    enqueue_vcycle(e, H, H->r, (T*)H->L[0].xb, true, s);
+    launch_level<T>(e, L0.n, k_cg_rz<T>, gr, NT, 0, s, L0.n, V, 0);
   }
+  return e;
 }
 
 template <typename T>
@@ -1830,7 +1838,12 @@ int gmg_cg(mrg_problem* p, Hier<T>* H, const T* J, const double* b, double* x, d
   CgVec<T> V = cgvec(H);
   k_cg_init<T><<<grid_for(n, RED_PER_SM), NT, 0, s>>>(n, b, V);
   MRG_CUDA(cudaGetLastError());
-  enqueue_vcycle(H, H->r, (T*)H->L[0].xb, false, s);
+  cudaError_t e = cudaSuccess;
+  enqueue_vcycle(e, H, H->r, (T*)H->L[0].xb, false, s);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // not to be found by the next launch's check
+    return mrg_cuda_check(e, "multigrid cycle launch");
+  }
   k_cg_rz<T><<<grid_for(n, RED_PER_SM), NT, 0, s>>>(n, V, 1);
   MRG_CUDA(cudaGetLastError());
   // captured chunk of iterations (re-captured when the Jacobian pointer or the stream changes)
@@ -1842,15 +1855,19 @@ int gmg_cg(mrg_problem* p, Hier<T>* H, const T* J, const double* b, double* x, d
     cudaStream_t cs = nullptr;
     MRG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
+    e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      enqueue_iters(H, GCHUNK, cs);
-      e = cudaStreamEndCapture(cs, &graph);
+      e = enqueue_iters(H, GCHUNK, cs);
+      const cudaError_t ended = cudaStreamEndCapture(cs, &graph);
+      if (e == cudaSuccess) e = ended;
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&H->graph, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     cudaStreamDestroy(cs);
-    if (e != cudaSuccess) return mrg_cuda_check(e, "multigrid CG graph capture");
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // not to be found by the next launch's check
+      return mrg_cuda_check(e, "multigrid CG graph capture");
+    }
     H->graph_A = J;
     H->graph_stream = s;
     H->graph_tail = H->tail;
@@ -1864,21 +1881,23 @@ BgVec<T> bgvec(Hier<T>* H) {
 }
 
 template <typename T>
-void enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
+cudaError_t enqueue_bg_iters(Hier<T>* H, int count, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   const HLevel& L0 = H->L[0];
   BgVec<T> V = bgvec(H);
   const unsigned ge = grid_for(L0.n, 16), gs = grid_for(L0.n, staged_per_sm<T>()), gr = grid_for(L0.n, RED_PER_SM);
   for (int it = 0; it < count; ++it) {
-    launch_level<T>(L0.n, k_bg_p<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
-    enqueue_vcycle(H, H->p, H->ph, true, s);
-    if (L0.pp.p[0] == 2) launch_whole(k_bg_spmv<2, T, 0>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
-    else launch_level<T>(L0.n, k_bg_spmv<1, T, 0>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_level<T>(L0.n, k_bg_s<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
-    enqueue_vcycle(H, H->sv, H->sh, true, s);
-    if (L0.pp.p[0] == 2) launch_whole(k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
-    else launch_level<T>(L0.n, k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
-    launch_level<T>(L0.n, k_bg_update<T>, gr, NT, 0, s, L0.n, V);
+    launch_level<T>(e, L0.n, k_bg_p<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
+    enqueue_vcycle(e, H, H->p, H->ph, true, s);
+    if (L0.pp.p[0] == 2) launch_q2(e, k_bg_spmv<2, T, 0>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    else launch_level<T>(e, L0.n, k_bg_spmv<1, T, 0>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_level<T>(e, L0.n, k_bg_s<T>, ge, NT, 0, s, L0.n, V, first_step(H, 0));
+    enqueue_vcycle(e, H, H->sv, H->sh, true, s);
+    if (L0.pp.p[0] == 2) launch_q2(e, k_bg_spmv<2, T, 1>, ge, NT, 0, s, L0.g, L0.n, (const T*)L0.A, V);
+    else launch_level<T>(e, L0.n, k_bg_spmv<1, T, 1>, gs, NT, staged_smem<T>(), s, L0.g, L0.n, (const T*)L0.A, V);
+    launch_level<T>(e, L0.n, k_bg_update<T>, gr, NT, 0, s, L0.n, V);
   }
+  return e;
 }
 
 template <typename T>
@@ -1909,13 +1928,17 @@ int gmg_bicgstab(mrg_problem* p, Hier<T>* H, const T* J, const double* b, double
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      enqueue_bg_iters(H, GCHUNK, cs);
-      e = cudaStreamEndCapture(cs, &graph);
+      e = enqueue_bg_iters(H, GCHUNK, cs);
+      const cudaError_t ended = cudaStreamEndCapture(cs, &graph);
+      if (e == cudaSuccess) e = ended;
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&H->bgraph, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     cudaStreamDestroy(cs);
-    if (e != cudaSuccess) return mrg_cuda_check(e, "multigrid BiCGStab graph capture");
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // not to be found by the next launch's check
+      return mrg_cuda_check(e, "multigrid BiCGStab graph capture");
+    }
     H->bgraph_A = J;
     H->bgraph_stream = s;
     H->bgraph_tail = H->tail;

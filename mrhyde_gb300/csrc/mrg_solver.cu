@@ -644,7 +644,10 @@ static int chunk_graph(cudaGraphExec_t* exec, const void** key, cudaStream_t* ks
   cudaGraph_t graph;
   MRG_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
   enqueue(p, V, cs);
-  cudaError_t e = cudaStreamEndCapture(cs, &graph);
+  cudaError_t e = cudaGetLastError();  // a refused launch leaves the capture intact, without that kernel
+  const cudaError_t ended = cudaStreamEndCapture(cs, &graph);
+  if (e == cudaSuccess) e = ended;
+  else if (ended == cudaSuccess) cudaGraphDestroy(graph);
   if (own) cudaStreamDestroy(cs);
   if (e != cudaSuccess) return mrg_cuda_check(e, "capture PCG chunk");
   e = cudaGraphInstantiate(exec, graph, 0);
