@@ -37,7 +37,9 @@
  *     workspace); a time-out inside the tensor-core kernel is reported by a later MRG_ASM_TENSOR_CORES
  *     call instead of synchronising.
  *   - Every call returns an mrg_status; no C++ exception crosses the ABI.  mrg_last_error() gives text.
- *   - A handle is thread-compatible (one host thread at a time per handle).
+ *   - A handle is thread-compatible (one host thread at a time per handle).  One exception: calls of mrg_assemble,
+ *     mrg_assemble_residual (without MRG_ASM_TENSOR_CORES) and mrg_spmv may come from several threads, and their work
+ *     may overlap on several streams, as long as no other call changes the handle meanwhile.
  */
 #ifndef MRHYDE_GB300_H
 #define MRHYDE_GB300_H
@@ -153,7 +155,8 @@ int mrg_problem_create(const mrg_mesh_desc* mesh, const mrg_physics_desc* phys, 
    (the serving loop).  mrg_problem_create is this call on the legacy default stream. */
 int mrg_problem_create_on_stream(const mrg_mesh_desc* mesh, const mrg_physics_desc* phys, mrg_stream_t stream,
                                  mrg_problem** out);
-/* Waits for the last stream the handle's work was enqueued on, then frees its memory in stream order. */
+/* Waits for the work that the handle's calls have enqueued, on whatever streams, then frees its memory in stream
+   order.  Graphs that hold captured calls must have ended and not be launched again. */
 int mrg_problem_destroy(mrg_problem* p);
 int mrg_problem_get_info(const mrg_problem* p, mrg_problem_info* info);
 
@@ -326,7 +329,7 @@ int mrg_measure_fma_rates(double* fp64_fma_per_s, double* fp32_fma_per_s, mrg_st
      limit_ns       the limit for this problem's kernels; 0 restores the defaults
      withhold_copy  testing only: nonzero makes the first staged copy of those kernels never be issued, so
                     that its wait runs out (exercises the time-out path without a fault); 0 for normal use
-   Waits for the handle's last stream and drops the problem's captured Krylov chunks and multigrid levels,
+   Waits for the handle's work on every stream and drops the problem's captured Krylov chunks and multigrid levels,
    which are rebuilt on their next use with the new policy. */
 #define MRG_WAIT_LIMIT_MAX_NS 60000000000ull /* 60 s */
 int mrg_set_wait_policy(mrg_problem* p, uint64_t limit_ns, int32_t withhold_copy);

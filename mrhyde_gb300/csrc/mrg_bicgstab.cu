@@ -351,7 +351,7 @@ extern "C" int mrg_solve_bicgstab(mrg_problem* p, const void* J, int32_t fp32, c
   if (!p || !J || !b || !x) return mrg_fail(MRG_EINVAL, "mrg_solve_bicgstab: null argument");
   if (!(rtol >= 0.0) || maxiter < 0) return mrg_fail(MRG_EINVAL, "mrg_solve_bicgstab: bad tolerance or iteration limit");
   cudaStream_t s = (cudaStream_t)stream;
-  p->last_stream = s;
+  const StreamNote note{p, s};
   if (mrg_gmg_kind(p) == MRG_PREC_GMG) {
     // multigrid-preconditioned BiCGStab on the correction: J dx = b - J x, x += dx
     double *res = nullptr, *dx = nullptr;

@@ -435,6 +435,10 @@ extern "C" int mrg_set_face_bc(mrg_problem* p, int32_t face, int32_t kind, const
   BoundaryData* B = reinterpret_cast<BoundaryData*>(p->bnd);
   FaceBC& f = B->f[face];
   cudaStream_t s = p->stream;
+  if (f.d_g) {  // assembly calls in flight read the face's tables
+    const int st = mrg_drain(p);
+    if (st) return st;
+  }
   if (f.d_g) { cudaFreeAsync(f.d_g, s); f.d_g = nullptr; }
   if (f.d_tab) { cudaFreeAsync(f.d_tab, s); f.d_tab = nullptr; }
   if (f.d_ctab) { cudaFreeAsync(f.d_ctab, s); f.d_ctab = nullptr; }

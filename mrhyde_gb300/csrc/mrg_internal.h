@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -125,7 +126,7 @@ struct mrg_problem {
   // Workspaces that one assembly call takes and returns in stream order (mrg_ws_take, mrg_ws_give), so that calls of
   // one handle may overlap on several streams or be captured
   struct WsPool* ws_pool = nullptr;
-  size_t ws_need = 0;            // largest request so far
+  std::atomic<size_t> ws_need{0};  // largest request so far
   void* general = nullptr;       // cell matrices with stored geometry (mrg_general.cu)
   void* nl1 = nullptr;           // 1 + u^2 Q1 hexahedra on identical affine cells (mrg_nonlinear_q1.cu)
   void* box_q2 = nullptr;        // thermal Q2 on identical affine cells (mrg_box_q2.cu)
@@ -133,8 +134,22 @@ struct mrg_problem {
   void* bnd = nullptr;           // face boundary conditions (mrg_boundary.cu)
   void* gmg = nullptr;           // multigrid hierarchy and preconditioner choice (mrg_gmg.cu)
   cudaStream_t stream = nullptr;       // creation stream: the handle's memory is allocated/freed in its order
-  cudaStream_t last_stream = nullptr;  // last stream work was enqueued on (drained before destroy)
+  struct StreamUse* used = nullptr;    // other streams that work was enqueued on (mrg_note_stream)
   SolverWork* work = nullptr;
+};
+
+// Every call that enqueues work on a stream notes it (StreamNote, as the call returns): an event of the handle is recorded
+// on it, unless it is the creation stream or is being captured.  mrg_drain waits for the creation stream and for all those
+// events, so memory that work in flight on any stream may read is not freed; the streams themselves need not exist any
+// more.  Safe from any thread.
+int mrg_streams_open(mrg_problem* p);
+void mrg_streams_close(mrg_problem* p);
+void mrg_note_stream(const mrg_problem* p, cudaStream_t s);
+int mrg_drain(const mrg_problem* p);
+struct StreamNote {
+  const mrg_problem* p;
+  cudaStream_t s;
+  ~StreamNote() { mrg_note_stream(p, s); }
 };
 
 // Layout of d_qtab for the per-cell path: [nq] weights, [npe*nq] phi, [npe*nq*dim] dphi,
@@ -159,8 +174,8 @@ void mrg_q2_free(mrg_problem* p);
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
 // Assembly workspaces come from one pool per device, shared by the handles on it: a new handle finds memory that is
 // mapped already (mapping 40 MB takes longer than most assembly calls).  Whenever a handle is destroyed the pool gives
-// back what exceeds the live handles' largest requests by more than 1 GiB, and everything with the last one.  Safe from any thread and
-// stream: take and give are ordered on the call's stream, and memory in use on one stream is never handed to another.
+// back what exceeds the live handles' largest requests by more than 1 GiB, and everything with the last one.  Safe from any
+// thread and stream: take and give are ordered on the call's stream, and memory in use on one stream is never handed to another.
 int mrg_ws_open(mrg_problem* p);   // at creation, on the current device
 void mrg_ws_close(mrg_problem* p); // after the handle's streams have drained
 cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, void** out);

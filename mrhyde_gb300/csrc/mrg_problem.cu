@@ -7,6 +7,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "mrg_internal.h"
@@ -220,13 +221,12 @@ static inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / 
 // ------------------------------------------------------------------------------------------------
 // create / destroy
 // ------------------------------------------------------------------------------------------------
-// Frees the handle's device memory in stream order on its creation stream, after the last stream the
-// handle's work was enqueued on has drained (no device-wide synchronisation, so concurrent solves on
-// other streams keep running).
+// Frees the handle's device memory in stream order on its creation stream, after the handle's work on every
+// stream has ended (no device-wide synchronisation, so concurrent solves on other streams keep running).
 static void free_problem(mrg_problem* p) {
   if (!p) return;
   cudaStream_t s = p->stream;
-  if (p->last_stream != s) cudaStreamSynchronize(p->last_stream);
+  mrg_drain(p);
   mrg_solver_free(p);
   mrg_bicg_free(p);
   mrg_q2_free(p);
@@ -249,7 +249,95 @@ static void free_problem(mrg_problem* p) {
   cudaFreeAsync(p->d_bload, s);
   cudaStreamSynchronize(s);
   mrg_ws_close(p);
+  mrg_streams_close(p);
   delete p;
+}
+
+// ------------------------------------------------------------------------------------------------
+// streams that a handle's work runs on
+// ------------------------------------------------------------------------------------------------
+struct StreamUse {
+  struct Mark {
+    cudaStream_t s;
+    std::thread::id t;  // cudaStreamPerThread is another stream in every thread
+    cudaEvent_t ev;
+  };
+  std::mutex mu;
+  std::vector<Mark> marks;
+};
+namespace {
+constexpr size_t MARKS = 16;  // from here on a finished mark is used again before another is made
+// Event queries and waits of this thread do not disturb a capture elsewhere.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+bool being_captured(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream while a blocking one is captured: it is not captured itself
+    return false;
+  }
+  return cap != cudaStreamCaptureStatusNone;
+}
+}  // namespace
+
+int mrg_streams_open(mrg_problem* p) {
+  p->used = new StreamUse();
+  return MRG_OK;
+}
+
+void mrg_streams_close(mrg_problem* p) {
+  if (!p->used) return;
+  for (StreamUse::Mark& m : p->used->marks) cudaEventDestroy(m.ev);
+  delete p->used;
+  p->used = nullptr;
+}
+
+void mrg_note_stream(const mrg_problem* p, cudaStream_t s) {
+  const bool per_thread = s == cudaStreamPerThread;
+  if (s == p->stream && !per_thread) return;
+  if (being_captured(s)) return;
+  const std::thread::id t = per_thread ? std::this_thread::get_id() : std::thread::id();
+  std::lock_guard<std::mutex> lk(p->used->mu);
+  std::vector<StreamUse::Mark>& marks = p->used->marks;
+  StreamUse::Mark* at = nullptr;
+  for (StreamUse::Mark& m : marks)
+    if (m.s == s && m.t == t) at = &m;
+  if (!at && marks.size() >= MARKS) {
+    RelaxedCapture relaxed;
+    for (StreamUse::Mark& m : marks)
+      if (!at && cudaEventQuery(m.ev) == cudaSuccess) at = &m;
+    if (!at) cudaGetLastError();
+  }
+  if (!at) {
+    cudaEvent_t ev = nullptr;
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) {
+      marks.push_back({s, t, ev});
+      at = &marks.back();
+    }
+  }
+  if (at) {
+    at->s = s;
+    at->t = t;
+    if (cudaEventRecord(at->ev, s) == cudaSuccess) return;
+  }
+  // no event to be had: the work is waited for now
+  cudaGetLastError();
+  RelaxedCapture relaxed;
+  cudaStreamSynchronize(s);
+}
+
+int mrg_drain(const mrg_problem* p) {
+  RelaxedCapture relaxed;
+  cudaError_t e = cudaStreamSynchronize(p->stream);
+  std::lock_guard<std::mutex> lk(p->used->mu);
+  for (StreamUse::Mark& m : p->used->marks) {
+    const cudaError_t w = cudaEventSynchronize(m.ev);
+    if (e == cudaSuccess) e = w;
+  }
+  return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "waiting for the handle's streams");
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -309,10 +397,13 @@ void mrg_ws_close(mrg_problem* p) {
 }
 
 cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, void** out) {
-  if (bytes > p->ws_need) {
+  if (bytes > p->ws_need.load(std::memory_order_relaxed)) {
     std::lock_guard<std::mutex> lk(g_ws_mu);
-    p->ws_pool->wanted += bytes - p->ws_need;
-    p->ws_need = bytes;
+    const size_t need = p->ws_need;
+    if (bytes > need) {
+      p->ws_pool->wanted += bytes - need;
+      p->ws_need = bytes;
+    }
   }
   return cudaMallocFromPoolAsync(out, bytes, p->ws_pool->pool, s);
 }
@@ -341,7 +432,7 @@ static int create_impl(const mrg_mesh_desc* m, const mrg_physics_desc* ph, cudaS
 
   mrg_problem* P = new mrg_problem();
   P->stream = cs;
-  P->last_stream = cs;
+  mrg_streams_open(P);
   Grid& g = P->g;
   g.dim = m->dim;
   g.p = p;
@@ -627,7 +718,8 @@ extern "C" int mrg_set_wait_policy(mrg_problem* p, uint64_t limit_ns, int32_t wi
     return mrg_fail(MRG_EINVAL, "mrg_set_wait_policy: limit above MRG_WAIT_LIMIT_MAX_NS");
   // captured graphs and multigrid levels hold copies of the grid description: let the work in flight
   // finish, then drop them so that the next solve records the new policy
-  MRG_CUDA(cudaStreamSynchronize(p->last_stream));
+  const int st = mrg_drain(p);
+  if (st) return st;
   p->g.wait_ns = (unsigned long long)limit_ns;
   p->g.withhold = withhold_copy ? 1 : 0;
   mrg_solver_drop_graphs(p);
@@ -651,6 +743,7 @@ extern "C" int mrg_problem_get_info(const mrg_problem* p, mrg_problem_info* info
 
 extern "C" int mrg_get_graph(const mrg_problem* p, int64_t* row_ptr, int32_t* col_idx, mrg_stream_t stream) {
   if (!p || !row_ptr || !col_idx) return mrg_fail(MRG_EINVAL, "mrg_get_graph: null argument");
+  const StreamNote note{p, (cudaStream_t)stream};
   k_graph<<<nblk(p->ndof + 1, 256), 256, 0, (cudaStream_t)stream>>>(p->g, p->ndof, row_ptr, col_idx);
   MRG_CUDA(cudaGetLastError());
   return MRG_OK;
@@ -658,6 +751,7 @@ extern "C" int mrg_get_graph(const mrg_problem* p, int64_t* row_ptr, int32_t* co
 
 extern "C" int mrg_get_dof_map(const mrg_problem* p, int32_t* lids, mrg_stream_t stream) {
   if (!p || !lids) return mrg_fail(MRG_EINVAL, "mrg_get_dof_map: null argument");
+  const StreamNote note{p, (cudaStream_t)stream};
   k_dof_map<<<nblk(p->ncell * p->npe, 256), 256, 0, (cudaStream_t)stream>>>(p->g, p->ncell, p->npe, lids);
   MRG_CUDA(cudaGetLastError());
   return MRG_OK;
@@ -666,6 +760,7 @@ extern "C" int mrg_get_dof_map(const mrg_problem* p, int32_t* lids, mrg_stream_t
 extern "C" int mrg_get_fixed_dofs(const mrg_problem* p, int32_t* dofs, double* values, mrg_stream_t stream) {
   if (!p || !dofs) return mrg_fail(MRG_EINVAL, "mrg_get_fixed_dofs: null argument");
   if (p->nfixed == 0) return MRG_OK;
+  const StreamNote note{p, (cudaStream_t)stream};
   k_copy_fixed<<<nblk(p->nfixed, 256), 256, 0, (cudaStream_t)stream>>>(p->d_fixed, p->d_fixed_vals, p->nfixed, dofs,
                                                                           values);
   MRG_CUDA(cudaGetLastError());
@@ -674,6 +769,7 @@ extern "C" int mrg_get_fixed_dofs(const mrg_problem* p, int32_t* dofs, double* v
 
 extern "C" int mrg_set_kappa(mrg_problem* p, const double* kappa_dev, mrg_stream_t stream) {
   if (!p || !kappa_dev) return mrg_fail(MRG_EINVAL, "mrg_set_kappa: null argument");
+  const StreamNote note{p, (cudaStream_t)stream};
   MRG_CUDA(cudaMemcpyAsync(p->d_kappa, kappa_dev, p->ncell * sizeof(double), cudaMemcpyDeviceToDevice,
                            (cudaStream_t)stream));
   return mrg_launch_kappa32(p, (cudaStream_t)stream);
@@ -682,6 +778,7 @@ extern "C" int mrg_set_kappa(mrg_problem* p, const double* kappa_dev, mrg_stream
 extern "C" int mrg_set_dirichlet(const mrg_problem* p, double* u, mrg_stream_t stream) {
   if (!p || !u) return mrg_fail(MRG_EINVAL, "mrg_set_dirichlet: null argument");
   if (p->nfixed == 0) return MRG_OK;
+  const StreamNote note{p, (cudaStream_t)stream};
   k_set_dirichlet<<<nblk(p->nfixed, 256), 256, 0, (cudaStream_t)stream>>>(p->d_fixed, p->d_fixed_vals, p->nfixed, u);
   MRG_CUDA(cudaGetLastError());
   return MRG_OK;
@@ -699,7 +796,7 @@ extern "C" int mrg_assemble(mrg_problem* p, const double* u, double* r, void* J,
   if (doJ && !J) return mrg_fail(MRG_EINVAL, "mrg_assemble: Jacobian requested but J_vals is null");
   if (doR && !r) return mrg_fail(MRG_EINVAL, "mrg_assemble: residual requested but r is null");
   cudaStream_t s = (cudaStream_t)stream;
-  p->last_stream = s;
+  const StreamNote note{p, s};
   const bool fp32 = flags & MRG_ASM_J_FP32;
   int st = MRG_NO_WORKSPACE;
   if (p->path == MRG_PATH_FACTORED && !(flags & MRG_ASM_FORCE_CELL)) {

@@ -743,6 +743,7 @@ static int pcg32(mrg_problem* p, const float* J, const double* b, double rtol, i
 extern "C" int mrg_spmv(const mrg_problem* p, const void* J, int32_t fp32, const double* x, double* y,
                         mrg_stream_t stream) {
   if (!p || !J || !x || !y) return mrg_fail(MRG_EINVAL, "mrg_spmv: null argument");
+  const StreamNote note{p, (cudaStream_t)stream};
   cudaStream_t s = (cudaStream_t)stream;
   static std::once_flag attr_once;
   static cudaError_t attr_err = cudaSuccess;
@@ -789,7 +790,7 @@ extern "C" int mrg_solve_pcg(mrg_problem* p, const void* J, int32_t fp32, const 
   if (!p || !J || !b || !x) return mrg_fail(MRG_EINVAL, "mrg_solve_pcg: null argument");
   if (!(rtol >= 0.0) || maxiter < 0) return mrg_fail(MRG_EINVAL, "mrg_solve_pcg: bad tolerance or iteration limit");
   cudaStream_t s = (cudaStream_t)stream;
-  p->last_stream = s;
+  const StreamNote note{p, s};
   if (mrg_gmg_kind(p) == MRG_PREC_GMG) {
     // multigrid CG on the correction: dx solves J dx = b - J x0, then x = x0 + dx
     int rc = ensure_work(p, true, false, s);
@@ -849,7 +850,7 @@ extern "C" int mrg_newton(mrg_problem* p, double* u, const mrg_newton_opts* o, m
   if (!p || !u || !o) return mrg_fail(MRG_EINVAL, "mrg_newton: null argument");
   if (o->max_iters < 1 || !(o->nl_tol > 0.0)) return mrg_fail(MRG_EINVAL, "mrg_newton: bad options");
   cudaStream_t s = (cudaStream_t)stream;
-  p->last_stream = s;
+  const StreamNote note{p, s};
   const bool mixed = o->mixed != 0;
   int rc = ensure_work(p, true, mixed, s);
   if (rc) return rc;
@@ -1032,6 +1033,7 @@ extern "C" int mrg_solve_pcg_noalloc(mrg_problem* p, const double* J, const doub
   // the SpMV stages two CSR tiles in more than 48 KB of dynamic shared memory
   MRG_CUDA(cudaFuncSetAttribute(k_pcg64_spmv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, spmv_smem<1, double>()));
   cudaStream_t s = (cudaStream_t)stream;
+  const StreamNote note{p, s};
   PcgVec64 V{x, S->vec[0], S->vec[1], S->vec[2], S->vec[3], S->vec[4], S->parts, b, J, &S->scal};
   k_na_init_scal<<<1, 1, 0, s>>>(&S->scal, rtol, maxiter);
   const unsigned nb = pcg_grid(p);
