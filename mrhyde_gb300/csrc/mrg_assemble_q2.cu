@@ -35,7 +35,7 @@
 
 namespace {
 
-constexpr int CB = 32;       // cells per CTA and per workspace block
+constexpr int CB = MRG_CELL_BLOCK;  // cells per CTA and per workspace block
 constexpr int LINES = 9;     // warps: lines of one direction, pairs (l_x, j_x)
 constexpr int ET = LINES * 32;
 constexpr int ENT = 729;     // entries of an element matrix
@@ -449,17 +449,21 @@ __global__ void __launch_bounds__(QRT) k_q2_row(const Grid g, const __grid_const
 // ------------------------------------------------------------------------------------------------
 struct Q2Data {
   Q2Args A;
-  std::vector<int> slab;            // cell layers at which the slabs begin, and the last one's end
-  std::vector<mrgq2::Kinds> kinds;  // the slabs' rows; kinds.back(): all rows
   std::mutex side_use;              // held by the call that launches on the side stream
   cudaStream_t side = nullptr;      // rows of a slab while the next slab's cells are worked on (several slabs only)
-  std::vector<cudaEvent_t> ev;      // a slab's cells are done; the last: all rows are
+  std::vector<cudaEvent_t> ev;      // MAXSLAB: a slab's cells are done; the last: all rows are
   int* d_err = nullptr;          // tensor-core kernel status (bounded waits), sticky until reported
   int* h_err = nullptr;          // pinned mirror, refreshed asynchronously after every tensor-core launch
   cudaEvent_t err_ev = nullptr;  // recorded after the refresh
   bool err_pending = false;
   Q2Tc* tc = nullptr;            // tensor-core element-matrix plan, built on its first use
 };
+
+// slabs of a piece of the mesh
+static int slabs_of(const mrg_problem* p, int layers) {
+  const int64_t cells = (int64_t)p->g.nc[0] * p->g.nc[1] * layers;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(layers, MAXSLAB), cells / SLAB_CELLS));
+}
 
 static Q2Data* q2data(mrg_problem* p) { return reinterpret_cast<Q2Data*>(p->q2); }
 
@@ -502,20 +506,14 @@ int mrg_q2_setup(mrg_problem* p) {
   const double* src = reinterpret_cast<const double*>(&t);
   float* dst = reinterpret_cast<float*>(&Q->A.t32);
   for (size_t k = 0; k < sizeof(t) / sizeof(double); ++k) dst[k] = (float)src[k];
-  const int nz = p->g.nc[2];
-  const int64_t layer = (int64_t)p->g.nc[0] * p->g.nc[1];
-  const int slabs = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(nz, MAXSLAB), layer * nz / SLAB_CELLS));
-  for (int k = 0; k <= slabs; ++k) Q->slab.push_back((int)((int64_t)nz * k / slabs));
-  if (slabs > 1) {
-    for (int k = 0; k < slabs; ++k) Q->kinds.push_back(mrgq2::make_kinds(p->g, QRT, Q->slab[k], Q->slab[k + 1]));
+  if (slabs_of(p, p->g.nc[2]) > 1) {
     MRG_CUDA(cudaStreamCreateWithFlags(&Q->side, cudaStreamNonBlocking));
-    for (int k = 0; k <= slabs; ++k) {
+    for (int k = 0; k <= MAXSLAB; ++k) {
       cudaEvent_t e = nullptr;
       MRG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       Q->ev.push_back(e);
     }
   }
-  Q->kinds.push_back(mrgq2::make_kinds(p->g, QRT));
   cudaStream_t s = p->stream;
   MRG_CUDA(cudaMallocAsync(&Q->d_err, sizeof(int), s));
   MRG_CUDA(cudaMemsetAsync(Q->d_err, 0, sizeof(int), s));
@@ -536,15 +534,14 @@ void mrg_q2_free(mrg_problem* p) {
 }
 
 template <typename JT, typename CT, int OUT, bool DOR>
-static cudaError_t launch_cell(const Q2Data& Q, const double* u, JT* out, double* rbuf, cudaStream_t s, int64_t b0 = 0,
-                               int64_t b1 = -1) {
+static cudaError_t launch_cell(const Q2Data& Q, const double* u, JT* out, double* rbuf, cudaStream_t s, int64_t b0,
+                               int64_t b1) {
   constexpr int smem = cell_smem<JT, CT, OUT>();
   auto kern = k_q2_cell<JT, CT, OUT, DOR>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   Q2Args A = Q.A;
   A.blk0 = b0;
-  if (b1 < 0) b1 = (Q.A.ncell + CB - 1) / CB;
   if (b1 > b0) kern<<<(unsigned)(b1 - b0), ET, smem, s>>>(A, u, out, rbuf);
   return cudaGetLastError();
 }
@@ -566,9 +563,9 @@ static cudaError_t launch_rows(const mrg_problem* p, const mrgq2::Kinds& K, cons
 // same either way.  The side stream and its events serve one call at a time: a call that finds them taken by another
 // thread's, or that is being captured (its graph would hold on to the stream until the capture ends), goes without.
 template <typename JT, typename CT, bool DOR>
-static cudaError_t launch_slabs(const mrg_problem* p, Q2Data& Q, const double* u, JT* eb, double* rb, double* r, JT* J,
-                                bool ovw, cudaStream_t s) {
-  const int slabs = (int)Q.slab.size() - 1;
+static cudaError_t launch_slabs(const mrg_problem* p, Q2Data& Q, const MrgPiece& q, const double* u, JT* eb, double* rb,
+                                double* r, JT* J, bool ovw, cudaStream_t s) {
+  const int slabs = slabs_of(p, q.b - q.a);
   std::unique_lock<std::mutex> use(Q.side_use, std::defer_lock);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (slabs > 1) {
@@ -576,22 +573,28 @@ static cudaError_t launch_slabs(const mrg_problem* p, Q2Data& Q, const double* u
     if (e != cudaSuccess) return e;
   }
   if (slabs == 1 || cap != cudaStreamCaptureStatusNone || !use.try_lock()) {
-    const cudaError_t e = launch_cell<JT, CT, OUT_MATRIX, DOR>(Q, u, eb, rb, s);
-    return e != cudaSuccess ? e : launch_rows<JT>(p, Q.kinds.back(), eb, rb, r, J, true, DOR, ovw, s);
+    const cudaError_t e = launch_cell<JT, CT, OUT_MATRIX, DOR>(Q, u, eb, rb, s, q.block0, q.block1);
+    const mrgq2::Kinds K = mrgq2::make_kinds(p->g, QRT, q.a, q.b);
+    return e != cudaSuccess ? e : launch_rows<JT>(p, K, eb, rb, r, J, true, DOR, ovw, s);
   }
   const int64_t layer = (int64_t)p->g.nc[0] * p->g.nc[1];
   cudaError_t e = cudaSuccess;
+  int64_t b0 = q.block0;
   for (int k = 0; k < slabs && e == cudaSuccess; ++k) {
+    const int64_t n = q.b - q.a;
+    const int z0 = q.a + (int)(n * k / slabs), z1 = q.a + (int)(n * (k + 1) / slabs);
     // blocks of 32 cells up to the slab's last cell (they may reach into the next layer)
-    const int64_t b0 = (layer * Q.slab[k] + CB - 1) / CB, b1 = (layer * Q.slab[k + 1] + CB - 1) / CB;
-    e = launch_cell<JT, CT, OUT_MATRIX, DOR>(Q, u, eb, rb, s, k ? b0 : 0, b1);
+    const int64_t b1 = (layer * z1 + CB - 1) / CB;
+    e = launch_cell<JT, CT, OUT_MATRIX, DOR>(Q, u, eb, rb, s, b0, b1);
+    b0 = b1;
     if (e == cudaSuccess) e = cudaEventRecord(Q.ev[k], s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(Q.side, Q.ev[k], 0);
-    if (e == cudaSuccess) e = launch_rows<JT>(p, Q.kinds[k], eb, rb, r, J, true, DOR, ovw, Q.side);
+    if (e == cudaSuccess)
+      e = launch_rows<JT>(p, mrgq2::make_kinds(p->g, QRT, z0, z1), eb, rb, r, J, true, DOR, ovw, Q.side);
   }
   // the caller's stream goes on when the rows are written, whatever was launched
-  cudaError_t j = cudaEventRecord(Q.ev[slabs], Q.side);
-  if (j == cudaSuccess) j = cudaStreamWaitEvent(s, Q.ev[slabs], 0);
+  cudaError_t j = cudaEventRecord(Q.ev[MAXSLAB], Q.side);
+  if (j == cudaSuccess) j = cudaStreamWaitEvent(s, Q.ev[MAXSLAB], 0);
   return e != cudaSuccess ? e : j;
 }
 
@@ -623,11 +626,12 @@ static int launch_tensor_cores(mrg_problem* p, const double* u, double* r, float
     MRG_CUDA(cudaEventCreateWithFlags(&Q.err_ev, cudaEventDisableTiming));
   }
   float* w = mrg_q2tc_w_image(Q.tc);
+  const int64_t blocks = (p->ncell + CB - 1) / CB;
   if (rbuf) {
-    MRG_CUDA((launch_cell<float, double, OUT_TF32, true>(Q, u, w, rbuf, s)));
-    MRG_CUDA(launch_rows<float>(p, Q.kinds.back(), nullptr, rbuf, r, nullptr, false, true, ovw, s));
+    MRG_CUDA((launch_cell<float, double, OUT_TF32, true>(Q, u, w, rbuf, s, 0, blocks)));
+    MRG_CUDA(launch_rows<float>(p, mrgq2::make_kinds(p->g, QRT), nullptr, rbuf, r, nullptr, false, true, ovw, s));
   } else {
-    MRG_CUDA((launch_cell<float, float, OUT_TF32, false>(Q, u, w, nullptr, s)));
+    MRG_CUDA((launch_cell<float, float, OUT_TF32, false>(Q, u, w, nullptr, s, 0, blocks)));
   }
   const int st = mrg_q2tc_launch(p, Q.tc, J, ovw, Q.d_err, s);
   if (st) return st;
@@ -644,30 +648,35 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
   const bool doJ = flags & MRG_ASM_JAC, doR = flags & MRG_ASM_RES, ovw = flags & MRG_ASM_OVERWRITE;
   const bool fp32 = (flags & MRG_ASM_J_FP32) && doJ;
   const bool tc = fp32 && (flags & MRG_ASM_TENSOR_CORES) && !(flags & MRG_ASM_CUDA_CORES);
-  const size_t slots = (size_t)((p->ncell + CB - 1) / CB) * CB;
-  const size_t ebytes = doJ && !tc ? slots * ENT * (fp32 ? sizeof(float) : sizeof(double)) : 0;
-  const size_t bytes = ebytes + (doR ? slots * 27 * sizeof(double) : 0);
-  void* ws = nullptr;
-  if (bytes) MRG_TAKE_WS(p, bytes, s, &ws);
-  double* rbuf = doR ? reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + ebytes) : nullptr;
-  int st = MRG_OK;
-  cudaError_t e = cudaSuccess;
-  if (tc) {
-    st = launch_tensor_cores(p, u, r, (float*)J, rbuf, ovw, s);
-  } else if (!doJ) {
-    e = launch_cell<double, double, OUT_NONE, true>(Q, u, nullptr, rbuf, s);
-    if (e == cudaSuccess) e = launch_rows<double>(p, Q.kinds.back(), nullptr, rbuf, r, nullptr, false, true, ovw, s);
-  } else if (fp32) {
-    e = doR ? launch_slabs<float, double, true>(p, Q, u, reinterpret_cast<float*>(ws), rbuf, r, (float*)J, ovw, s)
-            : launch_slabs<float, float, false>(p, Q, u, reinterpret_cast<float*>(ws), nullptr, r, (float*)J, ovw, s);
-  } else {
-    e = doR ? launch_slabs<double, double, true>(p, Q, u, reinterpret_cast<double*>(ws), rbuf, r, (double*)J, ovw, s)
-            : launch_slabs<double, double, false>(p, Q, u, reinterpret_cast<double*>(ws), nullptr, r, (double*)J, ovw, s);
+  const size_t rblock = doR ? (size_t)CB * 27 * sizeof(double) : 0;
+  if (tc) {  // the plan holds all cells' coefficients and matrices, and so does the call
+    void* ws = nullptr;
+    if (doR) {
+      const cudaError_t e = mrg_ws_take(p, (size_t)((p->ncell + CB - 1) / CB) * rblock, s, &ws);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return MRG_NO_WORKSPACE;
+      }
+      MRG_CUDA(e);
+    }
+    const int st = launch_tensor_cores(p, u, r, (float*)J, reinterpret_cast<double*>(ws), ovw, s);
+    if (ws) MRG_CUDA(mrg_ws_give(ws, s));
+    return st;
   }
-  if (ws) {
-    const cudaError_t ef = mrg_ws_give(ws, s);
-    if (e == cudaSuccess) e = ef;
-  }
-  if (st) return st;
-  return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "Q2 assembly launch");
+  const size_t eblock = doJ ? (size_t)CB * ENT * (fp32 ? sizeof(float) : sizeof(double)) : 0;
+  return mrg_in_pieces(p, eblock + rblock, s, [&](const MrgPiece& q) {
+    double* rb = doR ? mrg_piece_array<double>(q.ws + q.blocks * eblock, q, 27 * CB) : nullptr;
+    if (!doJ) {
+      const cudaError_t e = launch_cell<double, double, OUT_NONE, true>(Q, u, nullptr, rb, s, q.block0, q.block1);
+      const mrgq2::Kinds K = mrgq2::make_kinds(p->g, QRT, q.a, q.b);
+      return e != cudaSuccess ? e : launch_rows<double>(p, K, nullptr, rb, r, nullptr, false, true, ovw, s);
+    }
+    float* ef = mrg_piece_array<float>(q.ws, q, ENT * CB);
+    double* ed = mrg_piece_array<double>(q.ws, q, ENT * CB);
+    if (fp32)
+      return doR ? launch_slabs<float, double, true>(p, Q, q, u, ef, rb, r, (float*)J, ovw, s)
+                 : launch_slabs<float, float, false>(p, Q, q, u, ef, nullptr, r, (float*)J, ovw, s);
+    return doR ? launch_slabs<double, double, true>(p, Q, q, u, ed, rb, r, (double*)J, ovw, s)
+               : launch_slabs<double, double, false>(p, Q, q, u, ed, nullptr, r, (double*)J, ovw, s);
+  });
 }

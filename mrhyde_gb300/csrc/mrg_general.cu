@@ -21,7 +21,7 @@
 // Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 241 us (cells 214, FP64
 // pipe 87 % active, rows 27).
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
-// on several streams and may be captured.
+// on several streams and may be captured; a mesh that would need more than MRG_PIECE_BYTES is worked on in pieces.
 #include <cmath>
 #include <type_traits>
 
@@ -31,7 +31,7 @@
 
 namespace {
 
-constexpr int CB = 32;     // cells per workspace block
+constexpr int CB = MRG_CELL_BLOCK;  // cells per workspace block
 constexpr int CT_ = 64;    // cells per CTA (up to 255 registers a thread)
 constexpr int RT = 128;    // rows per CTA of the gather
 
@@ -46,7 +46,7 @@ struct GenArgs {
   const double* bnode;   // node loads
   const double* kap;
   int thermal;
-  int64_t ncell;
+  int64_t c0, c1;        // cells of the launch
 };
 
 __host__ __device__ constexpr int ipow(int b, int e) { return e == 0 ? 1 : b * ipow(b, e - 1); }
@@ -215,8 +215,8 @@ __device__ __forceinline__ void pair3(double aa, double bb, double ab, double v0
 template <typename JT, bool DOJ, bool DOR>
 __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenArgs A, const double* __restrict__ u_,
                                                    JT* __restrict__ ebuf, double* __restrict__ rbuf) {
-  const int64_t c = (int64_t)blockIdx.x * CT_ + threadIdx.x;
-  if (c >= A.ncell) return;
+  const int64_t c = A.c0 + (int64_t)blockIdx.x * CT_ + threadIdx.x;
+  if (c >= A.c1) return;
   const Grid& g = A.g;
   int cx, cy, cz;
   cell_of(g, c, cx, cy, cz);
@@ -383,8 +383,8 @@ template <int P, typename JT, bool DOJ, bool DOR, bool SPLIT>
 __global__ void __launch_bounds__(CT_) k_cell_quad(const __grid_constant__ GenArgs A, const double* __restrict__ u_,
                                                    JT* __restrict__ ebuf, double* __restrict__ rbuf) {
   constexpr int N1 = P + 1, NL = N1 * N1;
-  const int64_t c = (int64_t)blockIdx.x * CT_ + threadIdx.x;
-  if (c >= A.ncell) return;
+  const int64_t c = A.c0 + (int64_t)blockIdx.x * CT_ + threadIdx.x;
+  if (c >= A.c1) return;
   const Grid& g = A.g;
   const GenTab& T = A.t;
   int cx, cy, cz;
@@ -508,15 +508,15 @@ __global__ void __launch_bounds__(CT_) k_cell_quad(const __grid_constant__ GenAr
 // Row lengths of a CTA's 128 rows fit the staged segment; entries are added cell by cell (cz, cy, cx order) at
 // positions computed from the row's extents.
 template <int DIM, int P, typename JT, bool DOJ, bool DOR, bool OVW>
-__global__ void __launch_bounds__(RT) k_gather(const Grid g, int64_t nrows, const JT* __restrict__ ebuf,
+__global__ void __launch_bounds__(RT) k_gather(const Grid g, int64_t row0, int64_t row1, const JT* __restrict__ ebuf,
                                                const double* __restrict__ rbuf, const double* __restrict__ bnode,
                                                double* __restrict__ r, JT* __restrict__ J) {
   constexpr int N1 = P + 1, NL = Gen<DIM, P>::NL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int64_t s_seg[2];
-  const int64_t n0 = (int64_t)blockIdx.x * RT, n = n0 + threadIdx.x;
-  const int64_t nend = n0 + RT < nrows ? n0 + RT : nrows;
-  const bool active = n < nrows;
+  const int64_t n0 = row0 + (int64_t)blockIdx.x * RT, n = n0 + threadIdx.x;
+  const int64_t nend = n0 + RT < row1 ? n0 + RT : row1;
+  const bool active = n < row1;
   int ix = 0, iy = 0, iz = 0;
   mrgdev::RowInfo R{0, 0, 0, 1, 1, 1, 0};
   if (active) {
@@ -624,13 +624,16 @@ int setup_t(mrg_problem* p, General* Q, MetricArgs& M, cudaStream_t s) {
 constexpr int64_t FILL = 32 * 4 * 2 / 3 - 1;  // cells per SM
 
 template <int DIM, int P, typename JT, bool SPLIT>
-cudaError_t launch_t(const mrg_problem* p, const General& Q, const double* u, double* r, JT* J, JT* ebuf, double* rbuf,
-                     bool doJ, bool doR, bool ovw, cudaStream_t s) {
-  const dim3 gc(nblk(p->ncell, CT_), SPLIT && doJ ? P + 1 : 1);
-  const unsigned gr = nblk(p->ndof, RT);
+cudaError_t launch_t(const mrg_problem* p, const General& Q, const MrgPiece& q, const double* u, double* r, JT* J, JT* ebuf,
+                     double* rbuf, bool doJ, bool doR, bool ovw, cudaStream_t s) {
+  const dim3 gc(nblk(q.cell1 - q.cell0, CT_), SPLIT && doJ ? P + 1 : 1);
+  const unsigned gr = nblk(q.row1 - q.row0, RT);
+  GenArgs A = Q.A;
+  A.c0 = q.cell0;
+  A.c1 = q.cell1;
 #define MRG_GEN_CELL(DJ, DR, SP)                                                              \
-  if constexpr (DIM == 3) k_cell_hex1<JT, DJ, DR><<<gc, CT_, 0, s>>>(Q.A, u, ebuf, rbuf);     \
-  else k_cell_quad<P, JT, DJ, DR, SP><<<gc, CT_, 0, s>>>(Q.A, u, ebuf, rbuf)
+  if constexpr (DIM == 3) k_cell_hex1<JT, DJ, DR><<<gc, CT_, 0, s>>>(A, u, ebuf, rbuf);     \
+  else k_cell_quad<P, JT, DJ, DR, SP><<<gc, CT_, 0, s>>>(A, u, ebuf, rbuf)
   if (doJ && doR) { MRG_GEN_CELL(true, true, SPLIT); }
   else if (doJ) { MRG_GEN_CELL(true, false, SPLIT); }
   else { MRG_GEN_CELL(false, true, false); }
@@ -640,7 +643,7 @@ cudaError_t launch_t(const mrg_problem* p, const General& Q, const double* u, do
   const int smem = doJ ? (RT * ipow(2 * P + 1, DIM) + 16 / (int)sizeof(JT)) * (int)sizeof(JT) : 0;
   static_assert((RT * ipow(2 * P + 1, DIM) + 2) * (int)sizeof(JT) <= 48 * 1024, "staged rows fit the default shared memory");
 #define MRG_GEN_ROW(DJ, DR, OV) \
-  k_gather<DIM, P, JT, DJ, DR, OV><<<gr, RT, smem, s>>>(p->g, p->ndof, ebuf, rbuf, Q.d_bnode, r, J)
+  k_gather<DIM, P, JT, DJ, DR, OV><<<gr, RT, smem, s>>>(p->g, q.row0, q.row1, ebuf, rbuf, Q.d_bnode, r, J)
   if (doJ && doR) { if (ovw) MRG_GEN_ROW(true, true, true); else MRG_GEN_ROW(true, true, false); }
   else if (doJ) { if (ovw) MRG_GEN_ROW(true, false, true); else MRG_GEN_ROW(true, false, false); }
   else { if (ovw) MRG_GEN_ROW(false, true, true); else MRG_GEN_ROW(false, true, false); }
@@ -696,7 +699,6 @@ int mrg_general_setup(mrg_problem* p, cudaStream_t s) {
   Q->A.bnode = Q->d_bnode;
   Q->A.kap = p->d_kappa;
   Q->A.thermal = p->kind == MRG_THERMAL;
-  Q->A.ncell = p->ncell;
   return mrg_ws_open(p);
 }
 
@@ -713,26 +715,21 @@ int mrg_launch_general(mrg_problem* p, const double* u, double* r, void* J, uint
   const General& Q = *reinterpret_cast<General*>(p->general);
   const bool doJ = flags & MRG_ASM_JAC, doR = flags & MRG_ASM_RES, ovw = flags & MRG_ASM_OVERWRITE;
   const bool fp32 = flags & MRG_ASM_J_FP32;
-  const size_t cells = (size_t)((p->ncell + CB - 1) / CB) * CB;
-  const size_t ebytes = doJ ? cells * p->npe * p->npe * (fp32 ? sizeof(float) : sizeof(double)) : 0;
-  void* ws = nullptr;
-  MRG_TAKE_WS(p, ebytes + (doR ? cells * p->npe * sizeof(double) : 0), s, &ws);
-  double* rbuf = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + ebytes);
-  cudaError_t e;
-  auto go = [&](auto* Jt) {
-    using JT = std::remove_pointer_t<decltype(Jt)>;
-    JT* eb = reinterpret_cast<JT*>(ws);
-    if (p->g.dim == 3) return launch_t<3, 1, JT, false>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
-    const bool split = p->ncell < FILL * mrg_device_sms();
-    if (p->g.p == 1)
-      return split ? launch_t<2, 1, JT, true>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s)
-                   : launch_t<2, 1, JT, false>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
-    return split ? launch_t<2, 2, JT, true>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s)
-                 : launch_t<2, 2, JT, false>(p, Q, u, r, Jt, eb, rbuf, doJ, doR, ovw, s);
-  };
-  if (fp32) e = go(reinterpret_cast<float*>(J));
-  else e = go(reinterpret_cast<double*>(J));
-  const cudaError_t ef = mrg_ws_give(ws, s);
-  if (e == cudaSuccess) e = ef;
-  return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "general assembly launch");
+  const size_t ent = (size_t)CB * p->npe * p->npe, eblock = doJ ? ent * (fp32 ? sizeof(float) : sizeof(double)) : 0;
+  const size_t rblock = doR ? (size_t)CB * p->npe * sizeof(double) : 0;
+  return mrg_in_pieces(p, eblock + rblock, s, [&](const MrgPiece& q) {
+    double* rb = mrg_piece_array<double>(q.ws + q.blocks * eblock, q, (size_t)CB * p->npe);
+    auto go = [&](auto* Jt) {
+      using JT = std::remove_pointer_t<decltype(Jt)>;
+      JT* eb = mrg_piece_array<JT>(q.ws, q, ent);
+      if (p->g.dim == 3) return launch_t<3, 1, JT, false>(p, Q, q, u, r, Jt, eb, rb, doJ, doR, ovw, s);
+      const bool split = p->ncell < FILL * mrg_device_sms();
+      if (p->g.p == 1)
+        return split ? launch_t<2, 1, JT, true>(p, Q, q, u, r, Jt, eb, rb, doJ, doR, ovw, s)
+                     : launch_t<2, 1, JT, false>(p, Q, q, u, r, Jt, eb, rb, doJ, doR, ovw, s);
+      return split ? launch_t<2, 2, JT, true>(p, Q, q, u, r, Jt, eb, rb, doJ, doR, ovw, s)
+                   : launch_t<2, 2, JT, false>(p, Q, q, u, r, Jt, eb, rb, doJ, doR, ovw, s);
+    };
+    return fp32 ? go(reinterpret_cast<float*>(J)) : go(reinterpret_cast<double*>(J));
+  });
 }

@@ -183,15 +183,69 @@ cudaError_t mrg_ws_give(void* ws, cudaStream_t s);
 // A launcher's return when there is no memory for its workspace; nothing has been launched then, and the call takes the
 // per-cell kernels, which need none: a mesh whose matrix nearly fills the device is assembled all the same.
 constexpr int MRG_NO_WORKSPACE = -1;
-#define MRG_TAKE_WS(p, bytes, s, out)                                       \
-  do {                                                                      \
-    const cudaError_t e__ = mrg_ws_take(p, bytes, s, out);                  \
-    if (e__ == cudaErrorMemoryAllocation) {                                 \
-      cudaGetLastError(); /* not to be found by the next launch's check */  \
-      return MRG_NO_WORKSPACE;                                              \
-    }                                                                       \
-    if (e__ != cudaSuccess) return mrg_cuda_check(e__, "workspace");        \
-  } while (0)
+
+// Assembly in pieces of cell layers (along z, in 2-D along y), one after the other in one workspace: the cells' numbers or
+// matrices are kept for a piece of the mesh, not for all of it.  A piece holds the rows of the node layers that begin with
+// cell layers a .. b - 1 (with the last node layer when b is the last cell layer) and so the cells of layers a - 1 .. b - 1,
+// rounded down and up to blocks of 32 cells: one layer is worked on twice at each seam, with the same bits.
+constexpr int MRG_CELL_BLOCK = 32;
+constexpr size_t MRG_PIECE_BYTES = (size_t)4 << 30;  // 12 pieces on 128 x 128 x 512 Q2 cells in FP64: 2 % worked on twice
+struct MrgPiece {
+  int a, b;                // cell layers
+  int64_t block0, block1;  // blocks of cells
+  int64_t cell0, cell1;    // and the cells they hold
+  int64_t row0, row1;
+  unsigned char* ws;
+  size_t blocks;           // room in the workspace
+};
+template <typename F>
+int mrg_in_pieces(mrg_problem* p, size_t block_bytes, cudaStream_t s, F&& work) {
+  const int ax = p->g.dim - 1, layers = p->g.nc[ax];
+  const int64_t cells = p->ncell / layers, nodes = p->ndof / p->g.nn[ax];
+  auto blocks_of = [&](int per) -> size_t {
+    return per >= layers ? (size_t)((p->ncell + MRG_CELL_BLOCK - 1) / MRG_CELL_BLOCK)
+                         : (size_t)((per + 1) * cells / MRG_CELL_BLOCK + 2);
+  };
+  int per = layers;
+  if (blocks_of(per) * block_bytes > MRG_PIECE_BYTES) {
+    const int64_t fit = (int64_t)(MRG_PIECE_BYTES / block_bytes) * MRG_CELL_BLOCK / cells - 1;
+    per = fit < 1 ? 1 : (fit < layers ? (int)fit : layers);
+    const int n = (layers + per - 1) / per;
+    per = (layers + n - 1) / n;
+  }
+  void* ws = nullptr;
+  for (;;) {
+    const cudaError_t e = mrg_ws_take(p, blocks_of(per) * block_bytes, s, &ws);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation) return mrg_cuda_check(e, "workspace");
+    cudaGetLastError();  // not to be found by the next launch's check
+    if (per == 1) return MRG_NO_WORKSPACE;
+    per = (per + 1) / 2;
+  }
+  cudaError_t e = cudaSuccess;
+  for (int a = 0; a < layers && e == cudaSuccess; a += per) {
+    MrgPiece q;
+    q.a = a;
+    q.b = a + per < layers ? a + per : layers;
+    q.block0 = (a > 0 ? a - 1 : 0) * cells / MRG_CELL_BLOCK;
+    q.block1 = (q.b * cells + MRG_CELL_BLOCK - 1) / MRG_CELL_BLOCK;
+    q.cell0 = q.block0 * MRG_CELL_BLOCK;
+    q.cell1 = q.block1 * MRG_CELL_BLOCK < p->ncell ? q.block1 * MRG_CELL_BLOCK : p->ncell;
+    q.row0 = (int64_t)p->g.p * q.a * nodes;
+    q.row1 = q.b == layers ? p->ndof : (int64_t)p->g.p * q.b * nodes;
+    q.ws = static_cast<unsigned char*>(ws);
+    q.blocks = blocks_of(per);
+    e = work(q);
+  }
+  const cudaError_t ef = mrg_ws_give(ws, s);
+  if (e == cudaSuccess) e = ef;
+  return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "assembly launch");
+}
+// An array with `per_block` elements a block that holds a piece's blocks, to be indexed by the mesh's blocks
+template <typename T>
+T* mrg_piece_array(void* at, const MrgPiece& q, size_t per_block) {
+  return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(at) - (uintptr_t)q.block0 * per_block * sizeof(T));
+}
 // Cell matrices with stored geometry: the forms and shapes without a path of their own (mrg_general.cu)
 bool mrg_general_eligible(const mrg_problem* p, int points_per_axis);
 int mrg_general_setup(mrg_problem* p, cudaStream_t s);

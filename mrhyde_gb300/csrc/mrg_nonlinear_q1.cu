@@ -22,7 +22,7 @@
 // active; the row-by-row contraction took 2712 and eight coloured residual launches 780); FP32 Jacobian alone on
 // 96^3 cells 865 -> about 40 us.
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
-// on several streams and may be captured.
+// on several streams and may be captured; a mesh that would need more than MRG_PIECE_BYTES is worked on in pieces.
 #include <cmath>
 
 #include "mrg_device.cuh"
@@ -34,7 +34,7 @@ namespace {
 constexpr int CT_ = 128;  // cells per CTA
 constexpr int RT = 128;   // rows per CTA
 constexpr int NZ_ = 54;   // numbers per cell
-constexpr int CB = 32;    // cells per workspace block
+constexpr int CB = MRG_CELL_BLOCK;  // cells per workspace block
 
 // products and sums that must not be contracted differently from one instance to the next (the residual of the
 // separate and of the fused call has the same bits)
@@ -59,7 +59,7 @@ struct Nl1Args {
   float betaf, slopef, wf[3];
   double m[3], m02;  // L L at the Gauss point near node 0 for the pairs 00, 01, 11; m[0] + m[2]
   float m32[3][2];   // m in FP32: value and what it lacks
-  int64_t ncell;
+  int64_t c0, c1;    // cells of the launch
 };
 
 template <typename T>
@@ -107,8 +107,8 @@ __device__ __forceinline__ void pair3(const Nl1Args& A, float v0, float v1, floa
 template <typename JT, typename CT, bool DOJ, bool DOR>
 __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Args A, const double* __restrict__ u_,
                                                   JT* __restrict__ zbuf, double* __restrict__ rbuf) {
-  const int64_t cl = (int64_t)blockIdx.x * CT_ + threadIdx.x;
-  if (cl >= A.ncell) return;
+  const int64_t cl = A.c0 + (int64_t)blockIdx.x * CT_ + threadIdx.x;
+  if (cl >= A.c1) return;
   const Grid& g = A.g;
   const unsigned c32 = (unsigned)cl, t = c32 / (unsigned)g.nc[0];  // n_cells < n_dofs <= INT32_MAX
   const int cx = (int)(c32 - t * (unsigned)g.nc[0]), cz = (int)(t / (unsigned)g.nc[1]);
@@ -221,13 +221,13 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
 // FP64: 4 CTAs per SM (128 registers): 27 accumulators and a cell's 24 loads in flight; FP32 needs 80 registers
 template <typename JT, bool DOJ, bool DOR, bool OVW>
 __global__ void __launch_bounds__(RT, !DOJ ? 8 : (sizeof(JT) == 4 ? 6 : 4))
-    k_nl1_row(const Grid g, int64_t nrows, const JT* __restrict__ zbuf, const double* __restrict__ rbuf,
+    k_nl1_row(const Grid g, int64_t row0, int64_t row1, const JT* __restrict__ zbuf, const double* __restrict__ rbuf,
               double* __restrict__ r, JT* __restrict__ J) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int64_t s_seg[2];
-  const int64_t n0 = (int64_t)blockIdx.x * RT, n = n0 + threadIdx.x;
-  const int64_t nend = n0 + RT < nrows ? n0 + RT : nrows;
-  const bool active = n < nrows;
+  const int64_t n0 = row0 + (int64_t)blockIdx.x * RT, n = n0 + threadIdx.x;
+  const int64_t nend = n0 + RT < row1 ? n0 + RT : row1;
+  const bool active = n < row1;
   const int NX = g.nn[0], NY = g.nn[1], NZ = g.nn[2];
   int ix = 0, iy = 0, iz = 0, cx = 1, cy = 1, cz = 1;
   int64_t row = 0;
@@ -328,16 +328,16 @@ struct Nl1 {
 };
 
 template <typename JT>
-cudaError_t launch(const mrg_problem* p, const Nl1Args& A, const double* u, double* r, JT* J, JT* z, double* rb, bool doJ,
-                   bool doR, bool ovw, cudaStream_t s) {
-  const unsigned gc = nblk(p->ncell, CT_), gr = nblk(p->ndof, RT);
+cudaError_t launch(const mrg_problem* p, const Nl1Args& A, const MrgPiece& q, const double* u, double* r, JT* J, JT* z,
+                   double* rb, bool doJ, bool doR, bool ovw, cudaStream_t s) {
+  const unsigned gc = nblk(q.cell1 - q.cell0, CT_), gr = nblk(q.row1 - q.row0, RT);
   if (doJ && doR) k_nl1_cell<JT, double, true, true><<<gc, CT_, 0, s>>>(A, u, z, rb);
   else if (doJ) k_nl1_cell<JT, JT, true, false><<<gc, CT_, 0, s>>>(A, u, z, rb);
   else k_nl1_cell<double, double, false, true><<<gc, CT_, 0, s>>>(A, u, nullptr, rb);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int smem = doJ ? (RT * 27 + 16 / (int)sizeof(JT)) * (int)sizeof(JT) : 0;
-#define MRG_NL1_ROW(DJ, DR, OV) k_nl1_row<JT, DJ, DR, OV><<<gr, RT, smem, s>>>(p->g, p->ndof, z, rb, r, J)
+#define MRG_NL1_ROW(DJ, DR, OV) k_nl1_row<JT, DJ, DR, OV><<<gr, RT, smem, s>>>(p->g, q.row0, q.row1, z, rb, r, J)
   if (doJ && doR) { if (ovw) MRG_NL1_ROW(true, true, true); else MRG_NL1_ROW(true, true, false); }
   else if (doJ) { if (ovw) MRG_NL1_ROW(true, false, true); else MRG_NL1_ROW(true, false, false); }
   else { if (ovw) MRG_NL1_ROW(false, true, true); else MRG_NL1_ROW(false, true, false); }
@@ -352,7 +352,6 @@ int mrg_nl1_setup(mrg_problem* p) {
   p->nl1 = Q;
   Nl1Args& A = Q->A;
   A.g = p->g;
-  A.ncell = p->ncell;
   double l[2], dl[2];
   mrg_lagrange_1d(1, p->gx1[0], l, dl);
   A.beta = l[1];
@@ -386,14 +385,15 @@ int mrg_launch_nl1(mrg_problem* p, const double* u, double* r, void* J, uint32_t
   const Nl1Args& A = reinterpret_cast<Nl1*>(p->nl1)->A;
   const bool doJ = flags & MRG_ASM_JAC, doR = flags & MRG_ASM_RES, ovw = flags & MRG_ASM_OVERWRITE;
   const bool fp32 = flags & MRG_ASM_J_FP32;
-  const size_t cells = (size_t)((p->ncell + CB - 1) / CB) * CB;
-  const size_t zbytes = doJ ? cells * NZ_ * (fp32 ? sizeof(float) : sizeof(double)) : 0;
-  void* ws = nullptr;
-  MRG_TAKE_WS(p, zbytes + (doR ? cells * 8 * sizeof(double) : 0), s, &ws);
-  double* rb = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ws) + zbytes);
-  cudaError_t e = fp32 && doJ ? launch<float>(p, A, u, r, (float*)J, (float*)ws, rb, doJ, doR, ovw, s)
-                              : launch<double>(p, A, u, r, (double*)J, (double*)ws, rb, doJ, doR, ovw, s);
-  const cudaError_t ef = mrg_ws_give(ws, s);
-  if (e == cudaSuccess) e = ef;
-  return e == cudaSuccess ? MRG_OK : mrg_cuda_check(e, "nonlinear Q1 assembly launch");
+  const size_t zblock = doJ ? (size_t)CB * NZ_ * (fp32 ? sizeof(float) : sizeof(double)) : 0;
+  const size_t rblock = doR ? (size_t)CB * 8 * sizeof(double) : 0;
+  return mrg_in_pieces(p, zblock + rblock, s, [&](const MrgPiece& q) {
+    Nl1Args Q = A;
+    Q.c0 = q.cell0;
+    Q.c1 = q.cell1;
+    double* rb = mrg_piece_array<double>(q.ws + q.blocks * zblock, q, 8 * CB);
+    return fp32 && doJ
+               ? launch<float>(p, Q, q, u, r, (float*)J, mrg_piece_array<float>(q.ws, q, NZ_ * CB), rb, doJ, doR, ovw, s)
+               : launch<double>(p, Q, q, u, r, (double*)J, mrg_piece_array<double>(q.ws, q, NZ_ * CB), rb, doJ, doR, ovw, s);
+  });
 }
