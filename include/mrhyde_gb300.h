@@ -36,6 +36,11 @@
  *     in a CUDA graph (with MRG_ASM_TENSOR_CORES once a first call has created the tensor-core
  *     workspace); a time-out inside the tensor-core kernel is reported by a later MRG_ASM_TENSOR_CORES
  *     call instead of synchronising.
+ *   - The 1 + u^2 forms and the thermal Q2 quadrilaterals of general shape take device memory for the duration of
+ *     each assembly call, at most 4 GiB (more only where two layers of cells need more), from a pool of the library;
+ *     without memory the per-cell kernels, which need none, do the work.  A captured call's graph holds kernels only:
+ *     its workspace is allocated at the capture and given back after the graph and its executable copies are
+ *     destroyed; the copies share it, so one runs at a time.
  *   - Every call returns an mrg_status; no C++ exception crosses the ABI.  mrg_last_error() gives text.
  *   - A handle is thread-compatible (one host thread at a time per handle).  One exception: calls of mrg_assemble,
  *     mrg_assemble_residual (without MRG_ASM_TENSOR_CORES) and mrg_spmv may come from several threads, and their work

@@ -650,7 +650,7 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
   const bool tc = fp32 && (flags & MRG_ASM_TENSOR_CORES) && !(flags & MRG_ASM_CUDA_CORES);
   const size_t rblock = doR ? (size_t)CB * 27 * sizeof(double) : 0;
   if (tc) {  // the plan holds all cells' coefficients and matrices, and so does the call
-    void* ws = nullptr;
+    MrgWs ws;
     if (doR) {
       const cudaError_t e = mrg_ws_take(p, (size_t)((p->ncell + CB - 1) / CB) * rblock, s, &ws);
       if (e == cudaErrorMemoryAllocation) {
@@ -659,8 +659,8 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
       }
       MRG_CUDA(e);
     }
-    const int st = launch_tensor_cores(p, u, r, (float*)J, reinterpret_cast<double*>(ws), ovw, s);
-    if (ws) MRG_CUDA(mrg_ws_give(ws, s));
+    const int st = launch_tensor_cores(p, u, r, (float*)J, reinterpret_cast<double*>(ws.p), ovw, s);
+    if (ws.p) MRG_CUDA(mrg_ws_give(ws, s));
     return st;
   }
   const size_t eblock = doJ ? (size_t)CB * ENT * (fp32 ? sizeof(float) : sizeof(double)) : 0;

@@ -178,8 +178,15 @@ int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t 
 // thread and stream: take and give are ordered on the call's stream, and memory in use on one stream is never handed to another.
 int mrg_ws_open(mrg_problem* p);   // at creation, on the current device
 void mrg_ws_close(mrg_problem* p); // after the handle's streams have drained
-cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, void** out);
-cudaError_t mrg_ws_give(void* ws, cudaStream_t s);
+// In a capture the workspace belongs to the graph: it is allocated outside the capture, so that the graph holds kernels
+// only (a graph with allocation nodes can have one executable copy and no place in another graph), shared by the calls
+// captured on one stream, which run one after the other, and given back when the graph and its copies are gone.
+struct MrgWs {
+  void* p = nullptr;
+  bool of_graph = false;
+};
+cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, MrgWs* out);
+cudaError_t mrg_ws_give(const MrgWs& ws, cudaStream_t s);
 // A launcher's return when there is no memory for its workspace; nothing has been launched then, and the call takes the
 // per-cell kernels, which need none: a mesh whose matrix nearly fills the device is assembled all the same.
 constexpr int MRG_NO_WORKSPACE = -1;
@@ -213,7 +220,7 @@ int mrg_in_pieces(mrg_problem* p, size_t block_bytes, cudaStream_t s, F&& work) 
     const int n = (layers + per - 1) / per;
     per = (layers + n - 1) / n;
   }
-  void* ws = nullptr;
+  MrgWs ws;
   for (;;) {
     const cudaError_t e = mrg_ws_take(p, blocks_of(per) * block_bytes, s, &ws);
     if (e == cudaSuccess) break;
@@ -233,7 +240,7 @@ int mrg_in_pieces(mrg_problem* p, size_t block_bytes, cudaStream_t s, F&& work) 
     q.cell1 = q.block1 * MRG_CELL_BLOCK < p->ncell ? q.block1 * MRG_CELL_BLOCK : p->ncell;
     q.row0 = (int64_t)p->g.p * q.a * nodes;
     q.row1 = q.b == layers ? p->ndof : (int64_t)p->g.p * q.b * nodes;
-    q.ws = static_cast<unsigned char*>(ws);
+    q.ws = static_cast<unsigned char*>(ws.p);
     q.blocks = blocks_of(per);
     e = work(q);
   }

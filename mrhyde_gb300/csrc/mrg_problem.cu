@@ -345,14 +345,84 @@ int mrg_drain(const mrg_problem* p) {
 // ------------------------------------------------------------------------------------------------
 struct WsPool {
   cudaMemPool_t pool = nullptr;
+  cudaStream_t own = nullptr;  // graphs' workspaces are taken and given back in its order
   size_t wanted = 0;  // sum of the live handles' largest requests
   int users = 0;      // live handles
+  // the workspaces taken last in captures, by capture (its number is never used again) and stream
+  struct Captured {
+    unsigned long long id;
+    cudaStream_t s;
+    void* p;
+    size_t bytes;
+  };
+  std::vector<Captured> captured;
 };
+constexpr size_t WS_CAPTURED = 16;
 constexpr size_t WS_SLACK = (size_t)1 << 30;
 constexpr uint64_t WS_KEEP = 8ull << 30;
 namespace {
 std::mutex g_ws_mu;
 WsPool g_ws[SM_CACHE];  // by device ordinal
+
+// Workspaces whose graph is gone.  The runtime says so in a callback that may not call it, so they wait here for the next
+// call on the device.
+struct GraphWs {
+  void* p;
+  WsPool* w;
+};
+std::mutex g_gone_mu;
+std::vector<GraphWs>& g_gone = *new std::vector<GraphWs>();  // callbacks may come after the statics' destructors
+std::atomic<bool> g_any_gone{false};
+void CUDART_CB graph_ws_gone(void* arg) {
+  GraphWs* g = static_cast<GraphWs*>(arg);
+  std::lock_guard<std::mutex> lk(g_gone_mu);
+  g_gone.push_back(*g);
+  g_any_gone.store(true, std::memory_order_release);
+  delete g;
+}
+void collect_graph_ws(WsPool& w) {
+  if (!g_any_gone.load(std::memory_order_acquire)) return;
+  std::lock_guard<std::mutex> lk(g_gone_mu);
+  RelaxedCapture relaxed;  // the caller may be capturing
+  size_t kept = 0;
+  for (const GraphWs& g : g_gone)
+    if (g.w == &w) cudaFreeAsync(g.p, w.own);
+    else g_gone[kept++] = g;
+  g_gone.resize(kept);
+  g_any_gone.store(kept > 0, std::memory_order_release);
+}
+
+cudaError_t take_for_graph(WsPool& w, size_t bytes, cudaStream_t s, unsigned long long id, cudaGraph_t graph, MrgWs* out) {
+  out->of_graph = true;
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  for (const WsPool::Captured& c : w.captured)
+    if (c.id == id && c.s == s && c.bytes >= bytes) {
+      out->p = c.p;
+      return cudaSuccess;
+    }
+  RelaxedCapture relaxed;
+  void* ptr = nullptr;
+  cudaError_t e = cudaMallocFromPoolAsync(&ptr, bytes, w.pool, w.own);
+  if (e != cudaSuccess) return e;
+  e = cudaStreamSynchronize(w.own);
+  GraphWs* g = new GraphWs{ptr, &w};
+  cudaUserObject_t obj = nullptr;
+  if (e == cudaSuccess) e = cudaUserObjectCreate(&obj, g, graph_ws_gone, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    delete g;
+    cudaFreeAsync(ptr, w.own);
+    return e;
+  }
+  e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(obj, 1);  // hands the memory to graph_ws_gone
+    return e;
+  }
+  if (w.captured.size() >= WS_CAPTURED) w.captured.erase(w.captured.begin());
+  w.captured.push_back({id, s, ptr, bytes});
+  out->p = ptr;
+  return cudaSuccess;
+}
 }  // namespace
 
 int mrg_ws_open(mrg_problem* p) {
@@ -379,6 +449,11 @@ int mrg_ws_open(mrg_problem* p) {
       cudaMemPoolDestroy(pool);
       return mrg_cuda_check(e, "workspace pool");
     }
+    e = cudaStreamCreateWithFlags(&w.own, cudaStreamNonBlocking);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return mrg_cuda_check(e, "workspace pool's stream");
+    }
     w.pool = pool;
   }
   ++w.users;
@@ -392,23 +467,40 @@ void mrg_ws_close(mrg_problem* p) {
   WsPool& w = *p->ws_pool;
   w.wanted -= p->ws_need;
   --w.users;
+  collect_graph_ws(w);
+  if (!w.users) {
+    RelaxedCapture relaxed;
+    cudaStreamSynchronize(w.own);
+  }
   cudaMemPoolTrimTo(w.pool, w.users ? w.wanted + WS_SLACK : 0);
   p->ws_pool = nullptr;
 }
 
-cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, void** out) {
+cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, MrgWs* out) {
+  WsPool& w = *p->ws_pool;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(s, &cap, &id, &graph) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream while a blocking one is captured: it is not captured itself
+    cap = cudaStreamCaptureStatusNone;
+  }
+  if (cap == cudaStreamCaptureStatusInvalidated) return cudaErrorStreamCaptureInvalidated;
+  collect_graph_ws(w);
+  if (cap == cudaStreamCaptureStatusActive) return take_for_graph(w, bytes, s, id, graph, out);
   if (bytes > p->ws_need.load(std::memory_order_relaxed)) {
     std::lock_guard<std::mutex> lk(g_ws_mu);
     const size_t need = p->ws_need;
     if (bytes > need) {
-      p->ws_pool->wanted += bytes - need;
+      w.wanted += bytes - need;
       p->ws_need = bytes;
     }
   }
-  return cudaMallocFromPoolAsync(out, bytes, p->ws_pool->pool, s);
+  out->of_graph = false;
+  return cudaMallocFromPoolAsync(&out->p, bytes, w.pool, s);
 }
 
-cudaError_t mrg_ws_give(void* ws, cudaStream_t s) { return cudaFreeAsync(ws, s); }
+cudaError_t mrg_ws_give(const MrgWs& ws, cudaStream_t s) { return ws.of_graph ? cudaSuccess : cudaFreeAsync(ws.p, s); }
 
 static int create_impl(const mrg_mesh_desc* m, const mrg_physics_desc* ph, cudaStream_t cs, mrg_problem** out) {
   if (!m || !ph || !out) return mrg_fail(MRG_EINVAL, "mrg_problem_create: null argument");
