@@ -38,7 +38,8 @@
  *     call instead of synchronising.
  *   - The 1 + u^2 forms and the thermal Q2 quadrilaterals of general shape take device memory for the duration of
  *     each assembly call, at most 4 GiB (more only where two layers of cells need more), from a pool of the library;
- *     without memory the per-cell kernels, which need none, do the work.  A captured call's graph holds kernels only:
+ *     without memory the per-cell kernels, which need none, do the work.  Between calls the pool keeps what the
+ *     live handles have asked for and 1 GiB, at most 8 GiB in all, and nothing after the last handle.  A captured call's graph holds kernels only:
  *     its workspace is allocated at the capture and given back after the graph and its executable copies are
  *     destroyed; the copies share it, so one runs at a time.
  *   - Every call returns an mrg_status; no C++ exception crosses the ABI.  mrg_last_error() gives text.

@@ -173,9 +173,10 @@ int mrg_q2_setup(mrg_problem* p);
 void mrg_q2_free(mrg_problem* p);
 int mrg_launch_q2(mrg_problem* p, const double* u, double* r, void* J, uint32_t flags, cudaStream_t s);
 // Assembly workspaces come from one pool per device, shared by the handles on it: a new handle finds memory that is
-// mapped already (mapping 40 MB takes longer than most assembly calls).  Whenever a handle is destroyed the pool gives
-// back what exceeds the live handles' largest requests by more than 1 GiB, and everything with the last one.  Safe from any
-// thread and stream: take and give are ordered on the call's stream, and memory in use on one stream is never handed to another.
+// mapped already (mapping 40 MB takes longer than most assembly calls).  Over synchronisations the pool keeps the live
+// handles' largest requests and 1 GiB, at most 8 GiB, and nothing once the last handle is destroyed.  Safe from any
+// thread and stream: take and give are ordered on the call's stream, and memory in use on one stream is never handed to
+// another.
 int mrg_ws_open(mrg_problem* p);   // at creation, on the current device
 void mrg_ws_close(mrg_problem* p); // after the handle's streams have drained
 // In a capture the workspace belongs to the graph: it is allocated outside the capture, so that the graph holds kernels

@@ -358,6 +358,8 @@ struct WsPool {
   std::vector<Captured> captured;
 };
 constexpr size_t WS_CAPTURED = 16;
+// What the pool keeps over synchronisations: the live handles' largest requests, each taken by one call at a time, and a
+// little for calls that overlap; at most WS_KEEP.  Calls that need more map their memory anew.
 constexpr size_t WS_SLACK = (size_t)1 << 30;
 constexpr uint64_t WS_KEEP = 8ull << 30;
 namespace {
@@ -425,6 +427,12 @@ cudaError_t take_for_graph(WsPool& w, size_t bytes, cudaStream_t s, unsigned lon
 }
 }  // namespace
 
+static cudaError_t keep_wanted(cudaMemPool_t pool, size_t wanted) {
+  RelaxedCapture relaxed;
+  uint64_t keep = std::min<uint64_t>(WS_KEEP, wanted + WS_SLACK);
+  return cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
 int mrg_ws_open(mrg_problem* p) {
   int dev = 0;
   MRG_CUDA(cudaGetDevice(&dev));
@@ -438,13 +446,9 @@ int mrg_ws_open(mrg_problem* p) {
     props.location.id = dev;
     cudaMemPool_t pool = nullptr;
     MRG_CUDA(cudaMemPoolCreate(&pool, &props));
-    // keep up to WS_KEEP over synchronisations (less when a handle goes): beyond that a call takes tens of milliseconds
-    // and can afford to map its memory, which the caller may want back; never make one stream wait for another to reuse
-    // its memory
-    uint64_t keep = WS_KEEP;
-    int no = 0;
-    cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no);
+    int no = 0;  // never make one stream wait for another to reuse its memory
+    cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no);
+    if (e == cudaSuccess) e = keep_wanted(pool, 0);
     if (e != cudaSuccess) {
       cudaMemPoolDestroy(pool);
       return mrg_cuda_check(e, "workspace pool");
@@ -472,7 +476,8 @@ void mrg_ws_close(mrg_problem* p) {
     RelaxedCapture relaxed;
     cudaStreamSynchronize(w.own);
   }
-  cudaMemPoolTrimTo(w.pool, w.users ? w.wanted + WS_SLACK : 0);
+  keep_wanted(w.pool, w.wanted);
+  cudaMemPoolTrimTo(w.pool, w.users ? std::min<size_t>(WS_KEEP, w.wanted + WS_SLACK) : 0);
   p->ws_pool = nullptr;
 }
 
@@ -494,6 +499,7 @@ cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, MrgWs* out
     if (bytes > need) {
       w.wanted += bytes - need;
       p->ws_need = bytes;
+      keep_wanted(w.pool, w.wanted);
     }
   }
   out->of_graph = false;

@@ -42,14 +42,11 @@ CFGS = {
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", list(CFGS))
-@pytest.mark.parametrize("call", ["jacres", "jac", "res"])
-@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("call,fp32", [("jacres", False), ("jacres", True), ("jac", False), ("jac", True), ("res", False)])
 @pytest.mark.parametrize("overwrite", [False, True])
 def test_pieces_give_the_bits_of_the_whole(fake_lib, monkeypatch, name, call, fp32, overwrite):
     from mrhyde_gb300 import AssemblyManager
 
-    if call == "res" and fp32:
-        pytest.skip("the residual has one precision")
     monkeypatch.setattr(L, "_lib", fake_lib)
     fake = Fake(fake_lib)
     fake.pool_most.value = 2 ** 60
@@ -88,4 +85,28 @@ def test_pieces_give_the_bits_of_the_whole(fake_lib, monkeypatch, name, call, fp
     fake.pool_most.value = 2 ** 60
     for a, b in zip(run(), want):  # and the next call has its workspace again
         assert torch.equal(a, b)
+    G.close()
+
+
+@pytest.mark.gpu
+def test_idle_workspace_is_given_back(cuda):
+    """Calls overlapping on six streams take six workspaces; a synchronisation leaves the handle's own request and 1 GiB."""
+    from mrhyde_gb300 import AssemblyManager, Problem
+
+    G = Problem(dim=3, order=1, n=(120, 120, 120), kind="diffusion_1pu2")
+    need = 120 ** 3 * (54 + 8) * 8  # 857 MB
+    A = AssemblyManager(G)
+    u = G.new_vector()
+    out = [(G.new_vector(), G.new_matrix_values()) for _ in range(6)]
+    side = [torch.cuda.Stream() for _ in out]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for s, (r, J) in zip(side, out):
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(50_000_000)
+            A.assembleJacRes(u, r, J, overwrite=True)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= need + 2 ** 30 + 2 ** 27  # and what mapping rounds up
+    for r, J in out[1:]:
+        assert torch.equal(J, out[0][1]) and torch.equal(r, out[0][0])
     G.close()
