@@ -76,7 +76,8 @@ def poisson_stream(rate=200.0, count=400, edge=(16, 96), nonlinear_fraction=0.5,
 def estimate_bytes(req: Request) -> int:
     """Device bytes a request holds while admitted (problem data, Jacobian, Newton / Krylov vectors and
     the multigrid hierarchy: coarse operators ~1/7 of the fine nonzeros, six vectors per level, CG and
-    BiCGStab vectors on the fine level)."""
+    BiCGStab vectors on the fine level; nonlinear requests: the workspace of a Jacobian assembly, 54 numbers
+    for each cell of a piece of the mesh)."""
     n = req.n
     ndof = (n + 1) ** 3
     ncell = n ** 3
@@ -85,7 +86,8 @@ def estimate_bytes(req: Request) -> int:
     jbytes = nnz * w
     vec = ndof * 8 * 9 + (ndof * 4 * 6 if req.mixed else 0)
     hier = int(nnz * w / 7) + int(ndof * 1.15) * 6 * w + ndof * 10 * w
-    return int(jbytes + vec + hier + ncell * (8 + 4) + 4 * 1024 * 1024)
+    work = min((ncell + 31) // 32 * 32 * 54 * w, 4 << 30) if req.kind == "nonlinear" else 0
+    return int(jbytes + vec + hier + work + ncell * (8 + 4) + 4 * 1024 * 1024)
 
 
 # Per serving thread: one device generator (reseeded per request: the same sequence as a fresh generator
