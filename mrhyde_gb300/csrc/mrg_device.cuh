@@ -124,10 +124,11 @@ __device__ __forceinline__ double widen_any(float v) {
 // row's extents are loaded as zeros, so that a warp whose rows include boundary nodes (any tile of a short grid line)
 // runs the row once instead of once for its interior and once for its boundary lanes (y = J x on 80^3 cells: FP32 matrix
 // 92 -> 71 us, FP64 54 -> 46).  FP32 values against an FP64 vector are widened on the integer pipes: 27 conversions a row
-// took as long as its 27 FMAs (71 -> 39 us).  Terms in storage order.
+// took as long as its 27 FMAs (71 -> 39 us).  Terms in storage order.  x comes by plain loads: in a chain of programmatic
+// launches the kernel before may still be writing it when this one starts, and the read-only path is for data that
+// nothing writes while the grid exists.
 template <typename AT, typename JT, typename XT>
-__device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* __restrict__ vals,
-                                     const XT* __restrict__ x) {
+__device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* __restrict__ vals, const XT* x) {
   const int NX = g.nn[0];
   const int64_t plane = (int64_t)NX * g.nn[1];
   const XT* xb = x + R.lx + (int64_t)NX * R.ly + plane * R.lz;
@@ -140,7 +141,7 @@ __device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* 
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
         const bool in = (k % 3 < 2 || x2) && (k < 6 || y2);
-        b[z * 9 + k] = in ? __ldg(xr + NX * (k / 3) + k % 3) : XT(0);
+        b[z * 9 + k] = in ? xr[NX * (k / 3) + k % 3] : XT(0);
       }
     }
   }
@@ -174,8 +175,7 @@ __device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* 
 
 // y_i = sum_j J_ij x_j over the row (values contiguous at vals), accumulated in AT
 template <int P, typename JT, typename XT, typename AT>
-__device__ __forceinline__ AT row_dot(const Grid& g, const RowInfo& R, const JT* __restrict__ vals,
-                                      const XT* __restrict__ x) {
+__device__ __forceinline__ AT row_dot(const Grid& g, const RowInfo& R, const JT* __restrict__ vals, const XT* x) {
   if constexpr (P == 1) return row_q1<AT>(g, R, vals, x);
   constexpr int MC = 2 * P + 1;
   const int64_t NX = g.nn[0], plane = (int64_t)g.nn[0] * g.nn[1];
@@ -262,8 +262,7 @@ __device__ __forceinline__ int64_t row_ptr_at(const Grid& g, int64_t n, int64_t 
 
 // ---- row products: y_i = sum_j J_ij x_j over the row of node i --------------------------------
 template <int P, typename JT, typename XT>
-__device__ __forceinline__ double row_apply(const Grid& g, const RowInfo& R, const JT* __restrict__ vals,
-                                            const XT* __restrict__ x) {
+__device__ __forceinline__ double row_apply(const Grid& g, const RowInfo& R, const JT* __restrict__ vals, const XT* x) {
   if constexpr (P == 1) return row_q1<double>(g, R, vals, x);
   constexpr int MC = 2 * P + 1;
   const int64_t NX = g.nn[0], plane = (int64_t)g.nn[0] * g.nn[1];
@@ -291,8 +290,7 @@ __device__ __forceinline__ double row_apply(const Grid& g, const RowInfo& R, con
 
 // FP32 variant accumulating in FP32 (inner solve of the mixed path)
 template <int P>
-__device__ __forceinline__ float row_apply_f(const Grid& g, const RowInfo& R, const float* __restrict__ vals,
-                                             const float* __restrict__ x) {
+__device__ __forceinline__ float row_apply_f(const Grid& g, const RowInfo& R, const float* __restrict__ vals, const float* x) {
   if constexpr (P == 1) return row_q1<float>(g, R, vals, x);
   constexpr int MC = 2 * P + 1;
   const int64_t NX = g.nn[0], plane = (int64_t)g.nn[0] * g.nn[1];
@@ -413,7 +411,9 @@ __device__ __forceinline__ uintptr_t wtile_issue(const Grid& g, int64_t nrows, c
 // Programmatic dependent launch.  A kernel launched with launch_pdl may start while its predecessor still runs; it
 // calls pdl_wait before it touches anything that the predecessor reads or writes (the wait ends when the predecessor
 // has completed and its writes are visible), and pdl_trigger at its start, so that its own successor can be set up.
-// Every kernel of such a chain waits, so completion stays ordered along the chain.
+// Every kernel of such a chain waits, so completion stays ordered along the chain.  The grid is resident while its
+// predecessor writes, so what a kernel of the chain writes is read by plain loads (no __ldg, no const __restrict__): the
+// read-only path would be allowed to read it ahead of the wait.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -592,8 +592,8 @@ __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(
 // Chebyshev-Jacobi step k for row n given ax = (A x_in)_n: d = c_first z (k = 0) or c_old d + c_new z with
 // z = D^{-1} (b - ax); x_out = x_in + d (x_in = 0 when zero_x).  Shared by k_cheb and k_vcycle_tail.
 template <typename T>
-__device__ __forceinline__ void cheb_row(const LevDev<T>& L, int64_t n, T ax, const T* __restrict__ xin,
-                                         T* __restrict__ xout, int k, int zero_x, T c_first, T c_old, T c_new) {
+__device__ __forceinline__ void cheb_row(const LevDev<T>& L, int64_t n, T ax, const T* xin,
+                                         T* xout, int k, int zero_x, T c_first, T c_old, T c_new) {
   const T z = mul_rn(L.minv[n], sub_rn(L.b[n], ax));
   const T d = (k == 0) ? mul_rn(c_first, z) : fma(c_old, L.d[n], mul_rn(c_new, z));
   L.d[n] = d;
@@ -621,7 +621,7 @@ __device__ __forceinline__ void resid_row(const LevDev<T>& L, int64_t n, T ax) {
 }
 
 template <int P, typename T>
-__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cheb(LevDev<T> L, const T* __restrict__ xin, T* __restrict__ xout, int k,
+__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cheb(LevDev<T> L, const T* xin, T* xout, int k,
                                              int zero_x, const T* __restrict__ coef,
                                              const GScal* __restrict__ S, int* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_cheb(LevDev<T> L, co
 
 // r = b - A x
 template <int P, typename T>
-__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_resid(LevDev<T> L, const T* __restrict__ x, const GScal* __restrict__ S,
+__global__ void __launch_bounds__(NT, staged_per_sm<T>()) k_resid(LevDev<T> L, const T* x, const GScal* __restrict__ S,
                                               int* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar[2 * (NT / 32)];
@@ -701,7 +701,7 @@ __device__ __forceinline__ void parent_slots(int i, int nnf, int nnc, int co, bo
 // The free nodes are a Cartesian product, so a child counts if it exists and is free along each axis; the others are
 // loaded as zeros (no branches: the lanes of a warp have children missing at different places).
 template <typename T>
-__device__ __forceinline__ T restrict_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* __restrict__ rf, int64_t n) {
+__device__ __forceinline__ T restrict_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* rf, int64_t n) {
   int I[3];
   decompose(gc, n, I[0], I[1], I[2]);
   if (node_fixed(gc, I[0], I[1], I[2])) return T(0);
@@ -734,7 +734,7 @@ __device__ __forceinline__ T restrict_row(const Grid& gf, const Grid& gc, const 
 
 // and the coarse level's first smoothing step
 template <typename T>
-__global__ void __launch_bounds__(NT) k_restrict(Grid gf, Grid gc, Xfer X, const T* __restrict__ rf, T* __restrict__ bc,
+__global__ void __launch_bounds__(NT) k_restrict(Grid gf, Grid gc, Xfer X, const T* rf, T* bc,
                                                  FirstStep<T> first, const GScal* __restrict__ S) {
   pdl_trigger();
   pdl_wait();
@@ -749,8 +749,8 @@ __global__ void __launch_bounds__(NT) k_restrict(Grid gf, Grid gc, Xfer X, const
 
 // x_f += P x_c, fine row n (k_vcycle_tail; k_prolong takes two rows at once)
 template <typename T>
-__device__ __forceinline__ void prolong_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* __restrict__ xc,
-                                            T* __restrict__ xf, int64_t n) {
+__device__ __forceinline__ void prolong_row(const Grid& gf, const Grid& gc, const Xfer& X, const T* xc,
+                                            T* xf, int64_t n) {
   int i[3];
   decompose(gf, n, i[0], i[1], i[2]);
   if (node_fixed(gf, i[0], i[1], i[2])) return;
@@ -786,7 +786,7 @@ __device__ __forceinline__ void prolong_row(const Grid& gf, const Grid& gc, cons
 // Terms in prolong_row's order; those it multiplies by a weight of 0 are left out.  FP64: a row a thread; pairs halve the
 // warps that the FP64 pipe's latency is hidden behind (Newton solves on 48^3 cells with pairs 2 % slower).
 template <typename T>
-__global__ void __launch_bounds__(NT) k_prolong(Grid gf, Grid gc, Xfer X, const T* __restrict__ xc, T* __restrict__ xf,
+__global__ void __launch_bounds__(NT) k_prolong(Grid gf, Grid gc, Xfer X, const T* xc, T* xf,
                                                 const GScal* __restrict__ S) {
   pdl_trigger();
   pdl_wait();
@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(NT) k_prolong(Grid gf, Grid gc, Xfer X, const 
 
 // x = inv b on the coarsest level, row i (shared by k_coarse_apply and k_vcycle_tail)
 template <typename T>
-__device__ __forceinline__ void coarse_row(int n, const T* __restrict__ inv, const T* __restrict__ b, T* __restrict__ x,
+__device__ __forceinline__ void coarse_row(int n, const T* __restrict__ inv, const T* b, T* x,
                                            int i) {
   T s = T(0);
   for (int j = 0; j < n; ++j) s = fma(inv[i * n + j], b[j], s);
@@ -850,8 +850,8 @@ __device__ __forceinline__ void coarse_row(int n, const T* __restrict__ inv, con
 }
 
 template <typename T>
-__global__ void __launch_bounds__(NT) k_coarse_apply(int n, const T* __restrict__ inv, const T* __restrict__ b,
-                                                     T* __restrict__ x, const GScal* __restrict__ S) {
+__global__ void __launch_bounds__(NT) k_coarse_apply(int n, const T* __restrict__ inv, const T* b,
+                                                     T* x, const GScal* __restrict__ S) {
   pdl_trigger();
   pdl_wait();
   if (is_done(S)) return;
