@@ -36,7 +36,8 @@ struct BatchProb {
   int64_t cell_off, node_off, nnz_off;
   double Kp[8];
   float Kp32[8];
-  float Kc32[8];  // classes of the FP32 operator: multiples of one quantum, adding up to exactly 0
+  float Kc32[8];  // classes of the FP32 operator; class 0 balances the others
+  float Kc0_lo;   // and what it lacks
   double load;  // f * vol / 8
 };
 
@@ -173,9 +174,9 @@ __device__ __forceinline__ void class_sums(const Layer<T>& L, const Plane<T>& P,
 
 // f(k, (A v)_k, v_k) for the rows z0 .. z0 + n - 1 of a column: kap at the column's first cell of layer 0, v at the
 // column's node of plane 0.  A row takes the layer below and the layer above; each layer meets the planes below and
-// above it once.
+// above it once.  FP32: class 0 has a second part K0_lo.
 template <int U, int R, typename T, typename F>  // U: steps unrolled
-__device__ __forceinline__ void march(const T* K, const T* kap, int nx, int nxy, const T* v, int NX, int NXY, int z0, int n,
+__device__ __forceinline__ void march(const T* K, T K0_lo, const T* kap, int nx, int nxy, const T* v, int NX, int NXY, int z0, int n,
                                       F&& f) {
   Layer<T> L;
   Plane<T> lo, hi;
@@ -195,7 +196,9 @@ __device__ __forceinline__ void march(const T* K, const T* kap, int nx, int nxy,
     class_sums(L, hi, a1);
     hi.load(v + (z + 1) * NXY, NX);
     class_sums(L, hi, b1);
-    T q = K[0] * (b[0] + a1[0]);
+    const T c0 = b[0] + a1[0];
+    T q = K[0] * c0;
+    if constexpr (sizeof(T) == 4) q = fma(K0_lo, c0, q);
     q = fma(K[4], a[0] + b1[0], q);
 #pragma unroll
     for (int c = 1; c < 4; ++c) {
@@ -302,6 +305,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1) k_batch(const BatchArgs A
     float Kc[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) Kc[c] = P.Kc32[c];
+    const float Kc0_lo = P.Kc0_lo;
     for (;;) {
       // FP64 residual at u: b - A u, matrix-free
       double amax = 0.0;
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1) k_batch(const BatchArgs A
         for (int c = 0; c < 8; ++c) Kd[c] = P.Kp[c];
         const double b = P.load * 8.0;
         if (n > 0)
-          march<1, R, double>(Kd, kap + ct, nx, nxy, u + at, NX, NXY, z0, n, [&](int k, double q, double) {
+          march<1, R, double>(Kd, 0.0, kap + ct, nx, nxy, u + at, NX, NXY, z0, n, [&](int k, double q, double) {
             const double acc = b - q;
             x_own[k * T] = (float)acc;  // scaled below, once the max is known
             amax = fmax(amax, fabs(acc));
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1) k_batch(const BatchArgs A
         float q[R];
         float pqf = 0.0f;
         if (n > 0)
-          march<R, R, float>(Kc, k_sh + ct, nx, nxy, p_sh + at, NX, NXY, z0, n, [&](int k, float v, float own) {
+          march<R, R, float>(Kc, Kc0_lo, k_sh + ct, nx, nxy, p_sh + at, NX, NXY, z0, n, [&](int k, float v, float own) {
             q[k] = v;
             pqf = fmaf(v, own, pqf);
           });
@@ -398,20 +402,17 @@ __global__ void __launch_bounds__(T, T == 256 ? 2 : 1) k_batch(const BatchArgs A
   }
 }
 
-// Classes of the FP32 operator: rounded to multiples of 2^-23 of the largest one's binade and balanced by class 0,
-// so that they add up to exactly 0 (a row's kappa sums have the same total in every class) and the operator keeps a
-// stiffness matrix's zero row sums up to the rounding of the sums themselves.
-void balanced_classes(const double* Kp, float* Kc) {
-  double kmax = 0.0;
-  for (int c = 0; c < 8; ++c) kmax = std::max(kmax, std::fabs(Kp[c]));
-  const double quantum = std::ldexp(1.0, std::ilogb(kmax) - 23);
+// Classes of the FP32 operator: the rounded classes of the matrix, and minus their sum for class 0, in two parts, so that a
+// row adds up to 0 (its kappa sums have the same total in every class) as a stiffness matrix's does, up to the rounding of
+// the sums themselves.
+void balanced_classes(const double* Kp, float* Kc, float* Kc0_lo) {
   double total = 0.0;
   for (int c = 1; c < 8; ++c) {
-    const double v = std::nearbyint(Kp[c] / quantum) * quantum;
-    Kc[c] = (float)v;
-    total += v;
+    Kc[c] = (float)Kp[c];
+    total += Kc[c];
   }
   Kc[0] = (float)-total;
+  *Kc0_lo = (float)(-total - Kc[0]);
 }
 
 // box-cell stiffness classes K(|dx|,|dy|,|dz|) (exact integration of the trilinear element):
@@ -481,7 +482,7 @@ extern "C" int mrg_batch_create(const mrg_batch_desc* d, mrg_batch** out) {
     const double hx = 1.0 / P.nx, hy = 1.0 / P.ny, hz = 1.0 / P.nz;
     box_classes(hx, hy, hz, P.Kp);
     for (int c = 0; c < 8; ++c) P.Kp32[c] = (float)P.Kp[c];
-    balanced_classes(P.Kp, P.Kc32);
+    balanced_classes(P.Kp, P.Kc32, &P.Kc0_lo);
     P.load = d->source * hx * hy * hz / 8.0;
   }
   for (int64_t c = 0; c < B->ncell; ++c)
