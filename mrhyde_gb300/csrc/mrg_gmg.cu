@@ -1020,7 +1020,8 @@ __global__ void __launch_bounds__(TT) k_vcycle_tail(const __grid_constant__ Tail
 }
 
 // Vector updates with a dot product: RED_PER_SM CTAs per SM (each CTA's FP64 tree takes the FP64 pipe for 320 cycles, so
-// 16 per SM spent more time on the trees than on the vectors), four elements of a thread in flight.
+// 16 per SM spent more time on the trees than on the vectors), four elements of a thread in flight, each with a partial sum
+// of its own (Dot), so that a partial has no more terms than with 16 CTAs per SM.
 constexpr int RED_PER_SM = 4;
 template <typename L, typename F>
 __device__ __forceinline__ void each4(int64_t n, L&& load, F&& use) {
@@ -1032,11 +1033,34 @@ __device__ __forceinline__ void each4(int64_t n, L&& load, F&& use) {
       if (i + k * st < n) v[k] = load(i + k * st);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (i + k * st < n) use(i + k * st, v[k]);
+      if (i + k * st < n) use(i + k * st, v[k], k);
   }
 }
 template <typename T, int N>
 struct Vals { T v[N]; };
+
+// Four partial sums of products in the vectors' precision, added up in FP64.  FP32: with one FP64 addition, of the sum and
+// what it lacks (two-sum), where four conversions and three additions would hold the FP64 pipe.
+template <typename T>
+struct Dot {
+  T s[4] = {T(0), T(0), T(0), T(0)};
+  __device__ __forceinline__ void add(int k, T a, T b) { s[k] = fma(a, b, s[k]); }
+  __device__ __forceinline__ double total() const {
+    if constexpr (sizeof(T) == 8) {
+      return (s[0] + s[1]) + (s[2] + s[3]);
+    } else {
+      float t = s[0], c = 0.0f;
+#pragma unroll
+      for (int k = 1; k < 4; ++k) {
+        const float n = __fadd_rn(t, s[k]), z = __fsub_rn(n, t);
+        c = __fadd_rn(c, __fadd_rn(__fsub_rn(t, __fsub_rn(n, z)), __fsub_rn(s[k], z)));
+        t = n;
+      }
+      // c is not finite where t is not, and subnormal beside sums whose squares underflow
+      return (double)t + (mrgdev::widen_special(c) ? 0.0 : mrgdev::widen(c));
+    }
+  }
+};
 
 // ---- CG kernels -----------------------------------------------------------------------------------
 template <typename T>
@@ -1050,16 +1074,16 @@ struct CgVec {
 // x = 0, r = b (FP64 in, T out), p = q = 0; r0 = |r|
 template <typename T>
 __global__ void __launch_bounds__(NT) k_cg_init(int64_t n, const double* __restrict__ b, CgVec<T> V) {
-  T rr = T(0);  // per-thread partials in the vector precision (no per-element FP64 work for FP32)
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
-    const T r = (T)b[i];
-    V.x[i] = T(0);
-    V.r[i] = r;
-    V.p[i] = T(0);
-    V.q[i] = T(0);
-    rr = fma(r, r, rr);
-  }
-  double m[1] = {block_sum((double)rr)};
+  Dot<T> rr;  // per-thread partials in the vector precision (no per-element FP64 work for FP32)
+  each4(n, [&](int64_t i) { return (T)b[i]; },
+        [&](int64_t i, T r, int k) {
+          V.x[i] = T(0);
+          V.r[i] = r;
+          V.p[i] = T(0);
+          V.q[i] = T(0);
+          rr.add(k, r, r);
+        });
+  double m[1] = {block_sum(rr.total())};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
     double t[1];
     sum_parts<1>(V.parts, t, &V.S->counter);
@@ -1084,10 +1108,10 @@ __global__ void __launch_bounds__(NT) k_cg_rz(int64_t n, CgVec<T> V, int first) 
   pdl_trigger();
   pdl_wait();
   if (is_done(V.S)) return;
-  T rz = T(0);
+  Dot<T> rz;
   each4(n, [&](int64_t i) { return Vals<T, 2>{{V.r[i], V.z[i]}}; },
-        [&](int64_t, const Vals<T, 2>& e) { rz = fma(e.v[0], e.v[1], rz); });
-  double m[1] = {block_sum((double)rz)};
+        [&](int64_t, const Vals<T, 2>& e, int k) { rz.add(k, e.v[0], e.v[1]); });
+  double m[1] = {block_sum(rz.total())};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
     double t[1];
     sum_parts<1>(V.parts, t, &V.S->counter);
@@ -1148,16 +1172,16 @@ __global__ void __launch_bounds__(NT) k_cg_update(int64_t n, CgVec<T> V, FirstSt
   pdl_wait();
   if (is_done(V.S)) return;
   const T alpha = alpha_of<T>(V.S);
-  T rr = T(0);
+  Dot<T> rr;
   each4(n, [&](int64_t i) { return Vals<T, 5>{{V.x[i], V.p[i], V.r[i], V.q[i], first.diag(i)}}; },
-        [&](int64_t i, const Vals<T, 5>& e) {
+        [&](int64_t i, const Vals<T, 5>& e, int k) {
           V.x[i] = e.v[0] + alpha * e.v[1];
           const T r = e.v[2] - alpha * e.v[3];
           V.r[i] = r;
-          rr = fma(r, r, rr);
+          rr.add(k, r, r);
           first(i, r, e.v[4]);
         });
-  double m[1] = {block_sum((double)rr)};
+  double m[1] = {block_sum(rr.total())};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
     double t[1];
     sum_parts<1>(V.parts, t, &V.S->counter);
@@ -1188,17 +1212,17 @@ struct BgVec {
 // x = 0, r = rh = b, p = v = 0; rho = (rh . r), alpha = omega = 1, beta = 0
 template <typename T>
 __global__ void __launch_bounds__(NT) k_bg_init(int64_t n, const double* __restrict__ b, BgVec<T> V) {
-  T rr = T(0);
-  for (int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * NT) {
-    const T r = (T)b[i];
-    V.x[i] = T(0);
-    V.r[i] = r;
-    V.rh[i] = r;
-    V.p[i] = T(0);
-    V.v[i] = T(0);
-    rr = fma(r, r, rr);
-  }
-  double m[1] = {block_sum((double)rr)};
+  Dot<T> rr;
+  each4(n, [&](int64_t i) { return (T)b[i]; },
+        [&](int64_t i, T r, int k) {
+          V.x[i] = T(0);
+          V.r[i] = r;
+          V.rh[i] = r;
+          V.p[i] = T(0);
+          V.v[i] = T(0);
+          rr.add(k, r, r);
+        });
+  double m[1] = {block_sum(rr.total())};
   if (last_block<1>(V.parts, m, &V.S->counter)) {
     double t[1];
     sum_parts<1>(V.parts, t, &V.S->counter);
@@ -1305,16 +1329,16 @@ __global__ void __launch_bounds__(NT) k_bg_update(int64_t n, BgVec<T> V) {
   pdl_wait();
   if (is_done(V.S)) return;
   const T alpha = alpha_of<T>(V.S), omega = omega_of<T>(V.S);
-  T rr = T(0), rhr = T(0);
+  Dot<T> rr, rhr;
   each4(n, [&](int64_t i) { return Vals<T, 6>{{V.x[i], V.ph[i], V.sh[i], V.s[i], V.t[i], V.rh[i]}}; },
-        [&](int64_t i, const Vals<T, 6>& e) {
+        [&](int64_t i, const Vals<T, 6>& e, int k) {
           V.x[i] = e.v[0] + (alpha * e.v[1] + omega * e.v[2]);
           const T r = e.v[3] - omega * e.v[4];
           V.r[i] = r;
-          rr = fma(r, r, rr);
-          rhr = fma(e.v[5], r, rhr);
+          rr.add(k, r, r);
+          rhr.add(k, e.v[5], r);
         });
-  double m[2] = {block_sum((double)rr), block_sum((double)rhr)};
+  double m[2] = {block_sum(rr.total()), block_sum(rhr.total())};
   if (last_block<2>(V.parts, m, &V.S->counter)) {
     double t[2];
     sum_parts<2>(V.parts, t, &V.S->counter);
