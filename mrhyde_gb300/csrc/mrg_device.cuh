@@ -124,10 +124,16 @@ __device__ __forceinline__ double widen_any(float v) {
 // row's extents are loaded as zeros, so that a warp whose rows include boundary nodes (any tile of a short grid line)
 // runs the row once instead of once for its interior and once for its boundary lanes (y = J x on 80^3 cells: FP32 matrix
 // 92 -> 71 us, FP64 54 -> 46).  FP32 values against an FP64 vector are widened on the integer pipes: 27 conversions a row
-// took as long as its 27 FMAs (71 -> 39 us).  Terms in storage order.  x comes by plain loads: in a chain of programmatic
-// launches the kernel before may still be writing it when this one starts, and the read-only path is for data that
-// nothing writes while the grid exists.
-template <typename AT, typename JT, typename XT>
+// took as long as its 27 FMAs (71 -> 39 us).  Terms in storage order.
+// CHAIN: x comes by plain loads.  In a chain of programmatic launches the kernel before may still be writing it when this one
+// starts, and the read-only path is for data that nothing writes while the grid exists.  Elsewhere by read-only loads (y = J
+// x on 40 x 35 x 30 cells, FP32 matrix: 6.6 us, with plain ones 7.1).
+template <bool CHAIN, typename XT>
+__device__ __forceinline__ XT load_x(const XT* x) {
+  if constexpr (CHAIN) return *x;
+  else return __ldg(x);
+}
+template <typename AT, bool CHAIN, typename JT, typename XT>
 __device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* __restrict__ vals, const XT* x) {
   const int NX = g.nn[0];
   const int64_t plane = (int64_t)NX * g.nn[1];
@@ -141,7 +147,7 @@ __device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* 
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
         const bool in = (k % 3 < 2 || x2) && (k < 6 || y2);
-        b[z * 9 + k] = in ? xr[NX * (k / 3) + k % 3] : XT(0);
+        b[z * 9 + k] = in ? load_x<CHAIN>(xr + NX * (k / 3) + k % 3) : XT(0);
       }
     }
   }
@@ -176,7 +182,7 @@ __device__ __forceinline__ AT row_q1(const Grid& g, const RowInfo& R, const JT* 
 // y_i = sum_j J_ij x_j over the row (values contiguous at vals), accumulated in AT
 template <int P, typename JT, typename XT, typename AT>
 __device__ __forceinline__ AT row_dot(const Grid& g, const RowInfo& R, const JT* __restrict__ vals, const XT* x) {
-  if constexpr (P == 1) return row_q1<AT>(g, R, vals, x);
+  if constexpr (P == 1) return row_q1<AT, false>(g, R, vals, x);
   constexpr int MC = 2 * P + 1;
   const int64_t NX = g.nn[0], plane = (int64_t)g.nn[0] * g.nn[1];
   AT acc = AT(0);
@@ -261,9 +267,9 @@ __device__ __forceinline__ int64_t row_ptr_at(const Grid& g, int64_t n, int64_t 
 }
 
 // ---- row products: y_i = sum_j J_ij x_j over the row of node i --------------------------------
-template <int P, typename JT, typename XT>
+template <int P, typename JT, typename XT, bool CHAIN = false>
 __device__ __forceinline__ double row_apply(const Grid& g, const RowInfo& R, const JT* __restrict__ vals, const XT* x) {
-  if constexpr (P == 1) return row_q1<double>(g, R, vals, x);
+  if constexpr (P == 1) return row_q1<double, CHAIN>(g, R, vals, x);
   constexpr int MC = 2 * P + 1;
   const int64_t NX = g.nn[0], plane = (int64_t)g.nn[0] * g.nn[1];
   double acc = 0.0;
@@ -289,9 +295,9 @@ __device__ __forceinline__ double row_apply(const Grid& g, const RowInfo& R, con
 }
 
 // FP32 variant accumulating in FP32 (inner solve of the mixed path)
-template <int P>
+template <int P, bool CHAIN = false>
 __device__ __forceinline__ float row_apply_f(const Grid& g, const RowInfo& R, const float* __restrict__ vals, const float* x) {
-  if constexpr (P == 1) return row_q1<float>(g, R, vals, x);
+  if constexpr (P == 1) return row_q1<float, CHAIN>(g, R, vals, x);
   constexpr int MC = 2 * P + 1;
   const int64_t NX = g.nn[0], plane = (int64_t)g.nn[0] * g.nn[1];
   float acc = 0.0f;

@@ -116,8 +116,8 @@ __device__ __forceinline__ T omega_of(const GScal* S) {
 
 template <int P, typename T>
 __device__ __forceinline__ auto row_prod(const Grid& g, const RowInfo& R, const T* vals, const T* x) {
-  if constexpr (sizeof(T) == 4) return row_apply_f<P>(g, R, vals, x);
-  else return row_apply<P, double, double>(g, R, vals, x);
+  if constexpr (sizeof(T) == 4) return row_apply_f<P, true>(g, R, vals, x);
+  else return row_apply<P, double, double, true>(g, R, vals, x);
 }
 
 // f(n, R, vals) for every row: Q1 rows through the per-warp staged loop, Q2 rows (125-point) read directly.  gate
