@@ -507,8 +507,11 @@ __global__ void __launch_bounds__(CT_) k_cell_quad(const __grid_constant__ GenAr
 // ---- rows ------------------------------------------------------------------------------------------
 // Row lengths of a CTA's 128 rows fit the staged segment; entries are added cell by cell (cz, cy, cx order) at
 // positions computed from the row's extents.
+// With entries, 64 registers for 8 CTAs per SM (as many as their staged rows leave room for): left to itself the compiler
+// took 32 to 48 and loaded an element row in parts (300 x 400 Q2 quadrilaterals, FP64 Jacobian and residual, 504 us -> 500;
+// with the bounds of a piece among the arguments and 32 registers 522).
 template <int DIM, int P, typename JT, bool DOJ, bool DOR, bool OVW>
-__global__ void __launch_bounds__(RT) k_gather(const Grid g, int64_t row0, int64_t row1, const JT* __restrict__ ebuf,
+__global__ void __launch_bounds__(RT, DOJ ? 8 : 0) k_gather(const Grid g, int64_t row0, int64_t row1, const JT* __restrict__ ebuf,
                                                const double* __restrict__ rbuf, const double* __restrict__ bnode,
                                                double* __restrict__ r, JT* __restrict__ J) {
   constexpr int N1 = P + 1, NL = Gen<DIM, P>::NL;
