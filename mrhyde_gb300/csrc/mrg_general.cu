@@ -18,7 +18,7 @@
 //   k_cell_quad   lanes write and read consecutive addresses
 //   k_gather      one thread a CSR row: adds its cells' entries in a fixed order; rows staged in shared memory and
 //                 written once
-// Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 241 us (cells 214, FP64
+// Measured, FP64 Jacobian and residual: 47 x 45 x 50 hexahedra with every vertex moved 1783 -> 246 us (cells 220, FP64
 // pipe 87 % active, rows 27).
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
 // on several streams and may be captured; a mesh that would need more than MRG_PIECE_BYTES is worked on in pieces.
@@ -39,9 +39,15 @@ struct GenTab {  // 1-D tables at the Gauss points: values, derivatives, weights
   double l[3][3], d[3][3], w[3];
 };
 
+struct HexTab {  // Q1 hexahedra: weights of the pairs of nodes 00, 01, 11 at a Gauss point
+  double near, far;  // 00 / 01, 11 / 01
+  double scale;      // 2 (01)^2
+};
+
 struct GenArgs {
   Grid g;
   GenTab t;
+  HexTab hex;
   const double* metric;  // [cell / 32][components * points][32]
   const double* bnode;   // node loads
   const double* kap;
@@ -205,11 +211,17 @@ __device__ __forceinline__ void lerp2(double be, double al, double c0, double g0
   p0 = fma(be, d, f0);
   p1 = fma(al, d, f0);
 }
-__device__ __forceinline__ void pair3(double aa, double bb, double ab, double v0, double v1, double* t) {
-  const double s = v0 + v1;
-  t[0] = fma(bb, v1, aa * v0);
-  t[2] = fma(aa + bb, s, -t[0]);  // the two add up to (aa + bb)(v0 + v1): 5 operations for 6 (259 -> 249 us)
-  t[1] = ab * s;
+// Sums of two Gauss points' values against L[q][l] L[q][j]: (00, 01, 11), the pairs' weights w; and in units of the pair 01's
+// weight (near = 00 / 01, far = 11 / 01), an operation less.
+__device__ __forceinline__ void pair3(const double (&w)[3], double v0, double v1, double* t) {
+  t[0] = fma(w[2], v1, w[0] * v0);
+  t[1] = w[1] * (v0 + v1);
+  t[2] = fma(w[2], v0, w[0] * v1);
+}
+__device__ __forceinline__ void pair3(double near, double far, double v0, double v1, double* t) {
+  t[0] = fma(far, v1, near * v0);
+  t[1] = v0 + v1;
+  t[2] = fma(far, v0, near * v1);
 }
 
 template <typename JT, bool DOJ, bool DOR>
@@ -285,8 +297,12 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
     }
   }
   if constexpr (DOJ) {
-    const double aa = al * al, bb = be * be, ab = al * be;
-    double E[64];
+    const double w[3] = {al * al, al * be, be * be};  // of the pairs 00, 01, 11
+    // the same-axis parts' two sums over pairs leave the square of the pair 01's weight out (48 multiplications)
+    const double near = A.hex.near, far = A.hex.far, sc = A.hex.scale, hs = 0.5 * sc;
+    double E[64], su[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) su[q] = sc * u[q];
     // same-axis and advective parts: E[l][j] gets sigma(l_a) Z[j_a][pair b][pair c]
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -297,17 +313,17 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
         for (int p = 0; p < 2; ++p) {
           const int q0 = pt(a, q, p, 0), q1 = pt(a, q, p, 1), ca = a == 0 ? 0 : (a == 1 ? 3 : 5);
           const double C = fma(k[q1], m(ca, q1), k[q0] * m(ca, q0));
-          const double f0 = (u[q0] + u[q0]) * h[a][q0], d = fma(u[q1] + u[q1], h[a][q1], -f0);  // 2 u h
-          Z[0][q][p] = fma(be, d, f0 - C);
-          Z[1][q][p] = fma(al, d, f0 + C);
+          const double f0 = su[q0] * h[a][q0], d = fma(su[q1], h[a][q1], -f0);  // 2 u h
+          Z[0][q][p] = fma(be, d, fma(-hs, C, f0));
+          Z[1][q][p] = fma(al, d, fma(hs, C, f0));
         }
 #pragma unroll
       for (int ja = 0; ja < 2; ++ja) {
         double Pq[2][3], T[3][3];  // T[pair of the first other axis][pair of the second]
-        pair3(aa, bb, ab, Z[ja][0][0], Z[ja][0][1], Pq[0]);
-        pair3(aa, bb, ab, Z[ja][1][0], Z[ja][1][1], Pq[1]);
+        pair3(near, far, Z[ja][0][0], Z[ja][0][1], Pq[0]);
+        pair3(near, far, Z[ja][1][0], Z[ja][1][1], Pq[1]);
 #pragma unroll
-        for (int t = 0; t < 3; ++t) pair3(aa, bb, ab, Pq[0][t], Pq[1][t], T[t]);
+        for (int t = 0; t < 3; ++t) pair3(near, far, Pq[0][t], Pq[1][t], T[t]);
         const int p = a == 0 ? 1 : 0, q = a == 2 ? 1 : 2;
 #pragma unroll
         for (int l = 0; l < 8; ++l)
@@ -343,7 +359,7 @@ __global__ void __launch_bounds__(CT_) k_cell_hex1(const __grid_constant__ GenAr
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int j = 0; j < 2; ++j) pair3(aa, bb, ab, V[0][i][j], V[1][i][j], X[i][j]);
+          for (int j = 0; j < 2; ++j) pair3(w, V[0][i][j], V[1][i][j], X[i][j]);
         // the 16 combinations of (l_a, j_a, l_b, j_b), each with its mirror (l and j exchanged) at once
 #pragma unroll
         for (int s = 0; s < 16; ++s) {
@@ -679,6 +695,11 @@ int mrg_general_setup(mrg_problem* p, cudaStream_t s) {
     t.w[q] = p->gw1[q];
     M.gx[q] = p->gx1[q];
   }
+  const double l0 = t.l[0][0], l1 = t.l[0][1];
+  HexTab& x = Q->A.hex;
+  x.near = l0 / l1;
+  x.far = l1 / l0;
+  x.scale = 2.0 * (l0 * l1) * (l0 * l1);
   M.g = p->g;
   M.t = t;
   M.vcoord = p->d_vcoord;

@@ -18,7 +18,7 @@
 //                so that lanes write and read consecutive addresses and every offset is an immediate
 //   k_nl1_row    one thread a CSR row: 24 loads from each of its 8 cells, the CTA's rows staged in shared memory
 //                and written once; the residual adds the cells' entries in the same order
-// Measured, FP64 Jacobian and residual on 95^3 cells: 3506 -> 950 us (cells 610, rows 340, FP64 pipe 84 and 83 %
+// Measured, FP64 Jacobian and residual on 95^3 cells: 3506 -> 938 us (cells 600, rows 340, FP64 pipe 84 and 83 %
 // active; the row-by-row contraction took 2712 and eight coloured residual launches 780); FP32 Jacobian alone on
 // 96^3 cells 865 -> about 40 us.
 // The workspace is taken from the device's pool in stream order for each call, so calls of one handle may overlap
@@ -57,8 +57,10 @@ struct Nl1Args {
   double w[3];       // |J| w_q / h_a^2
   double load;       // f * int(phi_l) over one cell
   float betaf, slopef, wf[3];
-  double m[3], m02;  // L L at the Gauss point near node 0 for the pairs 00, 01, 11; m[0] + m[2]
-  float m32[3][2];   // m in FP32: value and what it lacks
+  // L L at the Gauss point near node 0 for the pairs 00, 01, 11.  FP64: in units of the pair 01's, which wj has twice
+  double near, far;  // 00 / 01 and 11 / 01
+  double wj[3];      // w times the pair 01's weight squared
+  float m32[3][2];   // FP32: value and what it lacks
   int64_t c0, c1;    // cells of the launch
 };
 
@@ -74,6 +76,10 @@ template <typename T>
 __device__ __forceinline__ T w_of(const Nl1Args& A, int a) {
   if constexpr (sizeof(T) == 4) return A.wf[a]; else return A.w[a];
 }
+template <typename T>
+__device__ __forceinline__ T wj_of(const Nl1Args& A, int a) {  // for the 54 numbers
+  if constexpr (sizeof(T) == 4) return A.wf[a]; else return A.wj[a];
+}
 
 // values at the two Gauss points from two nodes, or node sums from two Gauss points (the 2 x 2 table is
 // symmetric); d is the difference
@@ -84,15 +90,15 @@ __device__ __forceinline__ void lerp2(T beta, T a, T b, T& p0, T& p1, T& d) {
   p1 = fma(-beta, d, b);
 }
 
-// Sums of two Gauss points' values against L[q][l] L[q][j]: (00, 01, 11).  FP64: t00 and t11 add up to
-// (aa + bb)(v0 + v1), 5 operations.  FP32 is not short of operations: the table's values come in two parts, because
-// their rounding would shift every entry the same way (FP32 matrix's error at 16 x 16 x 16 cells 8.8e-8 with values
-// rounded once, 5.7e-8 so; 5.8e-8 for the row-by-row contraction).
+// Sums of two Gauss points' values against L[q][l] L[q][j]: (00, 01, 11).  FP64: in units of the pair 01's weight, so that
+// its sum takes no multiplication: 5 operations, none a difference (6 with the weights themselves).  FP32 is not short of
+// operations: the table's values come in two parts, because their rounding would shift every entry the same way (FP32
+// matrix at 16 x 16 x 16 cells, 2-norm of the error over that of the matrix: 8.8e-8 with values rounded once, 5.7e-8 so;
+// 5.8e-8 for the row-by-row contraction).
 __device__ __forceinline__ void pair3(const Nl1Args& A, double v0, double v1, double& t00, double& t01, double& t11) {
-  const double s = v0 + v1;
-  t00 = fma(A.m[2], v1, A.m[0] * v0);
-  t11 = fma(A.m02, s, -t00);
-  t01 = A.m[1] * s;
+  t00 = fma(A.far, v1, A.near * v0);
+  t11 = fma(A.far, v0, A.near * v1);
+  t01 = v0 + v1;
 }
 __device__ __forceinline__ void pair3(const Nl1Args& A, float v0, float v1, float& t00, float& t01, float& t11) {
   const float (&m)[3][2] = A.m32;
@@ -179,7 +185,7 @@ __global__ void __launch_bounds__(CT_) k_nl1_cell(const __grid_constant__ Nl1Arg
     }
     if constexpr (DOJ) {
       const JT kj = slope_of<JT>(A);
-      const JT w = w_of<JT>(A, a), w2 = JT(2) * w;
+      const JT w = wj_of<JT>(A, a), w2 = JT(2) * w;
       JT* out = zbuf + ((cl >> 5) * NZ_ + a * 18) * CB + (cl & 31);
       JT Z[2][2][2];  // [j][q][p]
 #pragma unroll
@@ -360,9 +366,9 @@ int mrg_nl1_setup(mrg_problem* p) {
   A.betaf = (float)A.beta;
   A.slopef = (float)A.slope;
   const double m[3] = {l[0] * l[0], l[0] * l[1], l[1] * l[1]};
-  A.m02 = m[0] + m[2];
+  A.near = l[0] / l[1];
+  A.far = l[1] / l[0];
   for (int k = 0; k < 3; ++k) {
-    A.m[k] = m[k];
     A.m32[k][0] = (float)m[k];
     A.m32[k][1] = (float)(m[k] - (double)A.m32[k][0]);
   }
@@ -371,6 +377,7 @@ int mrg_nl1_setup(mrg_problem* p) {
   for (int a = 0; a < 3; ++a) {
     A.w[a] = vol / (p->h[a] * p->h[a]);
     A.wf[a] = (float)A.w[a];
+    A.wj[a] = A.w[a] * (m[1] * m[1]);
   }
   A.load = p->source_amp * vol;  // the 8 basis values at the 8 equal-weight points add up to 1 for each node
   return mrg_ws_open(p);
