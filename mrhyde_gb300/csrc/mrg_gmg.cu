@@ -265,8 +265,7 @@ template <typename T>
 constexpr int rap_smem() { return RAP_W * RAP_BUF * (int)sizeof(T); }
 template <typename T, int A>
 __global__ void __launch_bounds__(RAP_W * 32) k_rap_line(Grid gf, Grid gc, int tiles, int64_t ntile,
-                                                         const T* __restrict__ Af, T* __restrict__ Ac,
-                                                         int* __restrict__ err) {
+                                                         const T* __restrict__ Af, T* __restrict__ Ac) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* buf = reinterpret_cast<T*>(smem_raw) + (threadIdx.x >> 5) * RAP_BUF;
   const int lane = threadIdx.x & 31;
@@ -1673,9 +1672,9 @@ int setup_values(Hier<T>* H, const T* J, cudaStream_t s) {
           const int64_t nt = (int64_t)tiles * gout.nn[1] * gout.nn[2];
           const unsigned nb = nblk(nt, RAP_W);
           constexpr int smem = rap_smem<T>();
-          if (L.sweep_axis[w] == 0) k_rap_line<T, 0><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout, H->err);
-          else if (L.sweep_axis[w] == 1) k_rap_line<T, 1><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout, H->err);
-          else k_rap_line<T, 2><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout, H->err);
+          if (L.sweep_axis[w] == 0) k_rap_line<T, 0><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout);
+          else if (L.sweep_axis[w] == 1) k_rap_line<T, 1><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout);
+          else k_rap_line<T, 2><<<nb, RAP_W * 32, smem, s>>>(*gin, gout, tiles, nt, ain, aout);
         } else {
           k_rap_axis<T><<<nblk(nout, NT), NT, 0, s>>>(*gin, pin, gout, pout, L.sweep_axis[w], ain, aout, H->err);
         }
