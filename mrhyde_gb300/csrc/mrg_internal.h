@@ -142,7 +142,7 @@ struct mrg_problem {
 // on it, unless it is the creation stream or is being captured.  mrg_drain waits for the creation stream and for all those
 // events, so memory that work in flight on any stream may read is not freed; the streams themselves need not exist any
 // more.  Safe from any thread.
-int mrg_streams_open(mrg_problem* p);
+void mrg_streams_open(mrg_problem* p);
 void mrg_streams_close(mrg_problem* p);
 void mrg_note_stream(const mrg_problem* p, cudaStream_t s);
 int mrg_drain(const mrg_problem* p);

@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -283,9 +284,9 @@ bool being_captured(cudaStream_t s) {
 }
 }  // namespace
 
-int mrg_streams_open(mrg_problem* p) {
+void mrg_streams_open(mrg_problem* p) {
   p->used = new StreamUse();
-  return MRG_OK;
+  p->used->marks.reserve(4 * MARKS);
 }
 
 void mrg_streams_close(mrg_problem* p) {
@@ -311,7 +312,7 @@ void mrg_note_stream(const mrg_problem* p, cudaStream_t s) {
       if (!at && cudaEventQuery(m.ev) == cudaSuccess) at = &m;
     if (!at) cudaGetLastError();
   }
-  if (!at) {
+  if (!at && marks.size() < marks.capacity()) {  // never more than reserved: no exception leaves a C entry from here
     cudaEvent_t ev = nullptr;
     if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) {
       marks.push_back({s, t, ev});
@@ -371,27 +372,33 @@ WsPool g_ws[SM_CACHE];  // by device ordinal
 struct GraphWs {
   void* p;
   WsPool* w;
+  GraphWs* next;
 };
 std::mutex g_gone_mu;
-std::vector<GraphWs>& g_gone = *new std::vector<GraphWs>();  // callbacks may come after the statics' destructors
+GraphWs* g_gone = nullptr;
 std::atomic<bool> g_any_gone{false};
 void CUDART_CB graph_ws_gone(void* arg) {
   GraphWs* g = static_cast<GraphWs*>(arg);
   std::lock_guard<std::mutex> lk(g_gone_mu);
-  g_gone.push_back(*g);
+  g->next = g_gone;
+  g_gone = g;
   g_any_gone.store(true, std::memory_order_release);
-  delete g;
 }
 void collect_graph_ws(WsPool& w) {
   if (!g_any_gone.load(std::memory_order_acquire)) return;
   std::lock_guard<std::mutex> lk(g_gone_mu);
   RelaxedCapture relaxed;  // the caller may be capturing
-  size_t kept = 0;
-  for (const GraphWs& g : g_gone)
-    if (g.w == &w) cudaFreeAsync(g.p, w.own);
-    else g_gone[kept++] = g;
-  g_gone.resize(kept);
-  g_any_gone.store(kept > 0, std::memory_order_release);
+  for (GraphWs** at = &g_gone; *at;) {
+    GraphWs* g = *at;
+    if (g->w != &w) {
+      at = &g->next;
+      continue;
+    }
+    cudaFreeAsync(g->p, w.own);
+    *at = g->next;
+    delete g;
+  }
+  g_any_gone.store(g_gone != nullptr, std::memory_order_release);
 }
 
 cudaError_t take_for_graph(WsPool& w, size_t bytes, cudaStream_t s, unsigned long long id, cudaGraph_t graph, MrgWs* out) {
@@ -407,7 +414,8 @@ cudaError_t take_for_graph(WsPool& w, size_t bytes, cudaStream_t s, unsigned lon
   cudaError_t e = cudaMallocFromPoolAsync(&ptr, bytes, w.pool, w.own);
   if (e != cudaSuccess) return e;
   e = cudaStreamSynchronize(w.own);
-  GraphWs* g = new GraphWs{ptr, &w};
+  GraphWs* g = new (std::nothrow) GraphWs{ptr, &w, nullptr};
+  if (!g && e == cudaSuccess) e = cudaErrorMemoryAllocation;
   cudaUserObject_t obj = nullptr;
   if (e == cudaSuccess) e = cudaUserObjectCreate(&obj, g, graph_ws_gone, 1, cudaUserObjectNoDestructorSync);
   if (e != cudaSuccess) {
@@ -459,6 +467,7 @@ int mrg_ws_open(mrg_problem* p) {
       return mrg_cuda_check(e, "workspace pool's stream");
     }
     w.pool = pool;
+    w.captured.reserve(WS_CAPTURED);
   }
   ++w.users;
   p->ws_pool = &w;
