@@ -16,7 +16,7 @@
 // What bounds it: the FP64 pipe (16 SM cycles a warp instruction), with about 64 multiplications and 87 FMAs a
 // row in 3-D; so warps are filled with rows of one kind (mrg_q2_rows.cuh), which keeps all 32 lanes on the same
 // unrolled code whatever the mesh size.  Measured, FP64 Jacobian and residual:
-// 33 x 30 x 27 cells 6081 -> 78 us (FP64 floor 66), 300 x 211 cells with two flux sides 1146 -> 39 us.
+// 33 x 30 x 27 cells 6081 -> 78 us (FP64 floor 66), 300 x 211 cells with two flux sides 1146 -> 33 us.
 #include <cmath>
 #include <type_traits>
 #include <vector>
