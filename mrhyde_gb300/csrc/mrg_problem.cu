@@ -502,7 +502,9 @@ cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, MrgWs* out
   if (cap == cudaStreamCaptureStatusInvalidated) return cudaErrorStreamCaptureInvalidated;
   collect_graph_ws(w);
   if (cap == cudaStreamCaptureStatusActive) return take_for_graph(w, bytes, s, id, graph, out);
-  if (bytes > p->ws_need.load(std::memory_order_relaxed)) {
+  out->of_graph = false;
+  const cudaError_t e = cudaMallocFromPoolAsync(&out->p, bytes, w.pool, s);
+  if (e == cudaSuccess && bytes > p->ws_need.load(std::memory_order_relaxed)) {  // only what could be had is kept for
     std::lock_guard<std::mutex> lk(g_ws_mu);
     const size_t need = p->ws_need;
     if (bytes > need) {
@@ -511,8 +513,7 @@ cudaError_t mrg_ws_take(mrg_problem* p, size_t bytes, cudaStream_t s, MrgWs* out
       keep_wanted(w.pool, w.wanted);
     }
   }
-  out->of_graph = false;
-  return cudaMallocFromPoolAsync(&out->p, bytes, w.pool, s);
+  return e;
 }
 
 cudaError_t mrg_ws_give(const MrgWs& ws, cudaStream_t s) { return ws.of_graph ? cudaSuccess : cudaFreeAsync(ws.p, s); }
